@@ -21,9 +21,10 @@ INCLUDE = ROOT / "include"
 
 LIB_NAME = "librlt_kv_handoff.so"
 OPS_NAME = "_C.so"
+HOST_NAME = "_host.so"
 
 CUDA_SOURCES = ["lib.cu", "kv_table_copy.cu", "kv_segment_copy.cu", "kv_finalize.cu", "tensor_transfer.cu",
-                "kv_signal.cu", "peer.cu"]
+                "kv_signal.cu", "peer.cu", "block_moves.cu", "host_staging.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 
@@ -78,7 +79,7 @@ def build_library(force: bool = False, verbose: bool = False) -> Path:
     """Compile the C-ABI library (no torch types, static cudart)."""
     target = PACKAGE / LIB_NAME
     sources = [CSRC / s for s in CUDA_SOURCES]
-    deps = sources + [CSRC / "common.cuh", INCLUDE / "rlt_kv_handoff.h"]
+    deps = sources + [CSRC / "common.cuh", CSRC / "table_params.cuh", CSRC / "block_moves.h", INCLUDE / "rlt_kv_handoff.h"]
     flags = [*ARCH, "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC,-fvisibility=hidden"]
     fingerprint = _fingerprint(flags, deps)
     if force or verbose or _stale(target, fingerprint):
@@ -90,37 +91,47 @@ def build_library(force: bool = False, verbose: bool = False) -> Path:
     return target
 
 
-def build_ops(force: bool = False) -> Path:
-    """Compile the torch op library that registers ``torch.ops.vllm_rlt.kv_*`` over the C ABI."""
+def _build_torch_module(name: str, source_name: str, headers: list[Path], force: bool, python: bool = False) -> Path:
+    import sysconfig
+
     import torch
     from torch.utils import cpp_extension
 
-    target = PACKAGE / OPS_NAME
-    source = CSRC / "torch_bindings.cpp"
-    deps = [source, CSRC / "ops.h", INCLUDE / "rlt_kv_handoff.h", PACKAGE / LIB_NAME]
+    target = PACKAGE / name
+    source = CSRC / source_name
+    deps = [source, *headers, INCLUDE / "rlt_kv_handoff.h", PACKAGE / LIB_NAME]
     abi = int(torch._C._GLIBCXX_USE_CXX11_ABI)
-    flags = ["-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={abi}", "-DTORCH_EXTENSION_NAME=_C",
-             f"torch={torch.__version__}"]
+    flags = ["-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={abi}",
+             f"-DTORCH_EXTENSION_NAME={target.stem}", f"torch={torch.__version__}"]
     fingerprint = _fingerprint(flags, deps)
     if force or _stale(target, fingerprint):
         includes = [f"-I{p}" for p in cpp_extension.include_paths("cuda")] + [f"-I{INCLUDE}", f"-I{CSRC}"]
-        import sysconfig
-
         includes.append(f"-I{sysconfig.get_paths()['include']}")
         torch_lib = Path(torch.__file__).parent / "lib"
+        libraries = ["-ltorch", "-ltorch_cpu", "-lc10", "-ltorch_cuda", "-lc10_cuda"] + (["-ltorch_python"] if python else [])
         cmd = ["g++", *flags[:-1], *includes, str(source), "-o", str(target),
-               f"-L{PACKAGE}", "-l:" + LIB_NAME, f"-L{torch_lib}", "-ltorch", "-ltorch_cpu", "-lc10",
-               "-ltorch_cuda", "-lc10_cuda", "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{torch_lib}"]
+               f"-L{PACKAGE}", "-l:" + LIB_NAME, f"-L{torch_lib}", *libraries, "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{torch_lib}"]
         _run(cmd)
         _record(target, fingerprint)
     return target
 
 
+def build_ops(force: bool = False) -> Path:
+    """Compile the torch op library that registers ``torch.ops.vllm_rlt.kv_*`` over the C ABI."""
+    return _build_torch_module(OPS_NAME, "torch_bindings.cpp", [CSRC / "ops.h"], force)
+
+
+def build_host(force: bool = False) -> Path:
+    """Compile the Python module that prepares and issues the launches of the Python entry points."""
+    return _build_torch_module(HOST_NAME, "host_module.cpp", [CSRC / "block_moves.h"], force, python=True)
+
+
 def build_all(force: bool = False) -> None:
     build_library(force)
     build_ops(force)
+    build_host(force)
 
 
 if __name__ == "__main__":
     build_all(force="--force" in sys.argv)
-    print("built", PACKAGE / LIB_NAME, PACKAGE / OPS_NAME)
+    print("built", PACKAGE / LIB_NAME, PACKAGE / OPS_NAME, PACKAGE / HOST_NAME)

@@ -18,6 +18,8 @@ RLT_E_INVALID, RLT_E_GEOMETRY, RLT_E_LIMIT, RLT_E_CUDA, RLT_E_ALIGN = -1, -2, -3
 STATUS_OK, STATUS_BAD_RANGE, STATUS_BAD_BLOCK, STATUS_BAD_PLANE, STATUS_TIMEOUT, STATUS_STALL = 0, 1, 2, 3, 4, 5
 STATUS_WORDS = 4
 MODE_ALL_PLANES, MODE_DEDUP, MODE_EXIT_ONLY = 0, 1, 2
+MOVE_DIRECT, MOVE_PACK, MOVE_SCATTER = 0, 1, 2
+MOVE_UNSUITED = 1  # a launch the record kernels do not serve: the table-driven entry points do
 MAX_REQUESTS = 4096
 MAX_SEGMENTS = 4096
 MAX_WAIT_NS = 2_000_000_000
@@ -164,6 +166,29 @@ def load_ops():
 
     torch.ops.load_library(str(OPS_PATH))
     return torch.ops.vllm_rlt
+
+
+HOST_PATH = PACKAGE / "_host.so"
+
+
+@cache
+def load_host():
+    """The compiled host side of the Python entry points (``csrc/host_module.cpp``). Built on first use if the tree holds
+    its sources only, like the C-ABI library it is linked to; there is no Python form of it."""
+    if not HOST_PATH.is_file() or not LIB_PATH.is_file():
+        from . import _build
+
+        _build.build_library()
+        _build.build_host()
+    import importlib.machinery
+    import importlib.util
+
+    import torch  # noqa: F401  (its libraries must be loaded before the module that links to them)
+
+    loader = importlib.machinery.ExtensionFileLoader("_host", str(HOST_PATH))
+    module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_host", loader))
+    loader.exec_module(module)
+    return module
 
 
 class RltError(RuntimeError):

@@ -1,0 +1,666 @@
+// Handoff, pack and scatter from per-page records (block_moves.h): the kernels of a batch whose tables the host holds.
+//
+// Work decomposition. Inside a KV block the rows lie [layer][token][row], so a layer slice of a block is one contiguous
+// byte range on every plane of either pool. A CTA takes one small piece of such a range, 8 or 16 KiB, of one page:
+// vector i of the piece sits at the same offset of the source and of the destination block, and which token it belongs
+// to matters only where a page is partly in range, where exit planes choose the source, or where a packed image is
+// compacted. There is no loop over units: the grid holds one CTA per piece, in address order.
+//
+// Why small pieces and no persistent loop: the memory system is fastest when the bytes in flight at any moment are
+// neighbours. The hardware hands pieces to SMs in order as they become free, which keeps all SMs within a few MB of each
+// other; CTAs that stride over the work drift apart. Measured on one B200 with 1 GiB per stream, against 444
+// persistent CTAs: one read per write 6.2 -> 6.9 TB/s, one read per two writes 5.7 -> 6.85, per three 5.65 -> 6.8, per seven
+// 5.4 -> 6.7 (pieces of 8 KiB; 16 KiB within 1 %, 64 KiB 4 % slower), of which 32-byte accesses are 1 - 3 %.
+//
+// What a CTA must know is read in one round from the page's record; for small batches the records are kernel parameters, so a
+// launch needs no staging copy before it. Block ids and exit planes are checked here and reported in the status words;
+// a row that fails is skipped.
+
+#include <algorithm>
+#include <cstring>
+
+#include "block_moves.h"
+#include "common.cuh"
+#include "table_params.cuh"
+
+namespace rlt {
+namespace {
+
+enum MoveKind {
+  kPlaneToPlane,   // ALL_PLANES handoff: plane p <- plane p
+  kExitToPlane,    // EXIT_ONLY handoff: the only plane <- the token's exit plane
+  kFanOut,         // DEDUP handoff: planes up to the exit plane are read once, deeper ones filled from the last
+  kPlaneToWire,    // pack, ALL_PLANES
+  kExitToWire,     // pack, EXIT_ONLY
+  kDedupToWire,    // pack, DEDUP
+  kWireToPlane,    // scatter of an image with every plane
+  kDedupFromWire   // scatter of a dedup image: like kFanOut with the rows taken from the image
+};
+
+__host__ __device__ constexpr bool loops_planes(MoveKind k) { return k == kFanOut || k == kDedupFromWire; }
+
+struct MoveRegion {
+  const char* src[2];  // K and V; the image for a scatter
+  char* dst[2];
+  long long block_bytes;
+  long long slice_at;  // byte offset of the layer slice inside a block
+  int token_bytes;
+  int vec_bytes;       // 32, 16, 4 or 1
+  int row_vecs;
+  unsigned row_magic;  // div_magic(row_vecs), 0 for one-vector rows
+  int slice_vecs;      // vectors of the layer slice of one block
+  int pieces;          // CTAs per (page, plane, K|V)
+  int per;             // vectors of one piece
+};
+
+struct MoveParams {
+  MoveRegion region[2];
+  int pieces;        // CTAs per (page, plane of the grid): 2 * (region[0].pieces + region[1].pieces)
+  int grid_planes;   // planes the grid enumerates (1 where a CTA walks the planes itself)
+  int plane_begin, plane_end;
+  int src_planes, dst_planes, src_blocks, dst_blocks;
+  int block_size;
+  unsigned block_magic;
+  int layer_begin, slice_layers;
+  unsigned long long deep_layer_mask;
+  long long packed_bytes, packed_token_bytes;
+  int words;         // int32 per record
+  int blocks;
+  int dst_at, exit_at;  // where a record's destination blocks and exit planes start
+  const int* records;
+  const int* wire;   // [blocks][planes]
+  long long* wire_header;
+  long long wire_tokens;
+  int* status;
+};
+
+template <int kWords>
+struct MoveArgs {
+  MoveParams p;
+  int inline_words[kWords];
+};
+
+// Vectors per thread of one piece, and how many of them are in flight together: 16 KiB pieces where a vector is read
+// and written once, 8 KiB per plane where the planes are walked (their loads are batched over planes instead). Narrow
+// vectors get smaller pieces.
+template <typename T>
+__host__ __device__ constexpr int unroll_of(bool planes) {
+  return sizeof(T) == 32 ? (planes ? 1 : 2) : sizeof(T) == 16 ? (planes ? 2 : 4) : sizeof(T) == 4 ? 8 : 16;
+}
+template <typename T>
+__host__ __device__ constexpr int flight_of() {
+  return sizeof(T) == 32 ? 2 : 4;
+}
+
+struct Piece {
+  const int* rec;
+  int g, kv, index, plane;
+  int t_lo, t_hi;
+  // read again where an error is reported, not kept in registers for it
+  __device__ int request() const { return rec[0]; }
+  __device__ int logical() const { return rec[1]; }
+};
+
+// A page's record as the kinds that choose planes per token use it: fetched by the CTA in one round, then looked up in
+// shared memory (a chain of global lookups, token -> exit plane -> block, would cost a CTA this short as much time as its
+// payload).
+constexpr int kMaxPlanes = 64;
+struct PageShared {
+  long long src[kMaxPlanes];  // byte offset of each plane's block, -1 if the id is outside the pool
+  long long dst[kMaxPlanes];
+  long long wire[kMaxPlanes];               // dedup image: where this page's rows of each plane start
+  unsigned long long carried[kMaxPlanes];   // dedup image: tokens of the page that the plane carries
+  int src_id[kMaxPlanes], dst_id[kMaxPlanes];
+  int exit_plane[kMaxBlockSize];
+};
+// kDedupToWire: the (token, plane) pairs of a page that are on the wire, token by token (plane << 8 | token).
+struct PagePairs {
+  unsigned short code[kMaxPlanes * kMaxBlockSize];
+};
+
+// Where vector `first + k` of a block's layer slice is: row (layer-major, token-minor), token, and vector inside the row.
+// k counts from the piece's first vector, whose row and offset are (row0, rem0): the multiplier split stays exact.
+struct RowAt {
+  int layer, token, within;
+};
+__device__ __forceinline__ RowAt row_at(const MoveParams& p, const MoveRegion& rg, int row0, int rem0, int k) {
+  const unsigned j = static_cast<unsigned>(rem0 + k);
+  const int q = rg.row_magic ? static_cast<int>(__umulhi(j, rg.row_magic)) : static_cast<int>(j);
+  const int row = row0 + q;
+  const int layer = p.block_size == 1 ? row : static_cast<int>(__umulhi(static_cast<unsigned>(row), p.block_magic));
+  return {layer, row - layer * p.block_size, static_cast<int>(j) - q * rg.row_vecs};
+}
+
+__device__ __forceinline__ bool deep_carried(const MoveParams& p, int layer_rel) {
+  return p.deep_layer_mask == 0 || ((p.deep_layer_mask >> (p.layer_begin + layer_rel)) & 1ull) != 0;
+}
+
+// The block's address offset, or -1 (reported) if its id is outside the pool.
+__device__ __forceinline__ long long block_at(const MoveParams& p, const MoveRegion& rg, const Piece& w, int id, int blocks) {
+  if (static_cast<unsigned>(id) < static_cast<unsigned>(blocks)) return id * rg.block_bytes;
+  report(p.status, RLT_STATUS_BAD_BLOCK, w.request(), w.logical(), id);
+  return -1;
+}
+
+// The same from the page's shared table.
+__device__ __forceinline__ long long used_block(const MoveParams& p, const Piece& w, long long offset, int id) {
+  if (offset < 0) report(p.status, RLT_STATUS_BAD_BLOCK, w.request(), w.logical(), id);
+  return offset;
+}
+
+// Offset in the image of the first row of (page, plane, region, K|V) when `tokens` of the page are carried there.
+__device__ __forceinline__ long long wire_base(const MoveParams& p, const Piece& w, const MoveRegion& rg, long long before,
+                                               int tokens) {
+  long long at = before * p.packed_token_bytes;
+  if (w.g == 1) at += 2ll * p.slice_layers * tokens * p.region[0].token_bytes;
+  return at + static_cast<long long>(w.kv) * p.slice_layers * tokens * rg.token_bytes;
+}
+
+template <MoveKind K>
+__device__ __forceinline__ void fetch_page(const MoveParams& p, const MoveRegion& rg, const Piece& w, const int* wire, PageShared& s) {
+  constexpr bool kImage = K == kDedupToWire || K == kDedupFromWire;
+  const int tid = static_cast<int>(threadIdx.x);
+  const int word = kRecordHeader + tid;
+  if (word < p.words) {
+    const int v = w.rec[word];
+    if (word >= p.exit_at) {
+      s.exit_plane[word - p.exit_at] = v;
+    } else if (word >= p.dst_at) {
+      s.dst_id[word - p.dst_at] = v;
+      s.dst[word - p.dst_at] = static_cast<unsigned>(v) < static_cast<unsigned>(p.dst_blocks) ? v * rg.block_bytes : -1;
+    } else {
+      s.src_id[tid] = v;
+      s.src[tid] = static_cast<unsigned>(v) < static_cast<unsigned>(p.src_blocks) ? v * rg.block_bytes : -1;
+    }
+  }
+  long long before = 0;
+  const int planes = p.src_planes;
+  const int lane = tid & 31, warp = tid >> 5;
+  // warp w looks after planes w, w + 8, ...; its lane k keeps the wire entry of the k-th of them
+  if (kImage && warp + lane * (kThreads / 32) < planes) before = wire[warp + lane * (kThreads / 32)];
+  __syncthreads();
+  if constexpr (kImage) {
+    const int e0 = lane >= w.t_lo && lane < w.t_hi ? s.exit_plane[lane] : -1;
+    const int e1 = lane + 32 >= w.t_lo && lane + 32 < w.t_hi ? s.exit_plane[lane + 32] : -1;
+    for (int k = 0, plane = warp; plane < planes; ++k, plane += kThreads / 32) {
+      const unsigned long long mask = static_cast<unsigned long long>(__ballot_sync(0xffffffffu, e0 >= plane)) |
+                                      static_cast<unsigned long long>(__ballot_sync(0xffffffffu, e1 >= plane)) << 32;
+      const long long first = __shfl_sync(0xffffffffu, before, k);
+      if (lane == 0) {
+        s.carried[plane] = mask;
+        s.wire[plane] = wire_base(p, w, rg, first, __popcll(mask));
+      }
+    }
+    __syncthreads();
+  }
+}
+
+template <typename T, MoveKind K>
+__device__ __forceinline__ void move_rows(const MoveParams& p, const MoveRegion& rg, const Piece& w, const PageShared& s) {
+  constexpr int kU = flight_of<T>();
+  const int first = w.index * rg.per;
+  const int n_tok = w.t_hi - w.t_lo;
+  const int sid = K == kWireToPlane || K == kExitToPlane || K == kExitToWire ? 0 : w.rec[kRecordHeader + w.plane];
+  const int did = K == kPlaneToWire || K == kExitToWire ? 0 : w.rec[p.dst_at + w.plane];
+  const char* src = rg.src[w.kv];
+  char* dst = rg.dst[w.kv];
+  long long image = 0;  // where the page's rows start in the image
+  if (K == kPlaneToWire || K == kExitToWire || K == kWireToPlane) {
+    const long long before = static_cast<long long>(w.rec[4]) * p.dst_planes + static_cast<long long>(w.plane) * w.rec[5] + w.rec[3];
+    image = wire_base(p, w, rg, before, n_tok);
+  }
+  if (K == kPlaneToPlane || K == kPlaneToWire) {
+    const long long at = block_at(p, rg, w, sid, p.src_blocks);
+    if (at < 0) return;
+    src += at + rg.slice_at;
+  } else if (K == kWireToPlane) {
+    src += image;
+  }
+  if (K == kPlaneToPlane || K == kExitToPlane || K == kWireToPlane) {
+    const long long at = block_at(p, rg, w, did, p.dst_blocks);
+    if (at < 0) return;
+    dst += at + rg.slice_at;
+  } else {
+    dst += image;
+  }
+  T regs[kU];
+  // A page that is carried whole is the same byte range on both sides, the image included.
+  const bool whole = n_tok == p.block_size && (w.plane == 0 || p.deep_layer_mask == 0) &&
+                     (K == kPlaneToPlane || K == kExitToPlane ||
+                      image + static_cast<long long>(rg.slice_vecs) * static_cast<int>(sizeof(T)) <= p.packed_bytes);
+  if (K != kExitToPlane && K != kExitToWire && whole) {
+    const T* from = reinterpret_cast<const T*>(src) + first;
+    T* to = reinterpret_cast<T*>(dst) + first;
+    const int left = rg.slice_vecs - first;
+    for (int k0 = static_cast<int>(threadIdx.x); k0 < rg.per; k0 += kThreads * kU) {
+#pragma unroll
+      for (int u = 0; u < kU; ++u) {
+        if (k0 + u * kThreads < left) regs[u] = ld_stream(from + k0 + u * kThreads);
+      }
+#pragma unroll
+      for (int u = 0; u < kU; ++u) {
+        if (k0 + u * kThreads < left) st_stream(to + k0 + u * kThreads, regs[u]);
+      }
+    }
+    return;
+  }
+  const int row0 = first / rg.row_vecs, rem0 = first - row0 * rg.row_vecs;
+  for (int k0 = static_cast<int>(threadIdx.x); k0 < rg.per; k0 += kThreads * kU) {
+    T* to[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const int k = k0 + u * kThreads;
+      to[u] = nullptr;
+      if (first + k >= rg.slice_vecs) continue;
+      const RowAt at = row_at(p, rg, row0, rem0, k);
+      if (at.token < w.t_lo || at.token >= w.t_hi) continue;
+      if (w.plane > 0 && !deep_carried(p, at.layer)) continue;
+      const long long in_slice = static_cast<long long>(first + k) * static_cast<int>(sizeof(T));
+      long long in_image = 0;
+      if (K == kPlaneToWire || K == kExitToWire || K == kWireToPlane) {
+        in_image = (static_cast<long long>(at.layer) * n_tok + (at.token - w.t_lo)) * rg.token_bytes;
+        if (image + in_image + rg.token_bytes > p.packed_bytes) {
+          report(p.status, RLT_STATUS_BAD_RANGE, w.request(), w.logical() * p.block_size + w.t_lo, w.logical() * p.block_size + w.t_hi);
+          continue;
+        }
+        in_image += static_cast<long long>(at.within) * static_cast<int>(sizeof(T));
+      }
+      const char* from = src + (K == kWireToPlane ? in_image : in_slice);
+      if (K == kExitToPlane || K == kExitToWire) {
+        const int e = s.exit_plane[at.token];
+        if (e < 0 || e >= p.src_planes) {
+          report(p.status, RLT_STATUS_BAD_PLANE, w.request(), w.logical() * p.block_size + at.token, e);
+          continue;
+        }
+        const long long block = used_block(p, w, s.src[e], s.src_id[e]);
+        if (block < 0) continue;
+        from += block + rg.slice_at;
+      }
+      to[u] = reinterpret_cast<T*>(dst + (K == kPlaneToWire || K == kExitToWire ? in_image : in_slice));
+      regs[u] = ld_stream(reinterpret_cast<const T*>(from));
+    }
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      if (to[u] != nullptr) st_stream(to[u], regs[u]);
+    }
+  }
+}
+
+// The kinds that walk the planes: every row of planes up to the token's exit plane is read once; the last one is also
+// what the deeper planes get (kFanOut, kDedupFromWire). kPlaneBatch loads of a thread are in flight before the
+// first store.
+constexpr int kPlaneBatch = 4;
+
+template <typename T, MoveKind K>
+__device__ __forceinline__ void walk_planes(const MoveParams& p, const MoveRegion& rg, const Piece& w, const PageShared& s) {
+  const int first = w.index * rg.per;
+  const int row0 = first / rg.row_vecs, rem0 = first - row0 * rg.row_vecs;
+  const int begin = p.plane_begin;
+  const int count = min(rg.per, rg.slice_vecs - first);
+  for (int k = static_cast<int>(threadIdx.x); k < count; k += kThreads) {
+    const RowAt at = row_at(p, rg, row0, rem0, k);
+    if (at.token < w.t_lo || at.token >= w.t_hi) continue;
+    const int e = s.exit_plane[at.token];
+    if (e < 0 || e >= p.src_planes) {
+      report(p.status, RLT_STATUS_BAD_PLANE, w.request(), w.logical() * p.block_size + at.token, e);
+      continue;
+    }
+    const char* src = rg.src[w.kv];
+    char* dst = rg.dst[w.kv];
+    const long long in_slice = rg.slice_at + static_cast<long long>(first + k) * static_cast<int>(sizeof(T));
+    const int end = p.plane_end > 1 && !deep_carried(p, at.layer) ? 1 : p.plane_end;  // planes this row reaches
+    if (begin >= end) continue;
+    // source rows are those of planes [begin, begin + loads): plane p <- min(p, e)
+    const int loads = max(1, min(e + 1, end) - begin);
+    const int within = at.within * static_cast<int>(sizeof(T));
+    const unsigned long long below = (1ull << at.token) - 1ull;
+    // this row's offset in the image for one of the planes that carry it, -1 (reported) past the image's end
+    auto image_at = [&](int plane) -> long long {
+      const unsigned long long mask = s.carried[plane];
+      const long long row = s.wire[plane] + (static_cast<long long>(at.layer) * __popcll(mask) + __popcll(mask & below)) * rg.token_bytes;
+      if (row + rg.token_bytes <= p.packed_bytes) return row + within;
+      report(p.status, RLT_STATUS_BAD_RANGE, w.request(), w.logical() * p.block_size + w.t_lo, w.logical() * p.block_size + w.t_hi);
+      return -1;
+    };
+    T last;
+    bool last_ok = false;
+    for (int j0 = 0; j0 < loads; j0 += kPlaneBatch) {
+      T regs[kPlaneBatch];
+      bool ok[kPlaneBatch];
+#pragma unroll
+      for (int j = 0; j < kPlaneBatch; ++j) {
+        const int plane = begin + j0 + j;
+        ok[j] = j0 + j < loads;
+        if (!ok[j]) continue;
+        long long from;
+        if (K == kDedupFromWire) {
+          from = image_at(plane);
+          ok[j] = from >= 0;
+        } else {
+          const int sp = min(plane, e);
+          from = used_block(p, w, s.src[sp], s.src_id[sp]);
+          ok[j] = from >= 0;
+          from += in_slice;
+        }
+        if (ok[j]) regs[j] = ld_stream(reinterpret_cast<const T*>(src + from));
+      }
+#pragma unroll
+      for (int j = 0; j < kPlaneBatch; ++j) {
+        const int plane = begin + j0 + j;
+        if (j0 + j >= loads) continue;
+        const long long to = used_block(p, w, s.dst[plane], s.dst_id[plane]);
+        if (ok[j] && to >= 0) st_stream(reinterpret_cast<T*>(dst + to + in_slice), regs[j]);
+        last_ok = ok[j];
+        if (ok[j]) last = regs[j];
+      }
+    }
+    if (last_ok) {
+      for (int plane = begin + loads; plane < end; ++plane) {
+        const long long to = used_block(p, w, s.dst[plane], s.dst_id[plane]);
+        if (to >= 0) st_stream(reinterpret_cast<T*>(dst + to + in_slice), last);
+      }
+    }
+  }
+}
+
+// Lists the pairs of the page; returns how many. Every warp scans the tokens' plane counts for itself.
+__device__ __forceinline__ int list_pairs(const MoveParams& p, const Piece& w, const PageShared& s, PagePairs& pairs) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int start[2], total = 0;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int t = lane + 32 * h;
+    int planes = 0;
+    if (t >= w.t_lo && t < w.t_hi) {
+      const int e = s.exit_plane[t];
+      planes = e < 0 ? 0 : min(e + 1, p.src_planes);
+    }
+    const int through = warp_inclusive_scan(planes);
+    start[h] = total + through - planes;
+    total += __shfl_sync(0xffffffffu, through, 31);
+  }
+  for (int t = warp; t < p.block_size; t += kThreads / 32) {
+    const int from = __shfl_sync(0xffffffffu, t < 32 ? start[0] : start[1], t & 31);
+    if (t < w.t_lo || t >= w.t_hi) continue;
+    const int planes = min(s.exit_plane[t] + 1, p.src_planes);
+    for (int plane = lane; plane < planes; plane += 32) pairs.code[from + plane] = static_cast<unsigned short>(plane << 8 | t);
+  }
+  __syncthreads();
+  return total;
+}
+
+// Dedup pack. What a page contributes differs from page to page, so its vectors - (layer, pair, vector of the row) - are
+// dealt to the page's CTAs in equal shares: every thread has something to copy, whatever the exit planes.
+template <typename T>
+__device__ __forceinline__ void pack_pairs(const MoveParams& p, const MoveRegion& rg, const Piece& w, const PageShared& s,
+                                           PagePairs& pairs) {
+  constexpr int kU = flight_of<T>();
+  const int n = list_pairs(p, w, s, pairs);
+  if (w.index == 0 && w.g == 0 && w.kv == 0) {  // one CTA of the page looks for tokens whose exit plane is no plane
+    const int t = static_cast<int>(threadIdx.x);
+    if (t >= w.t_lo && t < w.t_hi && (s.exit_plane[t] < 0 || s.exit_plane[t] >= p.src_planes))
+      report(p.status, RLT_STATUS_BAD_PLANE, w.request(), w.logical() * p.block_size + t, s.exit_plane[t]);
+  }
+  if (n == 0) return;
+  const unsigned n_magic = n == 1 ? 0u : static_cast<unsigned>((1ull << 32) / static_cast<unsigned>(n)) + 1u;
+  const long long all = static_cast<long long>(p.slice_layers) * n * rg.row_vecs;
+  const int first = static_cast<int>(all * w.index / rg.pieces);
+  const int count = static_cast<int>(all * (w.index + 1) / rg.pieces) - first;
+  const int row0 = first / rg.row_vecs, rem0 = first - row0 * rg.row_vecs;
+  const char* src = rg.src[w.kv] + rg.slice_at;
+  char* dst = rg.dst[w.kv];
+  for (int k0 = static_cast<int>(threadIdx.x); k0 < count; k0 += kThreads * kU) {
+    T regs[kU];
+    T* to[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const int k = k0 + u * kThreads;
+      to[u] = nullptr;
+      if (k >= count) continue;
+      const unsigned j = static_cast<unsigned>(rem0 + k);
+      const int q = rg.row_magic ? static_cast<int>(__umulhi(j, rg.row_magic)) : static_cast<int>(j);
+      const int row = row0 + q;
+      const int layer = n_magic ? static_cast<int>(__umulhi(static_cast<unsigned>(row), n_magic)) : row;
+      const int code = pairs.code[row - layer * n];
+      const int plane = code >> 8, token = code & 0xff;
+      if (s.exit_plane[token] >= p.src_planes) continue;  // reported above
+      const unsigned long long mask = s.carried[plane];
+      const long long image = s.wire[plane] + (static_cast<long long>(layer) * __popcll(mask) + __popcll(mask & ((1ull << token) - 1ull))) * rg.token_bytes;
+      if (image + rg.token_bytes > p.packed_bytes) {
+        report(p.status, RLT_STATUS_BAD_RANGE, w.request(), w.logical() * p.block_size + w.t_lo, w.logical() * p.block_size + w.t_hi);
+        continue;
+      }
+      const long long block = used_block(p, w, s.src[plane], s.src_id[plane]);
+      if (block < 0) continue;
+      const int within = (static_cast<int>(j) - q * rg.row_vecs) * static_cast<int>(sizeof(T));
+      regs[u] = ld_stream(reinterpret_cast<const T*>(src + block + (static_cast<long long>(layer) * p.block_size + token) * rg.token_bytes + within));
+      to[u] = reinterpret_cast<T*>(dst + image + within);
+    }
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      if (to[u] != nullptr) st_stream(to[u], regs[u]);
+    }
+  }
+}
+
+template <typename T, MoveKind K>
+__device__ __forceinline__ void move_piece(const MoveParams& p, const MoveRegion& rg, const Piece& w, const PageShared& s, PagePairs& pairs) {
+  if constexpr (K == kDedupToWire) {
+    pack_pairs<T>(p, rg, w, s, pairs);
+  } else if constexpr (loops_planes(K)) {
+    walk_planes<T, K>(p, rg, w, s);
+  } else {
+    move_rows<T, K>(p, rg, w, s);
+  }
+}
+
+template <MoveKind K, int kWords>
+__global__ void __launch_bounds__(kThreads, loops_planes(K) ? 3 : 6) move_kernel(const __grid_constant__ MoveArgs<kWords> args) {
+  const MoveParams& p = args.p;
+  const int* records = kWords > 1 ? args.inline_words : p.records;
+  const int* wire = kWords > 1 ? args.inline_words + p.blocks * p.words : p.wire;
+  unsigned at = blockIdx.x;
+  Piece w;
+  const unsigned page = at / (static_cast<unsigned>(p.pieces) * p.grid_planes);
+  at -= page * (static_cast<unsigned>(p.pieces) * p.grid_planes);
+  const unsigned plane = at / p.pieces;
+  at -= plane * p.pieces;
+  w.plane = p.plane_begin + static_cast<int>(plane);
+  w.g = at >= 2u * p.region[0].pieces;
+  if (w.g) at -= 2u * p.region[0].pieces;
+  const MoveRegion& rg = p.region[w.g];
+  w.kv = at >= static_cast<unsigned>(rg.pieces);
+  w.index = static_cast<int>(at) - w.kv * rg.pieces;
+  w.rec = records + static_cast<long long>(page) * p.words;
+  const int range = w.rec[2];
+  if ((K == kDedupToWire || K == kDedupFromWire) && blockIdx.x == 0 && threadIdx.x == 0) {
+    p.wire_header[0] = p.wire_tokens;
+    p.wire_header[1] = static_cast<long long>(p.blocks) * p.src_planes;
+  }
+  if (range == kRecordBad) {
+    if (threadIdx.x == 0) report(p.status, RLT_STATUS_BAD_RANGE, w.request(), w.rec[3], w.rec[4]);
+    return;
+  }
+  w.t_lo = range & 0xff;
+  w.t_hi = range >> 8;
+  __shared__ PageShared shared;  // not allocated where nothing touches it
+  __shared__ PagePairs pairs;
+  if constexpr (loops_planes(K) || K == kExitToPlane || K == kExitToWire || K == kDedupToWire)
+    fetch_page<K>(p, rg, w, wire + static_cast<long long>(page) * p.src_planes, shared);
+  if (rg.vec_bytes == 32) {
+    move_piece<Vec32, K>(p, rg, w, shared, pairs);
+  } else if (rg.vec_bytes == 16) {
+    move_piece<uint4, K>(p, rg, w, shared, pairs);
+  } else if (rg.vec_bytes == 4) {
+    move_piece<uint32_t, K>(p, rg, w, shared, pairs);
+  } else {
+    move_piece<uint8_t, K>(p, rg, w, shared, pairs);
+  }
+}
+
+template <MoveKind K, int kWords>
+void launch_move(const MoveParams& p, const RltBlockMoves& m, unsigned grid, cudaStream_t stream) {
+  MoveArgs<kWords> args;
+  args.p = p;
+  if (kWords > 1) {
+    const size_t n = static_cast<size_t>(m.blocks) * m.words;
+    std::memcpy(args.inline_words, m.host_records, n * sizeof(int));
+    if (m.host_wire != nullptr)
+      std::memcpy(args.inline_words + n, m.host_wire, static_cast<size_t>(m.blocks) * p.src_planes * sizeof(int));
+  }
+  move_kernel<K, kWords><<<grid, kThreads, 0, stream>>>(args);
+}
+
+template <MoveKind K>
+int launch_kind(const MoveParams& p, const RltBlockMoves& m, unsigned grid, cudaStream_t stream) {
+  const long long n = static_cast<long long>(m.blocks) * m.words + (m.host_wire ? static_cast<long long>(m.blocks) * p.src_planes : 0);
+  // A parameter block is copied into the launch whole, so two sizes of it: 3.5 KiB covers a few hundred tokens.
+  if (n <= kInlineSmallWords) {
+    launch_move<K, kInlineSmallWords>(p, m, grid, stream);
+  } else if (n <= kInlineWords) {
+    launch_move<K, kInlineWords>(p, m, grid, stream);
+  } else if (p.records != nullptr && (m.host_wire == nullptr || p.wire != nullptr)) {
+    launch_move<K, 1>(p, m, grid, stream);
+  } else {
+    return RLT_E_INVALID;
+  }
+  return RLT_OK;
+}
+
+int vectors_per_round(int vec_bytes, bool planes) {
+  return kThreads * (vec_bytes == 32 ? unroll_of<Vec32>(planes) : vec_bytes == 16 ? unroll_of<uint4>(planes)
+                     : vec_bytes == 4 ? unroll_of<uint32_t>(planes) : unroll_of<uint8_t>(planes));
+}
+
+}  // namespace
+}  // namespace rlt
+
+extern "C" int rlt_move_blocks(int direction, const RltPool* src, const RltPool* dst, const RltBlockMoves* m,
+                               const RltOptions* opt, void* packed, int64_t packed_bytes, rlt_stream_t stream) {
+  using namespace rlt;
+  const Direction dir = static_cast<Direction>(direction);
+  const NvtxRange range(dir == kDirect ? "rlt.kv_handoff" : dir == kPack ? "rlt.kv_pack" : "rlt.kv_scatter");
+  if (m == nullptr || opt == nullptr) return RLT_E_INVALID;
+  // The checks of the table-driven entry points, on a batch of the same shape (its arrays are never touched).
+  static const int32_t present = 0;
+  static const int64_t present64 = 0;
+  RltBatch shape = {};
+  shape.num_requests = m->num_requests;
+  shape.table_width = m->table_width;
+  shape.src_tables = m->src_planes ? &present : nullptr;
+  shape.dst_tables = m->dst_planes ? &present : nullptr;
+  shape.tok_begin = shape.tok_end = &present;
+  if (m->has_exit) {
+    shape.exit_planes = &present;
+    shape.exit_offsets = &present64;
+    shape.exit_count = 1;
+  }
+  TableCopyParams t;
+  const int checked = table_params(dir, src, dst, &shape, opt, packed, packed_bytes, t);
+  if (checked != RLT_OK) return checked;
+  const bool dedup = opt->mode == RLT_MODE_DEDUP;
+  if (t.dedup_wire) {
+    if (opt->workspace == nullptr) return RLT_E_INVALID;
+    if (reinterpret_cast<uintptr_t>(opt->workspace) & 15u) return RLT_E_ALIGN;
+    if (opt->workspace_bytes < dedup_workspace_bytes(m->num_requests, m->table_width, t.src_planes)) return RLT_E_LIMIT;
+  }
+  if (opt->variant != 0 || opt->grid_limit != 0 || t.src_planes > 64 || t.dst_planes > 64) return RLT_MOVE_UNSUITED;
+  if (dir != kDirect && (t.plane_begin != 0 || t.plane_count != t.dst_planes)) return RLT_MOVE_UNSUITED;
+  if (t.block_size != m->block_size || (dir != kScatter && m->src_planes != t.src_planes) ||
+      (dir != kPack && m->dst_planes != t.dst_planes))
+    return RLT_MOVE_UNSUITED;
+  if (t.dedup_wire && m->host_wire == nullptr) return RLT_MOVE_UNSUITED;
+  if (m->blocks == 0) return RLT_OK;
+
+  const MoveKind kind = dir == kDirect ? (dedup ? kFanOut : opt->mode == RLT_MODE_EXIT_ONLY ? kExitToPlane : kPlaneToPlane)
+                        : dir == kPack ? (dedup ? kDedupToWire : opt->mode == RLT_MODE_EXIT_ONLY ? kExitToWire : kPlaneToWire)
+                                       : (dedup ? kDedupFromWire : kWireToPlane);
+  const bool planes = loops_planes(kind), pairs = kind == kDedupToWire;
+  MoveParams p = {};
+  p.slice_layers = t.layer_end - t.layer_begin;
+  for (int g = 0; g < t.num_regions; ++g) {
+    const RegionParams& s = t.region[g];
+    MoveRegion& rg = p.region[g];
+    rg.src[0] = s.src_key;
+    rg.src[1] = s.src_value;
+    rg.dst[0] = s.dst_key;
+    rg.dst[1] = s.dst_value;
+    rg.block_bytes = s.block_bytes;
+    rg.slice_at = s.layer_bytes * t.layer_begin;
+    rg.token_bytes = static_cast<int>(s.token_bytes);
+    rg.vec_bytes = s.wide_ok ? 32 : s.vec_bytes;
+    const long long row_vecs = s.token_bytes / rg.vec_bytes;
+    const long long slice_vecs = row_vecs * t.block_size * p.slice_layers;
+    // the multiplier splits of row_at: (row_vecs + piece) * row_vecs and rows * block_size below 2^32
+    if ((row_vecs + 65536) * row_vecs >= (1ll << 32) || slice_vecs * t.src_planes >= (1ll << 30) ||
+        static_cast<long long>(t.block_size) * t.block_size * p.slice_layers >= (1ll << 32))
+      return RLT_MOVE_UNSUITED;
+    rg.row_vecs = static_cast<int>(row_vecs);
+    rg.row_magic = row_vecs == 1 ? 0u : div_magic(static_cast<uint32_t>(row_vecs));
+    rg.slice_vecs = static_cast<int>(slice_vecs);
+  }
+  p.plane_begin = t.plane_begin;
+  p.plane_end = t.plane_begin + t.plane_count;
+  p.grid_planes = planes || pairs ? 1 : t.plane_count;
+  p.src_planes = t.src_planes;
+  p.dst_planes = t.dst_planes;
+  p.src_blocks = t.src_blocks;
+  p.dst_blocks = t.dst_blocks;
+  p.block_size = t.block_size;
+  p.block_magic = t.block_size == 1 ? 0u : div_magic(static_cast<uint32_t>(t.block_size));
+  p.layer_begin = t.layer_begin;
+  p.deep_layer_mask = t.deep_layer_mask;
+  p.packed_bytes = t.packed_bytes;
+  p.packed_token_bytes = t.packed_token_bytes;
+  p.words = m->words;
+  p.blocks = m->blocks;
+  p.dst_at = kRecordHeader + m->src_planes;
+  p.exit_at = kRecordHeader + m->src_planes + m->dst_planes;
+  p.records = m->device_records;
+  p.wire = m->device_wire;
+  p.wire_header = static_cast<long long*>(opt->workspace);
+  p.wire_tokens = m->wire_tokens;
+  p.status = opt->status;
+  // Rounds of a piece. Where a plane's block is all a CTA looks up, one: the smaller the piece the closer the SMs stay
+  // together. Kinds that fetch the page's record and work out exit planes first need more payload behind that: measured
+  // best at 2 for exit-only (29k tokens: 1.84 -> 1.75 ms), at about 12 / planes where planes are walked (6.4k tokens, four planes:
+  // 1.36 -> 1.23 ms; at 32 planes one round is best), at 8 for a dedup pack (1.86 -> 0.95 ms). A launch of fewer than eight
+  // waves takes the smallest piece that a larger one would split into: it is short of CTAs, not of payload per CTA.
+  int sms = 0;
+  const int found = sm_count(&sms);
+  if (found != RLT_OK) return found;
+  const bool by_exit = kind == kExitToPlane || kind == kExitToWire;
+  int rounds = pairs ? 8 : planes ? std::max(1, std::min(4, 12 / p.dst_planes)) : by_exit ? 2 : 1;
+  long long grid = 0;
+  for (;; rounds /= 2) {
+    p.pieces = 0;
+    for (int g = 0; g < t.num_regions; ++g) {
+      MoveRegion& rg = p.region[g];
+      rg.per = vectors_per_round(rg.vec_bytes, planes) * rounds;
+      const long long most = static_cast<long long>(rg.slice_vecs) * (pairs ? p.src_planes : 1);
+      rg.pieces = static_cast<int>((most + rg.per - 1) / rg.per);
+      p.pieces += 2 * rg.pieces;
+    }
+    grid = static_cast<long long>(m->blocks) * p.grid_planes * p.pieces;
+    if (rounds == 1 || grid >= 8ll * sms * (planes ? 3 : 6)) break;
+  }
+  if (grid > 0x7fffffffll) return RLT_MOVE_UNSUITED;
+
+  const cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  const unsigned ctas = static_cast<unsigned>(grid);
+  int rc = RLT_E_INVALID;
+  switch (kind) {
+    case kPlaneToPlane: rc = launch_kind<kPlaneToPlane>(p, *m, ctas, s); break;
+    case kExitToPlane: rc = launch_kind<kExitToPlane>(p, *m, ctas, s); break;
+    case kFanOut: rc = launch_kind<kFanOut>(p, *m, ctas, s); break;
+    case kPlaneToWire: rc = launch_kind<kPlaneToWire>(p, *m, ctas, s); break;
+    case kExitToWire: rc = launch_kind<kExitToWire>(p, *m, ctas, s); break;
+    case kDedupToWire: rc = launch_kind<kDedupToWire>(p, *m, ctas, s); break;
+    case kWireToPlane: rc = launch_kind<kWireToPlane>(p, *m, ctas, s); break;
+    case kDedupFromWire: rc = launch_kind<kDedupFromWire>(p, *m, ctas, s); break;
+  }
+  if (rc != RLT_OK) return rc;
+  RLT_CUDA_TRY(cudaGetLastError());
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  return RLT_OK;
+}

@@ -1,0 +1,581 @@
+// vllm_rlt_b200._host: the host side of the Python calls that a serving loop makes per step or per chunk.
+//
+// A launch of this library takes a GPU a few to a few hundred microseconds, so the time Python needs to look over block
+// tables, fill structs and find the current stream decides how many of them a worker can issue. This module does that
+// part in C++: it reads tables (tuples, lists, int32 arrays) straight into the records of block_moves.h, reads tensors'
+// addresses and shapes without building Python objects, and calls the C ABI. Checks and messages are those of the
+// Python callers' documentation.
+
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <cstring>
+#include <memory>
+#include <string>
+#include <vector>
+
+#include "block_moves.h"
+#include "rlt_kv_handoff.h"
+
+namespace {
+
+struct Failure {};  // a Python error is set
+
+[[noreturn]] void fail(PyObject* type, const char* text) {
+  PyErr_SetString(type, text);
+  throw Failure{};
+}
+[[noreturn]] void bad_value(const char* text) { fail(PyExc_ValueError, text); }
+
+struct Ref {
+  PyObject* p;
+  explicit Ref(PyObject* q) : p(q) {
+    if (q == nullptr) throw Failure{};
+  }
+  ~Ref() { Py_DECREF(p); }
+  Ref(const Ref&) = delete;
+  Ref& operator=(const Ref&) = delete;
+};
+
+struct Buffer {
+  Py_buffer view;
+  bool held = false;
+  ~Buffer() {
+    if (held) PyBuffer_Release(&view);
+  }
+};
+
+long long integer(PyObject* o) {
+  if (PyLong_Check(o)) {
+    const long long v = PyLong_AsLongLong(o);
+    if (v == -1 && PyErr_Occurred()) throw Failure{};
+    return v;
+  }
+  const Ref n(PyNumber_Long(o));
+  const long long v = PyLong_AsLongLong(n.p);
+  if (v == -1 && PyErr_Occurred()) throw Failure{};
+  return v;
+}
+
+int32_t int32_of(long long v) {
+  if (v < INT32_MIN || v > INT32_MAX) fail(PyExc_OverflowError, "block id or exit plane out of bounds for int32");
+  return static_cast<int32_t>(v);
+}
+
+bool is_int32(const Py_buffer& v) {
+  return v.itemsize == 4 && v.format != nullptr && (std::strcmp(v.format, "i") == 0 || std::strcmp(v.format, "l") == 0);
+}
+
+// Appends the int32 values of one table (or exit-plane array) to `out`; returns how many.
+Py_ssize_t append_ints(PyObject* o, std::vector<int32_t>& out, const char* not_flat) {
+  if (PyTuple_CheckExact(o) || PyList_CheckExact(o)) {
+    const Py_ssize_t n = PySequence_Fast_GET_SIZE(o);
+    PyObject** items = PySequence_Fast_ITEMS(o);
+    const size_t at = out.size();
+    out.resize(at + static_cast<size_t>(n));
+    for (Py_ssize_t i = 0; i < n; ++i) {
+      PyObject* item = items[i];
+      if (PyTuple_Check(item) || PyList_Check(item)) bad_value(not_flat);
+      out[at + i] = int32_of(integer(item));
+    }
+    return n;
+  }
+  auto take = [&](PyObject* source) -> Py_ssize_t {
+    Buffer b;
+    if (PyObject_GetBuffer(source, &b.view, PyBUF_RECORDS_RO) != 0) {
+      PyErr_Clear();
+      return -1;
+    }
+    b.held = true;
+    if (b.view.ndim != 1) bad_value(not_flat);
+    if (!is_int32(b.view)) return -1;
+    const Py_ssize_t n = b.view.shape[0], stride = b.view.strides[0];
+    const size_t at = out.size();
+    out.resize(at + static_cast<size_t>(n));
+    const char* from = static_cast<const char*>(b.view.buf);
+    if (stride == 4) {
+      std::memcpy(out.data() + at, from, 4 * static_cast<size_t>(n));
+    } else {
+      for (Py_ssize_t i = 0; i < n; ++i) std::memcpy(&out[at + i], from + i * stride, 4);
+    }
+    return n;
+  };
+  Py_ssize_t n = take(o);
+  if (n >= 0) return n;
+  const Ref numpy(PyImport_ImportModule("numpy"));
+  const Ref array(PyObject_CallMethod(numpy.p, "asarray", "OO", o, Ref(PyObject_GetAttrString(numpy.p, "int32")).p));
+  n = take(array.p);
+  if (n < 0) fail(PyExc_TypeError, "block tables and exit planes must hold integers");
+  return n;
+}
+
+Py_ssize_t length(PyObject* o) {
+  const Py_ssize_t n = PyObject_Length(o);
+  if (n < 0) throw Failure{};
+  return n;
+}
+
+// ------------------------------------------------------------------------------------------------ batch plans
+
+struct Side {
+  bool given = false;
+  int planes = 0;
+  int width = 0;                       // pages of the longest table
+  std::vector<int32_t> flat;           // every table, back to back
+  std::vector<size_t> at;              // [n * planes] where each starts
+  std::vector<Py_ssize_t> pages;       // [n] of each request's tables
+  const int32_t* table(int r, int p) const { return flat.data() + at[static_cast<size_t>(r) * planes + p]; }
+};
+
+struct Plan {
+  int n = 0, block_size = 0, width = 1;
+  Side src, dst;
+  std::vector<int64_t> begin, end;
+  bool has_exit = false;
+  std::vector<int32_t> exits;
+  std::vector<int64_t> exit_at;  // [n] index in exits of each request's token 0
+  int blocks = 0, words = 0;
+  std::vector<int32_t> records;
+  int wire_planes = 0;
+  std::vector<int32_t> wire;
+  int64_t wire_tokens = 0;
+
+  void make_records();
+  void make_wire(int planes);
+};
+
+void read_side(PyObject* tables, Side& side, int n, int block_size, const std::vector<int64_t>& end) {
+  side.given = true;
+  if (length(tables) != n) bad_value("one table set per request is required");
+  const Ref requests(PySequence_Fast(tables, "block tables must be a sequence of requests"));
+  std::vector<std::unique_ptr<Ref>> sets;
+  sets.reserve(n);
+  for (int r = 0; r < n; ++r)
+    sets.push_back(std::make_unique<Ref>(PySequence_Fast(PySequence_Fast_GET_ITEM(requests.p, r), "a request's tables must be a sequence")));
+  side.planes = static_cast<int>(PySequence_Fast_GET_SIZE(sets[0]->p));
+  for (int r = 0; r < n; ++r) {
+    if (PySequence_Fast_GET_SIZE(sets[r]->p) != side.planes) bad_value("requests of one batch must have the same number of planes");
+  }
+  side.at.reserve(static_cast<size_t>(n) * side.planes);
+  side.pages.resize(n);
+  bool ragged = false;
+  for (int r = 0; r < n; ++r) {
+    Py_ssize_t first = 0, least = 0;
+    for (int p = 0; p < side.planes; ++p) {
+      side.at.push_back(side.flat.size());
+      const Py_ssize_t pages = append_ints(PySequence_Fast_GET_ITEM(sets[r]->p, p), side.flat, "a block table must be a flat sequence of block ids");
+      if (p == 0) first = least = pages;
+      ragged |= pages != first;
+      least = pages < least ? pages : least;
+    }
+    if (end[r] > static_cast<int64_t>(least) * block_size) bad_value("KV range exceeds allocation");
+    side.pages[r] = first;
+    if (first > side.width) side.width = static_cast<int>(first);
+  }
+  if (ragged) bad_value("the planes of one request must have tables of equal length");
+}
+
+// A block id outside the pool matters only on pages that the request's range touches.
+void check_blocks(const Side& side, const Plan& plan, long long limit) {
+  if (!side.given) return;
+  for (int r = 0; r < plan.n; ++r) {
+    const int64_t lo = plan.begin[r] / plan.block_size, hi = (plan.end[r] - 1) / plan.block_size;
+    for (int p = 0; p < side.planes; ++p) {
+      const int32_t* t = side.table(r, p);
+      bool bad = false;
+      if (limit < 0) {
+        for (int64_t i = lo; i <= hi; ++i) bad |= t[i] < 0;
+      } else {
+        for (int64_t i = lo; i <= hi; ++i) bad |= static_cast<long long>(static_cast<uint32_t>(t[i])) >= limit;
+      }
+      if (bad) bad_value("physical block outside registered pool");
+    }
+  }
+}
+
+void Plan::make_records() {
+  words = kRecordHeader + src.planes + dst.planes + (has_exit ? block_size : 0);
+  int64_t total = 0;
+  for (int r = 0; r < n; ++r) total += (end[r] - 1) / block_size - begin[r] / block_size + 1;
+  blocks = static_cast<int>(total);
+  records.resize(static_cast<size_t>(total) * words);
+  int32_t* w = records.data();
+  int64_t before = 0;
+  for (int r = 0; r < n; ++r) {
+    const int64_t b = begin[r], e = end[r];
+    for (int64_t page = b / block_size; page <= (e - 1) / block_size; ++page, w += words) {
+      const int64_t base = page * block_size;
+      const int64_t lo = b > base ? b - base : 0, hi = e < base + block_size ? e - base : block_size;
+      w[0] = r;
+      w[1] = static_cast<int32_t>(page);
+      w[2] = static_cast<int32_t>(lo | hi << 8);
+      w[3] = static_cast<int32_t>(base + lo - b);
+      w[4] = static_cast<int32_t>(before);
+      w[5] = static_cast<int32_t>(e - b);
+      int32_t* id = w + kRecordHeader;
+      for (const Side* side : {&src, &dst}) {
+        for (int p = 0; p < side->planes; ++p) *id++ = side->table(r, p)[page];
+      }
+      if (has_exit) {
+        std::memset(id, 0, 4 * static_cast<size_t>(block_size));
+        std::memcpy(id + lo, exits.data() + exit_at[r] + base + lo, 4 * static_cast<size_t>(hi - lo));
+      }
+    }
+    before += e - b;
+  }
+}
+
+// Wire order: request, plane, page; a page's tokens count on every plane up to their exit plane.
+void Plan::make_wire(int planes) {
+  if (wire_planes == planes) return;
+  std::vector<int32_t> at(static_cast<size_t>(blocks) * planes);
+  std::vector<int32_t> carried(planes + 1);
+  const int exit_word = kRecordHeader + src.planes + dst.planes;
+  for (int b = 0; b < blocks; ++b) {
+    const int32_t* w = records.data() + static_cast<size_t>(b) * words;
+    std::fill(carried.begin(), carried.end(), 0);
+    for (int t = w[2] & 0xff; t < w[2] >> 8; ++t) {
+      const int32_t e = w[exit_word + t];
+      if (e >= 0) ++carried[e < planes ? e : planes - 1];
+    }
+    int32_t sum = 0;
+    for (int p = planes - 1; p >= 0; --p) at[static_cast<size_t>(b) * planes + p] = sum += carried[p];
+  }
+  int64_t run = 0;
+  for (int b = 0; b < blocks;) {
+    int next = b;
+    while (next < blocks && records[static_cast<size_t>(next) * words] == records[static_cast<size_t>(b) * words]) ++next;
+    for (int p = 0; p < planes; ++p) {
+      for (int k = b; k < next; ++k) {
+        int32_t& slot = at[static_cast<size_t>(k) * planes + p];
+        const int32_t count = slot;
+        slot = static_cast<int32_t>(run);
+        run += count;
+      }
+    }
+    b = next;
+  }
+  wire = std::move(at);
+  wire_tokens = run;
+  wire_planes = planes;
+}
+
+constexpr const char* kPlanName = "vllm_rlt_b200.plan";
+void free_plan(PyObject* capsule) { delete static_cast<Plan*>(PyCapsule_GetPointer(capsule, kPlanName)); }
+Plan& plan_of(PyObject* capsule) {
+  auto* p = static_cast<Plan*>(PyCapsule_GetPointer(capsule, kPlanName));
+  if (p == nullptr) throw Failure{};
+  return *p;
+}
+
+// plan(src_tables | None, dst_tables | None, ranges, exit_planes | None, block_size, src_blocks | None, dst_blocks | None,
+//      most requests) -> (plan, requests, tokens, width, source planes, destination planes, exit entries, ranges, record bytes)
+PyObject* make_plan(PyObject* const* a) {
+  auto plan = std::make_unique<Plan>();
+  const Py_ssize_t n = length(a[2]);
+  const long long most = integer(a[7]);
+  if (n < 1) bad_value("a handoff batch needs at least one request");
+  if (n > most) bad_value(("a handoff batch holds at most " + std::to_string(most) + " requests").c_str());
+  plan->n = static_cast<int>(n);
+  plan->block_size = static_cast<int>(integer(a[4]));
+  if (plan->block_size < 1) bad_value("block_size must be positive");
+  const Ref ranges(PySequence_Fast(a[2], "ranges must be a sequence of (start, end)"));
+  int64_t tokens = 0;
+  for (int r = 0; r < n; ++r) {
+    const Ref pair(PySequence_Fast(PySequence_Fast_GET_ITEM(ranges.p, r), "a range is (start, end)"));
+    if (PySequence_Fast_GET_SIZE(pair.p) != 2) bad_value("a range is (start, end)");
+    const int64_t b = integer(PySequence_Fast_GET_ITEM(pair.p, 0)), e = integer(PySequence_Fast_GET_ITEM(pair.p, 1));
+    plan->begin.push_back(b);
+    plan->end.push_back(e);
+    tokens += e - b;
+  }
+  for (int r = 0; r < n; ++r) {
+    if (plan->begin[r] < 0 || plan->begin[r] >= plan->end[r]) bad_value("invalid KV range");
+  }
+  if (a[0] != Py_None) read_side(a[0], plan->src, plan->n, plan->block_size, plan->end);
+  if (a[1] != Py_None) read_side(a[1], plan->dst, plan->n, plan->block_size, plan->end);
+  for (const Side* side : {&plan->src, &plan->dst}) plan->width = side->width > plan->width ? side->width : plan->width;
+  check_blocks(plan->src, *plan, a[5] == Py_None ? -1 : integer(a[5]));
+  check_blocks(plan->dst, *plan, a[6] == Py_None ? -1 : integer(a[6]));
+  if (a[3] != Py_None) {
+    plan->has_exit = true;
+    if (length(a[3]) != n) bad_value("one exit-plane array per request is required");
+    const Ref parts(PySequence_Fast(a[3], "exit planes must be a sequence of per-request arrays"));
+    constexpr const char* kCover = "exit planes must cover every token position up to the range end";
+    for (int r = 0; r < n; ++r) {
+      plan->exit_at.push_back(static_cast<int64_t>(plan->exits.size()));
+      const Py_ssize_t count = append_ints(PySequence_Fast_GET_ITEM(parts.p, r), plan->exits, kCover);
+      if (count < plan->end[r]) bad_value(kCover);
+    }
+  }
+  plan->make_records();
+  const Ref list(PyList_New(n));
+  for (int r = 0; r < n; ++r) {
+    PyObject* pair = Py_BuildValue("LL", static_cast<long long>(plan->begin[r]), static_cast<long long>(plan->end[r]));
+    if (pair == nullptr) throw Failure{};
+    PyList_SET_ITEM(list.p, r, pair);
+  }
+  Plan* raw = plan.release();
+  PyObject* capsule = PyCapsule_New(raw, kPlanName, free_plan);
+  if (capsule == nullptr) {
+    delete raw;
+    throw Failure{};
+  }
+  return Py_BuildValue("NiLiiiLOL", capsule, raw->n, static_cast<long long>(tokens), raw->width, raw->src.planes, raw->dst.planes,
+                       static_cast<long long>(raw->exits.size()), list.p, static_cast<long long>(4 * raw->records.size()));
+}
+
+// plan_layout(plan) -> (bytes, {name: offset}) of the padded arrays an RltBatch points at.
+// plan_arrays(plan, writable buffer): writes them there.
+struct Layout {
+  size_t offsets = 0, src = 0, dst = 0, begin = 0, end = 0, exits = 0, bytes = 0;
+};
+Layout layout_of(const Plan& p) {
+  Layout l;
+  auto put = [&](size_t bytes) {
+    l.bytes = (l.bytes + 15) & ~size_t{15};
+    const size_t at = l.bytes;
+    l.bytes += bytes;
+    return at;
+  };
+  const size_t n = p.n, row = 4 * n * p.width;
+  if (p.has_exit) l.offsets = put(8 * n);
+  if (p.src.given) l.src = put(row * p.src.planes);
+  if (p.dst.given) l.dst = put(row * p.dst.planes);
+  l.begin = put(4 * n);
+  l.end = put(4 * n);
+  if (p.has_exit) l.exits = put(4 * p.exits.size());
+  return l;
+}
+
+PyObject* plan_layout(PyObject* const* a) {
+  const Plan& p = plan_of(a[0]);
+  const Layout l = layout_of(p);
+  const Ref names(PyDict_New());
+  auto name = [&](const char* key, size_t at) {
+    const Ref v(PyLong_FromSize_t(at));
+    if (PyDict_SetItemString(names.p, key, v.p) != 0) throw Failure{};
+  };
+  if (p.has_exit) name("exit_offsets", l.offsets);
+  if (p.src.given) name("src_tables", l.src);
+  if (p.dst.given) name("dst_tables", l.dst);
+  name("tok_begin", l.begin);
+  name("tok_end", l.end);
+  if (p.has_exit) name("exit_planes", l.exits);
+  return Py_BuildValue("nO", static_cast<Py_ssize_t>(l.bytes), names.p);
+}
+
+PyObject* plan_arrays(PyObject* const* a) {
+  const Plan& p = plan_of(a[0]);
+  const Layout l = layout_of(p);
+  Buffer b;
+  if (PyObject_GetBuffer(a[1], &b.view, PyBUF_WRITABLE) != 0) throw Failure{};
+  b.held = true;
+  if (static_cast<size_t>(b.view.len) < l.bytes) bad_value("staging buffer too small");
+  char* out = static_cast<char*>(b.view.buf);
+  std::memset(out, 0, l.bytes);
+  auto tables = [&](const Side& side, size_t at) {
+    for (int r = 0; r < p.n; ++r) {
+      for (int q = 0; q < side.planes; ++q)
+        std::memcpy(out + at + 4 * (static_cast<size_t>(r) * side.planes + q) * p.width, side.table(r, q), 4 * static_cast<size_t>(side.pages[r]));
+    }
+  };
+  if (p.src.given) tables(p.src, l.src);
+  if (p.dst.given) tables(p.dst, l.dst);
+  for (int r = 0; r < p.n; ++r) {
+    const int32_t lo = static_cast<int32_t>(p.begin[r]), hi = static_cast<int32_t>(p.end[r]);
+    std::memcpy(out + l.begin + 4 * static_cast<size_t>(r), &lo, 4);
+    std::memcpy(out + l.end + 4 * static_cast<size_t>(r), &hi, 4);
+  }
+  if (p.has_exit) {
+    std::memcpy(out + l.offsets, p.exit_at.data(), 8 * static_cast<size_t>(p.n));
+    if (!p.exits.empty()) std::memcpy(out + l.exits, p.exits.data(), 4 * p.exits.size());
+  }
+  Py_RETURN_NONE;
+}
+
+// plan_wire(plan, planes) -> bytes of the wire plan, made at the first call. Tells how a dedup image is laid out.
+PyObject* plan_wire(PyObject* const* a) {
+  Plan& p = plan_of(a[0]);
+  if (!p.has_exit) return PyLong_FromLong(0);
+  p.make_wire(static_cast<int>(integer(a[1])));
+  return PyLong_FromSize_t(4 * p.wire.size());
+}
+
+// plan_fits(plan, with wire): whether the launch takes the records as kernel parameters.
+PyObject* plan_fits(PyObject* const* a) {
+  const Plan& p = plan_of(a[0]);
+  const size_t words = p.records.size() + (PyObject_IsTrue(a[1]) ? p.wire.size() : 0);
+  return PyBool_FromLong(words <= static_cast<size_t>(kInlineWords));
+}
+
+void* address(PyObject* o) { return o == Py_None ? nullptr : PyLong_AsVoidPtr(o); }
+
+// plan_upload(plan, which, device address, stream) -> code: records (0) or wire plan (1) to device memory.
+PyObject* plan_upload(PyObject* const* a) {
+  const Plan& p = plan_of(a[0]);
+  const std::vector<int32_t>& v = integer(a[1]) == 0 ? p.records : p.wire;
+  return PyLong_FromLong(rlt_stage_upload(v.data(), 4 * v.size(), address(a[2]), static_cast<rlt_stream_t>(address(a[3]))));
+}
+
+rlt_stream_t stream_of(PyObject* o) {  // None: the current stream of the current device
+  if (o != Py_None) return static_cast<rlt_stream_t>(PyLong_AsVoidPtr(o));
+  return reinterpret_cast<rlt_stream_t>(c10::cuda::getCurrentCUDAStream().stream());
+}
+
+const at::Tensor* tensor_of(PyObject* o) {
+  if (o == Py_None) return nullptr;
+  if (!THPVariable_Check(o)) fail(PyExc_TypeError, "expected a tensor");
+  return &THPVariable_Unpack(o);
+}
+
+void* data_of(PyObject* o) {
+  const at::Tensor* t = tensor_of(o);
+  return t == nullptr ? nullptr : t->data_ptr();
+}
+
+// move(direction, source pool, destination pool, plan, records, wire plan, mode, layer_begin, layer_end, wire_planes,
+//      plane_begin, plane_end, deep mask, status, grid_limit, variant, workspace, packed address, packed bytes, stream) -> code
+PyObject* move(PyObject* const* a) {
+  Plan& p = plan_of(a[3]);
+  const long direction = PyLong_AsLong(a[0]);
+  RltOptions o = {};
+  o.mode = static_cast<int32_t>(integer(a[6]));
+  o.layer_begin = static_cast<int32_t>(integer(a[7]));
+  o.layer_end = static_cast<int32_t>(integer(a[8]));
+  o.wire_planes = static_cast<int32_t>(integer(a[9]));
+  o.plane_begin = static_cast<int32_t>(integer(a[10]));
+  o.plane_end = static_cast<int32_t>(integer(a[11]));
+  o.deep_layer_mask = PyLong_AsUnsignedLongLong(a[12]);
+  o.status = static_cast<int32_t*>(data_of(a[13]));
+  o.grid_limit = static_cast<int32_t>(integer(a[14]));
+  o.variant = static_cast<int32_t>(integer(a[15]));
+  if (const at::Tensor* w = tensor_of(a[16])) {
+    if (w->scalar_type() != at::kByte || !w->is_contiguous() || !w->is_cuda())
+      bad_value("workspace must be a contiguous CUDA uint8 tensor");
+    o.workspace = w->data_ptr();
+    o.workspace_bytes = w->numel();
+  }
+  if (PyErr_Occurred()) throw Failure{};
+  RltBlockMoves m = {};
+  m.host_records = p.records.data();
+  m.device_records = static_cast<const int32_t*>(address(a[4]));
+  m.blocks = p.blocks;
+  m.words = p.words;
+  m.src_planes = p.src.planes;
+  m.dst_planes = p.dst.planes;
+  m.block_size = p.block_size;
+  m.has_exit = p.has_exit;
+  m.num_requests = p.n;
+  m.table_width = p.width;
+  if (direction != RLT_MOVE_DIRECT && o.mode == RLT_MODE_DEDUP && !p.wire.empty()) {
+    m.host_wire = p.wire.data();
+    m.device_wire = static_cast<const int32_t*>(address(a[5]));
+    m.wire_tokens = p.wire_tokens;
+  }
+  return PyLong_FromLong(rlt_move_blocks(static_cast<int>(direction), static_cast<const RltPool*>(address(a[1])),
+                                         static_cast<const RltPool*>(address(a[2])), &m, &o, address(a[17]), integer(a[18]),
+                                         stream_of(a[19])));
+}
+
+// ------------------------------------------------------------------------------------------------ other ops
+
+// handoff_host(source pool, destination pool, source tables, destination tables, begin, end, layer_begin, layer_end,
+//              plane_begin, plane_end, status, stream) -> code
+PyObject* handoff_host(PyObject* const* a) {
+  Buffer b[4];
+  for (int i = 0; i < 4; ++i) {
+    if (PyObject_GetBuffer(a[2 + i], &b[i].view, PyBUF_FORMAT | PyBUF_STRIDES) != 0) {
+      PyErr_Clear();
+      bad_value("host tables and ranges must be C-contiguous int32 arrays");
+    }
+    b[i].held = true;
+    if (!is_int32(b[i].view) || !PyBuffer_IsContiguous(&b[i].view, 'C'))
+      bad_value("host tables and ranges must be C-contiguous int32 arrays");
+  }
+  const Py_buffer &s = b[0].view, &d = b[1].view;
+  if (s.ndim != 3) bad_value("host tables must be [requests, planes, width]");
+  const Py_ssize_t n = s.shape[0];
+  auto one_per_request = [&](const Py_buffer& v) { return v.ndim == 1 && v.shape[0] == n; };
+  if (d.ndim != 3 || d.shape[0] != n || d.shape[2] != s.shape[2] || !one_per_request(b[2].view) || !one_per_request(b[3].view))
+    bad_value("source and destination tables must agree in requests and width, one range per request");
+  RltHostBatch hb = {};
+  hb.num_requests = static_cast<int32_t>(n);
+  hb.table_width = static_cast<int32_t>(s.shape[2]);
+  hb.src_planes = static_cast<int32_t>(s.shape[1]);
+  hb.dst_planes = static_cast<int32_t>(d.shape[1]);
+  hb.src_tables = static_cast<const int32_t*>(s.buf);
+  hb.dst_tables = static_cast<const int32_t*>(d.buf);
+  hb.tok_begin = static_cast<const int32_t*>(b[2].view.buf);
+  hb.tok_end = static_cast<const int32_t*>(b[3].view.buf);
+  RltOptions o = {};
+  o.layer_begin = static_cast<int32_t>(integer(a[6]));
+  o.layer_end = static_cast<int32_t>(integer(a[7]));
+  o.plane_begin = static_cast<int32_t>(integer(a[8]));
+  o.plane_end = static_cast<int32_t>(integer(a[9]));
+  o.status = static_cast<int32_t*>(data_of(a[10]));
+  return PyLong_FromLong(rlt_kv_handoff_host(static_cast<const RltPool*>(address(a[0])), static_cast<const RltPool*>(address(a[1])),
+                                             &hb, &o, stream_of(a[11])));
+}
+
+// finalize(pool, planes, tables, rows, layer mask, status, stream) -> code
+PyObject* finalize(PyObject* const* a) {
+  const at::Tensor* tables = tensor_of(a[2]);
+  const at::Tensor* rows = tensor_of(a[3]);
+  if (tables == nullptr || rows == nullptr) fail(PyExc_TypeError, "expected a tensor");
+  if (tables->scalar_type() != at::kInt || !tables->is_contiguous() || !tables->is_cuda())
+    bad_value("tables must be a contiguous CUDA int32 tensor");
+  if (rows->scalar_type() != at::kInt || !rows->is_contiguous() || !rows->is_cuda())
+    bad_value("rows must be a contiguous CUDA int32 tensor");
+  if (tables->dim() != 3 || tables->size(1) != integer(a[1]))
+    bad_value("tables must be [requests, planes, width] with the pool's plane count");
+  if (rows->dim() != 2 || rows->size(1) != 3) bad_value("rows must be [n, 3]: request index, exit plane, token position");
+  return PyLong_FromLong(rlt_kv_finalize(static_cast<const RltPool*>(address(a[0])), tables->data_ptr<int32_t>(),
+                                         static_cast<int32_t>(tables->size(0)), static_cast<int32_t>(tables->size(2)),
+                                         rows->data_ptr<int32_t>(), static_cast<int32_t>(rows->size(0)),
+                                         PyLong_AsUnsignedLongLong(a[4]), static_cast<int32_t*>(data_of(a[5])), stream_of(a[6])));
+}
+
+// ------------------------------------------------------------------------------------------------ the module
+
+template <PyObject* (*kFunction)(PyObject* const*), int kArgs>
+PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != kArgs) {
+    PyErr_Format(PyExc_TypeError, "expected %d arguments, got %zd", kArgs, n);
+    return nullptr;
+  }
+  try {
+    return kFunction(args);
+  } catch (const Failure&) {
+    return nullptr;
+  } catch (const std::exception& e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what());
+    return nullptr;
+  }
+}
+
+#define RLT_ENTRY(name, function, args) \
+  {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(&entry<function, args>)), METH_FASTCALL, nullptr}
+
+PyMethodDef kMethods[] = {
+    RLT_ENTRY("plan", make_plan, 8),
+    RLT_ENTRY("plan_layout", plan_layout, 1),
+    RLT_ENTRY("plan_arrays", plan_arrays, 2),
+    RLT_ENTRY("plan_wire", plan_wire, 2),
+    RLT_ENTRY("plan_fits", plan_fits, 2),
+    RLT_ENTRY("plan_upload", plan_upload, 4),
+    RLT_ENTRY("move", move, 20),
+    RLT_ENTRY("handoff_host", handoff_host, 12),
+    RLT_ENTRY("finalize", finalize, 7),
+    {nullptr, nullptr, 0, nullptr},
+};
+
+PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__host(void) { return PyModule_Create(&kModule); }

@@ -41,59 +41,12 @@
 #include <cstring>
 #include <mutex>
 
+#include "block_moves.h"
 #include "common.cuh"
+#include "table_params.cuh"
 
 namespace rlt {
 namespace {
-
-struct RegionParams {
-  const char* src_key;
-  const char* src_value;
-  char* dst_key;
-  char* dst_value;
-  long long block_bytes;
-  long long layer_bytes;
-  long long token_bytes;
-  int vec_bytes;        // 16, 4 or 1
-  int row_vecs;         // token_bytes / vec_bytes
-  unsigned row_magic;   // div_magic(row_vecs)
-  int wide_ok;          // rows and bases are 32-byte multiples: the 32-byte vector flavour may be used
-  int layers_per_unit;  // layers one unit covers
-  int chunks;           // ceil(layers in slice / layers_per_unit)
-};
-
-struct TableCopyParams {
-  RegionParams region[2];
-  int num_regions;
-  int num_requests;
-  int table_width;
-  int src_planes;
-  int dst_planes;   // destination planes, or wire planes for pack
-  int plane_begin;  // planes iterated by this launch: [plane_begin, plane_begin + plane_count)
-  int plane_count;
-  int block_size;
-  int src_blocks;
-  int dst_blocks;
-  const int* src_tables;
-  const int* dst_tables;
-  const int* tok_begin;
-  const int* tok_end;
-  const int* exit_planes;
-  const long long* exit_offsets;
-  long long exit_count;  // entries in exit_planes
-  int plane_bias;   // 0: source plane = min(p, exit); src_planes: source plane = exit
-  int layer_begin;
-  int layer_end;
-  int src_packed;   // source is the packed image (scatter)
-  int dst_packed;   // destination is the packed image (pack)
-  long long packed_token_bytes;  // 2 * layers in slice * (codes row + scales row)
-  long long packed_bytes;        // size of the packed image; rows past it are skipped
-  unsigned long long deep_layer_mask;  // layers carried for planes >= 1; 0 = all
-  int dedup_wire;                // the packed image holds, per token, only planes up to its exit plane
-  const int* dedup_prefix;       // [planes * total blocks] wire tokens before each (request, plane, block)
-  int fan;                       // pool-to-pool dedup that reads each row once and stores it to every plane it fills
-  int* status;
-};
 
 template <typename T, int kUnroll, bool kStreaming>
 __device__ __forceinline__ void stream_rows(const char* __restrict__ src, char* __restrict__ dst,
@@ -897,12 +850,6 @@ __global__ void __launch_bounds__(kThreads) dedup_finish_kernel(const long long*
   }
 }
 
-long long dedup_workspace_bytes(long long requests, long long width, long long planes) {
-  const long long entries = requests * width * planes;
-  const long long tiles = (entries + kPlanTile - 1) / kPlanTile;
-  return kPlanHeaderBytes + 4 * entries + 4 * (tiles + 1);
-}
-
 // Launch the three plan kernels into `workspace`; fills p.dedup_prefix.
 int plan_dedup(TableCopyParams& p, void* workspace, long long workspace_bytes, int sms, size_t scan_smem,
                cudaStream_t stream) {
@@ -938,17 +885,17 @@ int vector_width(const void* a, const void* b, const void* c, const void* d, lon
   return 1;
 }
 
-enum Direction { kDirect, kPack, kScatter };
+}  // namespace
 
-int launch_table_copy(Direction dir, const RltPool* src, const RltPool* dst, const RltBatch* batch,
-                      const RltOptions* opt, void* packed, long long packed_bytes, cudaStream_t stream,
-                      void* workspace = nullptr, long long workspace_bytes = 0) {
-  const NvtxRange range(dir == kDirect ? "rlt.kv_handoff" : dir == kPack ? "rlt.kv_pack" : "rlt.kv_scatter");
+long long dedup_workspace_bytes(long long requests, long long width, long long planes) {
+  const long long entries = requests * width * planes;
+  const long long tiles = (entries + kPlanTile - 1) / kPlanTile;
+  return kPlanHeaderBytes + 4 * entries + 4 * (tiles + 1);
+}
+
+int table_params(Direction dir, const RltPool* src, const RltPool* dst, const RltBatch* batch, const RltOptions* opt,
+                 void* packed, long long packed_bytes, TableCopyParams& p) {
   if (batch == nullptr || opt == nullptr) return RLT_E_INVALID;
-  if (workspace == nullptr) {
-    workspace = opt->workspace;
-    workspace_bytes = opt->workspace_bytes;
-  }
   const RltPool* any = dir == kScatter ? dst : src;
   if (any == nullptr || (dir == kDirect && dst == nullptr)) return RLT_E_INVALID;
   if (batch->num_requests < 1 || batch->table_width < 1 || batch->tok_begin == nullptr ||
@@ -987,7 +934,8 @@ int launch_table_copy(Direction dir, const RltPool* src, const RltPool* dst, con
       return RLT_E_GEOMETRY;
   }
 
-  TableCopyParams p{};
+  p = TableCopyParams{};
+  p.dedup_wire = dedup_wire;
   p.num_regions = scales ? 2 : 1;
   p.num_requests = batch->num_requests;
   p.table_width = batch->table_width;
@@ -1098,7 +1046,22 @@ int launch_table_copy(Direction dir, const RltPool* src, const RltPool* dst, con
     rg.chunks = (slice_layers + rg.layers_per_unit - 1) / rg.layers_per_unit;
   }
   if (p.num_regions == 1) p.region[1].chunks = 0;
+  return RLT_OK;
+}
 
+namespace {
+
+int launch_table_copy(Direction dir, const RltPool* src, const RltPool* dst, const RltBatch* batch,
+                      const RltOptions* opt, void* packed, long long packed_bytes, cudaStream_t stream,
+                      void* workspace = nullptr, long long workspace_bytes = 0) {
+  const NvtxRange range(dir == kDirect ? "rlt.kv_handoff" : dir == kPack ? "rlt.kv_pack" : "rlt.kv_scatter");
+  TableCopyParams p;
+  const int checked = table_params(dir, src, dst, batch, opt, packed, packed_bytes, p);
+  if (checked != RLT_OK) return checked;
+  if (workspace == nullptr) {
+    workspace = opt->workspace;
+    workspace_bytes = opt->workspace_bytes;
+  }
   int sms = 0;
   const int rc = sm_count(&sms);
   if (rc != RLT_OK) return rc;
@@ -1107,8 +1070,8 @@ int launch_table_copy(Direction dir, const RltPool* src, const RltPool* dst, con
   int grid = sms * per_sm;
   if (opt->grid_limit > 0 && grid > opt->grid_limit) grid = opt->grid_limit;
   const size_t smem = 2 * (static_cast<size_t>(batch->num_requests) + 1) * sizeof(int);
+  const bool dedup_wire = p.dedup_wire != 0;
   if (dedup_wire) {
-    p.dedup_wire = 1;
     const int planned = plan_dedup(p, workspace, workspace_bytes, sms, smem, stream);
     if (planned != RLT_OK) return planned;
   }
@@ -1248,6 +1211,51 @@ int host_ring(HostRing** out) {
   return RLT_OK;
 }
 
+// rlt_kv_handoff_host as one launch whose page records are kernel parameters: no slot, no copy, no event. Records take
+// (6 + planes of both sides) words a page; a batch whose records do not fit goes through a slot.
+int handoff_from_records(const RltPool* src, const RltPool* dst, const RltHostBatch* hb, const RltOptions* options,
+                         rlt_stream_t stream) {
+  const int bs = src->block_size;
+  if (bs < 1 || bs > kMaxBlockSize || hb->src_planes < 1 || hb->dst_planes < 1) return RLT_MOVE_UNSUITED;
+  const int words = kRecordHeader + hb->src_planes + hb->dst_planes;
+  int32_t records[kInlineWords];
+  int at = 0;
+  long long before = 0;
+  for (int r = 0; r < hb->num_requests; ++r) {
+    const int b = hb->tok_begin[r], e = hb->tok_end[r];
+    if (e <= b) continue;
+    const bool bad = b < 0 || e > static_cast<long long>(hb->table_width) * bs;
+    const int first = bad ? 0 : b / bs, last = bad ? 0 : (e - 1) / bs;
+    if (at + static_cast<long long>(last - first + 1) * words > kInlineWords) return RLT_MOVE_UNSUITED;
+    for (int page = first; page <= last; ++page, at += words) {
+      int32_t* w = records + at;
+      const int base = page * bs;
+      const int lo = b > base ? b - base : 0, hi = e < base + bs ? e - base : bs;
+      w[0] = r;
+      w[1] = page;
+      w[2] = bad ? kRecordBad : lo | hi << 8;
+      w[3] = bad ? b : base + lo - b;
+      w[4] = bad ? e : static_cast<int32_t>(before);
+      w[5] = e - b;
+      for (int p = 0; p < hb->src_planes; ++p)
+        w[kRecordHeader + p] = hb->src_tables[(static_cast<size_t>(r) * hb->src_planes + p) * hb->table_width + page];
+      for (int p = 0; p < hb->dst_planes; ++p)
+        w[kRecordHeader + hb->src_planes + p] = hb->dst_tables[(static_cast<size_t>(r) * hb->dst_planes + p) * hb->table_width + page];
+    }
+    before += e - b;
+  }
+  RltBlockMoves m = {};
+  m.host_records = records;
+  m.blocks = at / words;
+  m.words = words;
+  m.src_planes = hb->src_planes;
+  m.dst_planes = hb->dst_planes;
+  m.block_size = bs;
+  m.num_requests = hb->num_requests;
+  m.table_width = hb->table_width;
+  return rlt_move_blocks(RLT_MOVE_DIRECT, src, dst, &m, options, nullptr, 0, stream);
+}
+
 }  // namespace
 }  // namespace rlt
 
@@ -1285,6 +1293,9 @@ int rlt_kv_handoff_host(const RltPool* src, const RltPool* dst, const RltHostBat
   const size_t range_bytes = n * sizeof(int32_t);
   const size_t total = src_bytes + dst_bytes + 2 * range_bytes;
   if (total > rlt::kHostSlotBytes) return RLT_E_LIMIT;
+
+  const int by_records = rlt::handoff_from_records(src, dst, hb, options, stream);
+  if (by_records != RLT_MOVE_UNSUITED) return by_records;
 
   const std::lock_guard<std::mutex> lock(rlt::g_host_ring_mutex);
   rlt::HostRing* ring = nullptr;

@@ -24,10 +24,15 @@ from .._lib import MODE_ALL_PLANES, MODE_DEDUP, MODE_EXIT_ONLY  # noqa: F401  (r
 
 def _stream_ptr(stream) -> int:
     if stream is None:
-        return torch.cuda.current_stream().cuda_stream
+        return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
     if isinstance(stream, int):
         return stream
     return stream.cuda_stream
+
+
+def _raw_stream(stream):
+    """``stream`` as the compiled host side takes it: an address, or None for the current stream."""
+    return stream if stream is None or isinstance(stream, int) else stream.cuda_stream
 
 
 # --------------------------------------------------------------------------- pools
@@ -116,6 +121,15 @@ class PoolView:
             self.num_planes,
         )
 
+    def _address(self) -> int:
+        """Address of a struct of this view that lives as long as the view: a launch needs no new one."""
+        hit = self.__dict__.get("_struct")
+        if hit is None:
+            struct = self.as_struct()
+            hit = (C.addressof(struct), struct)
+            object.__setattr__(self, "_struct", hit)
+        return hit[0]
+
     @property
     def row_bytes(self) -> int:
         return self.codes.token_bytes + (self.scales.token_bytes if self.scales is not None else 0)
@@ -165,12 +179,16 @@ _PINNED = _PinnedPool()
 
 
 class HandoffBatch:
-    """Per-request tables and ranges, staged in pinned memory and copied to the device once.
+    """Per-request tables and ranges of a batch, checked on the host and kept there as the records the kernels read.
 
     ``src_tables[r]`` / ``dst_tables[r]`` are the per-plane block tables of request
     ``r`` (``plane_block_tables``); ``ranges[r]`` is its token range; ``exit_planes[r]``
     (optional) holds one zero-based exit plane per token position of the request.
     Validation mirrors ``kv_segments``: same conditions, same messages.
+
+    Everything is copied out of the arguments. A batch of up to about a thousand tokens travels as kernel parameters of
+    the launches that use it; the records of a larger one are sent to the device here, on ``stream``, in one copy. The
+    padded arrays that an ``RltBatch`` points at are made and sent when something asks for them (``as_struct``).
     """
 
     def __init__(
@@ -186,125 +204,93 @@ class HandoffBatch:
         device=None,
         stream=None,
     ):
-        n = len(ranges)
-        if n < 1:
-            raise ValueError("a handoff batch needs at least one request")
-        if n > _lib.MAX_REQUESTS:
-            raise ValueError(f"a handoff batch holds at most {_lib.MAX_REQUESTS} requests")
-        self.num_requests = n
+        host = _lib.load_host()
+        (self._plan, self.num_requests, self.total_tokens, self.table_width, self.src_planes, self.dst_planes, self.exit_count,
+         self.ranges, self.metadata_bytes) = host.plan(src_tables, dst_tables, ranges, exit_planes, block_size, src_blocks,
+                                                       dst_blocks, _lib.MAX_REQUESTS)
         self.block_size = block_size
-        bounds = np.asarray(ranges, dtype=np.int64).reshape(n, 2)
-        begin, end = bounds[:, 0], bounds[:, 1]
-        if ((begin < 0) | (begin >= end)).any():
-            raise ValueError("invalid KV range")
-        self.ranges = [(int(s), int(e)) for s, e in bounds]
-        self.total_tokens = int((end - begin).sum())
-        # Per side: one int32 array [requests, planes, pages], zero-padded to the longest table. The checks are those of
-        # the reference's planner, done on whole arrays.
-        sides, width = [], 1
-        for tables, limit in ((src_tables, src_blocks), (dst_tables, dst_blocks)):
-            if tables is None:
-                sides.append(None)
-                continue
-            if len(tables) != n:
-                raise ValueError("one table set per request is required")
-            planes = len(tables[0])
-            if any(len(req) != planes for req in tables):
-                raise ValueError("requests of one batch must have the same number of planes")
-            pages0 = len(tables[0][0])
-            if all(len(table) == pages0 for req in tables for table in req):
-                # tables of one length (a single request, or a chunk's trimmed tables): one conversion, no padding
-                padded = np.asarray(tables, dtype=np.int32).reshape(n, planes, pages0)
-                if (end > pages0 * block_size).any():
-                    raise ValueError("KV range exceeds allocation")
-                pages_max = pages0
-            else:
-                rows = [table for req in tables for table in req]
-                lens = np.fromiter(map(len, rows), np.int64, count=n * planes).reshape(n, planes)
-                pages = lens[:, 0]
-                if (end > lens.min(axis=1) * block_size).any():
-                    raise ValueError("KV range exceeds allocation")
-                if (lens != pages[:, None]).any():
-                    raise ValueError("the planes of one request must have tables of equal length")
-                total = int(lens.sum())
-                if isinstance(rows[0], np.ndarray):
-                    flat = np.concatenate(rows).astype(np.int32, copy=False)
-                else:
-                    flat = np.fromiter((b for table in rows for b in table), np.int32, count=total)
-                pages_max = int(pages.max())
-                padded = np.zeros((n, planes, pages_max), np.int32)
-                # a boolean mask is filled in row-major order, which is the order of the flat array
-                padded.reshape(n * planes, pages_max)[np.arange(pages_max) < lens.reshape(-1)[:, None]] = flat
-            width = max(width, pages_max)
-            sides.append((padded, limit))
-        self.table_width = width
-        arrays = []
-        used = None
-        for side in sides:
-            if side is None:
-                arrays.append(None)
-                continue
-            a, limit = side
-            if a.shape[2] < width:  # the two sides share one width
-                wider = np.zeros((n, a.shape[1], width), np.int32)
-                wider[:, :, : a.shape[2]] = a
-                a = wider
-            # negative ids compare as huge unsigned numbers; the padding (0) is a valid id, so the mask of
-            # pages that the ranges touch is only needed when something looks wrong
-            bad = a < 0 if limit is None else a.view(np.uint32) >= limit
-            if bad.any():
-                if used is None:
-                    cols = np.arange(width)
-                    used = (cols >= (begin // block_size)[:, None]) & (cols <= ((end - 1) // block_size)[:, None])
-                if (bad & used[:, None, :]).any():
-                    raise ValueError("physical block outside registered pool")
-            arrays.append(np.ascontiguousarray(a))
-        self.src_planes = arrays[0].shape[1] if arrays[0] is not None else 0
-        self.dst_planes = arrays[1].shape[1] if arrays[1] is not None else 0
-        exit_parts = offsets = None
-        exit_count = 0
-        if exit_planes is not None:
-            if len(exit_planes) != n:
-                raise ValueError("one exit-plane array per request is required")
-            exit_parts = [np.asarray(e, np.int32) for e in exit_planes]
-            counts = np.fromiter(map(len, exit_parts), np.int64, count=n)
-            if any(e.ndim != 1 for e in exit_parts) or (counts < end).any():
-                raise ValueError("exit planes must cover every token position up to the range end")
-            offsets = np.cumsum(counts) - counts
-            exit_count = int(counts.sum())
-        # One pinned staging buffer, one host-to-device copy; int64 data first for alignment. The exit planes,
-        # the largest piece, are gathered straight into the staging buffer.
-        pieces = [("exit_offsets", offsets), ("src_tables", arrays[0]), ("dst_tables", arrays[1]),
-                  ("tok_begin", begin.astype(np.int32)), ("tok_end", end.astype(np.int32))]
-        layout, size = {}, 0
-        for name, a in pieces:
-            if a is None:
-                continue
-            size = (size + 15) & ~15
-            layout[name] = (size, a)
-            size += a.nbytes
-        if exit_parts is not None:
-            size = (size + 15) & ~15
-            layout["exit_planes"] = (size, None)
-            size += 4 * exit_count
-        self.metadata_bytes = size
-        device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
+        self.has_exit = exit_planes is not None
+        self._planned_exits = self.exit_count
+        self._device = device
+        self._arrays = None   # (device tensor, address of each array) of the RltBatch form
+        self._staged = {}     # what has been sent to the device: (tensor, stream it was sent on)
+        if not host.plan_fits(self._plan, False):
+            self._send(0, self.metadata_bytes, stream)
+
+    def _where(self):
+        return torch.device("cuda", torch.cuda.current_device()) if self._device is None else torch.device(self._device)
+
+    def _send(self, planes: int, nbytes: int, stream) -> int:
+        """The records (``planes`` 0), or the wire plan of ``planes`` planes, on the device: sent once; a use on another
+        stream than they were sent on waits for the copy."""
+        hit = self._staged.get(planes)
+        if hit is None:
+            with torch.cuda.device(self._where()):
+                at = _stream_ptr(stream)
+                tensor = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+                if stream is not None and at != _stream_ptr(None):
+                    # the allocator hands the memory out in the order of its current stream
+                    torch.cuda.ExternalStream(at).wait_stream(torch.cuda.current_stream())
+                _lib.check(_lib.load_host().plan_upload(self._plan, min(planes, 1), tensor.data_ptr(), at),
+                           "rlt_stage_upload")
+            self._staged[planes] = (tensor, at)
+            return tensor.data_ptr()
+        tensor, sent_on = hit
+        now = _stream_ptr(stream)
+        if now != sent_on:
+            torch.cuda.ExternalStream(now).wait_stream(torch.cuda.ExternalStream(sent_on))
+        return tensor.data_ptr()
+
+    def _move(self, direction, src, dst, *, mode, layer_begin=0, layer_end=0, wire_planes=0, plane_begin=0, plane_end=0,
+              mask=0, status=None, grid_limit=0, variant=0, workspace=None, packed=0, packed_bytes=0, stream=None) -> int:
+        """One launch from this batch's records; ``_lib.MOVE_UNSUITED`` (nothing launched) where they do not serve."""
+        if self._plan is None or self.exit_count != self._planned_exits or variant or grid_limit:
+            return _lib.MOVE_UNSUITED
+        host = _lib.load_host()
+        records = wire = wire_bytes = planes = 0
+        if direction != _lib.MOVE_DIRECT and mode == MODE_DEDUP:
+            planes = (src if direction == _lib.MOVE_PACK else dst).num_planes
+            wire_bytes = host.plan_wire(self._plan, planes)
+        if self._staged or (wire_bytes and not host.plan_fits(self._plan, True)):
+            records = self._send(0, self.metadata_bytes, stream)
+            if wire_bytes:
+                wire = self._send(planes, wire_bytes, stream)
+        return host.move(direction, src and src._address(), dst and dst._address(), self._plan, records, wire, mode, layer_begin,
+                         layer_end, wire_planes, plane_begin, plane_end, mask, status, grid_limit, variant, workspace, packed,
+                         packed_bytes, _raw_stream(stream))
+
+    def _send_arrays(self):
+        """The padded arrays of the RltBatch form, in one device buffer: one pinned staging buffer, one copy."""
+        host = _lib.load_host()
+        size, offsets = host.plan_layout(self._plan)
+        device = self._where()
         staging = _PINNED.acquire(size)
-        host = staging.buffer.numpy()
-        for name, (at, a) in layout.items():
-            if a is not None:
-                host[at : at + a.nbytes] = a.reshape(-1).view(np.uint8)
-            elif exit_count:
-                np.concatenate(exit_parts, out=host[at : at + 4 * exit_count].view(np.int32))
-        self._dev = torch.empty(size, dtype=torch.uint8, device=device)
-        with torch.cuda.device(device), torch.cuda.stream(stream if stream is not None else torch.cuda.current_stream(device)):
-            self._dev.copy_(staging.buffer[:size], non_blocking=True)
+        host.plan_arrays(self._plan, staging.buffer.numpy())
+        dev = torch.empty(size, dtype=torch.uint8, device=device)
+        with torch.cuda.device(device), torch.cuda.stream(torch.cuda.current_stream(device)):
+            dev.copy_(staging.buffer[:size], non_blocking=True)
             staging.release()
-        exits = exit_parts
-        base = self._dev.data_ptr()
-        self._ptr = {name: base + at for name, (at, _) in layout.items()}
-        self.has_exit = exits is not None
-        self.exit_count = exit_count
+        base = dev.data_ptr()
+        self._arrays = (dev, {name: base + at for name, at in offsets.items()})
+
+    def _struct_on(self, stream) -> _lib.RltBatch:
+        """``as_struct`` for a launch on ``stream``: arrays that are not on the device yet are sent on that stream."""
+        if self._arrays is None and stream is not None:
+            with torch.cuda.stream(torch.cuda.ExternalStream(_stream_ptr(stream))):
+                self._send_arrays()
+        return self.as_struct()
+
+    @property
+    def _dev(self):
+        if self._arrays is None:
+            self._send_arrays()
+        return self._arrays[0]
+
+    @property
+    def _ptr(self):
+        if self._arrays is None:
+            self._send_arrays()
+        return self._arrays[1]
 
     @classmethod
     def from_device(cls, src_tables, dst_tables, tok_begin, tok_end, *, block_size: int, exit_planes=None,
@@ -340,9 +326,10 @@ class HandoffBatch:
         self.src_planes = src_tables.shape[1] if src_tables is not None else 0
         self.dst_planes = dst_tables.shape[1] if dst_tables is not None else 0
         self.metadata_bytes = 0
-        self._dev = (src_tables, dst_tables, tok_begin, tok_end, exit_planes, exit_offsets)  # keeps them alive
+        arrays = (src_tables, dst_tables, tok_begin, tok_end, exit_planes, exit_offsets)  # kept alive with the batch
         names = ("src_tables", "dst_tables", "tok_begin", "tok_end", "exit_planes", "exit_offsets")
-        self._ptr = {name: t.data_ptr() for name, t in zip(names, self._dev) if t is not None}
+        self._plan = None
+        self._arrays = (arrays, {name: t.data_ptr() for name, t in zip(names, arrays) if t is not None})
         self.has_exit = exit_planes is not None
         self.exit_count = exit_planes.numel() if exit_planes is not None else 0
         return self
@@ -419,7 +406,6 @@ def kv_handoff(src: PoolView, dst: PoolView, batch: HandoffBatch, *, mode=MODE_A
     destination planes (0, 0 = everything), which is what layer-by-layer streaming uses. ``deep_layers`` lists
     the layers carried for planes >= 1 (a recurrent-depth model's recurrent layers); plane 0 carries them all.
     """
-    lib = _lib.load()
     mask = 0
     if deep_layers is not None:
         for layer in deep_layers:
@@ -428,7 +414,12 @@ def kv_handoff(src: PoolView, dst: PoolView, batch: HandoffBatch, *, mode=MODE_A
             mask |= 1 << layer
         if mask == 0:
             raise ValueError("recurrent_layers must be nonempty and unique")
-    s, d, b = src.as_struct(), dst.as_struct(), batch.as_struct()
+    rc = batch._move(_lib.MOVE_DIRECT, src, dst, mode=mode, layer_begin=layer_begin, layer_end=layer_end, plane_begin=plane_begin,
+                     plane_end=plane_end, mask=mask, status=status, grid_limit=grid_limit, variant=variant, stream=stream)
+    if rc != _lib.MOVE_UNSUITED:
+        return _lib.check(rc, "rlt_kv_handoff")
+    lib = _lib.load()
+    s, d, b = src.as_struct(), dst.as_struct(), batch._struct_on(stream)
     o = _options(mode, layer_begin, layer_end, 0, status, grid_limit, variant, None, plane_begin, plane_end, mask)
     _lib.check(lib.rlt_kv_handoff(C.byref(s), C.byref(d), C.byref(b), C.byref(o), _stream_ptr(stream)), "rlt_kv_handoff")
 
@@ -448,17 +439,8 @@ def kv_handoff_host(src: PoolView, dst: PoolView, src_tables: np.ndarray, dst_ta
     ``tok_end`` int32 ``[requests]``. Nothing is validated on the host beyond shapes; the kernel checks block ids and
     ranges and reports through ``status``. Raises ``ValueError`` with the library's limit message when the batch does
     not fit a staging slot."""
-    arrays = (src_tables, dst_tables, tok_begin, tok_end)
-    if any(a.dtype != np.int32 or not a.flags.c_contiguous for a in arrays):
-        raise ValueError("host tables and ranges must be C-contiguous int32 arrays")
-    n, src_planes, width = src_tables.shape
-    if dst_tables.shape[0] != n or dst_tables.shape[2] != width or tok_begin.shape != (n,) or tok_end.shape != (n,):
-        raise ValueError("source and destination tables must agree in requests and width, one range per request")
-    hb = _lib.RltHostBatch(n, width, src_planes, dst_tables.shape[1], src_tables.ctypes.data, dst_tables.ctypes.data,
-                           tok_begin.ctypes.data, tok_end.ctypes.data)
-    s, d = src.as_struct(), dst.as_struct()
-    o = _options(MODE_ALL_PLANES, layer_begin, layer_end, 0, status, 0, 0, None, plane_begin, plane_end, 0)
-    _lib.check(_lib.load().rlt_kv_handoff_host(C.byref(s), C.byref(d), C.byref(hb), C.byref(o), _stream_ptr(stream)),
+    _lib.check(_lib.load_host().handoff_host(src._address(), dst._address(), src_tables, dst_tables, tok_begin, tok_end,
+                                             layer_begin, layer_end, plane_begin, plane_end, status, _raw_stream(stream)),
                "rlt_kv_handoff_host")
 
 
@@ -476,18 +458,21 @@ def kv_pack(src: PoolView, batch: HandoffBatch, out: torch.Tensor, *, mode=MODE_
     """Gather a batch into ``out`` (uint8, contiguous) in the reference's segment order."""
     if out.dtype != torch.uint8 or not out.is_contiguous() or not out.is_cuda:
         raise ValueError("packed buffer must be a contiguous CUDA uint8 tensor")
-    lib = _lib.load()
-    s, b = src.as_struct(), batch.as_struct()
-    o = _options(mode, layer_begin, layer_end, wire_planes, status, grid_limit, variant, workspace)
-    _lib.check(lib.rlt_kv_pack(C.byref(s), C.byref(b), C.byref(o), out.data_ptr(), out.numel(), _stream_ptr(stream)), "rlt_kv_pack")
+    kv_pack_to(src, batch, out.data_ptr(), out.numel(), mode=mode, layer_begin=layer_begin, layer_end=layer_end,
+               wire_planes=wire_planes, status=status, stream=stream, grid_limit=grid_limit, variant=variant, workspace=workspace)
 
 
 def kv_pack_to(src: PoolView, batch: HandoffBatch, out_ptr: int, out_bytes: int, *, mode=MODE_ALL_PLANES, layer_begin=0,
                layer_end=0, wire_planes=0, status=None, stream=None, grid_limit=0, variant=0, workspace=None) -> None:
     """``kv_pack`` into raw memory, typically a staging buffer on the decode GPU mapped through a peer pointer:
     the gather and the push over NVLink become one kernel and nothing is staged on the prefill side."""
+    rc = batch._move(_lib.MOVE_PACK, src, None, mode=mode, layer_begin=layer_begin, layer_end=layer_end, wire_planes=wire_planes,
+                     status=status, grid_limit=grid_limit, variant=variant, workspace=workspace, packed=out_ptr,
+                     packed_bytes=out_bytes, stream=stream)
+    if rc != _lib.MOVE_UNSUITED:
+        return _lib.check(rc, "rlt_kv_pack")
     lib = _lib.load()
-    s, b = src.as_struct(), batch.as_struct()
+    s, b = src.as_struct(), batch._struct_on(stream)
     o = _options(mode, layer_begin, layer_end, wire_planes, status, grid_limit, variant, workspace)
     _lib.check(lib.rlt_kv_pack(C.byref(s), C.byref(b), C.byref(o), out_ptr, out_bytes, _stream_ptr(stream)), "rlt_kv_pack")
 
@@ -497,9 +482,15 @@ def kv_scatter(packed: torch.Tensor, dst: PoolView, batch: HandoffBatch, *, mode
     """Write a packed image into the destination blocks of a batch."""
     if packed.dtype != torch.uint8 or not packed.is_contiguous() or not packed.is_cuda:
         raise ValueError("packed buffer must be a contiguous CUDA uint8 tensor")
+    mode = mode if mode == MODE_DEDUP else MODE_ALL_PLANES
+    rc = batch._move(_lib.MOVE_SCATTER, None, dst, mode=mode, layer_begin=layer_begin, layer_end=layer_end,
+                     wire_planes=wire_planes, status=status, grid_limit=grid_limit, variant=variant, workspace=workspace,
+                     packed=packed.data_ptr(), packed_bytes=packed.numel(), stream=stream)
+    if rc != _lib.MOVE_UNSUITED:
+        return _lib.check(rc, "rlt_kv_scatter")
     lib = _lib.load()
-    d, b = dst.as_struct(), batch.as_struct()
-    o = _options(mode if mode == MODE_DEDUP else MODE_ALL_PLANES, layer_begin, layer_end, wire_planes, status,
+    d, b = dst.as_struct(), batch._struct_on(stream)
+    o = _options(mode, layer_begin, layer_end, wire_planes, status,
                  grid_limit, variant, workspace)
     _lib.check(lib.rlt_kv_scatter(packed.data_ptr(), packed.numel(), C.byref(d), C.byref(b), C.byref(o), _stream_ptr(stream)), "rlt_kv_scatter")
 
@@ -513,13 +504,6 @@ def kv_finalize(pool: PoolView, tables: torch.Tensor, rows: torch.Tensor, *, lay
     to be copied the view must carry them: build it with ``PoolView.from_tensors(..., key_scale,
     value_scale)`` also for a fixed-scale pool.
     """
-    for t, name, cols in ((tables, "tables", None), (rows, "rows", 3)):
-        if t.dtype != torch.int32 or not t.is_contiguous() or not t.is_cuda:
-            raise ValueError(f"{name} must be a contiguous CUDA int32 tensor")
-    if tables.dim() != 3 or tables.shape[1] != pool.num_planes:
-        raise ValueError("tables must be [requests, planes, width] with the pool's plane count")
-    if rows.dim() != 2 or rows.shape[1] != 3:
-        raise ValueError("rows must be [n, 3]: request index, exit plane, token position")
     mask = 0
     if layers is not None:
         for layer in layers:
@@ -528,13 +512,8 @@ def kv_finalize(pool: PoolView, tables: torch.Tensor, rows: torch.Tensor, *, lay
             mask |= 1 << layer
         if mask == 0:
             raise ValueError("recurrent_layers must be nonempty and unique")
-    s = pool.as_struct()
-    _lib.check(
-        _lib.load().rlt_kv_finalize(C.byref(s), tables.data_ptr(), tables.shape[0], tables.shape[2], rows.data_ptr(),
-                                    rows.shape[0], mask, status.data_ptr() if status is not None else None,
-                                    _stream_ptr(stream)),
-        "rlt_kv_finalize",
-    )
+    _lib.check(_lib.load_host().finalize(pool._address(), pool.num_planes, tables, rows, mask, status, _raw_stream(stream)),
+               "rlt_kv_finalize")
 
 
 def kv_push(src_ptr: int, dst_ptr: int, nbytes: int, *, stream=None) -> None:
