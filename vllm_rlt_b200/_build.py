@@ -79,7 +79,8 @@ def build_library(force: bool = False, verbose: bool = False) -> Path:
     """Compile the C-ABI library (no torch types, static cudart)."""
     target = PACKAGE / LIB_NAME
     sources = [CSRC / s for s in CUDA_SOURCES]
-    deps = sources + [CSRC / "common.cuh", CSRC / "table_params.cuh", CSRC / "block_moves.h", INCLUDE / "rlt_kv_handoff.h"]
+    deps = sources + [CSRC / "common.cuh", CSRC / "table_params.cuh", CSRC / "block_moves.h",
+                      CSRC / "internal.h", INCLUDE / "rlt_kv_handoff.h"]
     flags = [*ARCH, "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC,-fvisibility=hidden"]
     fingerprint = _fingerprint(flags, deps)
     if force or verbose or _stale(target, fingerprint):
@@ -123,7 +124,7 @@ def build_ops(force: bool = False) -> Path:
 
 def build_host(force: bool = False) -> Path:
     """Compile the Python module that prepares and issues the launches of the Python entry points."""
-    return _build_torch_module(HOST_NAME, "host_module.cpp", [CSRC / "block_moves.h"], force, python=True)
+    return _build_torch_module(HOST_NAME, "host_module.cpp", [CSRC / "block_moves.h", CSRC / "internal.h"], force, python=True)
 
 
 def build_all(force: bool = False) -> None:

@@ -49,10 +49,6 @@ enum { RLT_MOVE_DIRECT = 0, RLT_MOVE_PACK = 1, RLT_MOVE_SCATTER = 2 };
 RLT_API int rlt_move_blocks(int direction, const RltPool* src, const RltPool* dst, const RltBlockMoves* moves,
                             const RltOptions* options, void* packed, int64_t packed_bytes, rlt_stream_t stream);
 
-// Copies `bytes` bytes of ordinary host memory to the current device through a pinned buffer of the library, on `stream`;
-// the host memory is free again on return.
-RLT_API int rlt_stage_upload(const void* host, size_t bytes, void* device, rlt_stream_t stream);
-
 #ifdef __cplusplus
 }
 #endif

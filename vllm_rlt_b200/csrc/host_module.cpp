@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "block_moves.h"
+#include "internal.h"
 #include "rlt_kv_handoff.h"
 
 namespace {
@@ -540,6 +541,210 @@ PyObject* finalize(PyObject* const* a) {
                                          PyLong_AsUnsignedLongLong(a[4]), static_cast<int32_t*>(data_of(a[5])), stream_of(a[6])));
 }
 
+// ------------------------------------------------------------------------------------------------ tensor transfers
+
+// RLT_DTYPE_* of a tensor, -1 for the types that do not transfer.
+int transfer_type(const at::Tensor& t) {
+  switch (t.scalar_type()) {
+    case at::kInt: return RLT_DTYPE_I32;
+    case at::kLong: return RLT_DTYPE_I64;
+    case at::kHalf: return RLT_DTYPE_F16;
+    case at::kBFloat16: return RLT_DTYPE_BF16;
+    case at::kFloat: return RLT_DTYPE_F32;
+    default: return -1;
+  }
+}
+
+void check_source(const at::Tensor& source, const at::Device& device) {
+  if (source.is_cuda()) {
+    if (source.device() != device) bad_value("cross-device transfers require an explicit connector");
+  } else if (!source.is_pinned()) {
+    bad_value("host sources must be pinned: this transfer has no pageable-memory path");
+  }
+}
+
+const at::Tensor& some_tensor(PyObject* o) {
+  const at::Tensor* t = tensor_of(o);
+  if (t == nullptr) fail(PyExc_TypeError, "expected a tensor");
+  return *t;
+}
+
+// tensor_copy(source, target, secondary | None) -> code, on the current stream of the target's device
+PyObject* tensor_copy(PyObject* const* a) {
+  const at::Tensor &source = some_tensor(a[0]), &target = some_tensor(a[1]);
+  const at::Tensor* secondary = tensor_of(a[2]);
+  if (source.numel() != target.numel() || !source.is_contiguous() || !target.is_contiguous())
+    bad_value("copy_tensor requires equal-sized contiguous tensors");
+  if (secondary != nullptr &&
+      (secondary->numel() != source.numel() || !secondary->is_contiguous() || secondary->device() != target.device()))
+    bad_value("secondary output must match target size and device");
+  const int from = transfer_type(source), to = transfer_type(target), second = secondary ? transfer_type(*secondary) : 0;
+  if (from < 0 || to < 0 || second < 0) bad_value("unsupported transfer dtype");
+  if (!target.is_cuda()) bad_value("transfer destination must be a CUDA tensor");
+  check_source(source, target.device());
+  if (source.numel() == 0) return PyLong_FromLong(RLT_OK);
+  const c10::cuda::CUDAGuard guard(target.device());
+  return PyLong_FromLong(rlt_tensor_copy(source.data_ptr(), target.data_ptr(), secondary ? secondary->data_ptr() : nullptr,
+                                         source.numel(), from, to, second, stream_of(Py_None)));
+}
+
+// A TensorTransfer's descriptors, collected as copies are appended: the rows of rlt_tensor_transfer's table.
+struct Transfer {
+  std::vector<int64_t> rows;  // 8 per copy
+  int64_t max_rows = 0, max_cols = 0;
+};
+constexpr const char* kTransferName = "vllm_rlt_b200.transfer";
+void free_transfer(PyObject* capsule) { delete static_cast<Transfer*>(PyCapsule_GetPointer(capsule, kTransferName)); }
+Transfer& transfer_of(PyObject* capsule) {
+  auto* t = static_cast<Transfer*>(PyCapsule_GetPointer(capsule, kTransferName));
+  if (t == nullptr) throw Failure{};
+  return *t;
+}
+
+PyObject* transfer_new(PyObject* const*) {
+  auto* t = new Transfer;
+  PyObject* capsule = PyCapsule_New(t, kTransferName, free_transfer);
+  if (capsule == nullptr) {
+    delete t;
+    throw Failure{};
+  }
+  return capsule;
+}
+
+PyObject* transfer_reset(PyObject* const* a) {
+  Transfer& t = transfer_of(a[0]);
+  t.rows.clear();
+  t.max_rows = t.max_cols = 0;
+  Py_RETURN_NONE;
+}
+
+// transfer_append(transfer, capacity, source type, target type, device index, source, target) -> whether there is anything to copy
+PyObject* transfer_append(PyObject* const* a) {
+  Transfer& t = transfer_of(a[0]);
+  const at::Tensor &source = some_tensor(a[5]), &target = some_tensor(a[6]);
+  const int64_t dims = source.dim();
+  if (source.sizes() != target.sizes() || (dims != 1 && dims != 2)) bad_value("transfer requires matching 1D/2D shapes");
+  if (transfer_type(source) != integer(a[2]) || transfer_type(target) != integer(a[3])) bad_value("transfer dtype does not match its batch");
+  const at::Device device(at::kCUDA, static_cast<c10::DeviceIndex>(integer(a[4])));
+  if (target.device() != device) bad_value("transfer destination must be on the configured device");
+  if (source.is_cuda() && source.device() != device) bad_value("transfer source must be on the configured device");
+  check_source(source, device);
+  if (source.numel() == 0) Py_RETURN_FALSE;
+  if (static_cast<long long>(t.rows.size() / 8) >= integer(a[1])) bad_value("transfer batch is full");
+  const bool flat = dims == 1;
+  const int64_t rows = flat ? 1 : source.size(0), cols = source.size(dims - 1);
+  const int64_t row[8] = {reinterpret_cast<int64_t>(source.data_ptr()), reinterpret_cast<int64_t>(target.data_ptr()), rows, cols,
+                          flat ? cols * source.stride(0) : source.stride(0), source.stride(dims - 1),
+                          flat ? cols * target.stride(0) : target.stride(0), target.stride(dims - 1)};
+  t.rows.insert(t.rows.end(), row, row + 8);
+  t.max_rows = rows > t.max_rows ? rows : t.max_rows;
+  t.max_cols = cols > t.max_cols ? cols : t.max_cols;
+  Py_RETURN_TRUE;
+}
+
+// transfer_extent(transfer) -> rows and columns that bound its copies
+PyObject* transfer_extent(PyObject* const* a) {
+  const Transfer& t = transfer_of(a[0]);
+  return Py_BuildValue("LL", static_cast<long long>(t.max_rows), static_cast<long long>(t.max_cols));
+}
+
+// transfer_submit(transfer, source type, target type, device index, pinned table) -> code. A small batch between tensors of one
+// type travels with its launch; others are written into the table, which the kernel reads where it lies.
+PyObject* transfer_submit(PyObject* const* a) {
+  const Transfer& t = transfer_of(a[0]);
+  const int from = static_cast<int>(integer(a[1])), to = static_cast<int>(integer(a[2]));
+  const int count = static_cast<int>(t.rows.size() / 8);
+  if (count == 0) return PyLong_FromLong(RLT_OK);
+  const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(integer(a[3])));
+  const int32_t rows = static_cast<int32_t>(t.max_rows), cols = static_cast<int32_t>(t.max_cols);
+  if (from == to && count <= RLT_INLINE_TRANSFERS && t.max_cols <= INT32_MAX && t.max_rows <= INT32_MAX) {
+    const int rc = rlt_tensor_transfer_inline(t.rows.data(), count, rows, cols, from, stream_of(Py_None));
+    if (rc != RLT_E_LIMIT) return PyLong_FromLong(rc);
+  }
+  const at::Tensor& table = some_tensor(a[4]);
+  std::memcpy(table.data_ptr(), t.rows.data(), 8 * t.rows.size());
+  return PyLong_FromLong(rlt_tensor_transfer(table.data_ptr<int64_t>(), count, rows, cols, from, to, stream_of(Py_None)));
+}
+
+// ------------------------------------------------------------------------------------------------ staging helpers
+
+template <typename V, typename F>
+bool fill_from(PyObject** items, Py_ssize_t n, V* out, F convert) {
+  for (Py_ssize_t i = 0; i < n; ++i) {
+    if (!convert(items[i], &out[i])) return false;
+  }
+  return true;
+}
+
+// fill(flat CPU tensor, start, values) -> the slice that received them, or None where the values are not a list or tuple of plain
+// numbers of the tensor's kind, or do not fit: the caller's general path then does it, or says what is wrong.
+PyObject* fill(PyObject* const* a) {
+  const at::Tensor& t = some_tensor(a[0]);
+  PyObject* values = a[2];
+  if (!PyList_CheckExact(values) && !PyTuple_CheckExact(values)) Py_RETURN_NONE;
+  const int64_t start = integer(a[1]);
+  const Py_ssize_t n = PySequence_Fast_GET_SIZE(values);
+  if (!t.is_cpu() || t.dim() != 1 || !t.is_contiguous() || start < 0 || start + n > t.size(0)) Py_RETURN_NONE;
+  PyObject** items = PySequence_Fast_ITEMS(values);
+  auto whole = [](PyObject* o, long long* v) {
+    if (!PyLong_CheckExact(o)) return false;
+    int overflow = 0;
+    *v = PyLong_AsLongLongAndOverflow(o, &overflow);
+    return overflow == 0;
+  };
+  bool ok = false;
+  if (t.scalar_type() == at::kLong) {
+    ok = fill_from(items, n, t.data_ptr<int64_t>() + start, [&](PyObject* o, int64_t* v) {
+      long long x;
+      if (!whole(o, &x)) return false;
+      *v = x;
+      return true;
+    });
+  } else if (t.scalar_type() == at::kInt) {
+    ok = fill_from(items, n, t.data_ptr<int32_t>() + start, [&](PyObject* o, int32_t* v) {
+      long long x;
+      if (!whole(o, &x) || x < INT32_MIN || x > INT32_MAX) return false;
+      *v = static_cast<int32_t>(x);
+      return true;
+    });
+  } else if (t.scalar_type() == at::kFloat) {
+    ok = fill_from(items, n, t.data_ptr<float>() + start, [&](PyObject* o, float* v) {
+      if (!PyFloat_CheckExact(o)) return false;
+      *v = static_cast<float>(PyFloat_AS_DOUBLE(o));
+      return true;
+    });
+  }
+  if (!ok) Py_RETURN_NONE;
+  return THPVariable_Wrap(t.narrow(0, start, n));
+}
+
+// row_slice(tensor, index, start, count) -> tensor[index][start : start + count] for a 2-D tensor and an int in range; None otherwise
+PyObject* row_slice(PyObject* const* a) {
+  const at::Tensor& t = some_tensor(a[0]);
+  if (!PyLong_CheckExact(a[1]) || t.dim() != 2) Py_RETURN_NONE;
+  int64_t index = integer(a[1]);
+  const int64_t start = integer(a[2]), n = integer(a[3]);
+  index += index < 0 ? t.size(0) : 0;
+  if (index < 0 || index >= t.size(0) || start < 0 || start + n > t.size(1)) Py_RETURN_NONE;
+  return THPVariable_Wrap(t.as_strided({n}, {t.stride(1)}, t.storage_offset() + index * t.stride(0) + start * t.stride(1)));
+}
+
+// pieces(flat tensor, [targets]) -> consecutive slices of it, as long as the targets
+PyObject* pieces(PyObject* const* a) {
+  const at::Tensor& t = some_tensor(a[0]);
+  const Ref targets(PySequence_Fast(a[1], "targets must be a sequence of tensors"));
+  const Py_ssize_t n = PySequence_Fast_GET_SIZE(targets.p);
+  PyObject* out = PyList_New(n);
+  if (out == nullptr) throw Failure{};
+  int64_t at = 0;
+  for (Py_ssize_t i = 0; i < n; ++i) {
+    const int64_t count = some_tensor(PySequence_Fast_GET_ITEM(targets.p, i)).size(0);
+    PyList_SET_ITEM(out, i, THPVariable_Wrap(t.narrow(0, at, count)));
+    at += count;
+  }
+  return out;
+}
+
 // ------------------------------------------------------------------------------------------------ the module
 
 template <PyObject* (*kFunction)(PyObject* const*), int kArgs>
@@ -571,6 +776,15 @@ PyMethodDef kMethods[] = {
     RLT_ENTRY("move", move, 20),
     RLT_ENTRY("handoff_host", handoff_host, 12),
     RLT_ENTRY("finalize", finalize, 7),
+    RLT_ENTRY("tensor_copy", tensor_copy, 3),
+    RLT_ENTRY("transfer_new", transfer_new, 0),
+    RLT_ENTRY("transfer_reset", transfer_reset, 1),
+    RLT_ENTRY("transfer_append", transfer_append, 7),
+    RLT_ENTRY("transfer_extent", transfer_extent, 1),
+    RLT_ENTRY("transfer_submit", transfer_submit, 5),
+    RLT_ENTRY("fill", fill, 3),
+    RLT_ENTRY("row_slice", row_slice, 4),
+    RLT_ENTRY("pieces", pieces, 2),
     {nullptr, nullptr, 0, nullptr},
 };
 

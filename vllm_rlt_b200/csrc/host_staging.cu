@@ -8,8 +8,8 @@
 #include <mutex>
 #include <vector>
 
-#include "block_moves.h"
 #include "common.cuh"
+#include "internal.h"
 
 namespace rlt {
 namespace {

@@ -1,0 +1,25 @@
+// Entry points between the library and its own Python module: not part of the C ABI.
+#pragma once
+
+#include <stddef.h>
+#include <stdint.h>
+
+#include "rlt_kv_handoff.h"
+
+#ifdef __cplusplus
+extern "C" {
+#endif
+
+// Copies `bytes` bytes of ordinary host memory to the current device through a pinned buffer of the library, on `stream`;
+// the host memory is free again on return.
+RLT_API int rlt_stage_upload(const void* host, size_t bytes, void* device, rlt_stream_t stream);
+
+// rlt_tensor_transfer between tensors of one type, with the descriptor table in HOST memory: it travels as kernel
+// parameters, so nothing has to be kept for the launch. At most RLT_INLINE_TRANSFERS descriptors.
+#define RLT_INLINE_TRANSFERS 448
+RLT_API int rlt_tensor_transfer_inline(const int64_t* descriptors, int32_t count, int32_t max_rows, int32_t max_cols,
+                                       int32_t dtype, rlt_stream_t stream);
+
+#ifdef __cplusplus
+}
+#endif

@@ -13,7 +13,10 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <cstring>
+
 #include "common.cuh"
+#include "internal.h"
 
 namespace rlt {
 namespace {
@@ -88,6 +91,64 @@ __global__ void __launch_bounds__(kTile) segmented_transfer_kernel(const long lo
     const long long r = static_cast<long long>(blockIdx.y) * kRows + k;
     if (r < rows) dst[r * dr + c * dc] = Convert<D, S>::run(src[r * sr + c * sc]);
   }
+}
+
+// The same between tensors of one type, whose elements are only moved, with the descriptors in the kernel's parameters: a
+// step's handful of small copies waits neither for a table in host memory (a read over PCIe before every copy) nor for
+// a host-to-device copy of one. A CTA moves kRows rows of kTileBytes bytes, 16 bytes a thread where both sides are
+// contiguous and aligned.
+constexpr int kTileBytes = 4096;
+constexpr int kInlineSmall = 56;  // descriptors of the smaller parameter block (3.5 KiB)
+
+template <int kCount>
+struct InlineDescriptors {
+  long long d[kCount][8];
+};
+
+template <typename T>
+__device__ __forceinline__ void move_tile(const T* src, T* dst, int n, long long sc, long long dc) {
+  constexpr int kPer = 16 / sizeof(T);
+  const unsigned long long bits = reinterpret_cast<unsigned long long>(src) | reinterpret_cast<unsigned long long>(dst);
+  if (sc == 1 && dc == 1 && (bits & 15ull) == 0) {
+    const int vectors = n / kPer;
+    for (int i = threadIdx.x; i < vectors; i += kTile) reinterpret_cast<uint4*>(dst)[i] = reinterpret_cast<const uint4*>(src)[i];
+    for (int i = vectors * kPer + threadIdx.x; i < n; i += kTile) dst[i] = src[i];
+  } else {
+    for (int i = threadIdx.x; i < n; i += kTile) dst[i * dc] = src[i * sc];
+  }
+}
+
+template <typename T, int kCount>
+__global__ void __launch_bounds__(kTile) inline_transfer_kernel(const __grid_constant__ InlineDescriptors<kCount> table) {
+  constexpr long long kCols = kTileBytes / static_cast<long long>(sizeof(T));
+  const long long* d = table.d[blockIdx.x];
+  const long long rows = d[2], cols = d[3], sr = d[4], sc = d[5], dr = d[6], dc = d[7];
+  const long long c0 = blockIdx.z * kCols;
+  if (c0 >= cols) return;
+  const int n = static_cast<int>(cols - c0 < kCols ? cols - c0 : kCols);
+#pragma unroll
+  for (int k = 0; k < kRows; ++k) {
+    const long long r = static_cast<long long>(blockIdx.y) * kRows + k;
+    if (r < rows)
+      move_tile(reinterpret_cast<const T*>(d[0]) + r * sr + c0 * sc, reinterpret_cast<T*>(d[1]) + r * dr + c0 * dc, n, sc, dc);
+  }
+}
+
+template <typename T, int kCount>
+int launch_inline(const int64_t* descriptors, int count, dim3 grid, cudaStream_t stream) {
+  InlineDescriptors<kCount> table;
+  std::memcpy(table.d, descriptors, static_cast<size_t>(count) * sizeof(table.d[0]));
+  inline_transfer_kernel<T, kCount><<<grid, kTile, 0, stream>>>(table);
+  return RLT_OK;
+}
+
+template <typename T>
+int launch_inline(const int64_t* descriptors, int count, int max_rows, int max_cols, cudaStream_t stream) {
+  constexpr int kCols = kTileBytes / static_cast<int>(sizeof(T));
+  const dim3 grid(count, (max_rows + kRows - 1) / kRows, (max_cols + kCols - 1) / kCols);
+  if (grid.y > 65535u || grid.z > 65535u) return RLT_E_LIMIT;
+  return count <= kInlineSmall ? launch_inline<T, kInlineSmall>(descriptors, count, grid, stream)
+                               : launch_inline<T, RLT_INLINE_TRANSFERS>(descriptors, count, grid, stream);
 }
 
 // Flat copy with conversion. When every pointer is 16-byte aligned a thread handles N consecutive elements per
@@ -255,6 +316,26 @@ int rlt_tensor_transfer(const int64_t* descriptors, int32_t count, int32_t max_r
   const rlt::SegmentedCall call{reinterpret_cast<const long long*>(descriptors), count, max_rows, max_cols,
                                 reinterpret_cast<cudaStream_t>(stream)};
   const int rc = rlt::dispatch_pair(src_dtype, dst_dtype, call);
+  if (rc != RLT_OK) return rc;
+  RLT_CUDA_TRY(cudaGetLastError());
+  rlt::g_launches.fetch_add(1, std::memory_order_relaxed);
+  return RLT_OK;
+}
+
+int rlt_tensor_transfer_inline(const int64_t* descriptors, int32_t count, int32_t max_rows, int32_t max_cols, int32_t dtype,
+                               rlt_stream_t stream) {
+  if (count == 0) return RLT_OK;
+  if (descriptors == nullptr || count < 0 || max_rows < 1 || max_cols < 1) return RLT_E_INVALID;
+  if (count > RLT_INLINE_TRANSFERS) return RLT_E_LIMIT;
+  const cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  int rc = RLT_E_INVALID;
+  switch (dtype) {
+    case RLT_DTYPE_F16:
+    case RLT_DTYPE_BF16: rc = rlt::launch_inline<uint16_t>(descriptors, count, max_rows, max_cols, s); break;
+    case RLT_DTYPE_I32:
+    case RLT_DTYPE_F32: rc = rlt::launch_inline<uint32_t>(descriptors, count, max_rows, max_cols, s); break;
+    case RLT_DTYPE_I64: rc = rlt::launch_inline<unsigned long long>(descriptors, count, max_rows, max_cols, s); break;
+  }
   if (rc != RLT_OK) return rc;
   RLT_CUDA_TRY(cudaGetLastError());
   rlt::g_launches.fetch_add(1, std::memory_order_relaxed);
