@@ -514,9 +514,13 @@ void launch_move(const MoveParams& p, const RltBlockMoves& m, unsigned grid, cud
 template <MoveKind K>
 int launch_kind(const MoveParams& p, const RltBlockMoves& m, unsigned grid, cudaStream_t stream) {
   const long long n = static_cast<long long>(m.blocks) * m.words + (m.host_wire ? static_cast<long long>(m.blocks) * p.src_planes : 0);
-  // A parameter block is copied into the launch whole, so two sizes of it: 3.5 KiB covers a few hundred tokens.
+  // A parameter block is copied into the launch whole (a launch takes the host 2.4 us with 2 KiB, 3.6 with 8 and 6.6 with 32; a
+  // copy of the records, the launch and an event 4.5, and the GPU 6 us more), so three sizes of it: the small one covers a few
+  // hundred tokens, the medium one a thousand.
   if (n <= kInlineSmallWords) {
     launch_move<K, kInlineSmallWords>(p, m, grid, stream);
+  } else if (n <= kInlineMediumWords) {
+    launch_move<K, kInlineMediumWords>(p, m, grid, stream);
   } else if (n <= kInlineWords) {
     launch_move<K, kInlineWords>(p, m, grid, stream);
   } else if (p.records != nullptr && (m.host_wire == nullptr || p.wire != nullptr)) {

@@ -18,6 +18,7 @@ constexpr int kRecordBad = -1;
 
 // Records up to this many bytes travel as kernel parameters: no staging slot, no copy, no event.
 constexpr int kInlineWords = 7680;
+constexpr int kInlineMediumWords = 1920;
 constexpr int kInlineSmallWords = 896;
 
 struct RltBlockMoves {
@@ -48,6 +49,11 @@ enum { RLT_MOVE_DIRECT = 0, RLT_MOVE_PACK = 1, RLT_MOVE_SCATTER = 2 };
 // (nothing launched): options that steer the table-driven kernels, more than 64 planes, very long rows.
 RLT_API int rlt_move_blocks(int direction, const RltPool* src, const RltPool* dst, const RltBlockMoves* moves,
                             const RltOptions* options, void* packed, int64_t packed_bytes, rlt_stream_t stream);
+
+// The same for a direct handoff whose records are not staged: records that do not fit the kernel parameters go through a
+// slot of rlt_kv_handoff_host's staging ring, RLT_MOVE_UNSUITED if they do not fit that either.
+RLT_API int rlt_handoff_staged(const RltPool* src, const RltPool* dst, const RltBlockMoves* moves, const RltOptions* options,
+                               rlt_stream_t stream);
 
 #ifdef __cplusplus
 }

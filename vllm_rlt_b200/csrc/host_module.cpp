@@ -745,6 +745,217 @@ PyObject* pieces(PyObject* const* a) {
   return out;
 }
 
+// ------------------------------------------------------------------------------------------------ transport
+
+void put(std::string& out, const void* p, size_t n) { out.append(static_cast<const char*>(p), n); }
+template <typename V>
+void put(std::string& out, V v) {
+  put(out, &v, sizeof(v));
+}
+
+// Values [from, to) of a table, as int32.
+void append_range(PyObject* o, Py_ssize_t from, Py_ssize_t to, std::vector<int32_t>& out) {
+  if (PyTuple_CheckExact(o) || PyList_CheckExact(o)) {
+    PyObject** items = PySequence_Fast_ITEMS(o);
+    for (Py_ssize_t i = from; i < to; ++i) out.push_back(int32_of(integer(items[i])));
+    return;
+  }
+  const size_t at = out.size();
+  append_ints(o, out, "a block table must be a flat sequence of block ids");
+  out.erase(out.begin() + static_cast<std::ptrdiff_t>(at) + to, out.end());
+  out.erase(out.begin() + static_cast<std::ptrdiff_t>(at), out.begin() + static_cast<std::ptrdiff_t>(at) + from);
+}
+
+// encode_chunk(requests, extra, mode, layer_begin, layer_end, plane_begin, plane_end, page size | 0) -> bytes. With a page size, each
+// request's tables are cut to the pages its range touches and the range is rebased onto them.
+PyObject* encode_chunk(PyObject* const* a) {
+  const Ref requests(PySequence_Fast(a[0], "requests must be a sequence"));
+  const Ref extra(PySequence_Fast(a[1], "extra ranges must be a sequence"));
+  const long long page_size = integer(a[7]);
+  std::string out;
+  put(out, static_cast<uint32_t>(PySequence_Fast_GET_SIZE(requests.p)));
+  put(out, static_cast<uint32_t>(PySequence_Fast_GET_SIZE(extra.p)));
+  for (int i = 2; i < 7; ++i) put(out, static_cast<uint32_t>(integer(a[i])));
+  put(out, uint32_t{0});
+  std::vector<int32_t> ids;
+  for (Py_ssize_t r = 0; r < PySequence_Fast_GET_SIZE(requests.p); ++r) {
+    const Ref request(PySequence_Fast(PySequence_Fast_GET_ITEM(requests.p, r), "a request is (source, target, start, end)"));
+    if (PySequence_Fast_GET_SIZE(request.p) != 4) bad_value("a request is (source, target, start, end)");
+    const Ref source(PySequence_Fast(PySequence_Fast_GET_ITEM(request.p, 0), "block tables must be a sequence"));
+    const Ref target(PySequence_Fast(PySequence_Fast_GET_ITEM(request.p, 1), "block tables must be a sequence"));
+    const int64_t start = integer(PySequence_Fast_GET_ITEM(request.p, 2)), end = integer(PySequence_Fast_GET_ITEM(request.p, 3));
+    const Py_ssize_t ns = PySequence_Fast_GET_SIZE(source.p), nt = PySequence_Fast_GET_SIZE(target.p);
+    if (ns == 0 || nt == 0 || start < 0 || start >= end) bad_value("invalid KV range");
+    const int64_t first = page_size > 0 ? start / page_size : 0;
+    int64_t pages = INT64_MAX;  // of the shortest table, counted from the first page that is sent
+    for (const Ref* side : {&source, &target}) {
+      for (Py_ssize_t p = 0; p < PySequence_Fast_GET_SIZE(side->p); ++p) {
+        const int64_t n = length(PySequence_Fast_GET_ITEM(side->p, p)) - first;
+        pages = n < pages ? n : pages;
+      }
+    }
+    if (page_size > 0 && pages > (end - 1) / page_size - first + 1) pages = (end - 1) / page_size - first + 1;
+    if (pages < 0) pages = 0;
+    put(out, static_cast<uint32_t>(ns));
+    put(out, static_cast<uint32_t>(nt));
+    put(out, static_cast<int64_t>(start - first * page_size));
+    put(out, static_cast<int64_t>(end - first * page_size));
+    put(out, static_cast<uint32_t>(pages));
+    ids.clear();
+    for (const Ref* side : {&source, &target}) {
+      for (Py_ssize_t p = 0; p < PySequence_Fast_GET_SIZE(side->p); ++p) {
+        if (pages > 0) append_range(PySequence_Fast_GET_ITEM(side->p, p), first, first + pages, ids);
+      }
+    }
+    put(out, ids.data(), 4 * ids.size());
+  }
+  for (Py_ssize_t i = 0; i < PySequence_Fast_GET_SIZE(extra.p); ++i) {
+    const Ref triple(PySequence_Fast(PySequence_Fast_GET_ITEM(extra.p, i), "a range is (source, target, bytes)"));
+    if (PySequence_Fast_GET_SIZE(triple.p) != 3) bad_value("a range is (source, target, bytes)");
+    for (int k = 0; k < 3; ++k) put(out, static_cast<int64_t>(integer(PySequence_Fast_GET_ITEM(triple.p, k))));
+  }
+  return PyBytes_FromStringAndSize(out.data(), static_cast<Py_ssize_t>(out.size()));
+}
+
+// handoff_requests(source pool, destination pool, requests, layer_begin, layer_end, plane_begin, plane_end, device, stream) -> code of an
+// all-planes handoff of [(source tables, target tables, start, end)], or RLT_MOVE_UNSUITED (nothing queued) when something about the
+// requests looks wrong or their records do not fit the library's own staging: the general path then does it, or says what is wrong.
+PyObject* handoff_requests(PyObject* const* a) {
+  const auto* src = static_cast<const RltPool*>(address(a[0]));
+  const auto* dst = static_cast<const RltPool*>(address(a[1]));
+  const Ref requests(PySequence_Fast(a[2], "requests must be a sequence"));
+  const int64_t bs = src->block_size;
+  const Py_ssize_t n = PySequence_Fast_GET_SIZE(requests.p);
+  PyObject* unsuited = PyLong_FromLong(RLT_MOVE_UNSUITED);
+  if (n < 1 || n > RLT_MAX_REQUESTS || bs < 1) return unsuited;
+  std::vector<int32_t> records, ids;
+  const int words = kRecordHeader + src->num_planes + dst->num_planes;
+  int64_t before = 0, blocks = 0, width = 1;
+  for (Py_ssize_t r = 0; r < n; ++r) {
+    const Ref request(PySequence_Fast(PySequence_Fast_GET_ITEM(requests.p, r), "a request is (source, target, start, end)"));
+    if (PySequence_Fast_GET_SIZE(request.p) < 4) return unsuited;
+    const int64_t start = integer(PySequence_Fast_GET_ITEM(request.p, 2)), end = integer(PySequence_Fast_GET_ITEM(request.p, 3));
+    if (start < 0 || start >= end) return unsuited;
+    const int64_t first = start / bs, pages = (end - 1) / bs - first + 1;
+    if ((blocks + pages) * words * 4 > (1 << 20)) return unsuited;
+    ids.clear();
+    for (int side = 0; side < 2; ++side) {
+      const RltPool* pool = side == 0 ? src : dst;
+      const Ref tables(PySequence_Fast(PySequence_Fast_GET_ITEM(request.p, side), "block tables must be a sequence"));
+      if (PySequence_Fast_GET_SIZE(tables.p) != pool->num_planes) return unsuited;
+      Py_ssize_t of_request = -1;
+      for (int p = 0; p < pool->num_planes; ++p) {
+        PyObject* table = PySequence_Fast_GET_ITEM(tables.p, p);
+        const Py_ssize_t held = length(table);
+        if (held < first + pages || (of_request >= 0 && held != of_request)) return unsuited;
+        of_request = held;
+        width = held > width ? held : width;
+        const size_t at = ids.size();
+        append_range(table, first, first + pages, ids);
+        for (size_t i = at; i < ids.size(); ++i) {
+          if (static_cast<uint32_t>(ids[i]) >= static_cast<uint32_t>(pool->num_blocks)) return unsuited;
+        }
+      }
+    }
+    const int planes = src->num_planes + dst->num_planes;
+    for (int64_t k = 0; k < pages; ++k) {
+      const int64_t base = (first + k) * bs;
+      const int64_t lo = start > base ? start - base : 0, hi = end < base + bs ? end - base : bs;
+      const int32_t head[kRecordHeader] = {static_cast<int32_t>(r), static_cast<int32_t>(first + k), static_cast<int32_t>(lo | hi << 8),
+                                           static_cast<int32_t>(base + lo - start), static_cast<int32_t>(before), static_cast<int32_t>(end - start)};
+      records.insert(records.end(), head, head + kRecordHeader);
+      for (int p = 0; p < planes; ++p) records.push_back(ids[static_cast<size_t>(p) * pages + k]);
+    }
+    blocks += pages;
+    before += end - start;
+  }
+  Py_DECREF(unsuited);
+  RltOptions o = {};
+  o.layer_begin = static_cast<int32_t>(integer(a[3]));
+  o.layer_end = static_cast<int32_t>(integer(a[4]));
+  o.plane_begin = static_cast<int32_t>(integer(a[5]));
+  o.plane_end = static_cast<int32_t>(integer(a[6]));
+  RltBlockMoves m = {};
+  m.host_records = records.data();
+  m.blocks = static_cast<int32_t>(blocks);
+  m.words = words;
+  m.src_planes = src->num_planes;
+  m.dst_planes = dst->num_planes;
+  m.block_size = static_cast<int32_t>(bs);
+  m.num_requests = static_cast<int32_t>(n);
+  m.table_width = static_cast<int32_t>(width);
+  const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(integer(a[7])));
+  return PyLong_FromLong(rlt_handoff_staged(src, dst, &m, &o, stream_of(a[8])));
+}
+
+// pack_segments([(address, bytes, device)], [(address, bytes, device)], [(low, high, base)]) -> the (source, destination, bytes)
+// triples as int64, destinations translated by the span that holds them.
+PyObject* pack_segments(PyObject* const* a) {
+  const Ref local(PySequence_Fast(a[0], "descriptors must be a sequence")), remote(PySequence_Fast(a[1], "descriptors must be a sequence"));
+  const Ref spans(PySequence_Fast(a[2], "spans must be a sequence"));
+  std::vector<int64_t> span;
+  for (Py_ssize_t i = 0; i < PySequence_Fast_GET_SIZE(spans.p); ++i) {
+    const Ref s(PySequence_Fast(PySequence_Fast_GET_ITEM(spans.p, i), "a span is (low, high, base)"));
+    for (int k = 0; k < 3; ++k) span.push_back(integer(PySequence_Fast_GET_ITEM(s.p, k)));
+  }
+  const Py_ssize_t n = PySequence_Fast_GET_SIZE(local.p);
+  if (n != PySequence_Fast_GET_SIZE(remote.p)) bad_value("incompatible source/target KV geometry");
+  const Ref out(PyBytes_FromStringAndSize(nullptr, 24 * n));
+  auto* triple = reinterpret_cast<int64_t*>(PyBytes_AS_STRING(out.p));
+  size_t hit = 0;  // ranges of one tensor follow one another: try the last span first
+  for (Py_ssize_t i = 0; i < n; ++i, triple += 3) {
+    const Ref s(PySequence_Fast(PySequence_Fast_GET_ITEM(local.p, i), "a descriptor is (address, bytes, device)"));
+    const Ref d(PySequence_Fast(PySequence_Fast_GET_ITEM(remote.p, i), "a descriptor is (address, bytes, device)"));
+    if (PySequence_Fast_GET_SIZE(s.p) < 2 || PySequence_Fast_GET_SIZE(d.p) < 2) bad_value("a descriptor is (address, bytes, device)");
+    const int64_t bytes = integer(PySequence_Fast_GET_ITEM(s.p, 1)), to = integer(PySequence_Fast_GET_ITEM(d.p, 0));
+    if (bytes != integer(PySequence_Fast_GET_ITEM(d.p, 1))) bad_value("incompatible source/target KV geometry");
+    auto inside = [&](size_t k) { return span[k] <= to && to + bytes <= span[k + 1]; };
+    if (hit >= span.size() || !inside(hit)) {
+      for (hit = 0; hit < span.size() && !inside(hit); hit += 3) {
+      }
+      if (hit >= span.size()) bad_value("remote descriptor outside the peer's registered memory");
+    }
+    triple[0] = integer(PySequence_Fast_GET_ITEM(s.p, 0));
+    triple[1] = span[hit + 2] + (to - span[hit]);
+    triple[2] = bytes;
+  }
+  Py_INCREF(out.p);
+  return out.p;
+}
+
+// copy_segments(triples, device, stream) -> code
+PyObject* copy_segments(PyObject* const* a) {
+  char* data = nullptr;
+  Py_ssize_t n = 0;
+  if (PyBytes_AsStringAndSize(a[0], &data, &n) != 0) throw Failure{};
+  const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(integer(a[1])));
+  const auto* triples = reinterpret_cast<const int64_t*>(data);
+  for (Py_ssize_t left = n / 24; left > 0;) {
+    const int32_t count = static_cast<int32_t>(left < RLT_INLINE_SEGMENTS ? left : RLT_INLINE_SEGMENTS);
+    const int rc = rlt_copy_segments_inline(triples, count, stream_of(a[2]));
+    if (rc != RLT_OK) return PyLong_FromLong(rc);
+    triples += 3 * static_cast<ptrdiff_t>(count);
+    left -= count;
+  }
+  return PyLong_FromLong(RLT_OK);
+}
+
+// push(source, destination, bytes, device, stream) -> code
+PyObject* push(PyObject* const* a) {
+  const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(integer(a[3])));
+  return PyLong_FromLong(rlt_kv_push(address(a[0]), address(a[1]), integer(a[2]), stream_of(a[4])));
+}
+
+// post(slot address, 56-byte body, stamp, device, stream) -> code
+PyObject* post(PyObject* const* a) {
+  char* body = nullptr;
+  Py_ssize_t n = 0;
+  if (PyBytes_AsStringAndSize(a[1], &body, &n) != 0) throw Failure{};
+  if (n != 56) bad_value("a message body has 56 bytes");
+  const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(integer(a[3])));
+  return PyLong_FromLong(rlt_kv_post(address(a[0]), reinterpret_cast<const uint8_t*>(body), PyLong_AsUnsignedLongLong(a[2]), stream_of(a[4])));
+}
+
 // ------------------------------------------------------------------------------------------------ the module
 
 template <PyObject* (*kFunction)(PyObject* const*), int kArgs>
@@ -776,6 +987,12 @@ PyMethodDef kMethods[] = {
     RLT_ENTRY("move", move, 20),
     RLT_ENTRY("handoff_host", handoff_host, 12),
     RLT_ENTRY("finalize", finalize, 7),
+    RLT_ENTRY("encode_chunk", encode_chunk, 8),
+    RLT_ENTRY("handoff_requests", handoff_requests, 9),
+    RLT_ENTRY("pack_segments", pack_segments, 3),
+    RLT_ENTRY("copy_segments", copy_segments, 3),
+    RLT_ENTRY("push", push, 5),
+    RLT_ENTRY("post", post, 5),
     RLT_ENTRY("tensor_copy", tensor_copy, 3),
     RLT_ENTRY("transfer_new", transfer_new, 0),
     RLT_ENTRY("transfer_reset", transfer_reset, 1),

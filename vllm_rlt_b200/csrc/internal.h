@@ -20,6 +20,10 @@ RLT_API int rlt_stage_upload(const void* host, size_t bytes, void* device, rlt_s
 RLT_API int rlt_tensor_transfer_inline(const int64_t* descriptors, int32_t count, int32_t max_rows, int32_t max_cols,
                                        int32_t dtype, rlt_stream_t stream);
 
+// rlt_kv_copy_segments with the (source, destination, bytes) triples in HOST memory: they travel as kernel parameters.
+#define RLT_INLINE_SEGMENTS 1024
+RLT_API int rlt_copy_segments_inline(const int64_t* triples, int32_t count, rlt_stream_t stream);
+
 #ifdef __cplusplus
 }
 #endif

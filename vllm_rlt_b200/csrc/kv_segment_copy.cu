@@ -6,28 +6,34 @@
 // partition_segments produces (:95-112): up to a few hundred ranges whose sizes
 // differ by orders of magnitude (a 1.5 MiB block next to a 4 KiB partial row).
 //
-// Work split: the ranges are cut into tiles of 32 KiB (two passes of the copy loop) and the tiles of all
-// ranges form one flat index space that the persistent grid strides over: at any moment the CTAs work on
-// neighbouring tiles, so the DRAM channels see one dense window of addresses. Every CTA computes the
-// exclusive scan of the per-range tile counts with warp-shuffle prefix sums in shared memory and finds a tile's
-// range by binary search. Measured on a launch that moves 0.8 GB in 256 ranges: 0.128 ms, 0.96 of the HBM copy rate
-// (a plain device-to-device copy of the same bytes: 0.125 ms); tiles of 64 KiB leave up to 7 % of imbalance there
-// (0.132 ms), and giving each CTA one contiguous share of the bytes puts hundreds of far-apart streams on the memory
-// system (0.138 ms).
+// Work split: the ranges are cut into tiles, and the tiles of all ranges form one flat index space.
+//
+// Where the host knows the sizes (push, and ranges that come from the host, whose triples are kernel parameters) the grid
+// holds one CTA per 16 KiB tile, in order: the hardware then keeps all SMs within a few MB of each other, which DRAM
+// rewards (block_moves.cu has the measurements). 0.4 GB read and written in 256 ranges of 1.5 MiB: 136 us with the persistent kernel
+// below, 120 here; a push of 1 GiB 343 -> 312 us (6.9 TB/s).
+//
+// A list in device memory has sizes the host cannot see: a persistent grid strides over tiles of 32 KiB, every CTA computes the
+// exclusive scan of the per-range tile counts with warp-shuffle prefix sums in shared memory and finds a tile's range by
+// binary search.
 //
 // Roofline: one read and one write per byte. Local copies are HBM bound; a
 // destination on a peer GPU is bound by NVLink (one direction).
 
+#include <cstring>
+
 #include "common.cuh"
+#include "internal.h"
 
 namespace rlt {
 namespace {
 
-constexpr long long kTileBytes = 32 * 1024;  // 16, 64 and 128 KiB tiles, and 4 or 6 CTAs per SM, all measured slower
-constexpr int kUnroll = 4;  // four 16-byte loads in flight per thread and three CTAs per SM measured best on HBM
+constexpr long long kTileBytes = 32 * 1024;   // of the persistent kernel: 16, 64 and 128 KiB, and 4 or 6 CTAs per SM, all measured slower
+constexpr long long kShortTile = 16 * 1024;   // of one CTA per tile
+constexpr int kUnroll = 4;
 constexpr int kCtasPerSm = 3;
 
-template <typename T>
+template <typename T, int kUnroll = rlt::kUnroll>
 __device__ __forceinline__ void stream_range(const char* __restrict__ src, char* __restrict__ dst, long long n) {
   const T* s = reinterpret_cast<const T*>(src);
   T* d = reinterpret_cast<T*>(dst);
@@ -46,11 +52,17 @@ __device__ __forceinline__ void stream_range(const char* __restrict__ src, char*
   }
 }
 
-// One tile of one range. Pointers that are both 16-byte aligned take the vector path with a byte tail;
+// One tile of one range. kWide: 32-byte accesses where both pointers allow (the persistent kernel measured slower with
+// them: 136 -> 140 us for 0.8 GB). Pointers that are both 16-byte aligned take the vector path with a byte tail;
 // otherwise the widest element both pointers and the length allow.
+template <bool kWide>
 __device__ __forceinline__ void copy_piece(const char* src, char* dst, long long n) {
   const unsigned long long both = reinterpret_cast<unsigned long long>(src) | reinterpret_cast<unsigned long long>(dst);
-  if ((both & 15ull) == 0) {
+  if (kWide && (both & 31ull) == 0) {
+    const long long body = n & ~31ll;
+    stream_range<Vec32, 2>(src, dst, body >> 5);
+    if (static_cast<long long>(threadIdx.x) < n - body) dst[body + threadIdx.x] = src[body + threadIdx.x];
+  } else if ((both & 15ull) == 0) {
     const long long body = n & ~15ll;
     stream_range<uint4>(src, dst, body >> 4);
     if (static_cast<long long>(threadIdx.x) < n - body) dst[body + threadIdx.x] = src[body + threadIdx.x];
@@ -61,12 +73,54 @@ __device__ __forceinline__ void copy_piece(const char* src, char* dst, long long
   }
 }
 
-__global__ void __launch_bounds__(kThreads, 3) push_kernel(const char* src, char* dst, long long nbytes) {
-  const long long tiles = (nbytes + kTileBytes - 1) / kTileBytes;
-  for (long long t = blockIdx.x; t < tiles; t += gridDim.x) {
-    const long long at = t * kTileBytes;
-    copy_piece(src + at, dst + at, min(kTileBytes, nbytes - at));
+__global__ void __launch_bounds__(kThreads, 6) push_kernel(const char* src, char* dst, long long nbytes) {
+  const long long at = static_cast<long long>(blockIdx.x) * kShortTile;
+  copy_piece<true>(src + at, dst + at, min(kShortTile, nbytes - at));
+}
+
+struct Segment {
+  const char* src;
+  char* dst;
+  long long bytes;
+};
+template <int kCount>
+struct InlineSegments {
+  int count;
+  int first_tile[kCount + 1];
+  Segment segment[kCount];
+};
+
+template <int kCount>
+__global__ void __launch_bounds__(kThreads, 6) inline_segments_kernel(const __grid_constant__ InlineSegments<kCount> list) {
+  const int t = static_cast<int>(blockIdx.x);
+  int lo = 0, hi = list.count;  // last range whose first tile is at or before t
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (list.first_tile[mid] <= t) lo = mid; else hi = mid;
   }
+  const Segment s = list.segment[lo];
+  const long long at = static_cast<long long>(t - list.first_tile[lo]) * kShortTile;
+  copy_piece<true>(s.src + at, s.dst + at, min(kShortTile, s.bytes - at));
+}
+
+template <int kCount>
+int launch_inline(const int64_t* triples, int count, cudaStream_t stream) {
+  InlineSegments<kCount> list;
+  long long tiles = 0;
+  list.count = 0;
+  for (int i = 0; i < count; ++i) {
+    if (triples[3 * i + 2] <= 0) continue;
+    list.first_tile[list.count] = static_cast<int>(tiles);
+    list.segment[list.count++] = {reinterpret_cast<const char*>(triples[3 * i]), reinterpret_cast<char*>(triples[3 * i + 1]), triples[3 * i + 2]};
+    tiles += (triples[3 * i + 2] + kShortTile - 1) / kShortTile;
+    if (tiles > 0x7fffffffll) return RLT_E_LIMIT;
+  }
+  if (list.count == 0) return RLT_OK;
+  list.first_tile[list.count] = static_cast<int>(tiles);
+  inline_segments_kernel<kCount><<<static_cast<unsigned>(tiles), kThreads, 0, stream>>>(list);
+  RLT_CUDA_TRY(cudaGetLastError());
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  return RLT_OK;
 }
 
 __global__ void __launch_bounds__(kThreads, 3) segment_copy_kernel(const long long* __restrict__ segments, int count) {
@@ -105,7 +159,7 @@ __global__ void __launch_bounds__(kThreads, 3) segment_copy_kernel(const long lo
     }
     const long long at = static_cast<long long>(t - tile_off[lo]) * kTileBytes;
     const long long n = segments[3ll * lo + 2];
-    copy_piece(reinterpret_cast<const char*>(segments[3ll * lo]) + at, reinterpret_cast<char*>(segments[3ll * lo + 1]) + at,
+    copy_piece<false>(reinterpret_cast<const char*>(segments[3ll * lo]) + at, reinterpret_cast<char*>(segments[3ll * lo + 1]) + at,
                min(kTileBytes, n - at));
   }
 }
@@ -119,17 +173,25 @@ int rlt_kv_push(const void* src, void* dst, int64_t nbytes, rlt_stream_t stream)
   const rlt::NvtxRange range("rlt.kv_push");
   if (nbytes == 0) return RLT_OK;
   if (src == nullptr || dst == nullptr || nbytes < 0) return RLT_E_INVALID;
-  int sms = 0;
-  const int rc = rlt::sm_count(&sms);
-  if (rc != RLT_OK) return rc;
-  // one persistent wave; a small range gets one CTA per 16 KiB (one pass of the copy loop)
-  const long long passes = (nbytes + 16383) / 16384;
-  const int grid = static_cast<int>(passes < sms * static_cast<long long>(rlt::kCtasPerSm) ? passes : sms * static_cast<long long>(rlt::kCtasPerSm));
-  rlt::push_kernel<<<grid, rlt::kThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+  const long long tiles = (nbytes + rlt::kShortTile - 1) / rlt::kShortTile;
+  if (tiles > 0x7fffffffll) return RLT_E_LIMIT;
+  rlt::push_kernel<<<static_cast<unsigned>(tiles), rlt::kThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
       static_cast<const char*>(src), static_cast<char*>(dst), nbytes);
   RLT_CUDA_TRY(cudaGetLastError());
   rlt::g_launches.fetch_add(1, std::memory_order_relaxed);
   return RLT_OK;
+}
+
+int rlt_copy_segments_inline(const int64_t* triples, int32_t count, rlt_stream_t stream) {
+  const rlt::NvtxRange range("rlt.kv_copy_segments");
+  if (count == 0) return RLT_OK;
+  if (triples == nullptr || count < 0) return RLT_E_INVALID;
+  if (count > RLT_INLINE_SEGMENTS) return RLT_E_LIMIT;
+  const cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  // a parameter block is copied into the launch whole: 256 ranges are what one submission of the default configuration holds
+  return count <= 32    ? rlt::launch_inline<32>(triples, count, s)
+         : count <= 256 ? rlt::launch_inline<256>(triples, count, s)
+                        : rlt::launch_inline<RLT_INLINE_SEGMENTS>(triples, count, s);
 }
 
 int rlt_kv_copy_segments(const int64_t* segments, int32_t count, rlt_stream_t stream) {

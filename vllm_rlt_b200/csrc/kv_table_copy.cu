@@ -40,6 +40,7 @@
 
 #include <cstring>
 #include <mutex>
+#include <vector>
 
 #include "block_moves.h"
 #include "common.cuh"
@@ -1211,24 +1212,42 @@ int host_ring(HostRing** out) {
   return RLT_OK;
 }
 
-// rlt_kv_handoff_host as one launch whose page records are kernel parameters: no slot, no copy, no event. Records take
-// (6 + planes of both sides) words a page; a batch whose records do not fit goes through a slot.
+// The next slot of the current device's ring, free to be written: the launch that last read it (kHostSlots calls ago) is
+// over. The caller holds g_host_ring_mutex and records the slot's event behind the launch that reads it.
+struct HostSlot {
+  unsigned char* host;
+  unsigned char* device;
+  cudaEvent_t done;
+};
+int next_host_slot(HostSlot* out) {
+  HostRing* ring = nullptr;
+  const int rc = host_ring(&ring);
+  if (rc != RLT_OK) return rc;
+  const int slot = ring->next;
+  ring->next = (slot + 1) % kHostSlots;
+  RLT_CUDA_TRY(cudaEventSynchronize(ring->done[slot]));
+  *out = {ring->pinned + slot * kHostSlotBytes, ring->device + slot * kHostSlotBytes, ring->done[slot]};
+  return RLT_OK;
+}
+
+// rlt_kv_handoff_host as one launch from page records: kernel parameters, or a slot where they do not fit those. Records
+// take (6 + planes of both sides) words a page; a batch whose records do not fit a slot goes there as tables.
 int handoff_from_records(const RltPool* src, const RltPool* dst, const RltHostBatch* hb, const RltOptions* options,
                          rlt_stream_t stream) {
   const int bs = src->block_size;
   if (bs < 1 || bs > kMaxBlockSize || hb->src_planes < 1 || hb->dst_planes < 1) return RLT_MOVE_UNSUITED;
   const int words = kRecordHeader + hb->src_planes + hb->dst_planes;
-  int32_t records[kInlineWords];
-  int at = 0;
+  thread_local std::vector<int32_t> records(kHostSlotBytes / sizeof(int32_t));
+  size_t at = 0;
   long long before = 0;
   for (int r = 0; r < hb->num_requests; ++r) {
     const int b = hb->tok_begin[r], e = hb->tok_end[r];
     if (e <= b) continue;
     const bool bad = b < 0 || e > static_cast<long long>(hb->table_width) * bs;
     const int first = bad ? 0 : b / bs, last = bad ? 0 : (e - 1) / bs;
-    if (at + static_cast<long long>(last - first + 1) * words > kInlineWords) return RLT_MOVE_UNSUITED;
+    if (at + static_cast<size_t>(last - first + 1) * words > records.size()) return RLT_MOVE_UNSUITED;
     for (int page = first; page <= last; ++page, at += words) {
-      int32_t* w = records + at;
+      int32_t* w = records.data() + at;
       const int base = page * bs;
       const int lo = b > base ? b - base : 0, hi = e < base + bs ? e - base : bs;
       w[0] = r;
@@ -1245,15 +1264,15 @@ int handoff_from_records(const RltPool* src, const RltPool* dst, const RltHostBa
     before += e - b;
   }
   RltBlockMoves m = {};
-  m.host_records = records;
-  m.blocks = at / words;
+  m.host_records = records.data();
+  m.blocks = static_cast<int32_t>(at / words);
   m.words = words;
   m.src_planes = hb->src_planes;
   m.dst_planes = hb->dst_planes;
   m.block_size = bs;
   m.num_requests = hb->num_requests;
   m.table_width = hb->table_width;
-  return rlt_move_blocks(RLT_MOVE_DIRECT, src, dst, &m, options, nullptr, 0, stream);
+  return rlt_handoff_staged(src, dst, &m, options, stream);
 }
 
 }  // namespace
@@ -1279,6 +1298,26 @@ int64_t rlt_kv_static_plan_entries(void) { return rlt::kStaticPlanEntries; }
 
 int64_t rlt_kv_host_batch_limit(void) { return static_cast<int64_t>(rlt::kHostSlotBytes); }
 
+int rlt_handoff_staged(const RltPool* src, const RltPool* dst, const RltBlockMoves* moves, const RltOptions* options,
+                       rlt_stream_t stream) {
+  const size_t bytes = static_cast<size_t>(moves->blocks) * moves->words * sizeof(int32_t);
+  if (bytes <= kInlineWords * sizeof(int32_t))
+    return rlt_move_blocks(RLT_MOVE_DIRECT, src, dst, moves, options, nullptr, 0, stream);
+  if (bytes > rlt::kHostSlotBytes) return RLT_MOVE_UNSUITED;
+  const std::lock_guard<std::mutex> lock(rlt::g_host_ring_mutex);
+  rlt::HostSlot slot;
+  const int rc = rlt::next_host_slot(&slot);
+  if (rc != RLT_OK) return rc;
+  const cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  memcpy(slot.host, moves->host_records, bytes);
+  RLT_CUDA_TRY(cudaMemcpyAsync(slot.device, slot.host, bytes, cudaMemcpyHostToDevice, s));
+  RltBlockMoves staged = *moves;
+  staged.device_records = reinterpret_cast<const int32_t*>(slot.device);
+  const int launched = rlt_move_blocks(RLT_MOVE_DIRECT, src, dst, &staged, options, nullptr, 0, stream);
+  RLT_CUDA_TRY(cudaEventRecord(slot.done, s));
+  return launched;
+}
+
 int rlt_kv_handoff_host(const RltPool* src, const RltPool* dst, const RltHostBatch* hb, const RltOptions* options,
                         rlt_stream_t stream) {
   if (src == nullptr || dst == nullptr || hb == nullptr || options == nullptr) return RLT_E_INVALID;
@@ -1298,15 +1337,11 @@ int rlt_kv_handoff_host(const RltPool* src, const RltPool* dst, const RltHostBat
   if (by_records != RLT_MOVE_UNSUITED) return by_records;
 
   const std::lock_guard<std::mutex> lock(rlt::g_host_ring_mutex);
-  rlt::HostRing* ring = nullptr;
-  const int rc = rlt::host_ring(&ring);
+  rlt::HostSlot slot;
+  const int rc = rlt::next_host_slot(&slot);
   if (rc != RLT_OK) return rc;
-  const int slot = ring->next;
-  ring->next = (slot + 1) % rlt::kHostSlots;
-  // the launch that last read this slot (kHostSlots calls ago) must be over before the host overwrites it
-  RLT_CUDA_TRY(cudaEventSynchronize(ring->done[slot]));
-  unsigned char* host = ring->pinned + slot * rlt::kHostSlotBytes;
-  unsigned char* dev = ring->device + slot * rlt::kHostSlotBytes;
+  unsigned char* host = slot.host;
+  unsigned char* dev = slot.device;
   memcpy(host, hb->src_tables, src_bytes);
   memcpy(host + src_bytes, hb->dst_tables, dst_bytes);
   memcpy(host + src_bytes + dst_bytes, hb->tok_begin, range_bytes);
@@ -1322,7 +1357,7 @@ int rlt_kv_handoff_host(const RltPool* src, const RltPool* dst, const RltHostBat
   batch.tok_end = reinterpret_cast<const int32_t*>(dev + src_bytes + dst_bytes + range_bytes);
   const int launched = rlt::launch_table_copy(rlt::kDirect, src, dst, &batch, options, nullptr, 0, s);
   // recorded even when the launch was refused: the copy above still reads the slot
-  RLT_CUDA_TRY(cudaEventRecord(ring->done[slot], s));
+  RLT_CUDA_TRY(cudaEventRecord(slot.done, s));
   return launched;
 }
 

@@ -41,6 +41,8 @@ from multiprocessing import shared_memory
 
 import numpy as np
 
+from .. import _lib
+
 SLOT_BYTES = 64
 BODY_BYTES = 56
 LANES = 16
@@ -99,26 +101,18 @@ def _kv_region(key, value) -> dict:
 # ------------------------------------------------------------------------------------ chunk descriptors
 
 
-def encode_chunk(requests, extra, *, mode=0, layer_begin=0, layer_end=0, plane_begin=0, plane_end=0) -> bytes:
+def encode_chunk(requests, extra, *, mode=0, layer_begin=0, layer_end=0, plane_begin=0, plane_end=0, page_size=0) -> bytes:
     """A pull offer's descriptor: what the receiver needs to run the launch itself.
 
-    ``requests`` is ``[(source tables, target tables, start, end)]``; each request's tables are cut down to the
-    pages the range touches and the range is rebased onto them (block tables are only ever indexed by page, so
-    the kernel's result is the same), which keeps a descriptor proportional to the chunk, not to the prompt.
-    ``extra`` is ``[(source address, target address, bytes)]``.
+    ``requests`` is ``[(source tables, target tables, start, end)]``; given the page size, each request's tables are cut
+    down to the pages the range touches and the range is rebased onto them as ``trim_request`` does (block tables are only
+    ever indexed by page, so the kernel's result is the same), which keeps a descriptor proportional to the chunk, not
+    to the prompt. ``extra`` is ``[(source address, target address, bytes)]``.
+
+    Layout: ``<8I`` (requests, extra ranges, mode, layer and plane bounds, 0); per request ``<2I2qI`` (planes of either side,
+    start, end, pages) and the tables as int32; per extra range ``<3q``.
     """
-    out = [struct.pack("<8I", len(requests), len(extra), mode, layer_begin, layer_end, plane_begin, plane_end, 0)]
-    for source, target, start, end in requests:
-        if not source or not target or start < 0 or start >= end:
-            raise ValueError("invalid KV range")
-        page = min(len(table) for table in (*source, *target))
-        out.append(struct.pack("<2I2q", len(source), len(target), start, end))
-        out.append(struct.pack("<I", page))
-        for table in (*source, *target):
-            out.append(np.asarray(table[:page], dtype=np.int32).tobytes())
-    for src, dst, n in extra:
-        out.append(struct.pack("<3q", src, dst, n))
-    return b"".join(out)
+    return _lib.load_host().encode_chunk(requests, extra, mode, layer_begin, layer_end, plane_begin, plane_end, page_size)
 
 
 def decode_chunk(raw: bytes):
@@ -127,15 +121,12 @@ def decode_chunk(raw: bytes):
     at = 32
     requests = []
     for _ in range(n_req):
-        src_planes, dst_planes, start, end = struct.unpack_from("<2I2q", raw, at)
-        at += 24
-        (pages,) = struct.unpack_from("<I", raw, at)
-        at += 4
-        tables = []
-        for _ in range(src_planes + dst_planes):
-            tables.append(np.frombuffer(raw, dtype=np.int32, count=pages, offset=at))
-            at += 4 * pages
-        requests.append((tuple(tables[:src_planes]), tuple(tables[src_planes:]), start, end))
+        src_planes, dst_planes, start, end, pages = struct.unpack_from("<2I2qI", raw, at)
+        at += 28
+        planes = src_planes + dst_planes
+        tables = tuple(np.frombuffer(raw, dtype=np.int32, count=planes * pages, offset=at).reshape(planes, pages))
+        at += 4 * planes * pages
+        requests.append((tables[:src_planes], tables[src_planes:], start, end))
     extra = []
     for _ in range(n_extra):
         extra.append(struct.unpack_from("<3q", raw, at))
@@ -211,6 +202,7 @@ class Mailbox:
         self.name = self.shm.name
         self.words = np.frombuffer(self.shm.buf, dtype=np.uint64)
         self.bytes = np.frombuffer(self.shm.buf, dtype=np.uint8)
+        self._flags = self.shm.buf.cast("Q")  # the same words; one costs a third of a NumPy element to read
         self.next = [1] * LANES  # receiver: next stamp expected per lane
 
     @staticmethod
@@ -232,38 +224,45 @@ class Mailbox:
         return struct.pack("<IBBHII", sequence, len(raw), kind, count, *descriptor) + raw.ljust(TID_MAX, b"\0")
 
     def consumed(self, lane: int) -> int:
-        return int(self.words[lane * LANE_BYTES // 8])
+        return self._flags[lane * LANE_BYTES // 8]
 
     def write_descriptor(self, lane: int, offset: int, raw: bytes) -> None:
         at = lane * LANE_BYTES + RING_OFFSET + offset
-        self.bytes[at : at + len(raw)] = np.frombuffer(raw, dtype=np.uint8)
+        self.shm.buf[at : at + len(raw)] = raw
 
     def post_from_host(self, lane: int, n: int, body: bytes) -> None:
         """The CPU form of ``rlt_kv_post``: body first, stamp last (program order is store order on x86)."""
         at = self.slot_offset(lane, n)
-        self.bytes[at + 8 : at + SLOT_BYTES] = np.frombuffer(body, dtype=np.uint8)
-        self.words[at // 8] = n
+        self.shm.buf[at + 8 : at + SLOT_BYTES] = body
+        self._flags[at // 8] = n
+
+    def waiting(self, lane: int) -> bool:
+        """Receiver: whether ``drain`` would yield anything."""
+        n = self.next[lane]
+        return self._flags[self.slot_offset(lane, n) // 8] == n
 
     def drain(self, lane: int):
         """Receiver: yield a ``Message`` for everything that has arrived on a lane, in order."""
         while True:
             n = self.next[lane]
             at = self.slot_offset(lane, n)
-            if int(self.words[at // 8]) != n:
+            if self._flags[at // 8] != n:
                 return
-            sequence, length, kind, count, d_off, d_len = struct.unpack_from("<IBBHII", self.bytes, at + 8)
-            tid = bytes(self.bytes[at + 24 : at + 24 + min(length, TID_MAX)]).decode()
+            buf = self.shm.buf
+            sequence, length, kind, count, d_off, d_len = struct.unpack_from("<IBBHII", buf, at + 8)
+            tid = bytes(buf[at + 24 : at + 24 + min(length, TID_MAX)]).decode()
             descriptor = b""
             if d_len:
                 base = lane * LANE_BYTES + RING_OFFSET + d_off
-                descriptor = bytes(self.bytes[base : base + d_len])
+                descriptor = bytes(buf[base : base + d_len])
             self.next[lane] = n + 1
-            self.words[lane * LANE_BYTES // 8] = n  # lets the sender reuse the slot and the descriptor's bytes
+            self._flags[lane * LANE_BYTES // 8] = n  # lets the sender reuse the slot and the descriptor's bytes
             yield Message(kind, tid, sequence, descriptor, max(1, count))
 
     def close(self):
         if self.shm is None:
             return
+        self._flags.release()
         self.words = self.bytes = None
         shm, self.shm = self.shm, None
         try:
@@ -283,6 +282,19 @@ class Mailbox:
 
 
 # ------------------------------------------------------------------------------------ device backend
+
+
+class _Translation:
+    """Addresses of a peer's registered tensors as this process reaches them."""
+
+    def __init__(self, spans):
+        self.spans = spans  # (first address there, one past the last, first address here)
+
+    def __call__(self, address: int, nbytes: int) -> int:
+        for lo, hi, base in self.spans:
+            if lo <= address and address + nbytes <= hi:
+                return base + (address - lo)
+        raise ValueError("remote descriptor outside the peer's registered memory")
 
 
 class CudaBackend:
@@ -306,11 +318,10 @@ class CudaBackend:
         self.peerlib = peerlib
         self._mailboxes: dict[str, tuple[Mailbox, int]] = {}
         self._views: dict[tuple, tuple] = {}
-        self._host_limit = None  # bytes of tables one call of the library's own staging takes
+        self.lane = None  # the mailbox lane this worker writes on, once its transport has chosen it
         self.stream = torch.cuda.Stream(self.device)
-
-    def _on_stream(self):
-        return self.torch.cuda.stream(self.stream)
+        self._where = (self.stream.device.index, self.stream.cuda_stream)  # what the compiled calls launch on
+        self._host = _lib.load_host()
 
     def order_after(self, event) -> None:
         """Make everything submitted from now on wait (on the device) for ``event``."""
@@ -332,51 +343,38 @@ class CudaBackend:
         if same_process and peer_info["device"] != self.device.index:
             self.peerlib.enable_peer_access(self.device.index, peer_info["device"])
 
-        def translate(address: int, nbytes: int) -> int:
-            for lo, hi, base in spans:
-                if lo <= address and address + nbytes <= hi:
-                    return base + (address - lo)
-            raise ValueError("remote descriptor outside the peer's registered memory")
-
-        return translate
+        return _Translation(spans)
 
     def mailbox_pointer(self, name: str) -> tuple[Mailbox, int]:
         """Open a peer's mailbox and make it writable from this device."""
         import ctypes as C
 
-        from .. import _lib
-
         hit = self._mailboxes.get(name)
         if hit is None:
             box = Mailbox(name)
-            host = C.addressof(C.c_char.from_buffer(box.shm.buf))
+            # only the lane this worker writes on is made visible to its GPU: registering memory costs time per page
+            at = (self.lane or 0) * LANE_BYTES
+            size = LANE_BYTES if self.lane is not None else len(box.shm.buf)
+            host = C.addressof(C.c_char.from_buffer(box.shm.buf)) + at
             out = C.c_void_p()
             with self.torch.cuda.device(self.device):
-                _lib.check(_lib.load().rlt_host_register(host, len(box.shm.buf), C.byref(out)), "rlt_host_register")
-            hit = self._mailboxes[name] = (box, int(out.value), host)
+                _lib.check(_lib.load().rlt_host_register(host, size, C.byref(out)), "rlt_host_register")
+            hit = self._mailboxes[name] = (box, int(out.value) - at, host)
         return hit[0], hit[1]
 
-    def copy_segments(self, triples):
-        from ..kernels import kv_handoff as kh
+    def pair(self, local, remote, translate):
+        """Two descriptor lists as what ``copy_segments`` takes."""
+        return self._host.pack_segments(local, remote, translate.spans)
 
-        torch = self.torch
-        host = torch.tensor(triples, dtype=torch.int64).reshape(-1, 3).pin_memory()
-        keep = []
-        with torch.cuda.device(self.device), self._on_stream():
-            for at in range(0, len(host), kh._lib.MAX_SEGMENTS):
-                dev = host[at : at + kh._lib.MAX_SEGMENTS].to(self.device, non_blocking=True)
-                kh.kv_copy_segments(dev)
-                keep.append(dev)
-        return (host, *keep)
+    def copy_segments(self, triples):
+        _lib.check(self._host.copy_segments(triples, *self._where), "rlt_kv_copy_segments")
+        return ()
 
     def copy_ranges(self, triples):
         """A few plain (source, destination, bytes) ranges, one ``rlt_kv_push`` launch each: no descriptor table to
-        build, pin and upload, which matters for the single hidden-state row that rides on a chunk."""
-        from ..kernels import kv_handoff as kh
-
-        with self.torch.cuda.device(self.device), self._on_stream():
-            for src, dst, n in triples:
-                kh.kv_push(src, dst, n)
+        build, which matters for the single hidden-state row that rides on a chunk."""
+        for src, dst, n in triples:
+            _lib.check(self._host.push(src, dst, n, *self._where), "rlt_kv_push")
         return ()
 
     def handoff(self, cache, peer_info, translate, requests, *, mode=0, layer_begin=0, layer_end=0,
@@ -412,15 +410,14 @@ class CudaBackend:
             self._views[key] = views
         src, dst = views
         if exit_planes is None and status is None and mode == kh.MODE_ALL_PLANES:
-            host = self._host_tables(requests, src, dst)
-            if host is not None:  # a chunk's worth of tables: staged and launched by one call into the library
-                with self.torch.cuda.device(self.device):
-                    if before_launch is not None:
-                        before_launch()
-                    kh.kv_handoff_host(src, dst, *host, layer_begin=layer_begin, layer_end=layer_end,
-                                       plane_begin=plane_begin, plane_end=plane_end, stream=self.stream)
+            if before_launch is not None:
+                before_launch()
+            rc = self._host.handoff_requests(src._address(), dst._address(), requests, layer_begin, layer_end, plane_begin,
+                                             plane_end, *self._where)
+            if rc != _lib.MOVE_UNSUITED:
+                _lib.check(rc, "rlt_kv_handoff")
                 return ()
-        with self.torch.cuda.device(self.device), self._on_stream():
+        with self.torch.cuda.device(self.device), self.torch.cuda.stream(self.stream):
             batch = kh.HandoffBatch(
                 [r[0] for r in requests], [r[1] for r in requests], [(r[2], r[3]) for r in requests],
                 block_size=src.block_size, exit_planes=exit_planes, src_blocks=src.num_blocks,
@@ -431,55 +428,12 @@ class CudaBackend:
                           plane_begin=plane_begin, plane_end=plane_end, status=status)
         return (batch,)
 
-    def _host_tables(self, requests, src, dst):
-        """``(source tables, destination tables, begin, end)`` as int32 arrays for ``kv_handoff_host``, or None when
-        the batch is not of that kind (tables of different lengths, too large for a staging slot) or when anything
-        about it looks wrong: the general path then finds the error and words it as the reference does."""
-        import numpy as np
-
-        try:
-            source = np.asarray([r[0] for r in requests], dtype=np.int32)
-            target = np.asarray([r[1] for r in requests], dtype=np.int32)
-        except (ValueError, OverflowError):
-            return None
-        if source.ndim != 3 or target.ndim != 3 or source.shape[1] != src.num_planes or target.shape[1] != dst.num_planes:
-            return None
-        begin = np.asarray([r[2] for r in requests], dtype=np.int64)
-        end = np.asarray([r[3] for r in requests], dtype=np.int64)
-        # a decode worker reserves pages for the tokens it will generate, so its tables run past the prompt's: tables
-        # are only ever indexed by the pages a range touches, and both sides are cut to the shorter one
-        width = min(source.shape[2], target.shape[2])
-        if width < 1:
-            return None
-        if source.shape[2] != width:
-            source = np.ascontiguousarray(source[:, :, :width])
-        if target.shape[2] != width:
-            target = np.ascontiguousarray(target[:, :, :width])
-        if self._host_limit is None:
-            from ..kernels import kv_handoff as kh
-
-            self._host_limit = kh.host_batch_limit()
-        if source.nbytes + target.nbytes + 8 * len(requests) > self._host_limit:
-            return None
-        suspicious = ((begin < 0) | (begin >= end) | (end > source.shape[2] * src.block_size)).any() \
-            or (source.view(np.uint32) >= src.num_blocks).any() or (target.view(np.uint32) >= dst.num_blocks).any()
-        if suspicious:
-            return None
-        return source, target, begin.astype(np.int32), end.astype(np.int32)
-
     def post(self, slot_ptr: int, body: bytes, stamp: int):
-        import ctypes as C
-
-        from .. import _lib
-
-        with self.torch.cuda.device(self.device):
-            buf = (C.c_uint8 * BODY_BYTES).from_buffer_copy(body)
-            _lib.check(_lib.load().rlt_kv_post(slot_ptr, buf, stamp, self.stream.cuda_stream), "rlt_kv_post")
+        _lib.check(self._host.post(slot_ptr, body, stamp, *self._where), "rlt_kv_post")
 
     def event(self):
         ev = self.torch.cuda.Event()
-        with self.torch.cuda.device(self.device):
-            ev.record(self.stream)
+        ev.record(self.stream)
         return ev
 
     marker = event  # an event at the current end of the transfer stream, used to tell when queued work begins
@@ -487,13 +441,10 @@ class CudaBackend:
     def timed_event(self):
         """Like ``event`` but usable with ``elapsed_time`` (device time between two of them)."""
         ev = self.torch.cuda.Event(enable_timing=True)
-        with self.torch.cuda.device(self.device):
-            ev.record(self.stream)
+        ev.record(self.stream)
         return ev
 
     def close(self):
-        from .. import _lib
-
         boxes, self._mailboxes = self._mailboxes, {}
         self._views = {}
         for box, _, host in boxes.values():
@@ -542,6 +493,13 @@ def default_direction() -> str:
     return value
 
 
+def _pair(local, remote, translate):
+    """(source, destination here, bytes) of every descriptor pair, for backends without a compiled form of this."""
+    if len(local) != len(remote) or any(a[1] != b[1] for a, b in zip(local, remote)):
+        raise ValueError("incompatible source/target KV geometry")
+    return [(src, translate(dst, n), n) for (src, n, _), (dst, _, _) in zip(local, remote)]
+
+
 class B200Transport:
     def __init__(self, name, cache, hidden, config, *, backend=None, lane=None, direction=None):
         self.config = config
@@ -581,6 +539,7 @@ class B200Transport:
         # Mailbox lane this worker writes on at every receiver: its device index unless told otherwise
         # (workers of one deployment never share a device, vllm_rlt/pd/config.py:31-33).
         self.info["metadata"]["lane"] = Mailbox.lane_of(self.info["device"] if lane is None else lane)
+        self.backend.lane = self.info["metadata"]["lane"]
         self.peers: dict[str, dict] = {}
         self._lane_agent: dict[int, str] = {}
         self._link: dict[str, dict] = {}  # per peer: address translation, its mailbox, next stamp, descriptor ring
@@ -630,7 +589,7 @@ class B200Transport:
             box, box_ptr = self.backend.mailbox_pointer(peer["metadata"]["mailbox"])
             link = self._link[peer_name] = dict(
                 translate=self.backend.translator(peer), box=box, box_ptr=box_ptr,
-                lane=self.info["metadata"]["lane"], stamp=0, ring=_RingWriter(),
+                lane=self.info["metadata"]["lane"], stamp=0, ring=_RingWriter(), agent=peer_name,
             )
         return link
 
@@ -655,11 +614,12 @@ class B200Transport:
             at = Mailbox.slot_offset(link["lane"], link["stamp"])
             self.backend.post(link["box_ptr"] + at, body, link["stamp"])
 
-    def _ticket(self, handle, transfer_id, sequence, size, keepalive, started) -> bool:
+    def _tickets(self, handle, transfer_id, parts, keepalive, started) -> bool:
         now = time.monotonic()
         begun = now if started is None or started.query() else None  # nothing ahead of it on the transfer stream
-        self.pending.append(Transfer(handle, transfer_id, sequence, size, now, keepalive, started, begun))
-        self.inflight_bytes += size
+        for sequence, size in parts:
+            self.pending.append(Transfer(handle, transfer_id, sequence, size, now, keepalive, started, begun))
+            self.inflight_bytes += size
         return True
 
     def _order_after(self, event):
@@ -680,18 +640,11 @@ class B200Transport:
         if not self._admit(size, link):
             return False
         body = Mailbox.encode(transfer_id, sequence, LANDED)
-        if len(local) != len(remote):
-            raise ValueError("incompatible source/target KV geometry")
-        translate = link["translate"]
-        triples = []
-        for (src, n, _), (dst, m, _) in zip(local, remote):
-            if n != m:
-                raise ValueError("incompatible source/target KV geometry")
-            triples.append((src, translate(dst, n), n))
+        triples = getattr(self.backend, "pair", _pair)(local, remote, link["translate"])
         started = self._order_after(after)
         keep = self.backend.copy_segments(triples) if triples else ()
         self._post(link, body)
-        return self._ticket(self.backend.event(), transfer_id, sequence, size, keep, started)
+        return self._tickets(self.backend.event(), transfer_id, ((sequence, size),), keep, started)
 
     def submit_tables(self, transfer_id, sequence, peer, requests, size, *, mode=0, layer_begin=0, layer_end=0,
                       plane_begin=0, plane_end=0, exit_planes=None, extra=(), status=None, after=None, parts=None):
@@ -728,14 +681,11 @@ class B200Transport:
         if extra:
             keep += tuple(self.backend.copy_ranges([(s, translate(d, n), n) for s, d, n in extra]))
         self._post(link, body)
-        done = self.backend.event()
-        for seq, n in parts:
-            self._ticket(done, transfer_id, seq, n, keep, started)
-        return True
+        return self._tickets(self.backend.event(), transfer_id, parts, keep, started)
 
     def _offer(self, link, transfer_id, parts, requests, extra, where, after) -> bool:
         page = self.info["block_size"]
-        raw = encode_chunk([trim_request(*r, page) for r in requests], extra, **where)
+        raw = encode_chunk(requests, extra, page_size=page, **where)
         box = link["box"]
         at = link["ring"].reserve(len(raw), link["stamp"] + 1, box.consumed(link["lane"]))
         if at is None:
@@ -746,13 +696,8 @@ class B200Transport:
         started = self._order_after(after)  # the offer leaves when the producer's event has fired
         self._post(link, body)
         self._note("offer queued", transfer_id, first)
-        handle = self._offered[(self._agent_of(link), transfer_id, first)] = _RemoteCompletion()
-        for seq, n in parts:
-            self._ticket(handle, transfer_id, seq, n, (), started)
-        return True
-
-    def _agent_of(self, link) -> str:
-        return next(name for name, other in self._link.items() if other is link)
+        handle = self._offered[(link["agent"], transfer_id, first)] = _RemoteCompletion()
+        return self._tickets(handle, transfer_id, parts, (), started)
 
     # -- progress ----------------------------------------------------------------------------
 
@@ -771,16 +716,16 @@ class B200Transport:
 
         self._note("pull decoded", message.transfer_id, message.sequence)
         keep = ()
-        if requests:
-            keep = tuple(self.backend.handoff(self.cache, self.peers[agent], translate, requests, pull=True,
-                                              before_launch=staged, **where))
-        elif timed is not None:
-            begun = timed()
-        self._note("pull tables launched", message.transfer_id, message.sequence)
         size = 0
-        if extra:
+        if not requests and timed is not None:
+            begun = timed()
+        if extra:  # first: the GPU copies these few bytes while the host prepares the launch that matters
             keep += tuple(self.backend.copy_ranges([(translate(s, n), d, n) for s, d, n in extra]))
             size += sum(n for _, _, n in extra)
+        if requests:
+            keep += tuple(self.backend.handoff(self.cache, self.peers[agent], translate, requests, pull=True,
+                                              before_launch=staged, **where))
+        self._note("pull tables launched", message.transfer_id, message.sequence)
         layers = (where["layer_end"] or self.info["num_layers"]) - where["layer_begin"]
         row = self.info["token_bytes"] + (self.info["scale_region"]["token_bytes"] if self.info["scale_region"] else 0)
         for _, target, start, end in requests:
@@ -796,6 +741,8 @@ class B200Transport:
         finished = []
         notifications = []
         for lane, agent in self._lane_agent.items():
+            if not self.mailbox.waiting(lane):
+                continue
             for message in self.mailbox.drain(lane):
                 if message.kind == LANDED:
                     self._note("landed seen", message.transfer_id, message.sequence)
