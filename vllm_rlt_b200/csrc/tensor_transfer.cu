@@ -151,33 +151,45 @@ int launch_inline(const int64_t* descriptors, int count, int max_rows, int max_c
                                : launch_inline<T, RLT_INLINE_TRANSFERS>(descriptors, count, grid, stream);
 }
 
-// Flat copy with conversion. When every pointer is 16-byte aligned a thread handles N consecutive elements per
-// step, N = 16 / (size of the widest of the three types): the widest side moves as one 16-byte access per thread
-// and the narrower sides as 8-, 4- or 2-byte accesses, all of them contiguous across the warp, with kFlatUnroll
-// steps in flight per thread. The last n % N elements, and unaligned tensors, go one element at a time.
-constexpr int kFlatUnroll = 4;
+// Flat copy with conversion. A thread handles N consecutive elements, N = 32 / (size of the widest of the three types): the
+// widest side moves as 32-byte accesses and the narrower sides as 16-, 8- or 4-byte ones, all of them contiguous across
+// the warp. A CTA does two such groups per thread, both loaded before either is stored, and the grid holds one CTA per
+// 16 KiB of the widest side, in order (block_moves.cu says why that is faster than a persistent loop). Elements before the
+// first place where every pointer is aligned to its N elements, and the last few, go one at a time; tensors with no such
+// place go so altogether. Bound by HBM, by L2 for what fits there. Measured, persistent kernel -> this one:
+// 128 Mi elements int64 -> int32 253 -> 233 us (6.9 TB/s), float16 -> int32 143 -> 121, bfloat16 -> float16 and int64 303 -> 242;
+// int32 -> int32 views that start one element past an aligned one 233 -> 159.
+constexpr int kFlatGroups = 2;
+constexpr int kFlatSingles = 8;  // elements per thread where nothing is aligned
 
 template <int kBytes>
 struct Bits;
+template <>
+struct Bits<32> { using type = Vec32; };
 template <>
 struct Bits<16> { using type = uint4; };
 template <>
 struct Bits<8> { using type = uint2; };
 template <>
 struct Bits<4> { using type = uint32_t; };
-template <>
-struct Bits<2> { using type = uint16_t; };
 
 template <typename T, int N>
 struct alignas(sizeof(T) * N) Pack {
   T v[N];
 };
 
+__device__ __forceinline__ void load_bits(const Vec32* p, Vec32* out) { *out = ld_stream(p); }
+__device__ __forceinline__ void store_bits(Vec32* p, const Vec32& v) { st_stream(p, v); }
+template <typename B>
+__device__ __forceinline__ void load_bits(const B* p, B* out) { *out = *p; }
+template <typename B>
+__device__ __forceinline__ void store_bits(B* p, const B& v) { *p = v; }
+
 template <typename T, int N>
 __device__ __forceinline__ Pack<T, N> load_pack(const T* p) {
   using B = typename Bits<sizeof(T) * N>::type;
   union { B bits; Pack<T, N> pack; } u;
-  u.bits = *reinterpret_cast<const B*>(p);
+  load_bits(reinterpret_cast<const B*>(p), &u.bits);
   return u.pack;
 }
 
@@ -186,50 +198,75 @@ __device__ __forceinline__ void store_pack(T* p, const Pack<T, N>& pack) {
   using B = typename Bits<sizeof(T) * N>::type;
   union { B bits; Pack<T, N> pack; } u;
   u.pack = pack;
-  *reinterpret_cast<B*>(p) = u.bits;
+  store_bits(reinterpret_cast<B*>(p), u.bits);
 }
 
 template <typename S, typename D, typename E>
+constexpr int flat_width() {
+  constexpr size_t pair = sizeof(S) > sizeof(D) ? sizeof(S) : sizeof(D);
+  return static_cast<int>(32 / (pair > sizeof(E) ? pair : sizeof(E)));
+}
+
+template <typename S, typename D, typename E>
+__device__ __forceinline__ void one_element(const S* __restrict__ src, D* __restrict__ dst, E* __restrict__ secondary, long long i) {
+  const S v = src[i];
+  dst[i] = Convert<D, S>::run(v);
+  if (secondary != nullptr) secondary[i] = Convert<E, S>::run(v);
+}
+
+// head: elements before the first aligned one, -1 if there is no such place.
+template <typename S, typename D, typename E>
 __global__ void __launch_bounds__(kTile) flat_transfer_kernel(const S* __restrict__ src, D* __restrict__ dst,
-                                                              E* __restrict__ secondary, long long n, int vector_ok) {
-  constexpr int kWidest = sizeof(S) > sizeof(D) ? (sizeof(S) > sizeof(E) ? sizeof(S) : sizeof(E))
-                                                : (sizeof(D) > sizeof(E) ? sizeof(D) : sizeof(E));
-  constexpr int N = 16 / kWidest;
-  const long long first = static_cast<long long>(blockIdx.x) * kTile + threadIdx.x;
-  const long long stride = static_cast<long long>(gridDim.x) * kTile;
-  long long done = 0;
-  if (vector_ok) {
-    const long long groups = n / N;
-    for (long long base = first; base < groups; base += stride * kFlatUnroll) {
-      Pack<S, N> in[kFlatUnroll];
+                                                              E* __restrict__ secondary, long long n, int head) {
+  constexpr int N = 32 / (sizeof(S) > sizeof(D) ? (sizeof(S) > sizeof(E) ? sizeof(S) : sizeof(E))
+                                                : (sizeof(D) > sizeof(E) ? sizeof(D) : sizeof(E)));
+  if (head < 0) {
+    const long long first = static_cast<long long>(blockIdx.x) * (kTile * kFlatSingles) + threadIdx.x;
 #pragma unroll
-      for (int u = 0; u < kFlatUnroll; ++u) {
-        const long long g = base + u * stride;
-        if (g < groups) in[u] = load_pack<S, N>(src + g * N);
-      }
-#pragma unroll
-      for (int u = 0; u < kFlatUnroll; ++u) {
-        const long long g = base + u * stride;
-        if (g >= groups) continue;
-        Pack<D, N> out;
-#pragma unroll
-        for (int k = 0; k < N; ++k) out.v[k] = Convert<D, S>::run(in[u].v[k]);
-        store_pack<D, N>(dst + g * N, out);
-        if (secondary != nullptr) {
-          Pack<E, N> second;
-#pragma unroll
-          for (int k = 0; k < N; ++k) second.v[k] = Convert<E, S>::run(in[u].v[k]);
-          store_pack<E, N>(secondary + g * N, second);
-        }
-      }
+    for (int k = 0; k < kFlatSingles; ++k) {
+      if (first + k * kTile < n) one_element(src, dst, secondary, first + k * kTile);
     }
-    done = groups * N;
+    return;
   }
-  for (long long i = done + first; i < n; i += stride) {
-    const S v = src[i];
-    dst[i] = Convert<D, S>::run(v);
-    if (secondary != nullptr) secondary[i] = Convert<E, S>::run(v);
+  const long long groups = (n - head) / N;
+  const long long first = static_cast<long long>(blockIdx.x) * (kTile * kFlatGroups) + threadIdx.x;
+  Pack<S, N> in[kFlatGroups];
+#pragma unroll
+  for (int u = 0; u < kFlatGroups; ++u) {
+    if (first + u * kTile < groups) in[u] = load_pack<S, N>(src + head + (first + u * kTile) * N);
   }
+#pragma unroll
+  for (int u = 0; u < kFlatGroups; ++u) {
+    const long long g = first + u * kTile;
+    if (g >= groups) continue;
+    Pack<D, N> out;
+#pragma unroll
+    for (int k = 0; k < N; ++k) out.v[k] = Convert<D, S>::run(in[u].v[k]);
+    store_pack<D, N>(dst + head + g * N, out);
+    if (secondary != nullptr) {
+      Pack<E, N> second;
+#pragma unroll
+      for (int k = 0; k < N; ++k) second.v[k] = Convert<E, S>::run(in[u].v[k]);
+      store_pack<E, N>(secondary + head + g * N, second);
+    }
+  }
+  if (blockIdx.x == 0) {  // both ends: fewer than 2 N elements
+    const long long tail = head + groups * N;
+    const long long i = threadIdx.x < head ? threadIdx.x : tail + (threadIdx.x - head);
+    if (i < n && (i < head || i >= tail)) one_element(src, dst, secondary, i);
+  }
+}
+
+// Elements to skip until src, dst and secondary are all aligned to `width` elements of theirs; -1 if that never happens.
+int aligned_head(const void* src, size_t src_size, const void* dst, size_t dst_size, const void* secondary, size_t secondary_size,
+                 int width, long long n) {
+  auto aligned = [&](const void* p, size_t size, int skip) {
+    return p == nullptr || (reinterpret_cast<uintptr_t>(p) + skip * size) % (size * width) == 0;
+  };
+  for (int skip = 0; skip < width && skip <= n; ++skip) {
+    if (aligned(src, src_size, skip) && aligned(dst, dst_size, skip) && aligned(secondary, secondary_size, skip)) return skip;
+  }
+  return -1;
 }
 
 template <typename S, typename D>
@@ -240,26 +277,30 @@ int launch_segmented(const long long* descriptors, int count, int max_rows, int 
   return RLT_OK;
 }
 
+template <typename S, typename D, typename E>
+int launch_flat_typed(const void* src, void* dst, void* secondary, long long n, cudaStream_t stream) {
+  constexpr int kWidth = flat_width<S, D, E>();
+  const int head = aligned_head(src, sizeof(S), dst, sizeof(D), secondary, sizeof(E), kWidth, n);
+  const long long per = head < 0 ? kTile * kFlatSingles : static_cast<long long>(kTile) * kFlatGroups * kWidth;
+  const long long grid = (n + per - 1) / per;
+  if (grid > 0x7fffffffll) return RLT_E_LIMIT;
+  flat_transfer_kernel<S, D, E><<<static_cast<unsigned>(grid), kTile, 0, stream>>>(static_cast<const S*>(src), static_cast<D*>(dst),
+                                                                                 static_cast<E*>(secondary), n, head);
+  return RLT_OK;
+}
+
 template <typename S, typename D>
-int launch_flat(const void* src, void* dst, void* secondary, long long n, int secondary_dtype, int grid,
-                cudaStream_t stream) {
-  const S* s = static_cast<const S*>(src);
-  D* d = static_cast<D*>(dst);
-  const int vec = ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst) |
-                    reinterpret_cast<uintptr_t>(secondary)) & 15u) == 0;
-  if (secondary == nullptr) {  // no second output: its type must not narrow the vector width
-    flat_transfer_kernel<S, D, D><<<grid, kTile, 0, stream>>>(s, d, static_cast<D*>(nullptr), n, vec);
-    return RLT_OK;
-  }
+int launch_flat(const void* src, void* dst, void* secondary, long long n, int secondary_dtype, cudaStream_t stream) {
+  // no second output: its type must not narrow the vector width
+  if (secondary == nullptr) return launch_flat_typed<S, D, D>(src, dst, nullptr, n, stream);
   switch (secondary_dtype) {
-    case RLT_DTYPE_I32: flat_transfer_kernel<S, D, int><<<grid, kTile, 0, stream>>>(s, d, static_cast<int*>(secondary), n, vec); break;
-    case RLT_DTYPE_I64: flat_transfer_kernel<S, D, long long><<<grid, kTile, 0, stream>>>(s, d, static_cast<long long*>(secondary), n, vec); break;
-    case RLT_DTYPE_F16: flat_transfer_kernel<S, D, __half><<<grid, kTile, 0, stream>>>(s, d, static_cast<__half*>(secondary), n, vec); break;
-    case RLT_DTYPE_BF16: flat_transfer_kernel<S, D, __nv_bfloat16><<<grid, kTile, 0, stream>>>(s, d, static_cast<__nv_bfloat16*>(secondary), n, vec); break;
-    case RLT_DTYPE_F32: flat_transfer_kernel<S, D, float><<<grid, kTile, 0, stream>>>(s, d, static_cast<float*>(secondary), n, vec); break;
+    case RLT_DTYPE_I32: return launch_flat_typed<S, D, int>(src, dst, secondary, n, stream);
+    case RLT_DTYPE_I64: return launch_flat_typed<S, D, long long>(src, dst, secondary, n, stream);
+    case RLT_DTYPE_F16: return launch_flat_typed<S, D, __half>(src, dst, secondary, n, stream);
+    case RLT_DTYPE_BF16: return launch_flat_typed<S, D, __nv_bfloat16>(src, dst, secondary, n, stream);
+    case RLT_DTYPE_F32: return launch_flat_typed<S, D, float>(src, dst, secondary, n, stream);
     default: return RLT_E_INVALID;
   }
-  return RLT_OK;
 }
 
 // Calls f.template operator()<S, D>() for the pair of type codes.
@@ -298,10 +339,10 @@ struct FlatCall {
   void* dst;
   void* secondary;
   long long n;
-  int secondary_dtype, grid;
+  int secondary_dtype;
   cudaStream_t stream;
   template <typename S, typename D>
-  int operator()() const { return launch_flat<S, D>(src, dst, secondary, n, secondary_dtype, grid, stream); }
+  int operator()() const { return launch_flat<S, D>(src, dst, secondary, n, secondary_dtype, stream); }
 };
 
 }  // namespace
@@ -346,14 +387,7 @@ int rlt_tensor_copy(const void* src, void* dst, void* secondary, int64_t count, 
                     int32_t secondary_dtype, rlt_stream_t stream) {
   if (count == 0) return RLT_OK;
   if (src == nullptr || dst == nullptr || count < 0) return RLT_E_INVALID;
-  int sms = 0;
-  const int rc0 = rlt::sm_count(&sms);
-  if (rc0 != RLT_OK) return rc0;
-  // a thread of the vector path covers kFlatUnroll groups of at least two elements per step
-  const long long per_block = static_cast<long long>(rlt::kTile) * 2 * rlt::kFlatUnroll;
-  const long long blocks = (count + per_block - 1) / per_block;
-  const int grid = static_cast<int>(blocks < sms * 8ll ? blocks : sms * 8ll);
-  const rlt::FlatCall call{src, dst, secondary, count, secondary_dtype, grid, reinterpret_cast<cudaStream_t>(stream)};
+  const rlt::FlatCall call{src, dst, secondary, count, secondary_dtype, reinterpret_cast<cudaStream_t>(stream)};
   const int rc = rlt::dispatch_pair(src_dtype, dst_dtype, call);
   if (rc != RLT_OK) return rc;
   RLT_CUDA_TRY(cudaGetLastError());
