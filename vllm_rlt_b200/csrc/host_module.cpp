@@ -9,10 +9,12 @@
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
+#include <ATen/core/LegacyTypeDispatch.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <cstddef>
 #include <cstring>
 #include <memory>
 #include <string>
@@ -593,80 +595,90 @@ struct Transfer {
   std::vector<int64_t> rows;  // 8 per copy
   int64_t max_rows = 0, max_cols = 0;
 };
-constexpr const char* kTransferName = "vllm_rlt_b200.transfer";
-void free_transfer(PyObject* capsule) { delete static_cast<Transfer*>(PyCapsule_GetPointer(capsule, kTransferName)); }
-Transfer& transfer_of(PyObject* capsule) {
-  auto* t = static_cast<Transfer*>(PyCapsule_GetPointer(capsule, kTransferName));
-  if (t == nullptr) throw Failure{};
-  return *t;
-}
 
-PyObject* transfer_new(PyObject* const*) {
-  auto* t = new Transfer;
-  PyObject* capsule = PyCapsule_New(t, kTransferName, free_transfer);
-  if (capsule == nullptr) {
-    delete t;
-    throw Failure{};
-  }
-  return capsule;
-}
+// Base of TensorTransfer: the batch itself. `append` runs once per copy, so it is a method of this type.
+struct CopiesObject {
+  PyObject_HEAD
+  Transfer* batch;
+  PyObject* copies;  // [(source, target)]: what a submitted batch borrows
+  long long capacity;
+  int from, to, device;
+};
+CopiesObject* copies_of(PyObject* o) { return reinterpret_cast<CopiesObject*>(o); }
 
-PyObject* transfer_reset(PyObject* const* a) {
-  Transfer& t = transfer_of(a[0]);
-  t.rows.clear();
-  t.max_rows = t.max_cols = 0;
+// setup(capacity, source type, target type, device index)
+PyObject* copies_setup(PyObject* self, PyObject* const* a) {
+  CopiesObject* c = copies_of(self);
+  c->capacity = integer(a[0]);
+  c->from = static_cast<int>(integer(a[1]));
+  c->to = static_cast<int>(integer(a[2]));
+  c->device = static_cast<int>(integer(a[3]));
   Py_RETURN_NONE;
 }
 
-// transfer_append(transfer, capacity, source type, target type, device index, source, target) -> whether there is anything to copy
-PyObject* transfer_append(PyObject* const* a) {
-  Transfer& t = transfer_of(a[0]);
-  const at::Tensor &source = some_tensor(a[5]), &target = some_tensor(a[6]);
+PyObject* copies_reset(PyObject* self, PyObject* const*) {
+  CopiesObject* c = copies_of(self);
+  PyObject* fresh = PyList_New(0);
+  if (fresh == nullptr) throw Failure{};
+  PyObject* old = c->copies;
+  c->copies = fresh;
+  c->batch->rows.clear();
+  c->batch->max_rows = c->batch->max_cols = 0;
+  Py_XDECREF(old);
+  Py_RETURN_NONE;
+}
+
+PyObject* copies_append(PyObject* self, PyObject* const* a) {
+  CopiesObject* c = copies_of(self);
+  Transfer& t = *c->batch;
+  const at::Tensor &source = some_tensor(a[0]), &target = some_tensor(a[1]);
   const int64_t dims = source.dim();
   if (source.sizes() != target.sizes() || (dims != 1 && dims != 2)) bad_value("transfer requires matching 1D/2D shapes");
-  if (transfer_type(source) != integer(a[2]) || transfer_type(target) != integer(a[3])) bad_value("transfer dtype does not match its batch");
-  const at::Device device(at::kCUDA, static_cast<c10::DeviceIndex>(integer(a[4])));
+  if (transfer_type(source) != c->from || transfer_type(target) != c->to) bad_value("transfer dtype does not match its batch");
+  const at::Device device(at::kCUDA, static_cast<c10::DeviceIndex>(c->device));
   if (target.device() != device) bad_value("transfer destination must be on the configured device");
   if (source.is_cuda() && source.device() != device) bad_value("transfer source must be on the configured device");
   check_source(source, device);
-  if (source.numel() == 0) Py_RETURN_FALSE;
-  if (static_cast<long long>(t.rows.size() / 8) >= integer(a[1])) bad_value("transfer batch is full");
+  if (source.numel() == 0) Py_RETURN_NONE;
+  if (static_cast<long long>(t.rows.size() / 8) >= c->capacity) bad_value("transfer batch is full");
   const bool flat = dims == 1;
   const int64_t rows = flat ? 1 : source.size(0), cols = source.size(dims - 1);
   const int64_t row[8] = {reinterpret_cast<int64_t>(source.data_ptr()), reinterpret_cast<int64_t>(target.data_ptr()), rows, cols,
                           flat ? cols * source.stride(0) : source.stride(0), source.stride(dims - 1),
                           flat ? cols * target.stride(0) : target.stride(0), target.stride(dims - 1)};
+  const Ref pair(PyTuple_Pack(2, a[0], a[1]));
+  if (PyList_Append(c->copies, pair.p) != 0) throw Failure{};
   t.rows.insert(t.rows.end(), row, row + 8);
   t.max_rows = rows > t.max_rows ? rows : t.max_rows;
   t.max_cols = cols > t.max_cols ? cols : t.max_cols;
-  Py_RETURN_TRUE;
+  Py_RETURN_NONE;
 }
 
-// transfer_extent(transfer) -> rows and columns that bound its copies
-PyObject* transfer_extent(PyObject* const* a) {
-  const Transfer& t = transfer_of(a[0]);
-  return Py_BuildValue("LL", static_cast<long long>(t.max_rows), static_cast<long long>(t.max_cols));
-}
-
-// transfer_submit(transfer, source type, target type, device index, pinned table) -> code. A small batch between tensors of one
-// type travels with its launch; others are written into the table, which the kernel reads where it lies.
-PyObject* transfer_submit(PyObject* const* a) {
-  const Transfer& t = transfer_of(a[0]);
-  const int from = static_cast<int>(integer(a[1])), to = static_cast<int>(integer(a[2]));
+// launch(pinned table) -> code. A small batch between tensors of one type travels with its launch; others are written into
+// the table, which the kernel reads where it lies.
+PyObject* copies_launch(PyObject* self, PyObject* const* a) {
+  const CopiesObject* c = copies_of(self);
+  const Transfer& t = *c->batch;
   const int count = static_cast<int>(t.rows.size() / 8);
   if (count == 0) return PyLong_FromLong(RLT_OK);
-  const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(integer(a[3])));
+  const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(c->device));
   const int32_t rows = static_cast<int32_t>(t.max_rows), cols = static_cast<int32_t>(t.max_cols);
-  if (from == to && count <= RLT_INLINE_TRANSFERS && t.max_cols <= INT32_MAX && t.max_rows <= INT32_MAX) {
-    const int rc = rlt_tensor_transfer_inline(t.rows.data(), count, rows, cols, from, stream_of(Py_None));
+  if (c->from == c->to && count <= RLT_INLINE_TRANSFERS && t.max_cols <= INT32_MAX && t.max_rows <= INT32_MAX) {
+    const int rc = rlt_tensor_transfer_inline(t.rows.data(), count, rows, cols, c->from, stream_of(Py_None));
     if (rc != RLT_E_LIMIT) return PyLong_FromLong(rc);
   }
-  const at::Tensor& table = some_tensor(a[4]);
+  const at::Tensor& table = some_tensor(a[0]);
   std::memcpy(table.data_ptr(), t.rows.data(), 8 * t.rows.size());
-  return PyLong_FromLong(rlt_tensor_transfer(table.data_ptr<int64_t>(), count, rows, cols, from, to, stream_of(Py_None)));
+  return PyLong_FromLong(rlt_tensor_transfer(table.data_ptr<int64_t>(), count, rows, cols, c->from, c->to, stream_of(Py_None)));
 }
 
 // ------------------------------------------------------------------------------------------------ staging helpers
+
+// t[start : start + n] of a flat tensor. These slices never take part in autograd, whose bookkeeping is skipped.
+at::Tensor plain_slice(const at::Tensor& t, int64_t start, int64_t n) {
+  const at::AutoDispatchBelowADInplaceOrView guard;
+  return t.narrow(0, start, n);
+}
 
 template <typename V, typename F>
 bool fill_from(PyObject** items, Py_ssize_t n, V* out, F convert) {
@@ -715,7 +727,7 @@ PyObject* fill(PyObject* const* a) {
     });
   }
   if (!ok) Py_RETURN_NONE;
-  return THPVariable_Wrap(t.narrow(0, start, n));
+  return THPVariable_Wrap(plain_slice(t, start, n));
 }
 
 // row_slice(tensor, index, start, count) -> tensor[index][start : start + count] for a 2-D tensor and an int in range; None otherwise
@@ -726,7 +738,53 @@ PyObject* row_slice(PyObject* const* a) {
   const int64_t start = integer(a[2]), n = integer(a[3]);
   index += index < 0 ? t.size(0) : 0;
   if (index < 0 || index >= t.size(0) || start < 0 || start + n > t.size(1)) Py_RETURN_NONE;
+  const at::AutoDispatchBelowADInplaceOrView guard;
   return THPVariable_Wrap(t.as_strided({n}, {t.stride(1)}, t.storage_offset() + index * t.stride(0) + start * t.stride(1)));
+}
+
+// Base of StagedInputTensor: `append` of plain numbers that fit; everything else is the subclass's `append_values`.
+struct FilledObject {
+  PyObject_HEAD
+  PyObject* cpu;
+  Py_ssize_t count;
+};
+
+PyObject* filled_append(PyObject* self, PyObject* const* a) {
+  auto* f = reinterpret_cast<FilledObject*>(self);
+  if (f->cpu != nullptr && f->cpu != Py_None) {
+    const Ref start(PyLong_FromSsize_t(f->count));
+    PyObject* args[3] = {f->cpu, start.p, a[0]};
+    PyObject* piece = fill(args);
+    if (piece != Py_None) {
+      if (piece != nullptr) f->count += PySequence_Fast_GET_SIZE(a[0]);
+      return piece;
+    }
+    Py_DECREF(piece);
+  }
+  return PyObject_CallMethod(self, "append_values", "O", a[0]);
+}
+
+// Base of StagedWriteTensor: `stage_write` of a list of numbers into one row of a 2-D tensor; else the subclass's `stage_values`.
+struct WritesObject {
+  PyObject_HEAD
+  PyObject *gpu, *values, *targets;
+};
+
+PyObject* writes_stage(PyObject* self, PyObject* const* a) {
+  auto* w = reinterpret_cast<WritesObject*>(self);
+  if (PyList_CheckExact(a[2]) && PyList_GET_SIZE(a[2]) > 0 && w->gpu != nullptr && w->gpu != Py_None && w->values != nullptr &&
+      w->targets != nullptr && PyList_CheckExact(w->values) && PyList_CheckExact(w->targets)) {
+    const Py_ssize_t n = PyList_GET_SIZE(a[2]);
+    const Ref count(PyLong_FromSsize_t(n));
+    PyObject* args[4] = {w->gpu, a[0], a[1], count.p};
+    const Ref target(row_slice(args));
+    if (target.p != Py_None) {
+      const Py_ssize_t end = PyList_GET_SIZE(w->values);
+      if (PyList_SetSlice(w->values, end, end, a[2]) != 0 || PyList_Append(w->targets, target.p) != 0) throw Failure{};
+      Py_RETURN_NONE;
+    }
+  }
+  return PyObject_CallMethod(self, "stage_values", "OOO", a[0], a[1], a[2]);
 }
 
 // pieces(flat tensor, [targets]) -> consecutive slices of it, as long as the targets
@@ -739,7 +797,7 @@ PyObject* pieces(PyObject* const* a) {
   int64_t at = 0;
   for (Py_ssize_t i = 0; i < n; ++i) {
     const int64_t count = some_tensor(PySequence_Fast_GET_ITEM(targets.p, i)).size(0);
-    PyList_SET_ITEM(out, i, THPVariable_Wrap(t.narrow(0, at, count)));
+    PyList_SET_ITEM(out, i, THPVariable_Wrap(plain_slice(t, at, count)));
     at += count;
   }
   return out;
@@ -994,19 +1052,155 @@ PyMethodDef kMethods[] = {
     RLT_ENTRY("push", push, 5),
     RLT_ENTRY("post", post, 5),
     RLT_ENTRY("tensor_copy", tensor_copy, 3),
-    RLT_ENTRY("transfer_new", transfer_new, 0),
-    RLT_ENTRY("transfer_reset", transfer_reset, 1),
-    RLT_ENTRY("transfer_append", transfer_append, 7),
-    RLT_ENTRY("transfer_extent", transfer_extent, 1),
-    RLT_ENTRY("transfer_submit", transfer_submit, 5),
     RLT_ENTRY("fill", fill, 3),
     RLT_ENTRY("row_slice", row_slice, 4),
     RLT_ENTRY("pieces", pieces, 2),
     {nullptr, nullptr, 0, nullptr},
 };
 
+// ------------------------------------------------------------------------------------------------ types
+
+template <PyObject* (*kMethod)(PyObject*, PyObject* const*), int kArgs>
+PyObject* method(PyObject* self, PyObject* const* args, Py_ssize_t n) {
+  if (n != kArgs) {
+    PyErr_Format(PyExc_TypeError, "expected %d arguments, got %zd", kArgs, n);
+    return nullptr;
+  }
+  try {
+    return kMethod(self, args);
+  } catch (const Failure&) {
+    return nullptr;
+  } catch (const std::exception& e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what());
+    return nullptr;
+  }
+}
+#define RLT_METHOD(name, function, args) \
+  {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(&method<function, args>)), METH_FASTCALL, nullptr}
+
+// The same for methods whose arguments may be given by name. kNames: the parameters in order.
+template <PyObject* (*kMethod)(PyObject*, PyObject* const*), int kArgs, const char* const* kNames>
+PyObject* named_method(PyObject* self, PyObject* const* args, Py_ssize_t n, PyObject* names) {
+  const Py_ssize_t named = names == nullptr ? 0 : PyTuple_GET_SIZE(names);
+  if (named == 0) return method<kMethod, kArgs>(self, args, n);
+  PyObject* all[kArgs] = {};
+  for (Py_ssize_t i = 0; i < n && i < kArgs; ++i) all[i] = args[i];
+  for (Py_ssize_t k = 0; k < named; ++k) {
+    int at = 0;
+    while (at < kArgs && PyUnicode_CompareWithASCIIString(PyTuple_GET_ITEM(names, k), kNames[at]) != 0) ++at;
+    if (at == kArgs || all[at] != nullptr) {
+      PyErr_Format(PyExc_TypeError, "unexpected argument %R", PyTuple_GET_ITEM(names, k));
+      return nullptr;
+    }
+    all[at] = args[n + k];
+  }
+  return method<kMethod, kArgs>(self, all, n + named);
+}
+#define RLT_NAMED_METHOD(name, function, args, names)                                                                    \
+  {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(&named_method<function, args, names>)),           \
+   METH_FASTCALL | METH_KEYWORDS, nullptr}
+constexpr const char* kAppendNames[] = {"source", "target"};
+constexpr const char* kValuesNames[] = {"values"};
+constexpr const char* kWriteNames[] = {"index", "start", "values"};
+
+// The object fields of a type, for the collector: their offsets.
+template <size_t... kOffsets>
+struct Fields {
+  static PyObject*& at(PyObject* self, size_t offset) { return *reinterpret_cast<PyObject**>(reinterpret_cast<char*>(self) + offset); }
+  static int traverse(PyObject* self, visitproc visit, void* arg) {
+    Py_VISIT(Py_TYPE(self));
+    for (size_t offset : {kOffsets...}) Py_VISIT(at(self, offset));
+    return 0;
+  }
+  static int clear(PyObject* self) {
+    for (size_t offset : {kOffsets...}) Py_CLEAR(at(self, offset));
+    return 0;
+  }
+  static void dealloc(PyObject* self) {
+    PyTypeObject* type = Py_TYPE(self);
+    PyObject_GC_UnTrack(self);
+    clear(self);
+    reinterpret_cast<freefunc>(PyType_GetSlot(type, Py_tp_free))(self);
+    Py_DECREF(type);
+  }
+};
+
+using CopiesFields = Fields<offsetof(CopiesObject, copies)>;
+void copies_dealloc(PyObject* self) {
+  delete copies_of(self)->batch;
+  copies_of(self)->batch = nullptr;
+  CopiesFields::dealloc(self);
+}
+PyObject* copies_new(PyTypeObject* type, PyObject*, PyObject*) {
+  PyObject* self = type->tp_alloc(type, 0);
+  if (self == nullptr) return nullptr;
+  copies_of(self)->batch = new Transfer;
+  copies_of(self)->copies = PyList_New(0);
+  return self;
+}
+PyObject* copies_max_rows(PyObject* self, void*) { return PyLong_FromLongLong(copies_of(self)->batch->max_rows); }
+PyObject* copies_max_cols(PyObject* self, void*) { return PyLong_FromLongLong(copies_of(self)->batch->max_cols); }
+
+PyMethodDef kCopiesMethods[] = {RLT_METHOD("setup", copies_setup, 4), RLT_METHOD("reset", copies_reset, 0),
+                                RLT_NAMED_METHOD("append", copies_append, 2, kAppendNames), RLT_METHOD("launch", copies_launch, 1),
+                                {nullptr, nullptr, 0, nullptr}};
+PyMemberDef kCopiesMembers[] = {{"copies", Py_T_OBJECT_EX, offsetof(CopiesObject, copies), Py_READONLY, nullptr},
+                                {"capacity", Py_T_LONGLONG, offsetof(CopiesObject, capacity), Py_READONLY, nullptr},
+                                {nullptr, 0, 0, 0, nullptr}};
+PyGetSetDef kCopiesProperties[] = {{"max_rows", copies_max_rows, nullptr, nullptr, nullptr},
+                                   {"max_cols", copies_max_cols, nullptr, nullptr, nullptr},
+                                   {nullptr, nullptr, nullptr, nullptr, nullptr}};
+PyType_Slot kCopiesSlots[] = {{Py_tp_new, reinterpret_cast<void*>(copies_new)},
+                              {Py_tp_dealloc, reinterpret_cast<void*>(copies_dealloc)},
+                              {Py_tp_traverse, reinterpret_cast<void*>(CopiesFields::traverse)},
+                              {Py_tp_clear, reinterpret_cast<void*>(CopiesFields::clear)},
+                              {Py_tp_methods, kCopiesMethods},
+                              {Py_tp_members, kCopiesMembers},
+                              {Py_tp_getset, kCopiesProperties},
+                              {0, nullptr}};
+
+using FilledFields = Fields<offsetof(FilledObject, cpu)>;
+PyMethodDef kFilledMethods[] = {RLT_NAMED_METHOD("append", filled_append, 1, kValuesNames), {nullptr, nullptr, 0, nullptr}};
+PyMemberDef kFilledMembers[] = {{"cpu", Py_T_OBJECT_EX, offsetof(FilledObject, cpu), 0, nullptr},
+                                {"count", Py_T_PYSSIZET, offsetof(FilledObject, count), 0, nullptr},
+                                {nullptr, 0, 0, 0, nullptr}};
+PyType_Slot kFilledSlots[] = {{Py_tp_new, reinterpret_cast<void*>(PyType_GenericNew)},
+                              {Py_tp_dealloc, reinterpret_cast<void*>(FilledFields::dealloc)},
+                              {Py_tp_traverse, reinterpret_cast<void*>(FilledFields::traverse)},
+                              {Py_tp_clear, reinterpret_cast<void*>(FilledFields::clear)},
+                              {Py_tp_methods, kFilledMethods},
+                              {Py_tp_members, kFilledMembers},
+                              {0, nullptr}};
+
+using WritesFields = Fields<offsetof(WritesObject, gpu), offsetof(WritesObject, values), offsetof(WritesObject, targets)>;
+PyMethodDef kWritesMethods[] = {RLT_NAMED_METHOD("stage_write", writes_stage, 3, kWriteNames), {nullptr, nullptr, 0, nullptr}};
+PyMemberDef kWritesMembers[] = {{"gpu", Py_T_OBJECT_EX, offsetof(WritesObject, gpu), 0, nullptr},
+                                {"values", Py_T_OBJECT_EX, offsetof(WritesObject, values), 0, nullptr},
+                                {"targets", Py_T_OBJECT_EX, offsetof(WritesObject, targets), 0, nullptr},
+                                {nullptr, 0, 0, 0, nullptr}};
+PyType_Slot kWritesSlots[] = {{Py_tp_new, reinterpret_cast<void*>(PyType_GenericNew)},
+                              {Py_tp_dealloc, reinterpret_cast<void*>(WritesFields::dealloc)},
+                              {Py_tp_traverse, reinterpret_cast<void*>(WritesFields::traverse)},
+                              {Py_tp_clear, reinterpret_cast<void*>(WritesFields::clear)},
+                              {Py_tp_methods, kWritesMethods},
+                              {Py_tp_members, kWritesMembers},
+                              {0, nullptr}};
+
+constexpr unsigned kTypeFlags = Py_TPFLAGS_DEFAULT | Py_TPFLAGS_BASETYPE | Py_TPFLAGS_HAVE_GC;
+PyType_Spec kTypes[] = {{"_host.Copies", sizeof(CopiesObject), 0, kTypeFlags, kCopiesSlots},
+                        {"_host.Filled", sizeof(FilledObject), 0, kTypeFlags, kFilledSlots},
+                        {"_host.Writes", sizeof(WritesObject), 0, kTypeFlags, kWritesSlots}};
+
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__host(void) { return PyModule_Create(&kModule); }
+PyMODINIT_FUNC PyInit__host(void) {
+  PyObject* module = PyModule_Create(&kModule);
+  if (module == nullptr) return nullptr;
+  for (PyType_Spec& spec : kTypes) {
+    PyObject* type = PyType_FromSpec(&spec);
+    if (type == nullptr || PyModule_AddObject(module, spec.name + sizeof("_host.") - 1, type) != 0) return nullptr;
+  }
+  return module;
+}

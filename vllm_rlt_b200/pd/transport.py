@@ -622,13 +622,17 @@ class B200Transport:
             self.inflight_bytes += size
         return True
 
-    def _order_after(self, event):
-        """Queue what follows behind ``event`` on the transfer stream; returns an event that fires when the
-        transfer stream has got past that wait, i.e. when this submission's own work begins."""
+    def _wait_for(self, event) -> None:
+        """Queue what follows behind ``event`` on the transfer stream."""
         if event is not None:
             if not self.device_ordered:
                 raise ValueError("this backend cannot wait for an event on the device; submit once it has fired")
             self.backend.order_after(event)
+
+    def _order_after(self, event):
+        """``_wait_for``; returns an event that fires when the transfer stream has got past that wait, i.e. when this
+        submission's own work begins."""
+        self._wait_for(event)
         return self.backend.marker()
 
     def submit(self, transfer_id, sequence, peer, local, remote, size, *, after=None):
@@ -693,8 +697,9 @@ class B200Transport:
         first = parts[0][0]
         body = Mailbox.encode(transfer_id, first, OFFER, (at, len(raw)), count=len(parts))
         box.write_descriptor(link["lane"], at, raw)
-        started = self._order_after(after)  # the offer leaves when the producer's event has fired
+        self._wait_for(after)  # the offer leaves when the producer's event has fired
         self._post(link, body)
+        started = self.backend.marker()
         self._note("offer queued", transfer_id, first)
         handle = self._offered[(link["agent"], transfer_id, first)] = _RemoteCompletion()
         return self._tickets(handle, transfer_id, parts, (), started)
@@ -717,15 +722,15 @@ class B200Transport:
         self._note("pull decoded", message.transfer_id, message.sequence)
         keep = ()
         size = 0
-        if not requests and timed is not None:
-            begun = timed()
-        if extra:  # first: the GPU copies these few bytes while the host prepares the launch that matters
-            keep += tuple(self.backend.copy_ranges([(translate(s, n), d, n) for s, d, n in extra]))
-            size += sum(n for _, _, n in extra)
         if requests:
             keep += tuple(self.backend.handoff(self.cache, self.peers[agent], translate, requests, pull=True,
                                               before_launch=staged, **where))
+        elif timed is not None:
+            begun = timed()
         self._note("pull tables launched", message.transfer_id, message.sequence)
+        if extra:
+            keep += tuple(self.backend.copy_ranges([(translate(s, n), d, n) for s, d, n in extra]))
+            size += sum(n for _, _, n in extra)
         layers = (where["layer_end"] or self.info["num_layers"]) - where["layer_begin"]
         row = self.info["token_bytes"] + (self.info["scale_region"]["token_bytes"] if self.info["scale_region"] else 0)
         for _, target, start, end in requests:

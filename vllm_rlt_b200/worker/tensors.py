@@ -23,10 +23,11 @@ def copy_tensor(source: torch.Tensor, target: torch.Tensor, *, secondary: torch.
     return target
 
 
-class TensorTransfer:
+class TensorTransfer(_lib.load_host().Copies):
     """One typed batch of disjoint 1-D/2-D copies with borrowed tensor references.
 
-    ``append`` records a copy, ``submit`` launches the whole batch as one kernel, ``reset`` forgets it.
+    ``append(source, target)`` records a copy in ``copies``, ``submit`` launches the whole batch as one kernel, ``reset``
+    forgets it (``append`` and ``reset`` are the compiled base's, which holds the descriptors).
     The descriptors of a batch of up to 448 copies between tensors of one type are parameters of the launch; others are
     written into a pinned table that the kernel reads through its device mapping. Either way a submission needs no
     separate host-to-device copy. The table and the tensors of a submitted batch must stay untouched until the work
@@ -40,31 +41,9 @@ class TensorTransfer:
         self.device = torch.device(device)
         if self.device.type != "cuda":
             raise ValueError("transfer destination must be a CUDA device")
-        self._index = -1 if self.device.index is None else self.device.index  # no tensor is on a device without index
-        self.capacity = capacity
         self.table = torch.zeros((capacity, 8), dtype=torch.int64, pin_memory=True)
-        host = _lib.load_host()
-        self._rows = host.transfer_new()
-        self._append, self._submit, self._reset = host.transfer_append, host.transfer_submit, host.transfer_reset
-        self._types = _DTYPES[self.dtype], _DTYPES[self.target_dtype]
-        self.reset()
-
-    def reset(self) -> None:
-        self.copies: list[tuple[torch.Tensor, torch.Tensor]] = []
-        self._reset(self._rows)
-
-    def append(self, source: torch.Tensor, target: torch.Tensor) -> None:
-        if self._append(self._rows, self.capacity, *self._types, self._index, source, target):
-            self.copies.append((source, target))
+        # no tensor is on a device without index
+        self.setup(capacity, _DTYPES[self.dtype], _DTYPES[self.target_dtype], -1 if self.device.index is None else self.device.index)
 
     def submit(self) -> None:
-        if self.copies:
-            _lib.check(self._submit(self._rows, *self._types, self._index, self.table), "rlt_tensor_transfer")
-
-    @property
-    def max_rows(self) -> int:
-        return _lib.load_host().transfer_extent(self._rows)[0]
-
-    @property
-    def max_cols(self) -> int:
-        return _lib.load_host().transfer_extent(self._rows)[1]
+        _lib.check(self.launch(self.table), "rlt_tensor_transfer")
