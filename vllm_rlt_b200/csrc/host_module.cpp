@@ -875,6 +875,50 @@ PyObject* encode_chunk(PyObject* const* a) {
   return PyBytes_FromStringAndSize(out.data(), static_cast<Py_ssize_t>(out.size()));
 }
 
+// Records of an all-planes handoff, page by page, and their launch.
+struct RequestRecords {
+  const RltPool *src, *dst;
+  std::vector<int32_t> records;
+  int words;
+  int64_t requests = 0, before = 0, blocks = 0, width = 1;
+  RequestRecords(const RltPool* s, const RltPool* d) : src(s), dst(d), words(kRecordHeader + s->num_planes + d->num_planes) {}
+  bool fits(int64_t pages) const { return (blocks + pages) * words * 4 <= (1 << 20) && requests < RLT_MAX_REQUESTS; }
+  bool valid(const int32_t* ids, int64_t n, const RltPool* pool) const {
+    bool ok = true;
+    for (int64_t i = 0; i < n; ++i) ok &= static_cast<uint32_t>(ids[i]) < static_cast<uint32_t>(pool->num_blocks);
+    return ok;
+  }
+  // ids: [planes of both sides][stride], the range's first page at column `first_column`
+  void add(const int32_t* ids, int64_t stride, int64_t first_column, int64_t first_page, int64_t pages, int64_t start, int64_t end) {
+    const int64_t bs = src->block_size;
+    const int planes = src->num_planes + dst->num_planes;
+    records.reserve(records.size() + static_cast<size_t>(pages * words));
+    for (int64_t k = 0; k < pages; ++k) {
+      const int64_t base = (first_page + k) * bs;
+      const int64_t lo = start > base ? start - base : 0, hi = end < base + bs ? end - base : bs;
+      const int32_t head[kRecordHeader] = {static_cast<int32_t>(requests), static_cast<int32_t>(first_page + k), static_cast<int32_t>(lo | hi << 8),
+                                           static_cast<int32_t>(base + lo - start), static_cast<int32_t>(before), static_cast<int32_t>(end - start)};
+      records.insert(records.end(), head, head + kRecordHeader);
+      for (int p = 0; p < planes; ++p) records.push_back(ids[p * stride + first_column + k]);
+    }
+    ++requests;
+    blocks += pages;
+    before += end - start;
+  }
+  int launch(const RltOptions& o, rlt_stream_t stream) const {
+    RltBlockMoves m = {};
+    m.host_records = records.data();
+    m.blocks = static_cast<int32_t>(blocks);
+    m.words = words;
+    m.src_planes = src->num_planes;
+    m.dst_planes = dst->num_planes;
+    m.block_size = src->block_size;
+    m.num_requests = static_cast<int32_t>(requests);
+    m.table_width = static_cast<int32_t>(width);
+    return rlt_handoff_staged(src, dst, &m, &o, stream);
+  }
+};
+
 // handoff_requests(source pool, destination pool, requests, layer_begin, layer_end, plane_begin, plane_end, device, stream) -> code of an
 // all-planes handoff of [(source tables, target tables, start, end)], or RLT_MOVE_UNSUITED (nothing queued) when something about the
 // requests looks wrong or their records do not fit the library's own staging: the general path then does it, or says what is wrong.
@@ -884,66 +928,151 @@ PyObject* handoff_requests(PyObject* const* a) {
   const Ref requests(PySequence_Fast(a[2], "requests must be a sequence"));
   const int64_t bs = src->block_size;
   const Py_ssize_t n = PySequence_Fast_GET_SIZE(requests.p);
-  PyObject* unsuited = PyLong_FromLong(RLT_MOVE_UNSUITED);
-  if (n < 1 || n > RLT_MAX_REQUESTS || bs < 1) return unsuited;
-  std::vector<int32_t> records, ids;
-  const int words = kRecordHeader + src->num_planes + dst->num_planes;
-  int64_t before = 0, blocks = 0, width = 1;
+  auto unsuited = [] { return PyLong_FromLong(RLT_MOVE_UNSUITED); };
+  if (n < 1 || bs < 1) return unsuited();
+  RequestRecords out(src, dst);
+  std::vector<int32_t> ids;
   for (Py_ssize_t r = 0; r < n; ++r) {
     const Ref request(PySequence_Fast(PySequence_Fast_GET_ITEM(requests.p, r), "a request is (source, target, start, end)"));
-    if (PySequence_Fast_GET_SIZE(request.p) < 4) return unsuited;
+    if (PySequence_Fast_GET_SIZE(request.p) < 4) return unsuited();
     const int64_t start = integer(PySequence_Fast_GET_ITEM(request.p, 2)), end = integer(PySequence_Fast_GET_ITEM(request.p, 3));
-    if (start < 0 || start >= end) return unsuited;
+    if (start < 0 || start >= end) return unsuited();
     const int64_t first = start / bs, pages = (end - 1) / bs - first + 1;
-    if ((blocks + pages) * words * 4 > (1 << 20)) return unsuited;
+    if (!out.fits(pages)) return unsuited();
     ids.clear();
     for (int side = 0; side < 2; ++side) {
       const RltPool* pool = side == 0 ? src : dst;
       const Ref tables(PySequence_Fast(PySequence_Fast_GET_ITEM(request.p, side), "block tables must be a sequence"));
-      if (PySequence_Fast_GET_SIZE(tables.p) != pool->num_planes) return unsuited;
+      if (PySequence_Fast_GET_SIZE(tables.p) != pool->num_planes) return unsuited();
       Py_ssize_t of_request = -1;
+      const size_t at = ids.size();
       for (int p = 0; p < pool->num_planes; ++p) {
         PyObject* table = PySequence_Fast_GET_ITEM(tables.p, p);
         const Py_ssize_t held = length(table);
-        if (held < first + pages || (of_request >= 0 && held != of_request)) return unsuited;
+        if (held < first + pages || (of_request >= 0 && held != of_request)) return unsuited();
         of_request = held;
-        width = held > width ? held : width;
-        const size_t at = ids.size();
+        out.width = held > out.width ? held : out.width;
         append_range(table, first, first + pages, ids);
-        for (size_t i = at; i < ids.size(); ++i) {
-          if (static_cast<uint32_t>(ids[i]) >= static_cast<uint32_t>(pool->num_blocks)) return unsuited;
-        }
       }
+      if (!out.valid(ids.data() + at, static_cast<int64_t>(ids.size() - at), pool)) return unsuited();
     }
-    const int planes = src->num_planes + dst->num_planes;
-    for (int64_t k = 0; k < pages; ++k) {
-      const int64_t base = (first + k) * bs;
-      const int64_t lo = start > base ? start - base : 0, hi = end < base + bs ? end - base : bs;
-      const int32_t head[kRecordHeader] = {static_cast<int32_t>(r), static_cast<int32_t>(first + k), static_cast<int32_t>(lo | hi << 8),
-                                           static_cast<int32_t>(base + lo - start), static_cast<int32_t>(before), static_cast<int32_t>(end - start)};
-      records.insert(records.end(), head, head + kRecordHeader);
-      for (int p = 0; p < planes; ++p) records.push_back(ids[static_cast<size_t>(p) * pages + k]);
-    }
-    blocks += pages;
-    before += end - start;
+    out.add(ids.data(), pages, 0, first, pages, start, end);
   }
-  Py_DECREF(unsuited);
   RltOptions o = {};
   o.layer_begin = static_cast<int32_t>(integer(a[3]));
   o.layer_end = static_cast<int32_t>(integer(a[4]));
   o.plane_begin = static_cast<int32_t>(integer(a[5]));
   o.plane_end = static_cast<int32_t>(integer(a[6]));
-  RltBlockMoves m = {};
-  m.host_records = records.data();
-  m.blocks = static_cast<int32_t>(blocks);
-  m.words = words;
-  m.src_planes = src->num_planes;
-  m.dst_planes = dst->num_planes;
-  m.block_size = static_cast<int32_t>(bs);
-  m.num_requests = static_cast<int32_t>(n);
-  m.table_width = static_cast<int32_t>(width);
   const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(integer(a[7])));
-  return PyLong_FromLong(rlt_handoff_staged(src, dst, &m, &o, stream_of(a[8])));
+  return PyLong_FromLong(out.launch(o, stream_of(a[8])));
+}
+
+// A recorded event of the library's pool.
+struct EventObject {
+  PyObject_HEAD
+  RltEvent* event;
+};
+PyTypeObject* g_event_type = nullptr;
+
+void check_code(int code) {
+  if (code < 0) fail(PyExc_RuntimeError, rlt_error_string(code));
+}
+
+PyObject* record_event(bool timed, rlt_stream_t stream) {
+  RltEvent* event = nullptr;
+  check_code(rlt_event_record(timed, stream, &event));
+  auto* o = PyObject_New(EventObject, g_event_type);
+  if (o == nullptr) {
+    rlt_event_release(event);
+    throw Failure{};
+  }
+  o->event = event;
+  return reinterpret_cast<PyObject*>(o);
+}
+
+// event(timed, device, stream) -> an event recorded there
+PyObject* event(PyObject* const* a) {
+  const bool timed = PyObject_IsTrue(a[0]) == 1;
+  const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(integer(a[1])));
+  return record_event(timed, stream_of(a[2]));
+}
+
+template <typename V>
+bool take(const char*& at, const char* end, V* out) {
+  if (end - at < static_cast<ptrdiff_t>(sizeof(V))) return false;
+  std::memcpy(out, at, sizeof(V));
+  at += sizeof(V);
+  return true;
+}
+
+// pull_chunk(source pool, destination pool, descriptor, spans, device, stream) -> (begun, done, bytes): the launches that a chunk's
+// descriptor (encode_chunk) asks for, between two timing events; None (nothing queued) where handoff_requests would not do.
+PyObject* pull_chunk(PyObject* const* a) {
+  const auto* src = static_cast<const RltPool*>(address(a[0]));
+  const auto* dst = static_cast<const RltPool*>(address(a[1]));
+  char* raw = nullptr;
+  Py_ssize_t size = 0;
+  if (PyBytes_AsStringAndSize(a[2], &raw, &size) != 0) throw Failure{};
+  const char *at = raw, *end = raw + size;
+  uint32_t head[8];
+  if (!take(at, end, &head) || head[2] != RLT_MODE_ALL_PLANES || head[0] == 0) Py_RETURN_NONE;
+  const int64_t bs = src->block_size;
+  RequestRecords out(src, dst);
+  std::vector<int32_t> ids;
+  for (uint32_t r = 0; r < head[0]; ++r) {
+    uint32_t planes[2], columns;
+    int64_t range[2];
+    if (!take(at, end, &planes) || !take(at, end, &range) || !take(at, end, &columns)) Py_RETURN_NONE;
+    if (planes[0] != static_cast<uint32_t>(src->num_planes) || planes[1] != static_cast<uint32_t>(dst->num_planes) || range[0] < 0 ||
+        range[0] >= range[1])
+      Py_RETURN_NONE;
+    const int64_t first = range[0] / bs, pages = (range[1] - 1) / bs - first + 1;
+    const size_t count = static_cast<size_t>(planes[0] + planes[1]) * columns;
+    if (first + pages > columns || !out.fits(pages) || end - at < static_cast<ptrdiff_t>(4 * count)) Py_RETURN_NONE;
+    ids.resize(count);
+    std::memcpy(ids.data(), at, 4 * count);
+    at += 4 * count;
+    const size_t split = static_cast<size_t>(planes[0]) * columns;
+    if (!out.valid(ids.data(), static_cast<int64_t>(split), src) || !out.valid(ids.data() + split, static_cast<int64_t>(count - split), dst))
+      Py_RETURN_NONE;
+    out.width = columns > out.width ? columns : out.width;
+    out.add(ids.data(), columns, first, first, pages, range[0], range[1]);
+  }
+  std::vector<int64_t> extra(3 * static_cast<size_t>(head[1]));
+  if (end - at < static_cast<ptrdiff_t>(8 * extra.size())) Py_RETURN_NONE;
+  if (!extra.empty()) std::memcpy(extra.data(), at, 8 * extra.size());
+  if (!extra.empty()) {
+    const Ref spans(PySequence_Fast(a[3], "spans must be a sequence"));
+    for (size_t i = 0; i < extra.size(); i += 3) {
+      bool found = false;
+      for (Py_ssize_t k = 0; k < PySequence_Fast_GET_SIZE(spans.p) && !found; ++k) {
+        const Ref s(PySequence_Fast(PySequence_Fast_GET_ITEM(spans.p, k), "a span is (low, high, base)"));
+        const int64_t lo = integer(PySequence_Fast_GET_ITEM(s.p, 0)), hi = integer(PySequence_Fast_GET_ITEM(s.p, 1));
+        found = lo <= extra[i] && extra[i] + extra[i + 2] <= hi;
+        if (found) extra[i] += integer(PySequence_Fast_GET_ITEM(s.p, 2)) - lo;
+      }
+      if (!found) Py_RETURN_NONE;
+    }
+  }
+  RltOptions o = {};
+  o.layer_begin = static_cast<int32_t>(head[3]);
+  o.layer_end = static_cast<int32_t>(head[4]);
+  o.plane_begin = static_cast<int32_t>(head[5]);
+  o.plane_end = static_cast<int32_t>(head[6]);
+  const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(integer(a[4])));
+  const rlt_stream_t stream = stream_of(a[5]);
+  const Ref begun(record_event(true, stream));
+  const int code = out.launch(o, stream);
+  if (code == RLT_MOVE_UNSUITED) Py_RETURN_NONE;
+  if (code != RLT_OK) return PyLong_FromLong(code);
+  const int64_t layers = (head[4] ? head[4] : src->num_layers) - head[3], planes = (head[6] ? head[6] : dst->num_planes) - head[5];
+  int64_t bytes = out.before * planes * 2 * layers * (src->codes.token_bytes + (src->scales.key != nullptr ? src->scales.token_bytes : 0));
+  for (size_t i = 0; i < extra.size(); i += 3) {
+    check_code(rlt_kv_push(reinterpret_cast<void*>(extra[i]), reinterpret_cast<void*>(extra[i + 1]), extra[i + 2], stream));
+    bytes += extra[i + 2];
+  }
+  const Ref done(record_event(true, stream));
+  return Py_BuildValue("OOL", begun.p, done.p, static_cast<long long>(bytes));
 }
 
 // pack_segments([(address, bytes, device)], [(address, bytes, device)], [(low, high, base)]) -> the (source, destination, bytes)
@@ -1047,6 +1176,8 @@ PyMethodDef kMethods[] = {
     RLT_ENTRY("finalize", finalize, 7),
     RLT_ENTRY("encode_chunk", encode_chunk, 8),
     RLT_ENTRY("handoff_requests", handoff_requests, 9),
+    RLT_ENTRY("event", event, 3),
+    RLT_ENTRY("pull_chunk", pull_chunk, 6),
     RLT_ENTRY("pack_segments", pack_segments, 3),
     RLT_ENTRY("copy_segments", copy_segments, 3),
     RLT_ENTRY("push", push, 5),
@@ -1186,6 +1317,36 @@ PyType_Slot kWritesSlots[] = {{Py_tp_new, reinterpret_cast<void*>(PyType_Generic
                               {Py_tp_members, kWritesMembers},
                               {0, nullptr}};
 
+PyObject* event_query(PyObject* self, PyObject* const*) {
+  const int fired = rlt_event_query(reinterpret_cast<EventObject*>(self)->event);
+  check_code(fired);
+  return PyBool_FromLong(fired);
+}
+PyObject* event_synchronize(PyObject* self, PyObject* const*) {
+  int code = RLT_OK;
+  Py_BEGIN_ALLOW_THREADS;
+  code = rlt_event_wait(reinterpret_cast<EventObject*>(self)->event);
+  Py_END_ALLOW_THREADS;
+  check_code(code);
+  Py_RETURN_NONE;
+}
+PyObject* event_elapsed_time(PyObject* self, PyObject* const* a) {
+  if (Py_TYPE(a[0]) != g_event_type) fail(PyExc_TypeError, "expected an event");
+  float ms = 0.0f;
+  check_code(rlt_event_elapsed(reinterpret_cast<EventObject*>(self)->event, reinterpret_cast<EventObject*>(a[0])->event, &ms));
+  return PyFloat_FromDouble(ms);
+}
+void event_dealloc(PyObject* self) {
+  PyTypeObject* type = Py_TYPE(self);
+  rlt_event_release(reinterpret_cast<EventObject*>(self)->event);
+  PyObject_Free(self);
+  Py_DECREF(type);
+}
+PyMethodDef kEventMethods[] = {RLT_METHOD("query", event_query, 0), RLT_METHOD("synchronize", event_synchronize, 0),
+                               RLT_METHOD("elapsed_time", event_elapsed_time, 1), {nullptr, nullptr, 0, nullptr}};
+PyType_Slot kEventSlots[] = {{Py_tp_dealloc, reinterpret_cast<void*>(event_dealloc)}, {Py_tp_methods, kEventMethods}, {0, nullptr}};
+PyType_Spec kEventType = {"_host.Event", sizeof(EventObject), 0, Py_TPFLAGS_DEFAULT | Py_TPFLAGS_DISALLOW_INSTANTIATION, kEventSlots};
+
 constexpr unsigned kTypeFlags = Py_TPFLAGS_DEFAULT | Py_TPFLAGS_BASETYPE | Py_TPFLAGS_HAVE_GC;
 PyType_Spec kTypes[] = {{"_host.Copies", sizeof(CopiesObject), 0, kTypeFlags, kCopiesSlots},
                         {"_host.Filled", sizeof(FilledObject), 0, kTypeFlags, kFilledSlots},
@@ -1198,6 +1359,8 @@ PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, kMethods, nu
 PyMODINIT_FUNC PyInit__host(void) {
   PyObject* module = PyModule_Create(&kModule);
   if (module == nullptr) return nullptr;
+  g_event_type = reinterpret_cast<PyTypeObject*>(PyType_FromSpec(&kEventType));
+  if (g_event_type == nullptr) return nullptr;
   for (PyType_Spec& spec : kTypes) {
     PyObject* type = PyType_FromSpec(&spec);
     if (type == nullptr || PyModule_AddObject(module, spec.name + sizeof("_host.") - 1, type) != 0) return nullptr;

@@ -1,4 +1,4 @@
-// Pinned staging for host arrays on their way to the device.
+// What a call needs for a moment and the library keeps: pinned staging for host arrays on their way to the device, and events.
 //
 // Page-locked memory costs a driver call to get, so buffers are kept: per device and power-of-two size at most kKept of
 // them (eight of 1 MiB and more, two of 16 MiB and more), each free again when the copy that last read it has finished. When all of a size
@@ -67,8 +67,70 @@ int acquire(size_t bytes, Pinned** out) {
   return RLT_OK;
 }
 
+constexpr size_t kPooledEvents = 256;  // per device and kind; more than that are destroyed when given back
+std::mutex g_event_mutex;
+std::vector<cudaEvent_t> g_events[kMaxDevices][2];
+
 }  // namespace
 }  // namespace rlt
+
+struct RltEvent {
+  cudaEvent_t event;
+  int device, timed;
+};
+
+extern "C" int rlt_event_record(int timed, rlt_stream_t stream, RltEvent** out) {
+  int device = 0;
+  RLT_CUDA_TRY(cudaGetDevice(&device));
+  if (device < 0 || device >= rlt::kMaxDevices) return RLT_E_LIMIT;
+  cudaEvent_t event = nullptr;
+  {
+    const std::lock_guard<std::mutex> lock(rlt::g_event_mutex);
+    auto& pool = rlt::g_events[device][timed != 0];
+    if (!pool.empty()) {
+      event = pool.back();
+      pool.pop_back();
+    }
+  }
+  if (event == nullptr) RLT_CUDA_TRY(cudaEventCreateWithFlags(&event, timed ? cudaEventDefault : cudaEventDisableTiming));
+  if (const cudaError_t e = cudaEventRecord(event, reinterpret_cast<cudaStream_t>(stream)); e != cudaSuccess) {
+    cudaEventDestroy(event);
+    return rlt::cuda_fail(e);
+  }
+  *out = new RltEvent{event, device, timed != 0};
+  return RLT_OK;
+}
+
+extern "C" int rlt_event_query(RltEvent* event) {
+  const cudaError_t e = cudaEventQuery(event->event);
+  if (e == cudaSuccess) return 1;
+  if (e != cudaErrorNotReady) return rlt::cuda_fail(e);
+  cudaGetLastError();  // "not ready" is an answer, not an error to leave behind
+  return 0;
+}
+
+extern "C" int rlt_event_wait(RltEvent* event) {
+  RLT_CUDA_TRY(cudaEventSynchronize(event->event));
+  return RLT_OK;
+}
+
+extern "C" int rlt_event_elapsed(RltEvent* from, RltEvent* to, float* milliseconds) {
+  RLT_CUDA_TRY(cudaEventElapsedTime(milliseconds, from->event, to->event));
+  return RLT_OK;
+}
+
+extern "C" void rlt_event_release(RltEvent* event) {
+  {
+    const std::lock_guard<std::mutex> lock(rlt::g_event_mutex);
+    auto& pool = rlt::g_events[event->device][event->timed];
+    if (pool.size() < rlt::kPooledEvents) {
+      pool.push_back(event->event);
+      event->event = nullptr;
+    }
+  }
+  if (event->event != nullptr) cudaEventDestroy(event->event);
+  delete event;
+}
 
 extern "C" int rlt_stage_upload(const void* host, size_t bytes, void* device, rlt_stream_t stream) {
   if (bytes == 0) return RLT_OK;

@@ -24,6 +24,15 @@ RLT_API int rlt_tensor_transfer_inline(const int64_t* descriptors, int32_t count
 #define RLT_INLINE_SEGMENTS 1024
 RLT_API int rlt_copy_segments_inline(const int64_t* triples, int32_t count, rlt_stream_t stream);
 
+// Events of the current device that outlive the objects using them: taken from a pool, recorded on `stream`, given back. An
+// event that is given back before it has fired may be recorded again at once: nobody looks at it any more.
+typedef struct RltEvent RltEvent;
+RLT_API int rlt_event_record(int timed, rlt_stream_t stream, RltEvent** out);
+RLT_API int rlt_event_query(RltEvent* event);  // 1: fired, 0: not yet, negative: RLT_E_*
+RLT_API int rlt_event_wait(RltEvent* event);   // on the host
+RLT_API int rlt_event_elapsed(RltEvent* from, RltEvent* to, float* milliseconds);
+RLT_API void rlt_event_release(RltEvent* event);
+
 #ifdef __cplusplus
 }
 #endif

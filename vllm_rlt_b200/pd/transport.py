@@ -377,19 +377,13 @@ class CudaBackend:
             _lib.check(self._host.push(src, dst, n, *self._where), "rlt_kv_push")
         return ()
 
-    def handoff(self, cache, peer_info, translate, requests, *, mode=0, layer_begin=0, layer_end=0,
-                plane_begin=0, plane_end=0, exit_planes=None, status=None, pull=False, before_launch=None):
-        """One table-driven launch for ``requests`` = [(source tables, target tables, start, end), ...], optionally
-        of one slice of layers and destination planes (0, 0 = all).
-
-        Push: the local pool is the source and the peer's pool, behind translated pointers, the destination.
-        ``pull=True``: the peer's pool is the source and the local pool the destination (plain peer loads)."""
-        from ..kernels import kv_handoff as kh
-
-        # the two pool views of a (peer, direction, plane count) never change: build them once
-        key = (peer_info["agent"], pull, mode == kh.MODE_EXIT_ONLY)
+    def _views_of(self, cache, peer_info, translate, pull, exit_only):
+        """The (source, destination) pool views of a peer, a direction and a plane count: they never change."""
+        key = (peer_info["agent"], pull, exit_only)
         views = self._views.get(key)
         if views is None:
+            from ..kernels import kv_handoff as kh
+
             mine = kh.PoolView.from_cache(cache)
             codes = mine.codes.rebased(translate(peer_info["key_ptr"], 1), translate(peer_info["value_ptr"], 1))
             scales = None
@@ -399,16 +393,27 @@ class CudaBackend:
             if pull:
                 theirs = kh.PoolView(codes, scales, peer_info["num_blocks"], peer_info["block_size"], peer_info["num_layers"],
                                      peer_info["depths"], peer_info["device"])
-                if mode == kh.MODE_EXIT_ONLY and mine.num_planes != 1:
+                if exit_only and mine.num_planes != 1:
                     raise ValueError("an exit-only pull needs a single-plane destination pool")
                 views = (theirs, mine)
             else:
-                planes = 1 if mode == kh.MODE_EXIT_ONLY else peer_info["depths"]
+                planes = 1 if exit_only else peer_info["depths"]
                 theirs = kh.PoolView(codes, scales, peer_info["num_blocks"], peer_info["block_size"], peer_info["num_layers"],
                                      planes, peer_info["device"])
                 views = (mine, theirs)
             self._views[key] = views
-        src, dst = views
+        return views
+
+    def handoff(self, cache, peer_info, translate, requests, *, mode=0, layer_begin=0, layer_end=0,
+                plane_begin=0, plane_end=0, exit_planes=None, status=None, pull=False, before_launch=None):
+        """One table-driven launch for ``requests`` = [(source tables, target tables, start, end), ...], optionally
+        of one slice of layers and destination planes (0, 0 = all).
+
+        Push: the local pool is the source and the peer's pool, behind translated pointers, the destination.
+        ``pull=True``: the peer's pool is the source and the local pool the destination (plain peer loads)."""
+        from ..kernels import kv_handoff as kh
+
+        src, dst = self._views_of(cache, peer_info, translate, pull, mode == kh.MODE_EXIT_ONLY)
         if exit_planes is None and status is None and mode == kh.MODE_ALL_PLANES:
             if before_launch is not None:
                 before_launch()
@@ -432,17 +437,19 @@ class CudaBackend:
         _lib.check(self._host.post(slot_ptr, body, stamp, *self._where), "rlt_kv_post")
 
     def event(self):
-        ev = self.torch.cuda.Event()
-        ev.record(self.stream)
-        return ev
+        return self._host.event(False, *self._where)
 
     marker = event  # an event at the current end of the transfer stream, used to tell when queued work begins
 
     def timed_event(self):
         """Like ``event`` but usable with ``elapsed_time`` (device time between two of them)."""
-        ev = self.torch.cuda.Event(enable_timing=True)
-        ev.record(self.stream)
-        return ev
+        return self._host.event(True, *self._where)
+
+    def pull_chunk(self, cache, peer_info, translate, raw: bytes):
+        """What a chunk's descriptor asks for, queued by one compiled call: ``(begun, done, bytes)`` with timing events on
+        either side; None where the general path must do it or say what is wrong."""
+        src, dst = self._views_of(cache, peer_info, translate, True, False)
+        return self._host.pull_chunk(src._address(), dst._address(), raw, translate.spans, *self._where)
 
     def close(self):
         boxes, self._mailboxes = self._mailboxes, {}
@@ -708,9 +715,16 @@ class B200Transport:
 
     def _begin_pull(self, agent: str, message: Message) -> None:
         """Run the launch an offer describes, on this worker's transfer stream, reading the peer's pool."""
+        translate = self._peer_link(agent)["translate"]
+        at_once = None if self._trace_dir else getattr(self.backend, "pull_chunk", None)
+        queued = at_once(self.cache, self.peers[agent], translate, message.descriptor) if at_once is not None else None
+        if queued is not None:
+            if type(queued) is int:
+                _lib.check(queued, "rlt_kv_handoff")
+            begun, done, size = queued
+            self._pulls.append(_Pull(done, agent, message.transfer_id, message.sequence, size, count=message.count, begun=begun))
+            return
         requests, extra, where = decode_chunk(message.descriptor)
-        link = self._peer_link(agent)
-        translate = link["translate"]
         timed = getattr(self.backend, "timed_event", None)
         begun = None
 
