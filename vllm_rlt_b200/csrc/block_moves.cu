@@ -472,6 +472,7 @@ __global__ void __launch_bounds__(kThreads, loops_planes(K) ? 3 : 6) move_kernel
   w.kv = at >= static_cast<unsigned>(rg.pieces);
   w.index = static_cast<int>(at) - w.kv * rg.pieces;
   w.rec = records + static_cast<long long>(page) * p.words;
+  follow_stream();
   const int range = w.rec[2];
   if ((K == kDedupToWire || K == kDedupFromWire) && blockIdx.x == 0 && threadIdx.x == 0) {
     p.wire_header[0] = p.wire_tokens;
@@ -499,7 +500,7 @@ __global__ void __launch_bounds__(kThreads, loops_planes(K) ? 3 : 6) move_kernel
 }
 
 template <MoveKind K, int kWords>
-void launch_move(const MoveParams& p, const RltBlockMoves& m, unsigned grid, cudaStream_t stream) {
+cudaError_t launch_move(const MoveParams& p, const RltBlockMoves& m, unsigned grid, cudaStream_t stream) {
   MoveArgs<kWords> args;
   args.p = p;
   if (kWords > 1) {
@@ -508,7 +509,7 @@ void launch_move(const MoveParams& p, const RltBlockMoves& m, unsigned grid, cud
     if (m.host_wire != nullptr)
       std::memcpy(args.inline_words + n, m.host_wire, static_cast<size_t>(m.blocks) * p.src_planes * sizeof(int));
   }
-  move_kernel<K, kWords><<<grid, kThreads, 0, stream>>>(args);
+  return launch_following(move_kernel<K, kWords>, grid, kThreads, stream, args);
 }
 
 template <MoveKind K>
@@ -517,17 +518,19 @@ int launch_kind(const MoveParams& p, const RltBlockMoves& m, unsigned grid, cuda
   // A parameter block is copied into the launch whole (a launch takes the host 2.4 us with 2 KiB, 3.6 with 8 and 6.6 with 32; a
   // copy of the records, the launch and an event 4.5, and the GPU 6 us more), so three sizes of it: the small one covers a few
   // hundred tokens, the medium one a thousand.
+  cudaError_t launched;
   if (n <= kInlineSmallWords) {
-    launch_move<K, kInlineSmallWords>(p, m, grid, stream);
+    launched = launch_move<K, kInlineSmallWords>(p, m, grid, stream);
   } else if (n <= kInlineMediumWords) {
-    launch_move<K, kInlineMediumWords>(p, m, grid, stream);
+    launched = launch_move<K, kInlineMediumWords>(p, m, grid, stream);
   } else if (n <= kInlineWords) {
-    launch_move<K, kInlineWords>(p, m, grid, stream);
+    launched = launch_move<K, kInlineWords>(p, m, grid, stream);
   } else if (p.records != nullptr && (m.host_wire == nullptr || p.wire != nullptr)) {
-    launch_move<K, 1>(p, m, grid, stream);
+    launched = launch_move<K, 1>(p, m, grid, stream);
   } else {
     return RLT_E_INVALID;
   }
+  RLT_CUDA_TRY(launched);
   return RLT_OK;
 }
 
@@ -664,7 +667,6 @@ extern "C" int rlt_move_blocks(int direction, const RltPool* src, const RltPool*
     case kDedupFromWire: rc = launch_kind<kDedupFromWire>(p, *m, ctas, s); break;
   }
   if (rc != RLT_OK) return rc;
-  RLT_CUDA_TRY(cudaGetLastError());
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return RLT_OK;
 }

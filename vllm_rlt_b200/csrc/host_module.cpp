@@ -1184,7 +1184,6 @@ PyMethodDef kMethods[] = {
     RLT_ENTRY("post", post, 5),
     RLT_ENTRY("tensor_copy", tensor_copy, 3),
     RLT_ENTRY("fill", fill, 3),
-    RLT_ENTRY("row_slice", row_slice, 4),
     RLT_ENTRY("pieces", pieces, 2),
     {nullptr, nullptr, 0, nullptr},
 };

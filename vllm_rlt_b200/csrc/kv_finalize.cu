@@ -158,6 +158,7 @@ __global__ void __launch_bounds__(kThreads, 5) finalize_kernel(const __grid_cons
   __shared__ GroupShared s;
   const int group = static_cast<int>(blockIdx.x / p.parts);
   int at = static_cast<int>(blockIdx.x) - group * p.parts;
+  follow_stream();
   list_rows(p, group, at == 0, s);
   const int g = at >= 2 * p.region[0].parts;
   const FinalizeRegion& rg = p.region[g];
@@ -255,8 +256,8 @@ int rlt_kv_finalize(const RltPool* pool, const int32_t* tables, int32_t num_requ
   }
   const long long grid = groups * p.parts;
   if (grid > 0x7fffffffll) return RLT_E_LIMIT;
-  rlt::finalize_kernel<<<static_cast<unsigned>(grid), rlt::kThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(p);
-  RLT_CUDA_TRY(cudaGetLastError());
+  RLT_CUDA_TRY(rlt::launch_following(rlt::finalize_kernel, static_cast<unsigned>(grid), rlt::kThreads,
+                                     reinterpret_cast<cudaStream_t>(stream), p));
   rlt::g_launches.fetch_add(1, std::memory_order_relaxed);
   return RLT_OK;
 }

@@ -75,6 +75,7 @@ __device__ __forceinline__ void copy_piece(const char* src, char* dst, long long
 
 __global__ void __launch_bounds__(kThreads, 6) push_kernel(const char* src, char* dst, long long nbytes) {
   const long long at = static_cast<long long>(blockIdx.x) * kShortTile;
+  follow_stream();
   copy_piece<true>(src + at, dst + at, min(kShortTile, nbytes - at));
 }
 
@@ -100,6 +101,7 @@ __global__ void __launch_bounds__(kThreads, 6) inline_segments_kernel(const __gr
   }
   const Segment s = list.segment[lo];
   const long long at = static_cast<long long>(t - list.first_tile[lo]) * kShortTile;
+  follow_stream();
   copy_piece<true>(s.src + at, s.dst + at, min(kShortTile, s.bytes - at));
 }
 
@@ -117,8 +119,7 @@ int launch_inline(const int64_t* triples, int count, cudaStream_t stream) {
   }
   if (list.count == 0) return RLT_OK;
   list.first_tile[list.count] = static_cast<int>(tiles);
-  inline_segments_kernel<kCount><<<static_cast<unsigned>(tiles), kThreads, 0, stream>>>(list);
-  RLT_CUDA_TRY(cudaGetLastError());
+  RLT_CUDA_TRY(launch_following(inline_segments_kernel<kCount>, static_cast<unsigned>(tiles), kThreads, stream, list));
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return RLT_OK;
 }
@@ -175,9 +176,8 @@ int rlt_kv_push(const void* src, void* dst, int64_t nbytes, rlt_stream_t stream)
   if (src == nullptr || dst == nullptr || nbytes < 0) return RLT_E_INVALID;
   const long long tiles = (nbytes + rlt::kShortTile - 1) / rlt::kShortTile;
   if (tiles > 0x7fffffffll) return RLT_E_LIMIT;
-  rlt::push_kernel<<<static_cast<unsigned>(tiles), rlt::kThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      static_cast<const char*>(src), static_cast<char*>(dst), nbytes);
-  RLT_CUDA_TRY(cudaGetLastError());
+  RLT_CUDA_TRY(rlt::launch_following(rlt::push_kernel, static_cast<unsigned>(tiles), rlt::kThreads, reinterpret_cast<cudaStream_t>(stream),
+                                     static_cast<const char*>(src), static_cast<char*>(dst), static_cast<long long>(nbytes)));
   rlt::g_launches.fetch_add(1, std::memory_order_relaxed);
   return RLT_OK;
 }

@@ -220,6 +220,7 @@ __global__ void __launch_bounds__(kTile) flat_transfer_kernel(const S* __restric
                                                               E* __restrict__ secondary, long long n, int head) {
   constexpr int N = 32 / (sizeof(S) > sizeof(D) ? (sizeof(S) > sizeof(E) ? sizeof(S) : sizeof(E))
                                                 : (sizeof(D) > sizeof(E) ? sizeof(D) : sizeof(E)));
+  follow_stream();
   if (head < 0) {
     const long long first = static_cast<long long>(blockIdx.x) * (kTile * kFlatSingles) + threadIdx.x;
 #pragma unroll
@@ -284,8 +285,8 @@ int launch_flat_typed(const void* src, void* dst, void* secondary, long long n, 
   const long long per = head < 0 ? kTile * kFlatSingles : static_cast<long long>(kTile) * kFlatGroups * kWidth;
   const long long grid = (n + per - 1) / per;
   if (grid > 0x7fffffffll) return RLT_E_LIMIT;
-  flat_transfer_kernel<S, D, E><<<static_cast<unsigned>(grid), kTile, 0, stream>>>(static_cast<const S*>(src), static_cast<D*>(dst),
-                                                                                 static_cast<E*>(secondary), n, head);
+  RLT_CUDA_TRY(launch_following(flat_transfer_kernel<S, D, E>, static_cast<unsigned>(grid), kTile, stream, static_cast<const S*>(src),
+                                static_cast<D*>(dst), static_cast<E*>(secondary), n, head));
   return RLT_OK;
 }
 
