@@ -47,12 +47,12 @@ int sm_count(int* out);
 // stream has completed and is visible, and then lets the next such launch be set up behind this one. Saves most of the gap
 // between two short kernels; kernels launched the ordinary way, copies and events are ordered as ever.
 template <typename... P, typename... A>
-inline cudaError_t launch_following(void (*kernel)(P...), unsigned grid, unsigned block, cudaStream_t stream, const A&... args) {
+inline cudaError_t launch_following(void (*kernel)(P...), dim3 grid, unsigned block, cudaStream_t stream, const A&... args) {
   cudaLaunchAttribute attribute = {};
   attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attribute.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t config = {};
-  config.gridDim = dim3(grid);
+  config.gridDim = grid;
   config.blockDim = dim3(block);
   config.stream = stream;
   config.attrs = &attribute;

@@ -10,15 +10,15 @@
 // tensors: each row of every selected layer is loaded once and stored to every deeper plane.
 //
 // Work decomposition. kGroupRows consecutive rows of the batch form a group; they are usually consecutive tokens of one
-// request, so that the copies of one layer on one plane are neighbours in one block. The CTAs of a group share out
-// the vectors (selected layer, row, vector of the row) of one of its tensors in equal parts, rows that need no copy left
-// out. The grid holds one short CTA per part, in order of the groups: bound by HBM, the kernel is fastest while the
-// SMs work close together (block_moves.cu has the measurements), and a decode step of a few rows still reaches every SM.
-// A CTA's own preparation is two rounds of lookups: the rows, then the blocks of their planes.
+// request, so that the copies of one layer on one plane are neighbours in one block. A thread takes one vector of the group's
+// (selected layer, row, vector of the row) for one of its tensors, looks its row and its blocks up itself (the threads of a warp
+// mostly the same ones, so the lookups hit L1) and stores the vector to every deeper plane. The grid holds one CTA per 8 KiB
+// in that order: HBM is fastest while the SMs work close together (block_moves.cu has the measurements), and a decode step of
+// a few rows still reaches every SM. Nothing is shared inside a CTA: lists of rows and blocks in shared memory, with two
+// barriers before the first load, cost 7.4 us where this takes 6.2 (64 rows of four planes), 275 where it takes 271 (4,000 rows).
+// Measured before that, with persistent CTAs that scanned all rows' costs first: 12.6 and 324 us.
 //
 // HBM roofline: each selected (layer, tensor) row is read once and written once per deeper plane.
-
-#include <algorithm>
 
 #include "common.cuh"
 
@@ -41,6 +41,8 @@ struct FinalizeParams {
   int planes, block_size, num_blocks, num_layers;
   unsigned long long layer_mask;  // bit l set: layer l is copied (the recurrent layers)
   int layers;                     // bits set in layer_mask
+  int plane_chunk;                // planes one CTA stores to
+  int dense_layers;               // the selected layers are 0 .. layers - 1
   const int* tables;              // [requests, planes, table_width]
   int table_width, num_requests;
   const int* rows;                // [n][3]: request index, exit plane, token position
@@ -49,139 +51,91 @@ struct FinalizeParams {
 };
 
 constexpr int kGroupRows = 16;
-constexpr int kPlaneChunk = 64;  // planes whose blocks are looked up together
 
-struct GroupShared {
-  int layer_of[64];                               // the selected layers, in order
-  int carried;                                    // rows of the group with something to copy; the lists below hold those
-  int request[kGroupRows], page[kGroupRows], exit_plane[kGroupRows], token[kGroupRows];
-  long long src[kGroupRows];                      // byte offset of the exit plane's block, -1 if its id is bad
-  long long dst[kGroupRows][kPlaneChunk];         // the same for the planes of the chunk; -1 also where nothing is due
-};
-
-// The rows of the group that need copies, compacted by warp 0. An invalid row is reported by the group's first CTA.
-__device__ __forceinline__ void list_rows(const FinalizeParams& p, int group, bool say, GroupShared& s) {
-  const int tid = static_cast<int>(threadIdx.x);
-  if (tid < 64 && ((p.layer_mask >> tid) & 1ull)) s.layer_of[__popcll(p.layer_mask & ((1ull << tid) - 1ull))] = tid;
-  if (tid >= 32) return;
-  const long long row = static_cast<long long>(group) * kGroupRows + tid;
-  int request = -1, e = 0, position = 0;
-  bool carry = false;
-  if (tid < kGroupRows && row < p.n) {
-    request = p.rows[3 * row];
-    e = p.rows[3 * row + 1];
-    position = p.rows[3 * row + 2];
-    const bool valid = request >= 0 && request < p.num_requests && e >= 0 && e < p.planes && position >= 0 &&
-                       position < p.table_width * p.block_size;
-    if (!valid && say) report(p.status, RLT_STATUS_BAD_PLANE, static_cast<int>(row), position, e);
-    carry = valid && e + 1 < p.planes;
-  }
-  const unsigned keep = __ballot_sync(0xffffffffu, carry);
-  if (carry) {
-    const int slot = __popc(keep & ((1u << tid) - 1u));
-    s.request[slot] = request;
-    s.exit_plane[slot] = e;
-    s.page[slot] = position / p.block_size;
-    s.token[slot] = position % p.block_size;
-  }
-  if (tid == 0) s.carried = __popc(keep);
-}
-
-// The share of a group's vectors that one CTA copies: vectors [first, first + count) in the order layer, listed row,
-// vector of the row; the first lies `rem` vectors into line `line`, a line being one row of one layer.
-struct Share {
-  int first, count, line, rem, lines;
-};
-__device__ __forceinline__ Share share_of(const FinalizeParams& p, const FinalizeRegion& rg, int part, int carried) {
-  const long long all = static_cast<long long>(p.layers) * carried * rg.row_vecs;
-  Share h;
-  h.first = static_cast<int>(all * part / rg.parts);
-  h.count = static_cast<int>(all * (part + 1) / rg.parts) - h.first;
-  h.line = h.first / rg.row_vecs;
-  h.rem = h.first - h.line * rg.row_vecs;
-  h.lines = (h.rem + h.count + rg.row_vecs - 1) / rg.row_vecs;
-  return h;
-}
-
-// Blocks of planes [chunk, chunk + kPlaneChunk) of the listed rows that the share touches, and of their exit planes.
-__device__ __forceinline__ void look_up_blocks(const FinalizeParams& p, const FinalizeRegion& rg, const Share& h, int chunk,
-                                               GroupShared& s) {
-  const int width = min(kPlaneChunk, p.planes - chunk) + 1;  // the last column is the exit plane
-  const int n = s.carried, touched = min(h.lines, n), from = h.line % n;
-  for (int i = static_cast<int>(threadIdx.x); i < touched * width; i += kThreads) {
-    const int i_row = i / width, column = i - i_row * width;
-    const int r = from + i_row < n ? from + i_row : from + i_row - n;
-    const bool source = column == width - 1;
-    const int e = s.exit_plane[r], plane = source ? e : chunk + column;
-    long long at = -1;
-    if (source || plane > e) {
-      const int block = p.tables[(static_cast<long long>(s.request[r]) * p.planes + plane) * p.table_width + s.page[r]];
-      if (static_cast<unsigned>(block) < static_cast<unsigned>(p.num_blocks)) {
-        at = block * rg.block_bytes;
-      } else {
-        report(p.status, RLT_STATUS_BAD_BLOCK, s.request[r], s.page[r], block);
-      }
-    }
-    if (source) {
-      s.src[r] = at;
-    } else {
-      s.dst[r][column] = at;
-    }
-  }
-}
-
+// Vectors per thread: one of 32 or 16 bytes, more of the narrow ones.
 template <typename T>
-__device__ __forceinline__ void copy_share(const FinalizeParams& p, const FinalizeRegion& rg, char* pool, const Share& h, int chunk,
-                                           const GroupShared& s) {
-  const int n = s.carried;
-  const unsigned n_magic = n == 1 ? 0u : static_cast<unsigned>((1ull << 32) / static_cast<unsigned>(n)) + 1u;
-  const int chunk_planes = min(kPlaneChunk, p.planes - chunk);
-  for (int k = static_cast<int>(threadIdx.x); k < h.count; k += kThreads) {
-    const unsigned j = static_cast<unsigned>(h.rem + k);
-    const int q = rg.row_magic ? static_cast<int>(__umulhi(j, rg.row_magic)) : static_cast<int>(j);
-    const int line = h.line + q;
-    const int layer = n_magic ? static_cast<int>(__umulhi(static_cast<unsigned>(line), n_magic)) : line;
-    const int row = line - layer * n;
-    const long long src = s.src[row];
-    if (src < 0) continue;
-    char* at = pool + s.layer_of[layer] * rg.layer_bytes + s.token[row] * rg.token_bytes +
-               (static_cast<int>(j) - q * rg.row_vecs) * static_cast<int>(sizeof(T));
-    const T v = ld_stream(reinterpret_cast<const T*>(at + src));
-    for (int c = max(s.exit_plane[row] + 1 - chunk, 0); c < chunk_planes; ++c) {
-      const long long to = s.dst[row][c];
-      if (to >= 0) st_stream(reinterpret_cast<T*>(at + to), v);
+__host__ __device__ constexpr int vectors_of() {
+  return sizeof(T) >= 16 ? 1 : sizeof(T) == 4 ? 4 : 8;
+}
+
+// Position of the k-th (0-based) set bit.
+__device__ __forceinline__ int nth_set_bit(unsigned long long mask, int k) {
+  const unsigned lo = static_cast<unsigned>(mask), hi = static_cast<unsigned>(mask >> 32);
+  const int in_lo = __popc(lo);
+  return k < in_lo ? static_cast<int>(__fns(lo, 0, k + 1)) : 32 + static_cast<int>(__fns(hi, 0, k - in_lo + 1));
+}
+
+// Vector `k` of the part that begins at vector `first` of the group, to every deeper plane. `say`: this CTA reports invalid rows.
+template <typename T, bool kChunked>
+__device__ __forceinline__ void fill_deeper(const FinalizeParams& p, const FinalizeRegion& rg, int group, int kv, int first, int k, bool say) {
+  if (first + k >= p.layers * kGroupRows * rg.row_vecs) return;
+  const int row0 = first / rg.row_vecs;
+  const unsigned j = static_cast<unsigned>(first - row0 * rg.row_vecs + k);
+  const int q = rg.row_magic ? static_cast<int>(__umulhi(j, rg.row_magic)) : static_cast<int>(j);
+  const int slot = (row0 + q) / kGroupRows;
+  const int row = group * kGroupRows + (row0 + q) % kGroupRows;
+  if (row >= p.n) return;
+  const int request = p.rows[3 * row], e = p.rows[3 * row + 1], position = p.rows[3 * row + 2];
+  if (request < 0 || request >= p.num_requests || e < 0 || e >= p.planes || position < 0 || position >= p.table_width * p.block_size) {
+    if (say && slot == 0) report(p.status, RLT_STATUS_BAD_PLANE, row, position, e);
+    return;
+  }
+  // the deeper planes of this CTA's chunk (all of them, unless the launch is small)
+  const int from = kChunked ? max(e + 1, static_cast<int>(blockIdx.y) * p.plane_chunk) : e + 1;
+  const int to = kChunked ? min(p.planes, (static_cast<int>(blockIdx.y) + 1) * p.plane_chunk) : p.planes;
+  if (from >= to) return;
+  const int page = position / p.block_size;
+  const int* table = p.tables + static_cast<long long>(request) * p.planes * p.table_width + page;
+  const int source = table[static_cast<long long>(e) * p.table_width];
+  if (static_cast<unsigned>(source) >= static_cast<unsigned>(p.num_blocks)) {
+    report(p.status, RLT_STATUS_BAD_BLOCK, request, page, source);
+    return;
+  }
+  const int layer = p.dense_layers ? slot : nth_set_bit(p.layer_mask, slot);
+  char* at = (kv ? rg.value : rg.key) + layer * rg.layer_bytes + (position - page * p.block_size) * rg.token_bytes +
+             (static_cast<int>(j) - q * rg.row_vecs) * static_cast<int>(sizeof(T));
+  const T v = ld_stream(reinterpret_cast<const T*>(at + source * rg.block_bytes));
+  for (int t = from; t < to; ++t) {
+    const int block = table[static_cast<long long>(t) * p.table_width];
+    if (static_cast<unsigned>(block) < static_cast<unsigned>(p.num_blocks)) {
+      st_stream(reinterpret_cast<T*>(at + block * rg.block_bytes), v);
+    } else {
+      report(p.status, RLT_STATUS_BAD_BLOCK, request, page, block);
     }
   }
 }
 
-__global__ void __launch_bounds__(kThreads, 5) finalize_kernel(const __grid_constant__ FinalizeParams p) {
-  __shared__ GroupShared s;
+template <typename T, bool kChunked>
+__device__ __forceinline__ void copy_part(const FinalizeParams& p, const FinalizeRegion& rg, int group, int kv, int part, bool say) {
+  constexpr int kPer = kThreads * vectors_of<T>();
+  if constexpr (vectors_of<T>() == 1) {
+    fill_deeper<T, kChunked>(p, rg, group, kv, part * kPer, static_cast<int>(threadIdx.x), say);
+  } else {
+#pragma unroll 1
+    for (int k = static_cast<int>(threadIdx.x); k < kPer; k += kThreads) fill_deeper<T, kChunked>(p, rg, group, kv, part * kPer, k, say);
+  }
+}
+
+// kWide: every row is a multiple of 32 bytes. The loops of the narrow types would cost this kernel a fifth of its CTAs.
+template <bool kWide, bool kChunked>
+__global__ void __launch_bounds__(kThreads, kWide ? 8 : 6) finalize_kernel(const __grid_constant__ FinalizeParams p) {
   const int group = static_cast<int>(blockIdx.x / p.parts);
   int at = static_cast<int>(blockIdx.x) - group * p.parts;
-  follow_stream();
-  list_rows(p, group, at == 0, s);
   const int g = at >= 2 * p.region[0].parts;
   const FinalizeRegion& rg = p.region[g];
   if (g) at -= 2 * p.region[0].parts;
   const int kv = at >= rg.parts;
-  char* pool = kv ? rg.value : rg.key;
   const int part = at - kv * rg.parts;
-  __syncthreads();
-  if (s.carried == 0) return;
-  const Share h = share_of(p, rg, part, s.carried);
-  for (int chunk = 0; chunk < p.planes; chunk += kPlaneChunk) {
-    look_up_blocks(p, rg, h, chunk, s);
-    __syncthreads();
-    if (rg.vec_bytes == 32) {
-      copy_share<Vec32>(p, rg, pool, h, chunk, s);
-    } else if (rg.vec_bytes == 16) {
-      copy_share<uint4>(p, rg, pool, h, chunk, s);
-    } else if (rg.vec_bytes == 4) {
-      copy_share<uint32_t>(p, rg, pool, h, chunk, s);
-    } else {
-      copy_share<uint8_t>(p, rg, pool, h, chunk, s);
-    }
-    if (chunk + kPlaneChunk < p.planes) __syncthreads();
+  const bool say = g == 0 && kv == 0 && blockIdx.y == 0;
+  follow_stream();
+  if (kWide || rg.vec_bytes == 32) {
+    copy_part<Vec32, kChunked>(p, rg, group, kv, part, say);
+  } else if (rg.vec_bytes == 16) {
+    copy_part<uint4, kChunked>(p, rg, group, kv, part, say);
+  } else if (rg.vec_bytes == 4) {
+    copy_part<uint32_t, kChunked>(p, rg, group, kv, part, say);
+  } else {
+    copy_part<uint8_t, kChunked>(p, rg, group, kv, part, say);
   }
 }
 
@@ -208,6 +162,7 @@ int rlt_kv_finalize(const RltPool* pool, const int32_t* tables, int32_t num_requ
   p.layer_mask = layer_mask == 0 ? all : (layer_mask & all);
   p.layers = __builtin_popcountll(p.layer_mask);
   if (p.layers == 0) return RLT_OK;
+  p.dense_layers = (p.layer_mask & (p.layer_mask + 1)) == 0;
   for (int g = 0; g < regions; ++g) {
     const RltRegion& r = g == 0 ? pool->codes : pool->scales;
     if (r.token_bytes <= 0 || r.layer_bytes != r.token_bytes * pool->block_size ||
@@ -239,25 +194,29 @@ int rlt_kv_finalize(const RltPool* pool, const int32_t* tables, int32_t num_requ
   p.rows = rows;
   p.n = count;
   p.status = status;
-  int sms = 0;
-  const int rc = rlt::sm_count(&sms);
-  if (rc != RLT_OK) return rc;
   const long long groups = (static_cast<long long>(count) + rlt::kGroupRows - 1) / rlt::kGroupRows;
-  // Vectors per thread of a CTA's share: enough stores behind the two rounds of lookups, whatever the number of planes.
-  // 4,000 rows of four planes (Ouro-1.4B): 485 us at 1, 282 at 4, 277 at 6, 278 at 8; 483 rows of 32 planes (Huginn): 318 us at 1,
-  // 337 at 2. (The persistent kernel this one replaced: 324 and 369 us; 64 rows of a decode step 12.6 -> 8.5 us.)
-  const int rounds = std::clamp(24 / p.planes, 1, 8);
   for (int g = 0; g < regions; ++g) {
     rlt::FinalizeRegion& rg = p.region[g];
-    const long long per = static_cast<long long>(rlt::kThreads) * rounds * (rg.vec_bytes == 32 ? 1 : rg.vec_bytes == 16 ? 2 : rg.vec_bytes == 4 ? 4 : 8);
+    const int per = rlt::kThreads * (rg.vec_bytes == 32 ? rlt::vectors_of<rlt::Vec32>() : rg.vec_bytes == 16 ? rlt::vectors_of<uint4>()
+                                     : rg.vec_bytes == 4 ? rlt::vectors_of<uint32_t>() : rlt::vectors_of<uint8_t>());
     const long long vectors = static_cast<long long>(p.layers) * rlt::kGroupRows * rg.row_vecs;
     rg.parts = static_cast<int>((vectors + per - 1) / per);
     p.parts += 2 * rg.parts;
   }
   const long long grid = groups * p.parts;
   if (grid > 0x7fffffffll) return RLT_E_LIMIT;
-  RLT_CUDA_TRY(rlt::launch_following(rlt::finalize_kernel, static_cast<unsigned>(grid), rlt::kThreads,
-                                     reinterpret_cast<cudaStream_t>(stream), p));
+  // A launch too small to fill the GPU is short of stores in flight where each thread has many planes to fill: the planes
+  // are then dealt to several CTAs, each of which reads the source rows (from L2, after the first) for itself. 8 rows of 32
+  // planes: 13.3 -> 10.0 us.
+  int sms = 0;
+  const int rc = rlt::sm_count(&sms);
+  if (rc != RLT_OK) return rc;
+  p.plane_chunk = grid < 8ll * sms && p.planes > 8 ? 8 : p.planes;
+  const dim3 ctas(static_cast<unsigned>(grid), static_cast<unsigned>((p.planes + p.plane_chunk - 1) / p.plane_chunk));
+  const bool wide = p.region[0].vec_bytes == 32 && (regions == 1 || p.region[1].vec_bytes == 32);
+  auto* kernel = ctas.y > 1 ? (wide ? rlt::finalize_kernel<true, true> : rlt::finalize_kernel<false, true>)
+                            : (wide ? rlt::finalize_kernel<true, false> : rlt::finalize_kernel<false, false>);
+  RLT_CUDA_TRY(rlt::launch_following(kernel, ctas, rlt::kThreads, reinterpret_cast<cudaStream_t>(stream), p));
   rlt::g_launches.fetch_add(1, std::memory_order_relaxed);
   return RLT_OK;
 }
