@@ -536,7 +536,7 @@ def run_single(args):
                      "traffic": TRAFFIC_PER_ALGORITHMIC_BYTE * algorithmic, "peak_source": peak_note,
                      "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of a 2-request capture of the same "
                                        "kernel (traffic / algorithmic = 0.98), scaled by tokens",
-                     "kernel": "table_fan_kernel" if w.extra.get("mode") == "dedup" and args.variant & 0xf not in (3, 4, 6) else "table_copy_kernel",
+                     "kernel": "move_kernel" if args.variant == 0 else "table_fan_kernel" if w.extra.get("mode") == "dedup" and args.variant & 0xf not in (3, 4, 6) else "table_copy_kernel",
                      "algorithmic_bytes_per_launch": algorithmic, "kernel_ms": avg_kernel_ms},
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": batch.metadata_bytes,
                 "d2h_bytes_per_step": 16, "ms_per_step": statistics.mean(e2e_times) * 1e3,
@@ -633,14 +633,14 @@ def suite_kernels(args):
     copies = int((s.planes - 1 - exits).sum())
     sources = int((exits < s.planes - 1).sum())
     if wanted("finalize"):
-        # Finalize writes two to three rows for each one it reads, and HBM takes writes more slowly than the mix of
-        # the copy the peak was measured with. The same volume as pure writes (the library memset) is timed first;
+        # Finalize writes two to three rows for each one it reads; the same volume as pure writes (an element-wise fill) is timed
+        # first, for comparison:
         # each finalize line carries its own write rate next to it.
         scratch = dst.key_cache.view(torch.uint8).reshape(-1)
         size = min(scratch.numel(), 3 << 30)
         ms = _timed(lambda: scratch[:size].zero_())
         write_rate = size / ms / 1e6
-        report("finalize", "context: Tensor.zero_ of 3 GiB (writes only)", size, ms)
+        report("finalize", "context: Tensor.zero_ of 3 GiB (element-wise fill, writes only)", size, ms)
 
         def finalize_line(name, read_rows, written_rows, ms, **extra):
             written = written_rows * ptb / ms / 1e6
@@ -648,25 +648,25 @@ def suite_kernels(args):
                    memset_write_gbps=round(write_rate, 1), written_over_memset=round(written / write_rate, 3), **extra)
 
         ms = _timed(lambda: kh.kv_finalize(sv, tables, rows, status=status))
-        finalize_line("finalize_fan_kernel", sources, copies, ms, rows=len(rows), source_rows=sources, copied_rows=copies,
+        finalize_line("finalize_kernel", sources, copies, ms, rows=len(rows), source_rows=sources, copied_rows=copies,
                       note="each exit row with deeper planes is read once and written once per deeper plane")
         # the same launch with every token leaving at plane 0: whole pages read from one block and written to three,
         # no holes on any plane - separates the cost of the scattered pattern above from the kernel's own
         dense = rows.clone()
         dense[:, 1] = 0
         ms = _timed(lambda: kh.kv_finalize(sv, tables, dense, status=status))
-        finalize_line("finalize_fan_kernel, every token exits at plane 0 (dense pages)", len(rows),
+        finalize_line("finalize_kernel, every token exits at plane 0 (dense pages)", len(rows),
                       len(rows) * (s.planes - 1), ms, rows=len(rows))
         # and with every token leaving at plane 1: the same 1 : 2 mix of reads and writes as the U{0..3} launch, on whole pages
         dense[:, 1] = 1
         ms = _timed(lambda: kh.kv_finalize(sv, tables, dense, status=status))
-        finalize_line("finalize_fan_kernel, every token exits at plane 1 (dense pages, 1 read : 2 writes)", len(rows),
+        finalize_line("finalize_kernel, every token exits at plane 1 (dense pages, 1 read : 2 writes)", len(rows),
                       len(rows) * (s.planes - 2), ms, rows=len(rows))
         kh.kv_finalize(sv, tables, rows, status=status)  # restore the copies the dedup measurements below rely on
         few = rows[:256].contiguous()  # what one decode step finalizes
         ms = _timed(lambda: kh.kv_finalize(sv, tables, few, status=status))
         fe = exits[:256]
-        finalize_line("finalize_fan_kernel (256 rows, one decode step)", int((fe < s.planes - 1).sum()),
+        finalize_line("finalize_kernel (256 rows, one decode step)", int((fe < s.planes - 1).sum()),
                       int((s.planes - 1 - fe).sum()), ms, rows=256)
     else:
         kh.kv_finalize(sv, tables, rows, status=status)
@@ -676,14 +676,14 @@ def suite_kernels(args):
     wire = pairs * ptb
     if wanted("pack"):
         ms = _timed(lambda: kh.kv_pack(sv, batch, packed, status=status))
-        report("pack", "table_copy_kernel pack all planes", 2 * full, ms)
+        report("pack", "move_kernel pack all planes", 2 * full, ms)
         ms = _timed(lambda: kh.kv_scatter(packed, dv, batch, status=status))
-        report("pack", "table_copy_kernel scatter all planes", 2 * full, ms)
+        report("pack", "move_kernel scatter all planes", 2 * full, ms)
         ws = kh.dedup_workspace(batch, s.planes, dev)
         ms = _timed(lambda: kh.kv_pack(sv, batch, packed, mode=kh.MODE_DEDUP, status=status, workspace=ws))
-        report("pack", "dedup plan (3 kernels) + table_copy_kernel pack dedup", 2 * wire, ms, wire_fraction=round(wire / full, 3))
+        report("pack", "move_kernel pack dedup", 2 * wire, ms, wire_fraction=round(wire / full, 3))
         ms = _timed(lambda: kh.kv_scatter(packed[:wire], dv, batch, mode=kh.MODE_DEDUP, status=status, workspace=ws))
-        report("pack", "dedup plan (3 kernels) + table_fan_kernel scatter dedup", wire + full, ms,
+        report("pack", "move_kernel scatter dedup", wire + full, ms,
                note="reads the wire image once, writes every plane")
     kh.raise_for_status(status)
 
@@ -734,7 +734,7 @@ def suite_kernels(args):
         for i in range(64):
             tt.append(hidden[i * 64 : (i + 1) * 64], staged[(63 - i) * 64 : (64 - i) * 64])
         ms = _timed(tt.submit)
-        report("tensors", "segmented_transfer_kernel (64 copies of 64 x 2048 bf16)", 2 * hidden.numel() * 2, ms,
+        report("tensors", "inline_transfer_kernel (64 copies of 64 x 2048 bf16)", 2 * hidden.numel() * 2, ms,
                note="metadata-sized: launch latency, not bandwidth")
 
 

@@ -34,6 +34,24 @@ struct Failure {};  // a Python error is set
 }
 [[noreturn]] void bad_value(const char* text) { fail(PyExc_ValueError, text); }
 
+// Integers that grow without being zeroed first: every one is written before it is read.
+template <typename V>
+struct Uninitialised : std::allocator<V> {
+  template <typename U>
+  struct rebind {
+    using other = Uninitialised<U>;
+  };
+  template <typename U>
+  void construct(U* p) {
+    ::new (static_cast<void*>(p)) U;
+  }
+  template <typename U, typename... A>
+  void construct(U* p, A&&... a) {
+    ::new (static_cast<void*>(p)) U(std::forward<A>(a)...);
+  }
+};
+using Ints = std::vector<int32_t, Uninitialised<int32_t>>;
+
 struct Ref {
   PyObject* p;
   explicit Ref(PyObject* q) : p(q) {
@@ -74,7 +92,7 @@ bool is_int32(const Py_buffer& v) {
 }
 
 // Appends the int32 values of one table (or exit-plane array) to `out`; returns how many.
-Py_ssize_t append_ints(PyObject* o, std::vector<int32_t>& out, const char* not_flat) {
+Py_ssize_t append_ints(PyObject* o, Ints& out, const char* not_flat) {
   if (PyTuple_CheckExact(o) || PyList_CheckExact(o)) {
     const Py_ssize_t n = PySequence_Fast_GET_SIZE(o);
     PyObject** items = PySequence_Fast_ITEMS(o);
@@ -128,7 +146,7 @@ struct Side {
   bool given = false;
   int planes = 0;
   int width = 0;                       // pages of the longest table
-  std::vector<int32_t> flat;           // every table, back to back
+  Ints flat;                           // every table, back to back
   std::vector<size_t> at;              // [n * planes] where each starts
   std::vector<Py_ssize_t> pages;       // [n] of each request's tables
   const int32_t* table(int r, int p) const { return flat.data() + at[static_cast<size_t>(r) * planes + p]; }
@@ -139,12 +157,12 @@ struct Plan {
   Side src, dst;
   std::vector<int64_t> begin, end;
   bool has_exit = false;
-  std::vector<int32_t> exits;
+  Ints exits;
   std::vector<int64_t> exit_at;  // [n] index in exits of each request's token 0
   int blocks = 0, words = 0;
-  std::vector<int32_t> records;
+  Ints records;
   int wire_planes = 0;
-  std::vector<int32_t> wire;
+  Ints wire;
   int64_t wire_tokens = 0;
 
   void make_records();
@@ -208,8 +226,14 @@ void Plan::make_records() {
   records.resize(static_cast<size_t>(total) * words);
   int32_t* w = records.data();
   int64_t before = 0;
+  std::vector<const int32_t*> tables;
   for (int r = 0; r < n; ++r) {
     const int64_t b = begin[r], e = end[r];
+    tables.clear();
+    for (const Side* side : {&src, &dst}) {
+      for (int p = 0; p < side->planes; ++p) tables.push_back(side->table(r, p));
+    }
+    const int32_t* exit = has_exit ? exits.data() + exit_at[r] : nullptr;
     for (int64_t page = b / block_size; page <= (e - 1) / block_size; ++page, w += words) {
       const int64_t base = page * block_size;
       const int64_t lo = b > base ? b - base : 0, hi = e < base + block_size ? e - base : block_size;
@@ -220,12 +244,10 @@ void Plan::make_records() {
       w[4] = static_cast<int32_t>(before);
       w[5] = static_cast<int32_t>(e - b);
       int32_t* id = w + kRecordHeader;
-      for (const Side* side : {&src, &dst}) {
-        for (int p = 0; p < side->planes; ++p) *id++ = side->table(r, p)[page];
-      }
+      for (const int32_t* table : tables) *id++ = table[page];
       if (has_exit) {
-        std::memset(id, 0, 4 * static_cast<size_t>(block_size));
-        std::memcpy(id + lo, exits.data() + exit_at[r] + base + lo, 4 * static_cast<size_t>(hi - lo));
+        if (hi - lo != block_size) std::memset(id, 0, 4 * static_cast<size_t>(block_size));
+        std::memcpy(id + lo, exit + base + lo, 4 * static_cast<size_t>(hi - lo));
       }
     }
     before += e - b;
@@ -235,7 +257,7 @@ void Plan::make_records() {
 // Wire order: request, plane, page; a page's tokens count on every plane up to their exit plane.
 void Plan::make_wire(int planes) {
   if (wire_planes == planes) return;
-  std::vector<int32_t> at(static_cast<size_t>(blocks) * planes);
+  Ints at(static_cast<size_t>(blocks) * planes);
   std::vector<int32_t> carried(planes + 1);
   const int exit_word = kRecordHeader + src.planes + dst.planes;
   for (int b = 0; b < blocks; ++b) {
@@ -267,8 +289,37 @@ void Plan::make_wire(int planes) {
   wire_planes = planes;
 }
 
+// Plans that are no longer used, for their memory: fresh pages for a large batch's records cost more than writing them. A
+// few are kept, none above kKeptPlanBytes. The interpreter's lock guards the list.
+constexpr size_t kKeptPlans = 4;
+constexpr size_t kKeptPlanBytes = size_t{8} << 20;
+std::vector<std::unique_ptr<Plan>> g_plans;
+
+std::unique_ptr<Plan> fresh_plan() {
+  if (g_plans.empty()) return std::make_unique<Plan>();
+  std::unique_ptr<Plan> plan = std::move(g_plans.back());
+  g_plans.pop_back();
+  return plan;
+}
+
+void give_back(std::unique_ptr<Plan> plan) {
+  const size_t held = 4 * (plan->src.flat.capacity() + plan->dst.flat.capacity() + plan->exits.capacity() + plan->records.capacity());
+  if (g_plans.size() >= kKeptPlans || held > kKeptPlanBytes) return;
+  Plan clean;
+  for (auto list : {&Plan::exits, &Plan::records}) {
+    (clean.*list).swap((*plan).*list);
+    (clean.*list).clear();
+  }
+  for (auto side : {&Plan::src, &Plan::dst}) {
+    (clean.*side).flat.swap(((*plan).*side).flat);
+    (clean.*side).flat.clear();
+  }
+  *plan = std::move(clean);
+  g_plans.push_back(std::move(plan));
+}
+
 constexpr const char* kPlanName = "vllm_rlt_b200.plan";
-void free_plan(PyObject* capsule) { delete static_cast<Plan*>(PyCapsule_GetPointer(capsule, kPlanName)); }
+void free_plan(PyObject* capsule) { give_back(std::unique_ptr<Plan>(static_cast<Plan*>(PyCapsule_GetPointer(capsule, kPlanName)))); }
 Plan& plan_of(PyObject* capsule) {
   auto* p = static_cast<Plan*>(PyCapsule_GetPointer(capsule, kPlanName));
   if (p == nullptr) throw Failure{};
@@ -278,7 +329,7 @@ Plan& plan_of(PyObject* capsule) {
 // plan(src_tables | None, dst_tables | None, ranges, exit_planes | None, block_size, src_blocks | None, dst_blocks | None,
 //      most requests) -> (plan, requests, tokens, width, source planes, destination planes, exit entries, ranges, record bytes)
 PyObject* make_plan(PyObject* const* a) {
-  auto plan = std::make_unique<Plan>();
+  auto plan = fresh_plan();
   const Py_ssize_t n = length(a[2]);
   const long long most = integer(a[7]);
   if (n < 1) bad_value("a handoff batch needs at least one request");
@@ -421,7 +472,7 @@ void* address(PyObject* o) { return o == Py_None ? nullptr : PyLong_AsVoidPtr(o)
 // plan_upload(plan, which, device address, stream) -> code: records (0) or wire plan (1) to device memory.
 PyObject* plan_upload(PyObject* const* a) {
   const Plan& p = plan_of(a[0]);
-  const std::vector<int32_t>& v = integer(a[1]) == 0 ? p.records : p.wire;
+  const Ints& v = integer(a[1]) == 0 ? p.records : p.wire;
   return PyLong_FromLong(rlt_stage_upload(v.data(), 4 * v.size(), address(a[2]), static_cast<rlt_stream_t>(address(a[3]))));
 }
 
@@ -812,7 +863,7 @@ void put(std::string& out, V v) {
 }
 
 // Values [from, to) of a table, as int32.
-void append_range(PyObject* o, Py_ssize_t from, Py_ssize_t to, std::vector<int32_t>& out) {
+void append_range(PyObject* o, Py_ssize_t from, Py_ssize_t to, Ints& out) {
   if (PyTuple_CheckExact(o) || PyList_CheckExact(o)) {
     PyObject** items = PySequence_Fast_ITEMS(o);
     for (Py_ssize_t i = from; i < to; ++i) out.push_back(int32_of(integer(items[i])));
@@ -835,7 +886,7 @@ PyObject* encode_chunk(PyObject* const* a) {
   put(out, static_cast<uint32_t>(PySequence_Fast_GET_SIZE(extra.p)));
   for (int i = 2; i < 7; ++i) put(out, static_cast<uint32_t>(integer(a[i])));
   put(out, uint32_t{0});
-  std::vector<int32_t> ids;
+  Ints ids;
   for (Py_ssize_t r = 0; r < PySequence_Fast_GET_SIZE(requests.p); ++r) {
     const Ref request(PySequence_Fast(PySequence_Fast_GET_ITEM(requests.p, r), "a request is (source, target, start, end)"));
     if (PySequence_Fast_GET_SIZE(request.p) != 4) bad_value("a request is (source, target, start, end)");
@@ -878,7 +929,7 @@ PyObject* encode_chunk(PyObject* const* a) {
 // Records of an all-planes handoff, page by page, and their launch.
 struct RequestRecords {
   const RltPool *src, *dst;
-  std::vector<int32_t> records;
+  Ints records;
   int words;
   int64_t requests = 0, before = 0, blocks = 0, width = 1;
   RequestRecords(const RltPool* s, const RltPool* d) : src(s), dst(d), words(kRecordHeader + s->num_planes + d->num_planes) {}
@@ -931,7 +982,7 @@ PyObject* handoff_requests(PyObject* const* a) {
   auto unsuited = [] { return PyLong_FromLong(RLT_MOVE_UNSUITED); };
   if (n < 1 || bs < 1) return unsuited();
   RequestRecords out(src, dst);
-  std::vector<int32_t> ids;
+  Ints ids;
   for (Py_ssize_t r = 0; r < n; ++r) {
     const Ref request(PySequence_Fast(PySequence_Fast_GET_ITEM(requests.p, r), "a request is (source, target, start, end)"));
     if (PySequence_Fast_GET_SIZE(request.p) < 4) return unsuited();
@@ -1018,7 +1069,7 @@ PyObject* pull_chunk(PyObject* const* a) {
   if (!take(at, end, &head) || head[2] != RLT_MODE_ALL_PLANES || head[0] == 0) Py_RETURN_NONE;
   const int64_t bs = src->block_size;
   RequestRecords out(src, dst);
-  std::vector<int32_t> ids;
+  Ints ids;
   for (uint32_t r = 0; r < head[0]; ++r) {
     uint32_t planes[2], columns;
     int64_t range[2];
