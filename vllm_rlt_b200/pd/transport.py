@@ -18,7 +18,7 @@ with the same return values and exceptions. What differs is underneath:
 Two directions for ``submit_tables``. *Push*: the sender's GPU runs the handoff kernel with the receiver's pool
 behind peer pointers and then posts "landed". *Pull* (the default): the sender writes the chunk's descriptor
 (both sides' block tables, the token range, the hidden-state row) into a descriptor ring in the receiver's
-mailbox from the host and, behind the producer's event on its transfer stream, posts a 64-byte "offer"; the
+mailbox from the host and, behind the producer's event on its transfer stream (from the host if that has fired), posts a 64-byte "offer"; the
 receiver's ``poll()`` finds the offer, runs the same kernel on its own transfer stream with the *sender's* pool
 behind peer pointers, reports ``(peer, tid, seq)`` as received when that launch's event has fired, and posts
 "pulled" into the sender's mailbox, which completes the sender's ticket (``busy()`` stays true until then, so the
@@ -553,6 +553,7 @@ class B200Transport:
         self.pending: deque[Transfer] = deque()
         self._offered: dict[tuple[str, str, int], _RemoteCompletion] = {}
         self._pulls: list[_Pull] = []
+        self._behind = None  # marker of the last submission that waits for a producer's event on the device
         self.inflight_bytes = 0
         self.bytes_sent = 0
         self.bytes_received = 0
@@ -629,6 +630,15 @@ class B200Transport:
             self.inflight_bytes += size
         return True
 
+    def _ready(self, event) -> bool:
+        """Whether what is submitted with ``event`` would begin at once: the event has fired, and so have those that the
+        transfer stream was told to wait for before."""
+        if event is not None and not (self.device_ordered and event.query()):
+            return False
+        if self._behind is not None and self._behind.query():
+            self._behind = None
+        return self._behind is None
+
     def _wait_for(self, event) -> None:
         """Queue what follows behind ``event`` on the transfer stream."""
         if event is not None:
@@ -640,7 +650,10 @@ class B200Transport:
         """``_wait_for``; returns an event that fires when the transfer stream has got past that wait, i.e. when this
         submission's own work begins."""
         self._wait_for(event)
-        return self.backend.marker()
+        marker = self.backend.marker()
+        if event is not None:
+            self._behind = marker
+        return marker
 
     def submit(self, transfer_id, sequence, peer, local, remote, size, *, after=None):
         """WRITE the local ranges onto the remote ranges and notify the peer (vllm_rlt/pd/transport.py:182-201).
@@ -704,9 +717,13 @@ class B200Transport:
         first = parts[0][0]
         body = Mailbox.encode(transfer_id, first, OFFER, (at, len(raw)), count=len(parts))
         box.write_descriptor(link["lane"], at, raw)
-        self._wait_for(after)  # the offer leaves when the producer's event has fired
-        self._post(link, body)
-        started = self.backend.marker()
+        started = None
+        if self._ready(after):  # nothing to wait for: the host posts, which spares a launch and its way over the bus
+            self._post(link, body, from_host=True)
+        else:
+            self._wait_for(after)  # the offer leaves when the producer's event has fired
+            self._post(link, body)
+            started = self._behind = self.backend.marker()
         self._note("offer queued", transfer_id, first)
         handle = self._offered[(link["agent"], transfer_id, first)] = _RemoteCompletion()
         return self._tickets(handle, transfer_id, parts, (), started)
