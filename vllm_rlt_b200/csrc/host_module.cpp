@@ -9,7 +9,7 @@
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
-#include <ATen/core/LegacyTypeDispatch.h>
+#include <ATen/core/Tensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -61,6 +61,10 @@ struct Ref {
   Ref(const Ref&) = delete;
   Ref& operator=(const Ref&) = delete;
 };
+
+void check_code(int code) {
+  if (code < 0) fail(PyExc_RuntimeError, rlt_error_string(code));
+}
 
 struct Buffer {
   Py_buffer view;
@@ -596,6 +600,19 @@ PyObject* finalize(PyObject* const* a) {
 
 // ------------------------------------------------------------------------------------------------ tensor transfers
 
+// A 1-D view of `t`, as at::as_strided makes it, without the dispatcher and the bookkeeping of autograd (these slices never take
+// part in it): a step makes a few hundred of them. The caller has checked the bounds.
+at::Tensor plain_view(const at::Tensor& t, int64_t offset, int64_t n, int64_t stride) {
+  at::Tensor out = at::detail::make_tensor<c10::TensorImpl>(c10::TensorImpl::VIEW, c10::Storage(t.storage()), t.key_set(), t.dtype());
+  out.unsafeGetTensorImpl()->set_storage_offset(offset);
+  out.unsafeGetTensorImpl()->set_sizes_and_strides(c10::IntArrayRef(&n, 1), c10::IntArrayRef(&stride, 1));
+  return out;
+}
+// t[start : start + n] of a flat tensor
+at::Tensor plain_slice(const at::Tensor& t, int64_t start, int64_t n) {
+  return plain_view(t, t.storage_offset() + start * t.stride(0), n, t.stride(0));
+}
+
 // RLT_DTYPE_* of a tensor, -1 for the types that do not transfer.
 int transfer_type(const at::Tensor& t) {
   switch (t.scalar_type()) {
@@ -679,29 +696,48 @@ PyObject* copies_reset(PyObject* self, PyObject* const*) {
   Py_RETURN_NONE;
 }
 
-PyObject* copies_append(PyObject* self, PyObject* const* a) {
-  CopiesObject* c = copies_of(self);
+// Records source -> target; `keep_source` and `keep_target` are what the batch holds on to.
+void append_copy(CopiesObject* c, const at::Tensor& source, const at::Tensor& target, PyObject* keep_source, PyObject* keep_target,
+                 bool checked = false) {
   Transfer& t = *c->batch;
-  const at::Tensor &source = some_tensor(a[0]), &target = some_tensor(a[1]);
   const int64_t dims = source.dim();
   if (source.sizes() != target.sizes() || (dims != 1 && dims != 2)) bad_value("transfer requires matching 1D/2D shapes");
   if (transfer_type(source) != c->from || transfer_type(target) != c->to) bad_value("transfer dtype does not match its batch");
   const at::Device device(at::kCUDA, static_cast<c10::DeviceIndex>(c->device));
   if (target.device() != device) bad_value("transfer destination must be on the configured device");
   if (source.is_cuda() && source.device() != device) bad_value("transfer source must be on the configured device");
-  check_source(source, device);
-  if (source.numel() == 0) Py_RETURN_NONE;
+  if (!checked) check_source(source, device);
+  if (source.numel() == 0) return;
   if (static_cast<long long>(t.rows.size() / 8) >= c->capacity) bad_value("transfer batch is full");
   const bool flat = dims == 1;
   const int64_t rows = flat ? 1 : source.size(0), cols = source.size(dims - 1);
   const int64_t row[8] = {reinterpret_cast<int64_t>(source.data_ptr()), reinterpret_cast<int64_t>(target.data_ptr()), rows, cols,
                           flat ? cols * source.stride(0) : source.stride(0), source.stride(dims - 1),
                           flat ? cols * target.stride(0) : target.stride(0), target.stride(dims - 1)};
-  const Ref pair(PyTuple_Pack(2, a[0], a[1]));
+  const Ref pair(PyTuple_Pack(2, keep_source, keep_target));
   if (PyList_Append(c->copies, pair.p) != 0) throw Failure{};
   t.rows.insert(t.rows.end(), row, row + 8);
   t.max_rows = rows > t.max_rows ? rows : t.max_rows;
   t.max_cols = cols > t.max_cols ? cols : t.max_cols;
+}
+
+PyObject* copies_append(PyObject* self, PyObject* const* a) {
+  append_copy(copies_of(self), some_tensor(a[0]), some_tensor(a[1]), a[0], a[1]);
+  Py_RETURN_NONE;
+}
+
+// append_pieces(flat tensor, [targets]): appends the copies of consecutive slices of it, each as long as its target.
+PyObject* copies_append_pieces(PyObject* self, PyObject* const* a) {
+  const at::Tensor& source = some_tensor(a[0]);
+  const Ref targets(PySequence_Fast(a[1], "targets must be a sequence of tensors"));
+  int64_t at = 0;
+  for (Py_ssize_t i = 0; i < PySequence_Fast_GET_SIZE(targets.p); ++i) {
+    PyObject* target = PySequence_Fast_GET_ITEM(targets.p, i);
+    const int64_t n = some_tensor(target).size(0);
+    if (source.dim() != 1 || at + n > source.size(0)) bad_value("transfer requires matching 1D/2D shapes");
+    append_copy(copies_of(self), plain_slice(source, at, n), some_tensor(target), a[0], target, i > 0);  // slices of one tensor: looked at once
+    at += n;
+  }
   Py_RETURN_NONE;
 }
 
@@ -724,12 +760,6 @@ PyObject* copies_launch(PyObject* self, PyObject* const* a) {
 }
 
 // ------------------------------------------------------------------------------------------------ staging helpers
-
-// t[start : start + n] of a flat tensor. These slices never take part in autograd, whose bookkeeping is skipped.
-at::Tensor plain_slice(const at::Tensor& t, int64_t start, int64_t n) {
-  const at::AutoDispatchBelowADInplaceOrView guard;
-  return t.narrow(0, start, n);
-}
 
 template <typename V, typename F>
 bool fill_from(PyObject** items, Py_ssize_t n, V* out, F convert) {
@@ -789,8 +819,7 @@ PyObject* row_slice(PyObject* const* a) {
   const int64_t start = integer(a[2]), n = integer(a[3]);
   index += index < 0 ? t.size(0) : 0;
   if (index < 0 || index >= t.size(0) || start < 0 || start + n > t.size(1)) Py_RETURN_NONE;
-  const at::AutoDispatchBelowADInplaceOrView guard;
-  return THPVariable_Wrap(t.as_strided({n}, {t.stride(1)}, t.storage_offset() + index * t.stride(0) + start * t.stride(1)));
+  return THPVariable_Wrap(plain_view(t, t.storage_offset() + index * t.stride(0) + start * t.stride(1), n, t.stride(1)));
 }
 
 // Base of StagedInputTensor: `append` of plain numbers that fit; everything else is the subclass's `append_values`.
@@ -838,20 +867,20 @@ PyObject* writes_stage(PyObject* self, PyObject* const* a) {
   return PyObject_CallMethod(self, "stage_values", "OOO", a[0], a[1], a[2]);
 }
 
-// pieces(flat tensor, [targets]) -> consecutive slices of it, as long as the targets
-PyObject* pieces(PyObject* const* a) {
-  const at::Tensor& t = some_tensor(a[0]);
-  const Ref targets(PySequence_Fast(a[1], "targets must be a sequence of tensors"));
-  const Py_ssize_t n = PySequence_Fast_GET_SIZE(targets.p);
-  PyObject* out = PyList_New(n);
-  if (out == nullptr) throw Failure{};
-  int64_t at = 0;
-  for (Py_ssize_t i = 0; i < n; ++i) {
-    const int64_t count = some_tensor(PySequence_Fast_GET_ITEM(targets.p, i)).size(0);
-    PyList_SET_ITEM(out, i, THPVariable_Wrap(plain_slice(t, at, count)));
-    at += count;
+// upload(flat CPU tensor, pinned tensor, device tensor, count) -> the device tensor's first `count` elements, to which the CPU tensor's are
+// on their way through the pinned one; None where the three are not flat, of one type and large enough, on those devices.
+PyObject* upload(PyObject* const* a) {
+  const at::Tensor &source = some_tensor(a[0]), &pinned = some_tensor(a[1]), &target = some_tensor(a[2]);
+  const int64_t n = integer(a[3]);
+  const int type = transfer_type(source);
+  for (const at::Tensor* t : {&source, &pinned, &target}) {
+    if (t->dim() != 1 || !t->is_contiguous() || t->size(0) < n || transfer_type(*t) != type) Py_RETURN_NONE;
   }
-  return out;
+  if (type < 0 || n < 1 || !source.is_cpu() || !target.is_cuda() || !pinned.is_pinned()) Py_RETURN_NONE;
+  std::memcpy(pinned.data_ptr(), source.data_ptr(), static_cast<size_t>(n) * source.element_size());
+  const c10::cuda::CUDAGuard guard(target.device());
+  check_code(rlt_tensor_copy(pinned.data_ptr(), target.data_ptr(), nullptr, n, type, type, 0, stream_of(Py_None)));
+  return THPVariable_Wrap(plain_slice(target, 0, n));
 }
 
 // ------------------------------------------------------------------------------------------------ transport
@@ -1025,9 +1054,6 @@ struct EventObject {
 };
 PyTypeObject* g_event_type = nullptr;
 
-void check_code(int code) {
-  if (code < 0) fail(PyExc_RuntimeError, rlt_error_string(code));
-}
 
 PyObject* record_event(bool timed, rlt_stream_t stream) {
   RltEvent* event = nullptr;
@@ -1235,7 +1261,7 @@ PyMethodDef kMethods[] = {
     RLT_ENTRY("post", post, 5),
     RLT_ENTRY("tensor_copy", tensor_copy, 3),
     RLT_ENTRY("fill", fill, 3),
-    RLT_ENTRY("pieces", pieces, 2),
+    RLT_ENTRY("upload", upload, 4),
     {nullptr, nullptr, 0, nullptr},
 };
 
@@ -1323,7 +1349,7 @@ PyObject* copies_max_rows(PyObject* self, void*) { return PyLong_FromLongLong(co
 PyObject* copies_max_cols(PyObject* self, void*) { return PyLong_FromLongLong(copies_of(self)->batch->max_cols); }
 
 PyMethodDef kCopiesMethods[] = {RLT_METHOD("setup", copies_setup, 4), RLT_METHOD("reset", copies_reset, 0),
-                                RLT_NAMED_METHOD("append", copies_append, 2, kAppendNames), RLT_METHOD("launch", copies_launch, 1),
+                                RLT_NAMED_METHOD("append", copies_append, 2, kAppendNames), RLT_METHOD("append_pieces", copies_append_pieces, 2), RLT_METHOD("launch", copies_launch, 1),
                                 {nullptr, nullptr, 0, nullptr}};
 PyMemberDef kCopiesMembers[] = {{"copies", Py_T_OBJECT_EX, offsetof(CopiesObject, copies), Py_READONLY, nullptr},
                                 {"capacity", Py_T_LONGLONG, offsetof(CopiesObject, capacity), Py_READONLY, nullptr},
