@@ -316,7 +316,7 @@ class CudaBackend:
         self.device = torch.device(device)
         self.mapping = peerlib.PeerMapping()
         self.peerlib = peerlib
-        self._mailboxes: dict[str, tuple[Mailbox, int]] = {}
+        self._mailboxes: dict[str, list] = {}
         self._views: dict[tuple, tuple] = {}
         self.lane = None  # the mailbox lane this worker writes on, once its transport has chosen it
         self.stream = torch.cuda.Stream(self.device)
@@ -345,22 +345,29 @@ class CudaBackend:
 
         return _Translation(spans)
 
-    def mailbox_pointer(self, name: str) -> tuple[Mailbox, int]:
-        """Open a peer's mailbox and make it writable from this device."""
-        import ctypes as C
-
+    def mailbox_pointer(self, name: str) -> tuple[Mailbox, None]:
+        """Open a peer's mailbox. Its device address is asked for separately, by who posts from the device."""
         hit = self._mailboxes.get(name)
         if hit is None:
-            box = Mailbox(name)
-            # only the lane this worker writes on is made visible to its GPU: registering memory costs time per page
+            hit = self._mailboxes[name] = [Mailbox(name), None, None]  # box, device address, registered host address
+        return hit[0], None
+
+    def mailbox_address(self, name: str) -> int:
+        """Make an opened mailbox writable from this device. Registering memory costs milliseconds, which a worker that only ever
+        posts from its host (every worker that receives) does not pay; only the lane this worker writes on is registered."""
+        import ctypes as C
+
+        hit = self._mailboxes[name]
+        if hit[1] is None:
+            buf = hit[0].shm.buf
             at = (self.lane or 0) * LANE_BYTES
-            size = LANE_BYTES if self.lane is not None else len(box.shm.buf)
-            host = C.addressof(C.c_char.from_buffer(box.shm.buf)) + at
+            size = LANE_BYTES if self.lane is not None else len(buf)
+            host = C.addressof(C.c_char.from_buffer(buf)) + at
             out = C.c_void_p()
             with self.torch.cuda.device(self.device):
                 _lib.check(_lib.load().rlt_host_register(host, size, C.byref(out)), "rlt_host_register")
-            hit = self._mailboxes[name] = (box, int(out.value) - at, host)
-        return hit[0], hit[1]
+            hit[1:] = int(out.value) - at, host
+        return hit[1]
 
     def pair(self, local, remote, translate):
         """Two descriptor lists as what ``copy_segments`` takes."""
@@ -455,7 +462,8 @@ class CudaBackend:
         boxes, self._mailboxes = self._mailboxes, {}
         self._views = {}
         for box, _, host in boxes.values():
-            _lib.check(_lib.load().rlt_host_unregister(host), "rlt_host_unregister")
+            if host is not None:
+                _lib.check(_lib.load().rlt_host_unregister(host), "rlt_host_unregister")
             box.close()
         self.mapping.close()
 
@@ -615,6 +623,8 @@ class B200Transport:
         return self._slot_free(link)
 
     def _post(self, link: dict, body: bytes, *, from_host: bool = False) -> None:
+        if not from_host and link["box_ptr"] is None:
+            link["box_ptr"] = self.backend.mailbox_address(self.peers[link["agent"]]["metadata"]["mailbox"])
         link["stamp"] += 1
         if from_host:
             link["box"].post_from_host(link["lane"], link["stamp"], body)
