@@ -1115,8 +1115,8 @@ PyObject* pull_chunk(PyObject* const* a) {
     out.width = columns > out.width ? columns : out.width;
     out.add(ids.data(), columns, first, first, pages, range[0], range[1]);
   }
+  if (static_cast<size_t>(end - at) / 24 < head[1]) Py_RETURN_NONE;  // the count is another process's word: looked at before it is used
   std::vector<int64_t> extra(3 * static_cast<size_t>(head[1]));
-  if (end - at < static_cast<ptrdiff_t>(8 * extra.size())) Py_RETURN_NONE;
   if (!extra.empty()) std::memcpy(extra.data(), at, 8 * extra.size());
   if (!extra.empty()) {
     const Ref spans(PySequence_Fast(a[3], "spans must be a sequence"));
