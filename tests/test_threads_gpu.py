@@ -1,0 +1,93 @@
+"""Several threads and streams at once: a call that has to wait for the GPU holds up neither the threads that need not wait nor the
+one whose word the GPU is waiting for. Every wait on the GPU is bounded (``kv_wait``) and ends when the host sets its flag."""
+
+import ctypes as C
+import threading
+import time
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+LIMIT_NS = 1_500_000_000  # of the waits on the GPU; a test that passes sets their flags long before
+PAGES = 1000              # 8 words a page: more than the kernel parameters hold, and one staging slot
+
+
+class Waiting:
+    """A stream whose work waits until the host says ``go``."""
+
+    def __init__(self):
+        from vllm_rlt_b200.kernels import kv_handoff as kh
+
+        self.flag = torch.zeros(1, dtype=torch.int64, pin_memory=True)
+        self.status = kh.new_status()
+        self.stream = torch.cuda.Stream()
+        self.stream.wait_stream(torch.cuda.current_stream())
+        kh.kv_wait(self.flag.data_ptr(), 1, LIMIT_NS, self.status, stream=self.stream)
+
+    def go(self):
+        self.flag[0] = 1
+
+    def in_time(self):
+        self.stream.synchronize()
+        return self.status.tolist() == [0, 0, 0, 0]
+
+
+@pytest.fixture(scope="module")
+def pools():
+    """Two single-plane pools of PAGES + 1 blocks and tables over PAGES of them."""
+    from vllm_rlt_b200.core.kv_pool import KVPool
+    from vllm_rlt_b200.kernels import kv_handoff as kh
+
+    src, dst = (KVPool(1, 1, 16, PAGES + 1, 4, 1, device="cuda") for _ in range(2))
+    src.key_cache.normal_()
+    src.value_cache.normal_()
+    tables = np.random.default_rng(0).permutation(PAGES).astype(np.int32).reshape(1, 1, PAGES)
+    return src, dst, kh.PoolView.from_cache(src), kh.PoolView.from_cache(dst), tables
+
+
+def arrived(pools):
+    src, dst, _, _, tables = pools
+    at = torch.from_numpy(tables.reshape(-1)).cuda().long()
+    whole = all(torch.equal(a[at], b[at]) for a, b in ((src.key_cache, dst.key_cache), (src.value_cache, dst.value_cache)))
+    for t in (dst.key_cache, dst.value_cache):
+        t.zero_()
+    return whole
+
+
+def test_a_call_that_finds_a_free_slot_is_not_held_up_by_one_that_waits_for_its_own(pools):
+    from vllm_rlt_b200 import _lib
+
+    _, _, sv, dv, tables = pools
+    lib = _lib.load()  # through ctypes, which lets other threads run
+    s, d = sv.as_struct(), dv.as_struct()
+    begin, end = np.zeros(1, np.int32), np.full(1, 4 * PAGES, np.int32)
+    batch = _lib.RltHostBatch(1, PAGES, 1, 1, tables.ctypes.data, tables.ctypes.data, begin.ctypes.data, end.ctypes.data)
+    options = _lib.RltOptions()
+    device = torch.cuda.current_device()
+
+    def call(stream):
+        torch.cuda.set_device(device)
+        _lib.check(lib.rlt_kv_handoff_host(C.byref(s), C.byref(d), C.byref(batch), C.byref(options), stream.cuda_stream), "handoff")
+
+    call(torch.cuda.current_stream())
+    torch.cuda.synchronize()
+    a, b = Waiting(), Waiting()
+    for w in (a, b):
+        for _ in range(8):  # all 16 slots of the library
+            call(w.stream)
+    late = threading.Thread(target=call, args=(a.stream,))
+    late.start()
+    time.sleep(0.1)
+    assert late.is_alive()  # it waits for a slot of stream a's launches
+    b.go()
+    b.stream.synchronize()
+    began = time.monotonic()
+    call(b.stream)
+    took = time.monotonic() - began
+    a.go()
+    late.join(timeout=10)
+    assert not late.is_alive() and took < 0.5
+    assert a.in_time() and b.in_time() and arrived(pools)

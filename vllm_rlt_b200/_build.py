@@ -80,7 +80,7 @@ def build_library(force: bool = False, verbose: bool = False) -> Path:
     target = PACKAGE / LIB_NAME
     sources = [CSRC / s for s in CUDA_SOURCES]
     deps = sources + [CSRC / "common.cuh", CSRC / "table_params.cuh", CSRC / "block_moves.h",
-                      CSRC / "internal.h", INCLUDE / "rlt_kv_handoff.h"]
+                      CSRC / "internal.h", CSRC / "slot_pool.h", INCLUDE / "rlt_kv_handoff.h"]
     flags = [*ARCH, "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC,-fvisibility=hidden"]
     fingerprint = _fingerprint(flags, deps)
     if force or verbose or _stale(target, fingerprint):

@@ -1,8 +1,8 @@
 // What a call needs for a moment and the library keeps: pinned staging for host arrays on their way to the device, and events.
 //
 // Page-locked memory costs a driver call to get, so buffers are kept: per device and power-of-two size at most kKept of
-// them (eight of 1 MiB and more, two of 16 MiB and more), each free again when the copy that last read it has finished. When all of a size
-// are busy the call waits for the one that has been busy longest.
+// them (eight of 1 MiB and more, two of 16 MiB and more), each free again when the copy that last read it has finished. When all of a
+// size are busy the call waits for the one that has been busy longest.
 
 #include <cstring>
 #include <mutex>
@@ -10,6 +10,7 @@
 
 #include "common.cuh"
 #include "internal.h"
+#include "slot_pool.h"
 
 namespace rlt {
 namespace {
@@ -25,45 +26,31 @@ struct Pinned {
   void* host = nullptr;
   cudaEvent_t done = nullptr;
 };
-struct SizeClass {
-  std::vector<Pinned> buffers;
-  size_t next = 0;  // the one that was handed out longest ago
+
+int make_pinned(size_t bytes, Pinned* out) {
+  Pinned fresh;
+  RLT_CUDA_TRY(cudaHostAlloc(&fresh.host, bytes, cudaHostAllocDefault));
+  if (const cudaError_t e = cudaEventCreateWithFlags(&fresh.done, cudaEventDisableTiming); e != cudaSuccess) {
+    cudaFreeHost(fresh.host);
+    return cuda_fail(e);
+  }
+  *out = fresh;
+  return RLT_OK;
+}
+
+// Size class of `bytes` on the current device.
+struct PinnedClass {
+  SlotPool<Pinned>* pool;
+  size_t bytes, kept;
 };
-
-std::mutex g_mutex;
-
-// The buffer for `bytes` bytes on the current device; the caller holds g_mutex.
-int acquire(size_t bytes, Pinned** out) {
-  static SizeClass classes[kMaxDevices][kLargest + 1];
+int pinned_class(size_t bytes, PinnedClass* out) {
+  static auto* pools = new SlotPool<Pinned>[kMaxDevices][kLargest + 1];  // never destroyed: threads may outlive main
   int device = 0;
   RLT_CUDA_TRY(cudaGetDevice(&device));
   int log = kSmallest;
   while (log <= kLargest && (size_t{1} << log) < bytes) ++log;
   if (device < 0 || device >= kMaxDevices || log > kLargest) return RLT_E_LIMIT;
-  SizeClass& c = classes[device][log];
-  const size_t kept = log >= 24 ? kKeptHuge : log >= 20 ? kKeptLarge : kKept;
-  if (!c.buffers.empty()) {
-    Pinned& oldest = c.buffers[c.next];
-    const cudaError_t state = cudaEventQuery(oldest.done);
-    if (state != cudaSuccess && state != cudaErrorNotReady) return cuda_fail(state);
-    if (state == cudaErrorNotReady) cudaGetLastError();  // "not ready" is an answer, not an error to leave behind
-    if (state == cudaSuccess || c.buffers.size() >= kept) {
-      if (state != cudaSuccess) RLT_CUDA_TRY(cudaEventSynchronize(oldest.done));
-      c.next = (c.next + 1) % c.buffers.size();
-      *out = &oldest;
-      return RLT_OK;
-    }
-  }
-  Pinned fresh;
-  RLT_CUDA_TRY(cudaHostAlloc(&fresh.host, size_t{1} << log, cudaHostAllocDefault));
-  if (const cudaError_t e = cudaEventCreateWithFlags(&fresh.done, cudaEventDisableTiming); e != cudaSuccess) {
-    cudaFreeHost(fresh.host);
-    return cuda_fail(e);
-  }
-  // it takes the place just before the oldest: handed out now, it comes round last
-  c.buffers.insert(c.buffers.begin() + static_cast<std::ptrdiff_t>(c.next), fresh);
-  *out = &c.buffers[c.next];
-  c.next = (c.next + 1) % c.buffers.size();
+  *out = {&pools[device][log], size_t{1} << log, static_cast<size_t>(log >= 24 ? kKeptHuge : log >= 20 ? kKeptLarge : kKept)};
   return RLT_OK;
 }
 
@@ -135,13 +122,17 @@ extern "C" void rlt_event_release(RltEvent* event) {
 extern "C" int rlt_stage_upload(const void* host, size_t bytes, void* device, rlt_stream_t stream) {
   if (bytes == 0) return RLT_OK;
   if (host == nullptr || device == nullptr) return RLT_E_INVALID;
-  const std::lock_guard<std::mutex> lock(rlt::g_mutex);
-  rlt::Pinned* slot = nullptr;
-  const int rc = rlt::acquire(bytes, &slot);
+  rlt::PinnedClass size;
+  int rc = rlt::pinned_class(bytes, &size);
   if (rc != RLT_OK) return rc;
-  std::memcpy(slot->host, host, bytes);
+  rlt::Pinned slot;
+  rc = size.pool->take(&slot, size.kept, [&](rlt::Pinned* fresh) { return rlt::make_pinned(size.bytes, fresh); });
+  if (rc != RLT_OK) return rc;
+  std::memcpy(slot.host, host, bytes);
   const cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  RLT_CUDA_TRY(cudaMemcpyAsync(device, slot->host, bytes, cudaMemcpyHostToDevice, s));
-  RLT_CUDA_TRY(cudaEventRecord(slot->done, s));
+  cudaError_t e = cudaMemcpyAsync(device, slot.host, bytes, cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess) e = cudaEventRecord(slot.done, s);
+  size.pool->give(slot);
+  RLT_CUDA_TRY(e);
   return RLT_OK;
 }

@@ -44,6 +44,7 @@
 
 #include "block_moves.h"
 #include "common.cuh"
+#include "slot_pool.h"
 #include "table_params.cuh"
 
 namespace rlt {
@@ -1166,68 +1167,77 @@ int static_plan_address(void** out) {
 namespace rlt {
 namespace {
 
-// Staging of rlt_kv_handoff_host: per device a ring of slots, each a piece of pinned host memory and a piece of
-// device memory of the same size, allocated at the first call on that device. A slot is written by the host,
-// copied to the device on the caller's stream and read by the launch that follows; its event says when that
-// launch has finished, and the slot is reused only then.
+// Staging of rlt_kv_handoff_host: per device a few slots, each a piece of pinned host memory and a piece of device memory of
+// the same size, allocated together at the first call on that device. A slot is written by the host, copied to the device on the
+// caller's stream and read by the launch that follows; its event says when that launch has finished, and the slot is reused only then.
 constexpr int kHostSlots = 16;
 constexpr size_t kHostSlotBytes = 64 * 1024;
 
-struct HostRing {
-  unsigned char* pinned = nullptr;
+struct HostSlot {
+  unsigned char* host = nullptr;
   unsigned char* device = nullptr;
-  cudaEvent_t done[kHostSlots] = {};
-  int next = 0;
+  cudaEvent_t done = nullptr;
 };
 
-std::mutex g_host_ring_mutex;
+struct HostSlots {
+  std::mutex filling;
+  bool filled = false;
+  SlotPool<HostSlot> pool;
+};
 
-int host_ring(HostRing** out) {
-  constexpr int kMaxDevices = 64;
-  static HostRing rings[kMaxDevices];
-  int device = 0;
-  RLT_CUDA_TRY(cudaGetDevice(&device));
-  if (device < 0 || device >= kMaxDevices) return RLT_E_LIMIT;
-  HostRing& ring = rings[device];
-  if (ring.pinned == nullptr) {
-    void* host = nullptr;
-    void* dev = nullptr;
-    RLT_CUDA_TRY(cudaHostAlloc(&host, kHostSlots * kHostSlotBytes, cudaHostAllocDefault));
-    if (cudaError_t e = cudaMalloc(&dev, kHostSlots * kHostSlotBytes); e != cudaSuccess) {
+// All slots of the current device, into its pool.
+int fill_host_slots(HostSlots& slots) {
+  const std::lock_guard<std::mutex> lock(slots.filling);
+  if (slots.filled) return RLT_OK;
+  void* host = nullptr;
+  void* dev = nullptr;
+  RLT_CUDA_TRY(cudaHostAlloc(&host, kHostSlots * kHostSlotBytes, cudaHostAllocDefault));
+  if (cudaError_t e = cudaMalloc(&dev, kHostSlots * kHostSlotBytes); e != cudaSuccess) {
+    cudaFreeHost(host);
+    return cuda_fail(e);
+  }
+  HostSlot made[kHostSlots];
+  for (int i = 0; i < kHostSlots; ++i) {
+    if (cudaError_t e = cudaEventCreateWithFlags(&made[i].done, cudaEventDisableTiming); e != cudaSuccess) {
+      for (int j = 0; j < i; ++j) cudaEventDestroy(made[j].done);
+      cudaFree(dev);
       cudaFreeHost(host);
       return cuda_fail(e);
     }
-    for (int i = 0; i < kHostSlots; ++i) {
-      if (cudaError_t e = cudaEventCreateWithFlags(&ring.done[i], cudaEventDisableTiming); e != cudaSuccess) {
-        for (int j = 0; j < i; ++j) cudaEventDestroy(ring.done[j]);
-        cudaFree(dev);
-        cudaFreeHost(host);
-        return cuda_fail(e);
-      }
-    }
-    ring.device = static_cast<unsigned char*>(dev);
-    ring.pinned = static_cast<unsigned char*>(host);
+    made[i].host = static_cast<unsigned char*>(host) + i * kHostSlotBytes;
+    made[i].device = static_cast<unsigned char*>(dev) + i * kHostSlotBytes;
   }
-  *out = &ring;
+  for (const HostSlot& slot : made) slots.pool.give(slot);
+  slots.filled = true;
   return RLT_OK;
 }
 
-// The next slot of the current device's ring, free to be written: the launch that last read it (kHostSlots calls ago) is
-// over. The caller holds g_host_ring_mutex and records the slot's event behind the launch that reads it.
-struct HostSlot {
-  unsigned char* host;
-  unsigned char* device;
-  cudaEvent_t done;
-};
-int next_host_slot(HostSlot* out) {
-  HostRing* ring = nullptr;
-  const int rc = host_ring(&ring);
+// A slot of the current device that is free to be written. Its event is recorded behind the launch that reads it, and then it is
+// given back to `pool`.
+int take_host_slot(HostSlot* out, SlotPool<HostSlot>** pool) {
+  constexpr int kMaxDevices = 64;
+  static auto* devices = new HostSlots[kMaxDevices];  // never destroyed: threads may outlive main
+  int device = 0;
+  RLT_CUDA_TRY(cudaGetDevice(&device));
+  if (device < 0 || device >= kMaxDevices) return RLT_E_LIMIT;
+  const int rc = fill_host_slots(devices[device]);
   if (rc != RLT_OK) return rc;
-  const int slot = ring->next;
-  ring->next = (slot + 1) % kHostSlots;
-  RLT_CUDA_TRY(cudaEventSynchronize(ring->done[slot]));
-  *out = {ring->pinned + slot * kHostSlotBytes, ring->device + slot * kHostSlotBytes, ring->done[slot]};
-  return RLT_OK;
+  *pool = &devices[device].pool;
+  return (*pool)->take(out, 0, [](HostSlot*) { return RLT_E_INVALID; });
+}
+
+// Copies a filled slot's first `bytes` bytes to its device memory, runs `launch` behind the copy and gives the slot back.
+template <typename Launch>
+int copy_and_launch(const HostSlot& slot, SlotPool<HostSlot>* pool, size_t bytes, cudaStream_t stream, Launch launch) {
+  cudaError_t e = cudaMemcpyAsync(slot.device, slot.host, bytes, cudaMemcpyHostToDevice, stream);
+  int launched = RLT_E_CUDA;
+  if (e == cudaSuccess) {
+    launched = launch();
+    e = cudaEventRecord(slot.done, stream);  // also when the launch was refused: the copy still reads the slot
+  }
+  pool->give(slot);
+  RLT_CUDA_TRY(e);
+  return launched;
 }
 
 // rlt_kv_handoff_host as one launch from page records: kernel parameters, or a slot where they do not fit those. Records
@@ -1304,18 +1314,16 @@ int rlt_handoff_staged(const RltPool* src, const RltPool* dst, const RltBlockMov
   if (bytes <= kInlineWords * sizeof(int32_t))
     return rlt_move_blocks(RLT_MOVE_DIRECT, src, dst, moves, options, nullptr, 0, stream);
   if (bytes > rlt::kHostSlotBytes) return RLT_MOVE_UNSUITED;
-  const std::lock_guard<std::mutex> lock(rlt::g_host_ring_mutex);
   rlt::HostSlot slot;
-  const int rc = rlt::next_host_slot(&slot);
+  rlt::SlotPool<rlt::HostSlot>* pool = nullptr;
+  const int rc = rlt::take_host_slot(&slot, &pool);
   if (rc != RLT_OK) return rc;
-  const cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   memcpy(slot.host, moves->host_records, bytes);
-  RLT_CUDA_TRY(cudaMemcpyAsync(slot.device, slot.host, bytes, cudaMemcpyHostToDevice, s));
-  RltBlockMoves staged = *moves;
-  staged.device_records = reinterpret_cast<const int32_t*>(slot.device);
-  const int launched = rlt_move_blocks(RLT_MOVE_DIRECT, src, dst, &staged, options, nullptr, 0, stream);
-  RLT_CUDA_TRY(cudaEventRecord(slot.done, s));
-  return launched;
+  return rlt::copy_and_launch(slot, pool, bytes, reinterpret_cast<cudaStream_t>(stream), [&] {
+    RltBlockMoves staged = *moves;
+    staged.device_records = reinterpret_cast<const int32_t*>(slot.device);
+    return rlt_move_blocks(RLT_MOVE_DIRECT, src, dst, &staged, options, nullptr, 0, stream);
+  });
 }
 
 int rlt_kv_handoff_host(const RltPool* src, const RltPool* dst, const RltHostBatch* hb, const RltOptions* options,
@@ -1336,29 +1344,27 @@ int rlt_kv_handoff_host(const RltPool* src, const RltPool* dst, const RltHostBat
   const int by_records = rlt::handoff_from_records(src, dst, hb, options, stream);
   if (by_records != RLT_MOVE_UNSUITED) return by_records;
 
-  const std::lock_guard<std::mutex> lock(rlt::g_host_ring_mutex);
   rlt::HostSlot slot;
-  const int rc = rlt::next_host_slot(&slot);
+  rlt::SlotPool<rlt::HostSlot>* pool = nullptr;
+  const int rc = rlt::take_host_slot(&slot, &pool);
   if (rc != RLT_OK) return rc;
   unsigned char* host = slot.host;
-  unsigned char* dev = slot.device;
   memcpy(host, hb->src_tables, src_bytes);
   memcpy(host + src_bytes, hb->dst_tables, dst_bytes);
   memcpy(host + src_bytes + dst_bytes, hb->tok_begin, range_bytes);
   memcpy(host + src_bytes + dst_bytes + range_bytes, hb->tok_end, range_bytes);
   const cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  RLT_CUDA_TRY(cudaMemcpyAsync(dev, host, total, cudaMemcpyHostToDevice, s));
-  RltBatch batch = {};
-  batch.num_requests = hb->num_requests;
-  batch.table_width = hb->table_width;
-  batch.src_tables = reinterpret_cast<const int32_t*>(dev);
-  batch.dst_tables = reinterpret_cast<const int32_t*>(dev + src_bytes);
-  batch.tok_begin = reinterpret_cast<const int32_t*>(dev + src_bytes + dst_bytes);
-  batch.tok_end = reinterpret_cast<const int32_t*>(dev + src_bytes + dst_bytes + range_bytes);
-  const int launched = rlt::launch_table_copy(rlt::kDirect, src, dst, &batch, options, nullptr, 0, s);
-  // recorded even when the launch was refused: the copy above still reads the slot
-  RLT_CUDA_TRY(cudaEventRecord(slot.done, s));
-  return launched;
+  return rlt::copy_and_launch(slot, pool, total, s, [&] {
+    unsigned char* dev = slot.device;
+    RltBatch batch = {};
+    batch.num_requests = hb->num_requests;
+    batch.table_width = hb->table_width;
+    batch.src_tables = reinterpret_cast<const int32_t*>(dev);
+    batch.dst_tables = reinterpret_cast<const int32_t*>(dev + src_bytes);
+    batch.tok_begin = reinterpret_cast<const int32_t*>(dev + src_bytes + dst_bytes);
+    batch.tok_end = reinterpret_cast<const int32_t*>(dev + src_bytes + dst_bytes + range_bytes);
+    return rlt::launch_table_copy(rlt::kDirect, src, dst, &batch, options, nullptr, 0, s);
+  });
 }
 
 int rlt_kv_handoff(const RltPool* src, const RltPool* dst, const RltBatch* batch,
