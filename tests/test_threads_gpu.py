@@ -91,3 +91,43 @@ def test_a_call_that_finds_a_free_slot_is_not_held_up_by_one_that_waits_for_its_
     late.join(timeout=10)
     assert not late.is_alive() and took < 0.5
     assert a.in_time() and b.in_time() and arrived(pools)
+
+
+def test_a_batch_whose_image_another_thread_lays_out_for_other_planes_packs_its_own(monkeypatch):
+    """Between a pack's look at the layout of its image and its launch another thread may use the same batch for an image of another
+    plane count. (Here the launch itself lets that happen, at the one point where it matters.)"""
+    import random
+
+    from oracle import handoff_oracle as ho
+    from tests.conftest import oracle_pool
+    from tests.gpu_support import GpuPool
+    from vllm_rlt_b200.kernels import kv_handoff as kh
+
+    planes, page, lengths = 4, 4, [30, 11]
+    P = oracle_pool("bf16", (2, 1, 16, 64, page, planes))
+    P.fill_random(np.random.default_rng(3))
+    rng, exits = random.Random(3), []
+    for i, n in enumerate(lengths):
+        assert P.allocate(f"r{i}", n)
+        exits.append([rng.randrange(planes) for _ in range(n)])
+    tables = [P.plane_block_tables(f"r{i}") for i in range(len(lengths))]
+    want = np.concatenate([ho.pack_rows(P, t, 0, n, mode=ho.MODE_DEDUP, exit_planes=e) for t, n, e in zip(tables, lengths, exits)])
+    gp = GpuPool(P)
+    batch = kh.HandoffBatch(tables, None, [(0, n) for n in lengths], block_size=page, exit_planes=exits)
+    workspace, status = kh.dedup_workspace(batch, planes), kh.new_status()
+    packed = torch.zeros(kh.packed_bytes(gp.view(), batch.total_tokens, planes), dtype=torch.uint8, device="cuda")
+    host = kh._lib.load_host()
+
+    class Interrupted:
+        def __getattr__(self, name):
+            return getattr(host, name)
+
+        def move(self, *arguments):
+            host.plan_wire(batch._plan, 2)
+            return host.move(*arguments)
+
+    monkeypatch.setattr(kh._lib, "load_host", Interrupted)
+    kh.kv_pack(gp.view(), batch, packed, mode=kh.MODE_DEDUP, status=status, workspace=workspace)
+    kh.raise_for_status(status)
+    assert np.array_equal(packed.cpu().numpy()[: want.size], want)
+    assert kh.dedup_wire_tokens(workspace) == sum(e + 1 for row in exits for e in row)

@@ -16,6 +16,7 @@
 
 #include <cstddef>
 #include <cstring>
+#include <map>
 #include <memory>
 #include <string>
 #include <vector>
@@ -165,12 +166,16 @@ struct Plan {
   std::vector<int64_t> exit_at;  // [n] index in exits of each request's token 0
   int blocks = 0, words = 0;
   Ints records;
-  int wire_planes = 0;
-  Ints wire;
-  int64_t wire_tokens = 0;
+  // Where the rows of a dedup image lie, by the image's planes: made once each and never changed, because several threads may use
+  // the batch at once, for images of different plane counts.
+  struct Wire {
+    Ints at;
+    int64_t tokens = 0;
+  };
+  std::map<int, Wire> wires;
 
   void make_records();
-  void make_wire(int planes);
+  const Wire& wire(int planes);
 };
 
 void read_side(PyObject* tables, Side& side, int n, int block_size, const std::vector<int64_t>& end) {
@@ -259,8 +264,8 @@ void Plan::make_records() {
 }
 
 // Wire order: request, plane, page; a page's tokens count on every plane up to their exit plane.
-void Plan::make_wire(int planes) {
-  if (wire_planes == planes) return;
+const Plan::Wire& Plan::wire(int planes) {
+  if (const auto made = wires.find(planes); made != wires.end()) return made->second;
   Ints at(static_cast<size_t>(blocks) * planes);
   std::vector<int32_t> carried(planes + 1);
   const int exit_word = kRecordHeader + src.planes + dst.planes;
@@ -288,9 +293,10 @@ void Plan::make_wire(int planes) {
     }
     b = next;
   }
-  wire = std::move(at);
-  wire_tokens = run;
-  wire_planes = planes;
+  Wire& made = wires[planes];
+  made.at = std::move(at);
+  made.tokens = run;
+  return made;
 }
 
 // Plans that are no longer used, for their memory: fresh pages for a large batch's records cost more than writing them. A
@@ -459,24 +465,23 @@ PyObject* plan_arrays(PyObject* const* a) {
 // plan_wire(plan, planes) -> bytes of the wire plan, made at the first call. Tells how a dedup image is laid out.
 PyObject* plan_wire(PyObject* const* a) {
   Plan& p = plan_of(a[0]);
-  if (!p.has_exit) return PyLong_FromLong(0);
-  p.make_wire(static_cast<int>(integer(a[1])));
-  return PyLong_FromSize_t(4 * p.wire.size());
+  const int planes = static_cast<int>(integer(a[1]));
+  return PyLong_FromSize_t(p.has_exit && planes > 0 ? 4 * p.wire(planes).at.size() : 0);
 }
 
-// plan_fits(plan, with wire): whether the launch takes the records as kernel parameters.
+// plan_fits(plan, bytes of the wire plan that goes along): whether the launch takes the records as kernel parameters.
 PyObject* plan_fits(PyObject* const* a) {
   const Plan& p = plan_of(a[0]);
-  const size_t words = p.records.size() + (PyObject_IsTrue(a[1]) ? p.wire.size() : 0);
-  return PyBool_FromLong(words <= static_cast<size_t>(kInlineWords));
+  return PyBool_FromLong(4 * p.records.size() + static_cast<size_t>(integer(a[1])) <= 4 * static_cast<size_t>(kInlineWords));
 }
 
 void* address(PyObject* o) { return o == Py_None ? nullptr : PyLong_AsVoidPtr(o); }
 
-// plan_upload(plan, which, device address, stream) -> code: records (0) or wire plan (1) to device memory.
+// plan_upload(plan, planes, device address, stream) -> code: records (0 planes) or the wire plan of that many to device memory.
 PyObject* plan_upload(PyObject* const* a) {
-  const Plan& p = plan_of(a[0]);
-  const Ints& v = integer(a[1]) == 0 ? p.records : p.wire;
+  Plan& p = plan_of(a[0]);
+  const int planes = static_cast<int>(integer(a[1]));
+  const Ints& v = planes == 0 ? p.records : p.wire(planes).at;
   return PyLong_FromLong(rlt_stage_upload(v.data(), 4 * v.size(), address(a[2]), static_cast<rlt_stream_t>(address(a[3]))));
 }
 
@@ -530,14 +535,16 @@ PyObject* move(PyObject* const* a) {
   m.has_exit = p.has_exit;
   m.num_requests = p.n;
   m.table_width = p.width;
-  if (direction != RLT_MOVE_DIRECT && o.mode == RLT_MODE_DEDUP && !p.wire.empty()) {
-    m.host_wire = p.wire.data();
+  const auto* src = static_cast<const RltPool*>(address(a[1]));
+  const auto* dst = static_cast<const RltPool*>(address(a[2]));
+  const RltPool* image = direction == RLT_MOVE_PACK ? src : direction == RLT_MOVE_SCATTER ? dst : nullptr;
+  if (image != nullptr && o.mode == RLT_MODE_DEDUP && p.has_exit && image->num_planes > 0) {
+    const Plan::Wire& wire = p.wire(image->num_planes);
+    m.host_wire = wire.at.data();
     m.device_wire = static_cast<const int32_t*>(address(a[5]));
-    m.wire_tokens = p.wire_tokens;
+    m.wire_tokens = wire.tokens;
   }
-  return PyLong_FromLong(rlt_move_blocks(static_cast<int>(direction), static_cast<const RltPool*>(address(a[1])),
-                                         static_cast<const RltPool*>(address(a[2])), &m, &o, address(a[17]), integer(a[18]),
-                                         stream_of(a[19])));
+  return PyLong_FromLong(rlt_move_blocks(static_cast<int>(direction), src, dst, &m, &o, address(a[17]), integer(a[18]), stream_of(a[19])));
 }
 
 // ------------------------------------------------------------------------------------------------ other ops

@@ -214,7 +214,7 @@ class HandoffBatch:
         self._device = device
         self._arrays = None   # (device tensor, address of each array) of the RltBatch form
         self._staged = {}     # what has been sent to the device: (tensor, stream it was sent on)
-        if not host.plan_fits(self._plan, False):
+        if not host.plan_fits(self._plan, 0):
             self._send(0, self.metadata_bytes, stream)
 
     def _where(self):
@@ -231,7 +231,7 @@ class HandoffBatch:
                 if stream is not None and at != _stream_ptr(None):
                     # the allocator hands the memory out in the order of its current stream
                     torch.cuda.ExternalStream(at).wait_stream(torch.cuda.current_stream())
-                _lib.check(_lib.load_host().plan_upload(self._plan, min(planes, 1), tensor.data_ptr(), at),
+                _lib.check(_lib.load_host().plan_upload(self._plan, planes, tensor.data_ptr(), at),
                            "rlt_stage_upload")
             self._staged[planes] = (tensor, at)
             return tensor.data_ptr()
@@ -251,7 +251,7 @@ class HandoffBatch:
         if direction != _lib.MOVE_DIRECT and mode == MODE_DEDUP:
             planes = (src if direction == _lib.MOVE_PACK else dst).num_planes
             wire_bytes = host.plan_wire(self._plan, planes)
-        if self._staged or (wire_bytes and not host.plan_fits(self._plan, True)):
+        if self._staged or (wire_bytes and not host.plan_fits(self._plan, wire_bytes)):
             records = self._send(0, self.metadata_bytes, stream)
             if wire_bytes:
                 wire = self._send(planes, wire_bytes, stream)
