@@ -131,3 +131,73 @@ def test_a_batch_whose_image_another_thread_lays_out_for_other_planes_packs_its_
     kh.raise_for_status(status)
     assert np.array_equal(packed.cpu().numpy()[: want.size], want)
     assert kh.dedup_wire_tokens(workspace) == sum(e + 1 for row in exits for e in row)
+
+
+@pytest.mark.parametrize("what", ["host tables", "batch records", "transport tables"])
+def test_the_thread_that_the_gpu_waits_for_runs_while_another_waits_for_the_gpu(pools, what):
+    """More calls than there are staging slots, on a stream that waits for a word another Python thread writes: the calls wait for a
+    slot, and that thread has to get the interpreter meanwhile."""
+    from vllm_rlt_b200 import _lib
+    from vllm_rlt_b200.kernels import kv_handoff as kh
+
+    _, _, sv, dv, tables = pools
+    begin, end = np.zeros(1, np.int32), np.full(1, 4 * PAGES, np.int32)
+    w = Waiting()
+    keep = []
+
+    def call():
+        if what == "host tables":
+            kh.kv_handoff_host(sv, dv, tables, tables, begin, end, stream=w.stream)
+        elif what == "transport tables":
+            side = (tables[0, 0],)
+            _lib.check(_lib.load_host().handoff_requests(sv._address(), dv._address(), [(side, side, 0, 4 * PAGES)], 0, 0, 0, 0, 0,
+                                                         w.stream.cuda_stream), "handoff")
+        else:
+            keep.append(kh.HandoffBatch(tables, tables, [(0, 4 * PAGES)], block_size=4, stream=w.stream))
+
+    def release():
+        time.sleep(0.3)
+        w.go()
+
+    other = threading.Thread(target=release)
+    other.start()
+    began = time.monotonic()
+    for _ in range(70 if what == "batch records" else 20):
+        call()
+    took = time.monotonic() - began
+    other.join(timeout=10)
+    assert w.in_time() and 0.2 < took < 1.2  # the calls did have to wait
+    if what == "batch records":
+        kh.kv_handoff(sv, dv, keep[-1], stream=w.stream)
+        w.stream.synchronize()
+    assert arrived(pools)
+
+
+def test_copies_appended_while_another_thread_submits_do_not_disturb_the_submission():
+    from vllm_rlt_b200.worker.tensors import TensorTransfer
+
+    rows = 256
+    source = torch.arange(rows * 64, dtype=torch.int32, device="cuda").reshape(rows, 64)
+    target = torch.zeros_like(source)
+    mover = TensorTransfer(4096, torch.int32, "cuda:0")
+    for i in range(rows):
+        mover.append(source[i], target[i])
+    torch.cuda.synchronize()
+    stop, wrong = threading.Event(), []
+
+    def submitting():
+        torch.cuda.set_device(0)
+        while not stop.is_set():
+            mover.submit()
+            if not stop.is_set() and mover.max_cols != 64:
+                wrong.append(mover.max_cols)
+
+    thread = threading.Thread(target=submitting)
+    thread.start()
+    for _ in range(2000):
+        mover.append(source[3], target[3])
+    stop.set()
+    thread.join(timeout=20)
+    mover.submit()
+    torch.cuda.synchronize()
+    assert not thread.is_alive() and not wrong and torch.equal(source, target)

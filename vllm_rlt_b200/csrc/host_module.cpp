@@ -67,6 +67,18 @@ void check_code(int code) {
   if (code < 0) fail(PyExc_RuntimeError, rlt_error_string(code));
 }
 
+// f() without the interpreter's lock: every call into the CUDA runtime, for any of them may wait for the GPU (a launch where the
+// launch queue is full, an upload where all staging slots are busy), and the thread that the GPU waits for may be one of this
+// interpreter. Nothing in f touches a Python object; what it reads is held by the caller's arguments and changed by nobody.
+template <typename F>
+auto unlocked(F f) {
+  struct Away {
+    PyThreadState* state = PyEval_SaveThread();
+    ~Away() { PyEval_RestoreThread(state); }
+  } away;
+  return f();
+}
+
 struct Buffer {
   Py_buffer view;
   bool held = false;
@@ -482,7 +494,9 @@ PyObject* plan_upload(PyObject* const* a) {
   Plan& p = plan_of(a[0]);
   const int planes = static_cast<int>(integer(a[1]));
   const Ints& v = planes == 0 ? p.records : p.wire(planes).at;
-  return PyLong_FromLong(rlt_stage_upload(v.data(), 4 * v.size(), address(a[2]), static_cast<rlt_stream_t>(address(a[3]))));
+  void* to = address(a[2]);
+  const auto stream = static_cast<rlt_stream_t>(address(a[3]));
+  return PyLong_FromLong(unlocked([&] { return rlt_stage_upload(v.data(), 4 * v.size(), to, stream); }));
 }
 
 rlt_stream_t stream_of(PyObject* o) {  // None: the current stream of the current device
@@ -544,7 +558,10 @@ PyObject* move(PyObject* const* a) {
     m.device_wire = static_cast<const int32_t*>(address(a[5]));
     m.wire_tokens = wire.tokens;
   }
-  return PyLong_FromLong(rlt_move_blocks(static_cast<int>(direction), src, dst, &m, &o, address(a[17]), integer(a[18]), stream_of(a[19])));
+  void* packed = address(a[17]);
+  const int64_t packed_bytes = integer(a[18]);
+  const rlt_stream_t stream = stream_of(a[19]);
+  return PyLong_FromLong(unlocked([&] { return rlt_move_blocks(static_cast<int>(direction), src, dst, &m, &o, packed, packed_bytes, stream); }));
 }
 
 // ------------------------------------------------------------------------------------------------ other ops
@@ -583,8 +600,10 @@ PyObject* handoff_host(PyObject* const* a) {
   o.plane_begin = static_cast<int32_t>(integer(a[8]));
   o.plane_end = static_cast<int32_t>(integer(a[9]));
   o.status = static_cast<int32_t*>(data_of(a[10]));
-  return PyLong_FromLong(rlt_kv_handoff_host(static_cast<const RltPool*>(address(a[0])), static_cast<const RltPool*>(address(a[1])),
-                                             &hb, &o, stream_of(a[11])));
+  const auto* src = static_cast<const RltPool*>(address(a[0]));
+  const auto* dst = static_cast<const RltPool*>(address(a[1]));
+  const rlt_stream_t stream = stream_of(a[11]);
+  return PyLong_FromLong(unlocked([&] { return rlt_kv_handoff_host(src, dst, &hb, &o, stream); }));
 }
 
 // finalize(pool, planes, tables, rows, layer mask, status, stream) -> code
@@ -599,10 +618,14 @@ PyObject* finalize(PyObject* const* a) {
   if (tables->dim() != 3 || tables->size(1) != integer(a[1]))
     bad_value("tables must be [requests, planes, width] with the pool's plane count");
   if (rows->dim() != 2 || rows->size(1) != 3) bad_value("rows must be [n, 3]: request index, exit plane, token position");
-  return PyLong_FromLong(rlt_kv_finalize(static_cast<const RltPool*>(address(a[0])), tables->data_ptr<int32_t>(),
-                                         static_cast<int32_t>(tables->size(0)), static_cast<int32_t>(tables->size(2)),
-                                         rows->data_ptr<int32_t>(), static_cast<int32_t>(rows->size(0)),
-                                         PyLong_AsUnsignedLongLong(a[4]), static_cast<int32_t*>(data_of(a[5])), stream_of(a[6])));
+  const auto* pool = static_cast<const RltPool*>(address(a[0]));
+  const int32_t *table_data = tables->data_ptr<int32_t>(), *row_data = rows->data_ptr<int32_t>();
+  const auto requests = static_cast<int32_t>(tables->size(0)), width = static_cast<int32_t>(tables->size(2));
+  const auto count = static_cast<int32_t>(rows->size(0));
+  const uint64_t mask = PyLong_AsUnsignedLongLong(a[4]);
+  auto* status = static_cast<int32_t*>(data_of(a[5]));
+  const rlt_stream_t stream = stream_of(a[6]);
+  return PyLong_FromLong(unlocked([&] { return rlt_kv_finalize(pool, table_data, requests, width, row_data, count, mask, status, stream); }));
 }
 
 // ------------------------------------------------------------------------------------------------ tensor transfers
@@ -661,14 +684,23 @@ PyObject* tensor_copy(PyObject* const* a) {
   check_source(source, target.device());
   if (source.numel() == 0) return PyLong_FromLong(RLT_OK);
   const c10::cuda::CUDAGuard guard(target.device());
-  return PyLong_FromLong(rlt_tensor_copy(source.data_ptr(), target.data_ptr(), secondary ? secondary->data_ptr() : nullptr,
-                                         source.numel(), from, to, second, stream_of(Py_None)));
+  const void* in = source.data_ptr();
+  void *out = target.data_ptr(), *also = secondary ? secondary->data_ptr() : nullptr;
+  const int64_t count = source.numel();
+  const rlt_stream_t stream = stream_of(Py_None);
+  return PyLong_FromLong(unlocked([&] { return rlt_tensor_copy(in, out, also, count, from, to, second, stream); }));
 }
 
 // A TensorTransfer's descriptors, collected as copies are appended: the rows of rlt_tensor_transfer's table.
 struct Transfer {
-  std::vector<int64_t> rows;  // 8 per copy
+  using Rows = std::vector<int64_t>;  // 8 per copy
+  std::shared_ptr<Rows> rows = std::make_shared<Rows>();
   int64_t max_rows = 0, max_cols = 0;
+  // The rows to change: a copy of them while a launch, in another thread, still reads the ones there are.
+  Rows& own_rows() {
+    if (rows.use_count() > 1) rows = std::make_shared<Rows>(*rows);
+    return *rows;
+  }
 };
 
 // Base of TensorTransfer: the batch itself. `append` runs once per copy, so it is a method of this type.
@@ -697,7 +729,7 @@ PyObject* copies_reset(PyObject* self, PyObject* const*) {
   if (fresh == nullptr) throw Failure{};
   PyObject* old = c->copies;
   c->copies = fresh;
-  c->batch->rows.clear();
+  c->batch->own_rows().clear();
   c->batch->max_rows = c->batch->max_cols = 0;
   Py_XDECREF(old);
   Py_RETURN_NONE;
@@ -715,7 +747,7 @@ void append_copy(CopiesObject* c, const at::Tensor& source, const at::Tensor& ta
   if (source.is_cuda() && source.device() != device) bad_value("transfer source must be on the configured device");
   if (!checked) check_source(source, device);
   if (source.numel() == 0) return;
-  if (static_cast<long long>(t.rows.size() / 8) >= c->capacity) bad_value("transfer batch is full");
+  if (static_cast<long long>(t.rows->size() / 8) >= c->capacity) bad_value("transfer batch is full");
   const bool flat = dims == 1;
   const int64_t rows = flat ? 1 : source.size(0), cols = source.size(dims - 1);
   const int64_t row[8] = {reinterpret_cast<int64_t>(source.data_ptr()), reinterpret_cast<int64_t>(target.data_ptr()), rows, cols,
@@ -723,7 +755,8 @@ void append_copy(CopiesObject* c, const at::Tensor& source, const at::Tensor& ta
                           flat ? cols * target.stride(0) : target.stride(0), target.stride(dims - 1)};
   const Ref pair(PyTuple_Pack(2, keep_source, keep_target));
   if (PyList_Append(c->copies, pair.p) != 0) throw Failure{};
-  t.rows.insert(t.rows.end(), row, row + 8);
+  Transfer::Rows& list = t.own_rows();
+  list.insert(list.end(), row, row + 8);
   t.max_rows = rows > t.max_rows ? rows : t.max_rows;
   t.max_cols = cols > t.max_cols ? cols : t.max_cols;
 }
@@ -753,17 +786,20 @@ PyObject* copies_append_pieces(PyObject* self, PyObject* const* a) {
 PyObject* copies_launch(PyObject* self, PyObject* const* a) {
   const CopiesObject* c = copies_of(self);
   const Transfer& t = *c->batch;
-  const int count = static_cast<int>(t.rows.size() / 8);
+  const std::shared_ptr<const Transfer::Rows> list = t.rows;
+  const int count = static_cast<int>(list->size() / 8), from = c->from, to = c->to;
   if (count == 0) return PyLong_FromLong(RLT_OK);
   const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(c->device));
+  const rlt_stream_t stream = stream_of(Py_None);
   const int32_t rows = static_cast<int32_t>(t.max_rows), cols = static_cast<int32_t>(t.max_cols);
-  if (c->from == c->to && count <= RLT_INLINE_TRANSFERS && t.max_cols <= INT32_MAX && t.max_rows <= INT32_MAX) {
-    const int rc = rlt_tensor_transfer_inline(t.rows.data(), count, rows, cols, c->from, stream_of(Py_None));
+  if (from == to && count <= RLT_INLINE_TRANSFERS && t.max_cols <= INT32_MAX && t.max_rows <= INT32_MAX) {
+    const int rc = unlocked([&] { return rlt_tensor_transfer_inline(list->data(), count, rows, cols, from, stream); });
     if (rc != RLT_E_LIMIT) return PyLong_FromLong(rc);
   }
   const at::Tensor& table = some_tensor(a[0]);
-  std::memcpy(table.data_ptr(), t.rows.data(), 8 * t.rows.size());
-  return PyLong_FromLong(rlt_tensor_transfer(table.data_ptr<int64_t>(), count, rows, cols, c->from, c->to, stream_of(Py_None)));
+  int64_t* entries = table.data_ptr<int64_t>();
+  std::memcpy(entries, list->data(), 8 * list->size());
+  return PyLong_FromLong(unlocked([&] { return rlt_tensor_transfer(entries, count, rows, cols, from, to, stream); }));
 }
 
 // ------------------------------------------------------------------------------------------------ staging helpers
@@ -886,7 +922,10 @@ PyObject* upload(PyObject* const* a) {
   if (type < 0 || n < 1 || !source.is_cpu() || !target.is_cuda() || !pinned.is_pinned()) Py_RETURN_NONE;
   std::memcpy(pinned.data_ptr(), source.data_ptr(), static_cast<size_t>(n) * source.element_size());
   const c10::cuda::CUDAGuard guard(target.device());
-  check_code(rlt_tensor_copy(pinned.data_ptr(), target.data_ptr(), nullptr, n, type, type, 0, stream_of(Py_None)));
+  const void* from = pinned.data_ptr();
+  void* to = target.data_ptr();
+  const rlt_stream_t stream = stream_of(Py_None);
+  check_code(unlocked([&] { return rlt_tensor_copy(from, to, nullptr, n, type, type, 0, stream); }));
   return THPVariable_Wrap(plain_slice(target, 0, n));
 }
 
@@ -1051,7 +1090,8 @@ PyObject* handoff_requests(PyObject* const* a) {
   o.plane_begin = static_cast<int32_t>(integer(a[5]));
   o.plane_end = static_cast<int32_t>(integer(a[6]));
   const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(integer(a[7])));
-  return PyLong_FromLong(out.launch(o, stream_of(a[8])));
+  const rlt_stream_t stream = stream_of(a[8]);
+  return PyLong_FromLong(unlocked([&] { return out.launch(o, stream); }));
 }
 
 // A recorded event of the library's pool.
@@ -1062,23 +1102,29 @@ struct EventObject {
 PyTypeObject* g_event_type = nullptr;
 
 
-PyObject* record_event(bool timed, rlt_stream_t stream) {
+// An event of the library until a Python object owns it.
+struct RecordedEvent {
   RltEvent* event = nullptr;
-  check_code(rlt_event_record(timed, stream, &event));
-  auto* o = PyObject_New(EventObject, g_event_type);
-  if (o == nullptr) {
-    rlt_event_release(event);
-    throw Failure{};
+  ~RecordedEvent() {
+    if (event != nullptr) rlt_event_release(event);
   }
-  o->event = event;
-  return reinterpret_cast<PyObject*>(o);
-}
+  PyObject* object() {
+    auto* o = PyObject_New(EventObject, g_event_type);
+    if (o == nullptr) throw Failure{};
+    o->event = event;
+    event = nullptr;
+    return reinterpret_cast<PyObject*>(o);
+  }
+};
 
 // event(timed, device, stream) -> an event recorded there
 PyObject* event(PyObject* const* a) {
   const bool timed = PyObject_IsTrue(a[0]) == 1;
   const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(integer(a[1])));
-  return record_event(timed, stream_of(a[2]));
+  const rlt_stream_t stream = stream_of(a[2]);
+  RecordedEvent recorded;
+  check_code(unlocked([&] { return rlt_event_record(timed, stream, &recorded.event); }));
+  return recorded.object();
 }
 
 template <typename V>
@@ -1145,18 +1191,21 @@ PyObject* pull_chunk(PyObject* const* a) {
   o.plane_end = static_cast<int32_t>(head[6]);
   const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(integer(a[4])));
   const rlt_stream_t stream = stream_of(a[5]);
-  const Ref begun(record_event(true, stream));
-  const int code = out.launch(o, stream);
+  RecordedEvent begun, done;
+  const int code = unlocked([&] {
+    int rc = rlt_event_record(true, stream, &begun.event);
+    if (rc == RLT_OK) rc = out.launch(o, stream);
+    for (size_t i = 0; rc == RLT_OK && i < extra.size(); i += 3)
+      rc = rlt_kv_push(reinterpret_cast<void*>(extra[i]), reinterpret_cast<void*>(extra[i + 1]), extra[i + 2], stream);
+    return rc != RLT_OK ? rc : rlt_event_record(true, stream, &done.event);
+  });
   if (code == RLT_MOVE_UNSUITED) Py_RETURN_NONE;
   if (code != RLT_OK) return PyLong_FromLong(code);
   const int64_t layers = (head[4] ? head[4] : src->num_layers) - head[3], planes = (head[6] ? head[6] : dst->num_planes) - head[5];
   int64_t bytes = out.before * planes * 2 * layers * (src->codes.token_bytes + (src->scales.key != nullptr ? src->scales.token_bytes : 0));
-  for (size_t i = 0; i < extra.size(); i += 3) {
-    check_code(rlt_kv_push(reinterpret_cast<void*>(extra[i]), reinterpret_cast<void*>(extra[i + 1]), extra[i + 2], stream));
-    bytes += extra[i + 2];
-  }
-  const Ref done(record_event(true, stream));
-  return Py_BuildValue("OOL", begun.p, done.p, static_cast<long long>(bytes));
+  for (size_t i = 0; i < extra.size(); i += 3) bytes += extra[i + 2];
+  const Ref first(begun.object()), last(done.object());
+  return Py_BuildValue("OOL", first.p, last.p, static_cast<long long>(bytes));
 }
 
 // pack_segments([(address, bytes, device)], [(address, bytes, device)], [(low, high, base)]) -> the (source, destination, bytes)
@@ -1201,20 +1250,27 @@ PyObject* copy_segments(PyObject* const* a) {
   if (PyBytes_AsStringAndSize(a[0], &data, &n) != 0) throw Failure{};
   const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(integer(a[1])));
   const auto* triples = reinterpret_cast<const int64_t*>(data);
-  for (Py_ssize_t left = n / 24; left > 0;) {
-    const int32_t count = static_cast<int32_t>(left < RLT_INLINE_SEGMENTS ? left : RLT_INLINE_SEGMENTS);
-    const int rc = rlt_copy_segments_inline(triples, count, stream_of(a[2]));
-    if (rc != RLT_OK) return PyLong_FromLong(rc);
-    triples += 3 * static_cast<ptrdiff_t>(count);
-    left -= count;
-  }
-  return PyLong_FromLong(RLT_OK);
+  const rlt_stream_t stream = stream_of(a[2]);
+  return PyLong_FromLong(unlocked([&] {
+    int rc = RLT_OK;
+    for (Py_ssize_t left = n / 24; rc == RLT_OK && left > 0;) {
+      const int32_t count = static_cast<int32_t>(left < RLT_INLINE_SEGMENTS ? left : RLT_INLINE_SEGMENTS);
+      rc = rlt_copy_segments_inline(triples, count, stream);
+      triples += 3 * static_cast<ptrdiff_t>(count);
+      left -= count;
+    }
+    return rc;
+  }));
 }
 
 // push(source, destination, bytes, device, stream) -> code
 PyObject* push(PyObject* const* a) {
   const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(integer(a[3])));
-  return PyLong_FromLong(rlt_kv_push(address(a[0]), address(a[1]), integer(a[2]), stream_of(a[4])));
+  const void* from = address(a[0]);
+  void* to = address(a[1]);
+  const int64_t bytes = integer(a[2]);
+  const rlt_stream_t stream = stream_of(a[4]);
+  return PyLong_FromLong(unlocked([&] { return rlt_kv_push(from, to, bytes, stream); }));
 }
 
 // post(slot address, 56-byte body, stamp, device, stream) -> code
@@ -1224,7 +1280,10 @@ PyObject* post(PyObject* const* a) {
   if (PyBytes_AsStringAndSize(a[1], &body, &n) != 0) throw Failure{};
   if (n != 56) bad_value("a message body has 56 bytes");
   const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(integer(a[3])));
-  return PyLong_FromLong(rlt_kv_post(address(a[0]), reinterpret_cast<const uint8_t*>(body), PyLong_AsUnsignedLongLong(a[2]), stream_of(a[4])));
+  void* slot = address(a[0]);
+  const uint64_t stamp = PyLong_AsUnsignedLongLong(a[2]);
+  const rlt_stream_t stream = stream_of(a[4]);
+  return PyLong_FromLong(unlocked([&] { return rlt_kv_post(slot, reinterpret_cast<const uint8_t*>(body), stamp, stream); }));
 }
 
 // ------------------------------------------------------------------------------------------------ the module
@@ -1401,16 +1460,14 @@ PyType_Slot kWritesSlots[] = {{Py_tp_new, reinterpret_cast<void*>(PyType_Generic
                               {0, nullptr}};
 
 PyObject* event_query(PyObject* self, PyObject* const*) {
-  const int fired = rlt_event_query(reinterpret_cast<EventObject*>(self)->event);
+  RltEvent* event = reinterpret_cast<EventObject*>(self)->event;
+  const int fired = unlocked([&] { return rlt_event_query(event); });
   check_code(fired);
   return PyBool_FromLong(fired);
 }
 PyObject* event_synchronize(PyObject* self, PyObject* const*) {
-  int code = RLT_OK;
-  Py_BEGIN_ALLOW_THREADS;
-  code = rlt_event_wait(reinterpret_cast<EventObject*>(self)->event);
-  Py_END_ALLOW_THREADS;
-  check_code(code);
+  RltEvent* event = reinterpret_cast<EventObject*>(self)->event;
+  check_code(unlocked([&] { return rlt_event_wait(event); }));
   Py_RETURN_NONE;
 }
 PyObject* event_elapsed_time(PyObject* self, PyObject* const* a) {
