@@ -16,14 +16,14 @@ PAGES = 1000              # 8 words a page: more than the kernel parameters hold
 
 
 class Waiting:
-    """A stream whose work waits until the host says ``go``."""
+    """A stream whose work, from now on, waits until the host says ``go``."""
 
-    def __init__(self):
+    def __init__(self, stream=None):
         from vllm_rlt_b200.kernels import kv_handoff as kh
 
         self.flag = torch.zeros(1, dtype=torch.int64, pin_memory=True)
         self.status = kh.new_status()
-        self.stream = torch.cuda.Stream()
+        self.stream = stream or torch.cuda.Stream()
         self.stream.wait_stream(torch.cuda.current_stream())
         kh.kv_wait(self.flag.data_ptr(), 1, LIMIT_NS, self.status, stream=self.stream)
 
@@ -201,3 +201,61 @@ def test_copies_appended_while_another_thread_submits_do_not_disturb_the_submiss
     mover.submit()
     torch.cuda.synchronize()
     assert not thread.is_alive() and not wrong and torch.equal(source, target)
+
+
+def test_a_batch_used_on_another_stream_waits_for_its_records_and_for_nothing_else(pools):
+    from vllm_rlt_b200.kernels import kv_handoff as kh
+
+    _, _, sv, dv, tables = pools
+    for variant in (0, 5):  # the records, and the padded arrays of the table-driven kernels
+        own, third = torch.cuda.Stream(), torch.cuda.Stream()
+        batch = kh.HandoffBatch(tables, tables, [(0, 4 * PAGES)], block_size=4, stream=own)
+        if variant:
+            kh.kv_handoff(sv, dv, batch, variant=variant, stream=own)
+        w = Waiting(own)  # work that has nothing to do with the batch
+        for stream in (third, torch.cuda.current_stream()):
+            kh.kv_handoff(sv, dv, batch, variant=variant, stream=stream)
+            done = stream.record_event()
+            began = time.monotonic()
+            while not done.query() and time.monotonic() - began < 0.5:
+                time.sleep(0.001)
+            assert done.query() and arrived(pools)
+        w.go()
+        assert w.in_time()
+
+
+@pytest.mark.parametrize("default", [True, False])
+def test_a_use_on_any_other_stream_does_wait_for_the_records(pools, default):
+    from vllm_rlt_b200.kernels import kv_handoff as kh
+
+    _, _, sv, dv, tables = pools
+    w = Waiting()
+    batch = kh.HandoffBatch(tables, tables, [(0, 4 * PAGES)], block_size=4, stream=w.stream)  # sent behind the wait
+    user = torch.cuda.current_stream() if default else torch.cuda.Stream()
+    kh.kv_handoff(sv, dv, batch, stream=user)
+    done = user.record_event()
+    time.sleep(0.2)
+    assert not done.query()
+    w.go()
+    user.synchronize()
+    assert w.in_time() and arrived(pools)
+
+
+def test_a_batch_that_is_dropped_keeps_its_records_until_every_stream_has_used_them(pools):
+    from vllm_rlt_b200.kernels import kv_handoff as kh
+
+    _, _, sv, dv, tables = pools
+    own = torch.cuda.Stream()
+    batch = kh.HandoffBatch(tables, tables, [(0, 4 * PAGES)], block_size=4, stream=own)
+    size = batch.metadata_bytes
+    w = Waiting()
+    kh.kv_handoff(sv, dv, batch, stream=w.stream)
+    del batch
+    with torch.cuda.stream(own):
+        # the memory's next owner writes it; records of zeros name no token
+        others = [torch.zeros(size, dtype=torch.uint8, device="cuda") for _ in range(8)]
+    time.sleep(0.1)
+    w.go()
+    assert w.in_time() and arrived(pools)
+    own.synchronize()
+    assert not any(bool(t.any()) for t in others)

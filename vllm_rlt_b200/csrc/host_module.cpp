@@ -1470,6 +1470,12 @@ PyObject* event_synchronize(PyObject* self, PyObject* const*) {
   check_code(unlocked([&] { return rlt_event_wait(event); }));
   Py_RETURN_NONE;
 }
+PyObject* event_order(PyObject* self, PyObject* const* a) {
+  RltEvent* event = reinterpret_cast<EventObject*>(self)->event;
+  const rlt_stream_t stream = stream_of(a[0]);
+  check_code(unlocked([&] { return rlt_event_order(event, stream); }));
+  Py_RETURN_NONE;
+}
 PyObject* event_elapsed_time(PyObject* self, PyObject* const* a) {
   if (Py_TYPE(a[0]) != g_event_type) fail(PyExc_TypeError, "expected an event");
   float ms = 0.0f;
@@ -1482,7 +1488,7 @@ void event_dealloc(PyObject* self) {
   PyObject_Free(self);
   Py_DECREF(type);
 }
-PyMethodDef kEventMethods[] = {RLT_METHOD("query", event_query, 0), RLT_METHOD("synchronize", event_synchronize, 0),
+PyMethodDef kEventMethods[] = {RLT_METHOD("query", event_query, 0), RLT_METHOD("synchronize", event_synchronize, 0), RLT_METHOD("order", event_order, 1),
                                RLT_METHOD("elapsed_time", event_elapsed_time, 1), {nullptr, nullptr, 0, nullptr}};
 PyType_Slot kEventSlots[] = {{Py_tp_dealloc, reinterpret_cast<void*>(event_dealloc)}, {Py_tp_methods, kEventMethods}, {0, nullptr}};
 PyType_Spec kEventType = {"_host.Event", sizeof(EventObject), 0, Py_TPFLAGS_DEFAULT | Py_TPFLAGS_DISALLOW_INSTANTIATION, kEventSlots};

@@ -101,6 +101,11 @@ extern "C" int rlt_event_wait(RltEvent* event) {
   return RLT_OK;
 }
 
+extern "C" int rlt_event_order(RltEvent* event, rlt_stream_t stream) {
+  RLT_CUDA_TRY(cudaStreamWaitEvent(reinterpret_cast<cudaStream_t>(stream), event->event, 0));
+  return RLT_OK;
+}
+
 extern "C" int rlt_event_elapsed(RltEvent* from, RltEvent* to, float* milliseconds) {
   RLT_CUDA_TRY(cudaEventElapsedTime(milliseconds, from->event, to->event));
   return RLT_OK;

@@ -30,6 +30,7 @@ typedef struct RltEvent RltEvent;
 RLT_API int rlt_event_record(int timed, rlt_stream_t stream, RltEvent** out);
 RLT_API int rlt_event_query(RltEvent* event);  // 1: fired, 0: not yet, negative: RLT_E_*
 RLT_API int rlt_event_wait(RltEvent* event);   // on the host
+RLT_API int rlt_event_order(RltEvent* event, rlt_stream_t stream);  // what is queued on `stream` from now on comes after it
 RLT_API int rlt_event_elapsed(RltEvent* from, RltEvent* to, float* milliseconds);
 RLT_API void rlt_event_release(RltEvent* event);
 

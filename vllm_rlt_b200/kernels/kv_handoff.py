@@ -11,7 +11,9 @@ with the messages of ``kv_segments`` (vllm_rlt/pd/transport.py:29-47).
 
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
+import threading
 from dataclasses import dataclass, field
 from typing import Sequence
 
@@ -28,6 +30,14 @@ def _stream_ptr(stream) -> int:
     if isinstance(stream, int):
         return stream
     return stream.cuda_stream
+
+
+def _on_stream(address: int):
+    """Context in which the stream at ``address`` is the current device's current one. (``ExternalStream`` takes no address of 0: it
+    makes a new stream then.)"""
+    if address == _stream_ptr(None):
+        return contextlib.nullcontext()
+    return torch.cuda.stream(torch.cuda.default_stream() if address in (0, 1) else torch.cuda.ExternalStream(address))
 
 
 def _raw_stream(stream):
@@ -178,6 +188,35 @@ class _PinnedPool:
 _PINNED = _PinnedPool()
 
 
+class _Sent:
+    """Device memory of a batch and the stream it was filled on, which is also the one the allocator takes it back in the order of.
+
+    A use on another stream comes behind the fill alone (``before``), not behind what else that stream has been given since, and the
+    memory goes back behind that use (``after``)."""
+
+    def __init__(self, tensor, stream: int):
+        self.tensor, self.stream = tensor, stream
+        self._event = _lib.load_host().event
+        self._filled = self._event(False, tensor.device.index, stream)
+        self._used = {}  # other streams: an event behind the last use there
+
+    def before(self, stream: int) -> int:
+        if stream != self.stream:
+            self._filled.order(stream)
+        return self.tensor.data_ptr()
+
+    def after(self, stream: int) -> None:
+        if stream != self.stream:
+            self._used[stream] = self._event(False, self.tensor.device.index, stream)
+
+    def __del__(self):
+        try:
+            for event in self._used.values():
+                event.order(self.stream)
+        except Exception:  # the caller's stream is gone, and with it whatever was queued there
+            pass
+
+
 class HandoffBatch:
     """Per-request tables and ranges of a batch, checked on the host and kept there as the records the kernels read.
 
@@ -213,33 +252,27 @@ class HandoffBatch:
         self._planned_exits = self.exit_count
         self._device = device
         self._arrays = None   # (device tensor, address of each array) of the RltBatch form
-        self._staged = {}     # what has been sent to the device: (tensor, stream it was sent on)
+        self._arrays_sent = None
+        self._staged = {}     # what has been sent to the device, by the image's planes (0: the records)
+        self._sending = threading.Lock()
         if not host.plan_fits(self._plan, 0):
             self._send(0, self.metadata_bytes, stream)
 
     def _where(self):
         return torch.device("cuda", torch.cuda.current_device()) if self._device is None else torch.device(self._device)
 
-    def _send(self, planes: int, nbytes: int, stream) -> int:
-        """The records (``planes`` 0), or the wire plan of ``planes`` planes, on the device: sent once; a use on another
-        stream than they were sent on waits for the copy."""
-        hit = self._staged.get(planes)
-        if hit is None:
-            with torch.cuda.device(self._where()):
-                at = _stream_ptr(stream)
-                tensor = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
-                if stream is not None and at != _stream_ptr(None):
-                    # the allocator hands the memory out in the order of its current stream
-                    torch.cuda.ExternalStream(at).wait_stream(torch.cuda.current_stream())
-                _lib.check(_lib.load_host().plan_upload(self._plan, planes, tensor.data_ptr(), at),
-                           "rlt_stage_upload")
-            self._staged[planes] = (tensor, at)
-            return tensor.data_ptr()
-        tensor, sent_on = hit
-        now = _stream_ptr(stream)
-        if now != sent_on:
-            torch.cuda.ExternalStream(now).wait_stream(torch.cuda.ExternalStream(sent_on))
-        return tensor.data_ptr()
+    def _send(self, planes: int, nbytes: int, stream) -> _Sent:
+        """The records (``planes`` 0), or the wire plan of ``planes`` planes, on the device: sent once."""
+        with self._sending:
+            sent = self._staged.get(planes)
+            if sent is None:
+                with torch.cuda.device(self._where()):
+                    at = _stream_ptr(stream)
+                    with _on_stream(at):  # memory of the stream that fills it
+                        tensor = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+                    _lib.check(_lib.load_host().plan_upload(self._plan, planes, tensor.data_ptr(), at), "rlt_stage_upload")
+                    sent = self._staged[planes] = _Sent(tensor, at)
+        return sent
 
     def _move(self, direction, src, dst, *, mode, layer_begin=0, layer_end=0, wire_planes=0, plane_begin=0, plane_end=0,
               mask=0, status=None, grid_limit=0, variant=0, workspace=None, packed=0, packed_bytes=0, stream=None) -> int:
@@ -251,13 +284,20 @@ class HandoffBatch:
         if direction != _lib.MOVE_DIRECT and mode == MODE_DEDUP:
             planes = (src if direction == _lib.MOVE_PACK else dst).num_planes
             wire_bytes = host.plan_wire(self._plan, planes)
+        used, on = (), 0
         if self._staged or (wire_bytes and not host.plan_fits(self._plan, wire_bytes)):
-            records = self._send(0, self.metadata_bytes, stream)
+            on = _stream_ptr(stream)
+            used = (self._send(0, self.metadata_bytes, stream),)
+            records = used[0].before(on)
             if wire_bytes:
-                wire = self._send(planes, wire_bytes, stream)
-        return host.move(direction, src and src._address(), dst and dst._address(), self._plan, records, wire, mode, layer_begin,
+                used += (self._send(planes, wire_bytes, stream),)
+                wire = used[1].before(on)
+        code = host.move(direction, src and src._address(), dst and dst._address(), self._plan, records, wire, mode, layer_begin,
                          layer_end, wire_planes, plane_begin, plane_end, mask, status, grid_limit, variant, workspace, packed,
                          packed_bytes, _raw_stream(stream))
+        for sent in used:
+            sent.after(on)
+        return code
 
     def _send_arrays(self):
         """The padded arrays of the RltBatch form, in one device buffer: one pinned staging buffer, one copy."""
@@ -270,15 +310,24 @@ class HandoffBatch:
         with torch.cuda.device(device), torch.cuda.stream(torch.cuda.current_stream(device)):
             dev.copy_(staging.buffer[:size], non_blocking=True)
             staging.release()
+            if dev.is_cuda:
+                self._arrays_sent = _Sent(dev, _stream_ptr(None))
         base = dev.data_ptr()
         self._arrays = (dev, {name: base + at for name, at in offsets.items()})
 
-    def _struct_on(self, stream) -> _lib.RltBatch:
-        """``as_struct`` for a launch on ``stream``: arrays that are not on the device yet are sent on that stream."""
-        if self._arrays is None and stream is not None:
-            with torch.cuda.stream(torch.cuda.ExternalStream(_stream_ptr(stream))):
-                self._send_arrays()
-        return self.as_struct()
+    @contextlib.contextmanager
+    def _struct_on(self, stream):
+        """``as_struct`` for one launch on ``stream``: arrays that are not on the device yet are sent on that stream."""
+        on = _stream_ptr(stream)
+        with self._sending if self._plan is not None else contextlib.nullcontext():
+            if self._arrays is None:
+                with _on_stream(on):
+                    self._send_arrays()
+        if self._arrays_sent is not None:
+            self._arrays_sent.before(on)
+        yield self.as_struct()
+        if self._arrays_sent is not None:
+            self._arrays_sent.after(on)
 
     @property
     def _dev(self):
@@ -328,7 +377,7 @@ class HandoffBatch:
         self.metadata_bytes = 0
         arrays = (src_tables, dst_tables, tok_begin, tok_end, exit_planes, exit_offsets)  # kept alive with the batch
         names = ("src_tables", "dst_tables", "tok_begin", "tok_end", "exit_planes", "exit_offsets")
-        self._plan = None
+        self._plan = self._arrays_sent = None
         self._arrays = (arrays, {name: t.data_ptr() for name, t in zip(names, arrays) if t is not None})
         self.has_exit = exit_planes is not None
         self.exit_count = exit_planes.numel() if exit_planes is not None else 0
@@ -419,9 +468,10 @@ def kv_handoff(src: PoolView, dst: PoolView, batch: HandoffBatch, *, mode=MODE_A
     if rc != _lib.MOVE_UNSUITED:
         return _lib.check(rc, "rlt_kv_handoff")
     lib = _lib.load()
-    s, d, b = src.as_struct(), dst.as_struct(), batch._struct_on(stream)
+    s, d = src.as_struct(), dst.as_struct()
     o = _options(mode, layer_begin, layer_end, 0, status, grid_limit, variant, None, plane_begin, plane_end, mask)
-    _lib.check(lib.rlt_kv_handoff(C.byref(s), C.byref(d), C.byref(b), C.byref(o), _stream_ptr(stream)), "rlt_kv_handoff")
+    with batch._struct_on(stream) as b:
+        _lib.check(lib.rlt_kv_handoff(C.byref(s), C.byref(d), C.byref(b), C.byref(o), _stream_ptr(stream)), "rlt_kv_handoff")
 
 
 def host_batch_limit() -> int:
@@ -472,9 +522,10 @@ def kv_pack_to(src: PoolView, batch: HandoffBatch, out_ptr: int, out_bytes: int,
     if rc != _lib.MOVE_UNSUITED:
         return _lib.check(rc, "rlt_kv_pack")
     lib = _lib.load()
-    s, b = src.as_struct(), batch._struct_on(stream)
+    s = src.as_struct()
     o = _options(mode, layer_begin, layer_end, wire_planes, status, grid_limit, variant, workspace)
-    _lib.check(lib.rlt_kv_pack(C.byref(s), C.byref(b), C.byref(o), out_ptr, out_bytes, _stream_ptr(stream)), "rlt_kv_pack")
+    with batch._struct_on(stream) as b:
+        _lib.check(lib.rlt_kv_pack(C.byref(s), C.byref(b), C.byref(o), out_ptr, out_bytes, _stream_ptr(stream)), "rlt_kv_pack")
 
 
 def kv_scatter(packed: torch.Tensor, dst: PoolView, batch: HandoffBatch, *, mode=MODE_ALL_PLANES, layer_begin=0,
@@ -489,10 +540,11 @@ def kv_scatter(packed: torch.Tensor, dst: PoolView, batch: HandoffBatch, *, mode
     if rc != _lib.MOVE_UNSUITED:
         return _lib.check(rc, "rlt_kv_scatter")
     lib = _lib.load()
-    d, b = dst.as_struct(), batch._struct_on(stream)
-    o = _options(mode, layer_begin, layer_end, wire_planes, status,
-                 grid_limit, variant, workspace)
-    _lib.check(lib.rlt_kv_scatter(packed.data_ptr(), packed.numel(), C.byref(d), C.byref(b), C.byref(o), _stream_ptr(stream)), "rlt_kv_scatter")
+    d = dst.as_struct()
+    o = _options(mode, layer_begin, layer_end, wire_planes, status, grid_limit, variant, workspace)
+    with batch._struct_on(stream) as b:
+        _lib.check(lib.rlt_kv_scatter(packed.data_ptr(), packed.numel(), C.byref(d), C.byref(b), C.byref(o), _stream_ptr(stream)),
+                   "rlt_kv_scatter")
 
 
 def kv_finalize(pool: PoolView, tables: torch.Tensor, rows: torch.Tensor, *, layers=None, status=None, stream=None) -> None:
