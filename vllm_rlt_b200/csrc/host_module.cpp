@@ -445,14 +445,7 @@ PyObject* plan_layout(PyObject* const* a) {
   return Py_BuildValue("nO", static_cast<Py_ssize_t>(l.bytes), names.p);
 }
 
-PyObject* plan_arrays(PyObject* const* a) {
-  const Plan& p = plan_of(a[0]);
-  const Layout l = layout_of(p);
-  Buffer b;
-  if (PyObject_GetBuffer(a[1], &b.view, PyBUF_WRITABLE) != 0) throw Failure{};
-  b.held = true;
-  if (static_cast<size_t>(b.view.len) < l.bytes) bad_value("staging buffer too small");
-  char* out = static_cast<char*>(b.view.buf);
+void write_arrays(const Plan& p, const Layout& l, char* out) {
   std::memset(out, 0, l.bytes);
   auto tables = [&](const Side& side, size_t at) {
     for (int r = 0; r < p.n; ++r) {
@@ -471,6 +464,16 @@ PyObject* plan_arrays(PyObject* const* a) {
     std::memcpy(out + l.offsets, p.exit_at.data(), 8 * static_cast<size_t>(p.n));
     if (!p.exits.empty()) std::memcpy(out + l.exits, p.exits.data(), 4 * p.exits.size());
   }
+}
+
+PyObject* plan_arrays(PyObject* const* a) {
+  const Plan& p = plan_of(a[0]);
+  const Layout l = layout_of(p);
+  Buffer b;
+  if (PyObject_GetBuffer(a[1], &b.view, PyBUF_WRITABLE) != 0) throw Failure{};
+  b.held = true;
+  if (static_cast<size_t>(b.view.len) < l.bytes) bad_value("staging buffer too small");
+  write_arrays(p, l, static_cast<char*>(b.view.buf));
   Py_RETURN_NONE;
 }
 
@@ -489,14 +492,23 @@ PyObject* plan_fits(PyObject* const* a) {
 
 void* address(PyObject* o) { return o == Py_None ? nullptr : PyLong_AsVoidPtr(o); }
 
-// plan_upload(plan, planes, device address, stream) -> code: records (0 planes) or the wire plan of that many to device memory.
+// plan_upload(plan, planes, device address, stream) -> code: records (0 planes), the wire plan of that many or the padded arrays (-1) to
+// device memory.
 PyObject* plan_upload(PyObject* const* a) {
   Plan& p = plan_of(a[0]);
   const int planes = static_cast<int>(integer(a[1]));
-  const Ints& v = planes == 0 ? p.records : p.wire(planes).at;
   void* to = address(a[2]);
   const auto stream = static_cast<rlt_stream_t>(address(a[3]));
-  return PyLong_FromLong(unlocked([&] { return rlt_stage_upload(v.data(), 4 * v.size(), to, stream); }));
+  std::vector<char> arrays;
+  if (planes < 0) {
+    const Layout l = layout_of(p);
+    arrays.resize(l.bytes);
+    write_arrays(p, l, arrays.data());
+  }
+  const Ints* list = planes < 0 ? nullptr : planes == 0 ? &p.records : &p.wire(planes).at;
+  return PyLong_FromLong(unlocked([&] {
+    return list == nullptr ? rlt_stage_upload(arrays.data(), arrays.size(), to, stream) : rlt_stage_upload(list->data(), 4 * list->size(), to, stream);
+  }));
 }
 
 rlt_stream_t stream_of(PyObject* o) {  // None: the current stream of the current device
@@ -513,6 +525,14 @@ const at::Tensor* tensor_of(PyObject* o) {
 void* data_of(PyObject* o) {
   const at::Tensor* t = tensor_of(o);
   return t == nullptr ? nullptr : t->data_ptr();
+}
+
+// capture(stream) -> the id of the graph capture that it takes part in, 0 if it does not
+PyObject* capture(PyObject* const* a) {
+  const rlt_stream_t stream = stream_of(a[0]);
+  uint64_t id = 0;
+  check_code(unlocked([&] { return rlt_capture_id(stream, &id); }));
+  return PyLong_FromUnsignedLongLong(id);
 }
 
 // move(direction, source pool, destination pool, plan, records, wire plan, mode, layer_begin, layer_end, wire_planes,
@@ -1314,6 +1334,7 @@ PyMethodDef kMethods[] = {
     RLT_ENTRY("plan_wire", plan_wire, 2),
     RLT_ENTRY("plan_fits", plan_fits, 2),
     RLT_ENTRY("plan_upload", plan_upload, 4),
+    RLT_ENTRY("capture", capture, 1),
     RLT_ENTRY("move", move, 20),
     RLT_ENTRY("handoff_host", handoff_host, 12),
     RLT_ENTRY("finalize", finalize, 7),

@@ -54,6 +54,70 @@ int pinned_class(size_t bytes, PinnedClass* out) {
   return RLT_OK;
 }
 
+// Buffers that captured copies read: a replay may come at any time, so they are the graph's until it is destroyed. Then they are kept
+// for later captures, as many as were in graphs at once: the runtime allows no call of its own, like one that frees memory, where it
+// tells of a graph's end.
+struct GraphBuffers {
+  std::mutex mutex;
+  std::vector<void*> idle;
+};
+GraphBuffers& graph_buffers(int log) {
+  static auto* all = new GraphBuffers[kLargest + 1];
+  return all[log];
+}
+struct GraphBuffer {
+  void* host;
+  int log;
+};
+void graph_is_gone(void* p) {
+  auto* buffer = static_cast<GraphBuffer*>(p);
+  GraphBuffers& of = graph_buffers(buffer->log);
+  {
+    const std::lock_guard<std::mutex> lock(of.mutex);
+    of.idle.push_back(buffer->host);
+  }
+  delete buffer;
+}
+
+int upload_in_capture(const void* host, size_t bytes, void* device, cudaStream_t stream, cudaGraph_t graph) {
+  int log = kSmallest;
+  while (log <= kLargest && (size_t{1} << log) < bytes) ++log;
+  if (log > kLargest) return RLT_E_LIMIT;
+  auto* buffer = new GraphBuffer{nullptr, log};
+  GraphBuffers& of = graph_buffers(log);
+  {
+    const std::lock_guard<std::mutex> lock(of.mutex);
+    if (!of.idle.empty()) {
+      buffer->host = of.idle.back();
+      of.idle.pop_back();
+    }
+  }
+  const OutsideCapture outside;
+  cudaError_t e = cudaSuccess;
+  // portable: graphs of another device may get it after this one
+  if (buffer->host == nullptr) e = cudaHostAlloc(&buffer->host, size_t{1} << log, cudaHostAllocPortable);
+  cudaUserObject_t owner = nullptr;
+  if (e == cudaSuccess) {
+    std::memcpy(buffer->host, host, bytes);
+    e = cudaUserObjectCreate(&owner, buffer, graph_is_gone, 1, cudaUserObjectNoDestructorSync);
+  }
+  if (e != cudaSuccess) {
+    if (buffer->host != nullptr) {
+      graph_is_gone(buffer);
+    } else {
+      delete buffer;
+    }
+    return cuda_fail(e);
+  }
+  e = cudaGraphRetainUserObject(graph, owner, 1, cudaGraphUserObjectMove);
+  if (e != cudaSuccess) {
+    cudaUserObjectRelease(owner, 1);
+    return cuda_fail(e);
+  }
+  RLT_CUDA_TRY(cudaMemcpyAsync(device, buffer->host, bytes, cudaMemcpyHostToDevice, stream));
+  return RLT_OK;
+}
+
 constexpr size_t kPooledEvents = 256;  // per device and kind; more than that are destroyed when given back
 std::mutex g_event_mutex;
 std::vector<cudaEvent_t> g_events[kMaxDevices][2];
@@ -79,6 +143,7 @@ extern "C" int rlt_event_record(int timed, rlt_stream_t stream, RltEvent** out) 
       pool.pop_back();
     }
   }
+  const rlt::OutsideCapture outside;
   if (event == nullptr) RLT_CUDA_TRY(cudaEventCreateWithFlags(&event, timed ? cudaEventDefault : cudaEventDisableTiming));
   if (const cudaError_t e = cudaEventRecord(event, reinterpret_cast<cudaStream_t>(stream)); e != cudaSuccess) {
     cudaEventDestroy(event);
@@ -89,6 +154,7 @@ extern "C" int rlt_event_record(int timed, rlt_stream_t stream, RltEvent** out) 
 }
 
 extern "C" int rlt_event_query(RltEvent* event) {
+  const rlt::OutsideCapture outside;
   const cudaError_t e = cudaEventQuery(event->event);
   if (e == cudaSuccess) return 1;
   if (e != cudaErrorNotReady) return rlt::cuda_fail(e);
@@ -97,6 +163,7 @@ extern "C" int rlt_event_query(RltEvent* event) {
 }
 
 extern "C" int rlt_event_wait(RltEvent* event) {
+  const rlt::OutsideCapture outside;
   RLT_CUDA_TRY(cudaEventSynchronize(event->event));
   return RLT_OK;
 }
@@ -127,6 +194,11 @@ extern "C" void rlt_event_release(RltEvent* event) {
 extern "C" int rlt_stage_upload(const void* host, size_t bytes, void* device, rlt_stream_t stream) {
   if (bytes == 0) return RLT_OK;
   if (host == nullptr || device == nullptr) return RLT_E_INVALID;
+  const cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  cudaGraph_t graph = nullptr;
+  RLT_CUDA_TRY(cudaStreamGetCaptureInfo(s, &capturing, nullptr, &graph));
+  if (capturing != cudaStreamCaptureStatusNone) return rlt::upload_in_capture(host, bytes, device, s, graph);
   rlt::PinnedClass size;
   int rc = rlt::pinned_class(bytes, &size);
   if (rc != RLT_OK) return rc;
@@ -134,10 +206,17 @@ extern "C" int rlt_stage_upload(const void* host, size_t bytes, void* device, rl
   rc = size.pool->take(&slot, size.kept, [&](rlt::Pinned* fresh) { return rlt::make_pinned(size.bytes, fresh); });
   if (rc != RLT_OK) return rc;
   std::memcpy(slot.host, host, bytes);
-  const cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   cudaError_t e = cudaMemcpyAsync(device, slot.host, bytes, cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaEventRecord(slot.done, s);
   size.pool->give(slot);
   RLT_CUDA_TRY(e);
+  return RLT_OK;
+}
+
+extern "C" int rlt_capture_id(rlt_stream_t stream, uint64_t* id) {
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  unsigned long long of = 0;
+  RLT_CUDA_TRY(cudaStreamGetCaptureInfo(reinterpret_cast<cudaStream_t>(stream), &capturing, &of));
+  *id = capturing == cudaStreamCaptureStatusNone ? 0 : of;
   return RLT_OK;
 }

@@ -11,8 +11,10 @@ extern "C" {
 #endif
 
 // Copies `bytes` bytes of ordinary host memory to the current device through a pinned buffer of the library, on `stream`;
-// the host memory is free again on return.
+// the host memory is free again on return. On a stream that is capturing a graph the buffer belongs to that graph for as long as it
+// lives: every replay copies it again.
 RLT_API int rlt_stage_upload(const void* host, size_t bytes, void* device, rlt_stream_t stream);
+RLT_API int rlt_capture_id(rlt_stream_t stream, uint64_t* id);  // of the capture that `stream` takes part in; 0: none
 
 // rlt_tensor_transfer between tensors of one type, with the descriptor table in HOST memory: it travels as kernel
 // parameters, so nothing has to be kept for the launch. At most RLT_INLINE_TRANSFERS descriptors.

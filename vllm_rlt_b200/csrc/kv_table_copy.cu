@@ -1189,6 +1189,7 @@ struct HostSlots {
 int fill_host_slots(HostSlots& slots) {
   const std::lock_guard<std::mutex> lock(slots.filling);
   if (slots.filled) return RLT_OK;
+  const OutsideCapture outside;
   void* host = nullptr;
   void* dev = nullptr;
   RLT_CUDA_TRY(cudaHostAlloc(&host, kHostSlots * kHostSlotBytes, cudaHostAllocDefault));
@@ -1212,9 +1213,12 @@ int fill_host_slots(HostSlots& slots) {
   return RLT_OK;
 }
 
-// A slot of the current device that is free to be written. Its event is recorded behind the launch that reads it, and then it is
-// given back to `pool`.
-int take_host_slot(HostSlot* out, SlotPool<HostSlot>** pool) {
+// A slot of the current device that is free to be written, for work on `stream`. Its event is recorded behind the launch that reads
+// it, and then it is given back to `pool`. None for a graph that is being captured: its replays would read what is there by then.
+int take_host_slot(cudaStream_t stream, HostSlot* out, SlotPool<HostSlot>** pool) {
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  RLT_CUDA_TRY(cudaStreamIsCapturing(stream, &capturing));
+  if (capturing != cudaStreamCaptureStatusNone) return cuda_fail(cudaErrorStreamCaptureUnsupported);
   constexpr int kMaxDevices = 64;
   static auto* devices = new HostSlots[kMaxDevices];  // never destroyed: threads may outlive main
   int device = 0;
@@ -1316,7 +1320,7 @@ int rlt_handoff_staged(const RltPool* src, const RltPool* dst, const RltBlockMov
   if (bytes > rlt::kHostSlotBytes) return RLT_MOVE_UNSUITED;
   rlt::HostSlot slot;
   rlt::SlotPool<rlt::HostSlot>* pool = nullptr;
-  const int rc = rlt::take_host_slot(&slot, &pool);
+  const int rc = rlt::take_host_slot(reinterpret_cast<cudaStream_t>(stream), &slot, &pool);
   if (rc != RLT_OK) return rc;
   memcpy(slot.host, moves->host_records, bytes);
   return rlt::copy_and_launch(slot, pool, bytes, reinterpret_cast<cudaStream_t>(stream), [&] {
@@ -1346,7 +1350,7 @@ int rlt_kv_handoff_host(const RltPool* src, const RltPool* dst, const RltHostBat
 
   rlt::HostSlot slot;
   rlt::SlotPool<rlt::HostSlot>* pool = nullptr;
-  const int rc = rlt::take_host_slot(&slot, &pool);
+  const int rc = rlt::take_host_slot(reinterpret_cast<cudaStream_t>(stream), &slot, &pool);
   if (rc != RLT_OK) return rc;
   unsigned char* host = slot.host;
   memcpy(host, hb->src_tables, src_bytes);

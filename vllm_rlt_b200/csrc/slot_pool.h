@@ -11,6 +11,13 @@
 
 namespace rlt {
 
+// Lets the thread make calls that are not allowed while a stream is capturing a graph, about things that the capture has no part in.
+struct OutsideCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  OutsideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~OutsideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // `Slot` has a `done` event, recorded behind the last work that reads the slot. A slot belongs to the thread that took it until it
 // gives it back, so nothing is locked while that thread fills it, queues the work, or waits for the GPU to let go of it.
 template <typename Slot>
@@ -20,6 +27,7 @@ class SlotPool {
   // `make(Slot*)` while fewer than `most` exist; else the one given back longest ago, once its work is over.
   template <typename Make>
   int take(Slot* out, size_t most, Make make) {
+    const OutsideCapture outside;
     std::unique_lock<std::mutex> lock(mutex_);
     for (;;) {
       for (auto it = idle_.begin(); it != idle_.end(); ++it) {

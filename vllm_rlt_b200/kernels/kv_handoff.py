@@ -192,21 +192,23 @@ class _Sent:
     """Device memory of a batch and the stream it was filled on, which is also the one the allocator takes it back in the order of.
 
     A use on another stream comes behind the fill alone (``before``), not behind what else that stream has been given since, and the
-    memory goes back behind that use (``after``)."""
+    memory goes back behind that use (``after``). ``capture``: the graph capture that the fill is part of, 0 for none."""
 
-    def __init__(self, tensor, stream: int):
-        self.tensor, self.stream = tensor, stream
+    def __init__(self, tensor, stream: int, capture: int = 0):
+        self.tensor, self.stream, self.capture = tensor, stream, capture
         self._event = _lib.load_host().event
         self._filled = self._event(False, tensor.device.index, stream)
         self._used = {}  # other streams: an event behind the last use there
 
-    def before(self, stream: int) -> int:
-        if stream != self.stream:
+    def before(self, stream: int, capture: int) -> int:
+        if capture != self.capture:
+            self._filled.synchronize()  # a graph cannot wait for what lies before it: its replays find the memory filled
+        elif stream != self.stream:
             self._filled.order(stream)
         return self.tensor.data_ptr()
 
-    def after(self, stream: int) -> None:
-        if stream != self.stream:
+    def after(self, stream: int, capture: int) -> None:
+        if stream != self.stream and not capture:  # (a batch outlives the graphs that use it)
             self._used[stream] = self._event(False, self.tensor.device.index, stream)
 
     def __del__(self):
@@ -228,6 +230,9 @@ class HandoffBatch:
     Everything is copied out of the arguments. A batch of up to about a thousand tokens travels as kernel parameters of
     the launches that use it; the records of a larger one are sent to the device here, on ``stream``, in one copy. The
     padded arrays that an ``RltBatch`` points at are made and sent when something asks for them (``as_struct``).
+
+    Any stream and any thread may use a batch. A CUDA graph may use one that was built before it or within its capture; such
+    a batch has to be kept, like the pools, for as long as the graph is replayed.
     """
 
     def __init__(
@@ -251,9 +256,8 @@ class HandoffBatch:
         self.has_exit = exit_planes is not None
         self._planned_exits = self.exit_count
         self._device = device
-        self._arrays = None   # (device tensor, address of each array) of the RltBatch form
-        self._arrays_sent = None
-        self._staged = {}     # what has been sent to the device, by the image's planes (0: the records)
+        self._arrays = {}     # of the RltBatch form, by graph capture (0: none): (device tensor, address of each array, _Sent)
+        self._staged = {}     # what has been sent to the device, by the image's planes (0: the records) and graph capture (0: none)
         self._sending = threading.Lock()
         if not host.plan_fits(self._plan, 0):
             self._send(0, self.metadata_bytes, stream)
@@ -262,16 +266,20 @@ class HandoffBatch:
         return torch.device("cuda", torch.cuda.current_device()) if self._device is None else torch.device(self._device)
 
     def _send(self, planes: int, nbytes: int, stream) -> _Sent:
-        """The records (``planes`` 0), or the wire plan of ``planes`` planes, on the device: sent once."""
+        """The records (``planes`` 0), or the wire plan of ``planes`` planes, on the device: sent once, and once more by each graph that
+        cannot count on that."""
         with self._sending:
-            sent = self._staged.get(planes)
+            sent = self._staged.get((planes, 0))
             if sent is None:
                 with torch.cuda.device(self._where()):
                     at = _stream_ptr(stream)
-                    with _on_stream(at):  # memory of the stream that fills it
-                        tensor = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
-                    _lib.check(_lib.load_host().plan_upload(self._plan, planes, tensor.data_ptr(), at), "rlt_stage_upload")
-                    sent = self._staged[planes] = _Sent(tensor, at)
+                    capture = _lib.load_host().capture(at)
+                    sent = self._staged.get((planes, capture))
+                    if sent is None:
+                        with _on_stream(at):  # memory of the stream that fills it
+                            tensor = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+                        _lib.check(_lib.load_host().plan_upload(self._plan, planes, tensor.data_ptr(), at), "rlt_stage_upload")
+                        sent = self._staged[planes, capture] = _Sent(tensor, at, capture)
         return sent
 
     def _move(self, direction, src, dst, *, mode, layer_begin=0, layer_end=0, wire_planes=0, plane_begin=0, plane_end=0,
@@ -284,62 +292,76 @@ class HandoffBatch:
         if direction != _lib.MOVE_DIRECT and mode == MODE_DEDUP:
             planes = (src if direction == _lib.MOVE_PACK else dst).num_planes
             wire_bytes = host.plan_wire(self._plan, planes)
-        used, on = (), 0
+        used, on, capture = (), 0, 0
         if self._staged or (wire_bytes and not host.plan_fits(self._plan, wire_bytes)):
             on = _stream_ptr(stream)
+            capture = host.capture(on)
             used = (self._send(0, self.metadata_bytes, stream),)
-            records = used[0].before(on)
+            records = used[0].before(on, capture)
             if wire_bytes:
                 used += (self._send(planes, wire_bytes, stream),)
-                wire = used[1].before(on)
+                wire = used[1].before(on, capture)
         code = host.move(direction, src and src._address(), dst and dst._address(), self._plan, records, wire, mode, layer_begin,
                          layer_end, wire_planes, plane_begin, plane_end, mask, status, grid_limit, variant, workspace, packed,
                          packed_bytes, _raw_stream(stream))
         for sent in used:
-            sent.after(on)
+            sent.after(on, capture)
         return code
 
-    def _send_arrays(self):
-        """The padded arrays of the RltBatch form, in one device buffer: one pinned staging buffer, one copy."""
+    def _send_arrays(self, capture: int = 0):
+        """The padded arrays of the RltBatch form, in one device buffer: one pinned staging buffer, one copy on the current stream."""
         host = _lib.load_host()
         size, offsets = host.plan_layout(self._plan)
         device = self._where()
-        staging = _PINNED.acquire(size)
-        host.plan_arrays(self._plan, staging.buffer.numpy())
         dev = torch.empty(size, dtype=torch.uint8, device=device)
         with torch.cuda.device(device), torch.cuda.stream(torch.cuda.current_stream(device)):
-            dev.copy_(staging.buffer[:size], non_blocking=True)
-            staging.release()
-            if dev.is_cuda:
-                self._arrays_sent = _Sent(dev, _stream_ptr(None))
+            if capture:
+                _lib.check(host.plan_upload(self._plan, -1, dev.data_ptr(), _stream_ptr(None)), "rlt_stage_upload")
+            else:
+                staging = _PINNED.acquire(size)
+                host.plan_arrays(self._plan, staging.buffer.numpy())
+                dev.copy_(staging.buffer[:size], non_blocking=True)
+                staging.release()
+            sent = _Sent(dev, _stream_ptr(None), capture) if dev.is_cuda else None
         base = dev.data_ptr()
-        self._arrays = (dev, {name: base + at for name, at in offsets.items()})
+        return dev, {name: base + at for name, at in offsets.items()}, sent
+
+    def _arrays_on(self, on: int, capture: int):
+        """``_arrays`` for a use on a stream: sent once, on that stream, and once more by each graph that cannot count on that."""
+        if self._plan is None:
+            return self._arrays[0]
+        with self._sending:
+            arrays = self._arrays.get(0) or self._arrays.get(capture)
+            if arrays is None:
+                with _on_stream(on):
+                    arrays = self._arrays[capture] = self._send_arrays(capture)
+        return arrays
 
     @contextlib.contextmanager
     def _struct_on(self, stream):
-        """``as_struct`` for one launch on ``stream``: arrays that are not on the device yet are sent on that stream."""
+        """The RltBatch for one launch on ``stream``."""
         on = _stream_ptr(stream)
-        with self._sending if self._plan is not None else contextlib.nullcontext():
-            if self._arrays is None:
-                with _on_stream(on):
-                    self._send_arrays()
-        if self._arrays_sent is not None:
-            self._arrays_sent.before(on)
-        yield self.as_struct()
-        if self._arrays_sent is not None:
-            self._arrays_sent.after(on)
+        capture = _lib.load_host().capture(on)
+        _, addresses, sent = self._arrays_on(on, capture)
+        if sent is not None:
+            sent.before(on, capture)
+        yield self._struct(addresses)
+        if sent is not None:
+            sent.after(on, capture)
 
-    @property
-    def _dev(self):
-        if self._arrays is None:
-            self._send_arrays()
+    def _array_set(self):
+        with self._sending if self._plan is not None else contextlib.nullcontext():
+            if 0 not in self._arrays:
+                self._arrays[0] = self._send_arrays()
         return self._arrays[0]
 
     @property
+    def _dev(self):
+        return self._array_set()[0]
+
+    @property
     def _ptr(self):
-        if self._arrays is None:
-            self._send_arrays()
-        return self._arrays[1]
+        return self._array_set()[1]
 
     @classmethod
     def from_device(cls, src_tables, dst_tables, tok_begin, tok_end, *, block_size: int, exit_planes=None,
@@ -377,14 +399,19 @@ class HandoffBatch:
         self.metadata_bytes = 0
         arrays = (src_tables, dst_tables, tok_begin, tok_end, exit_planes, exit_offsets)  # kept alive with the batch
         names = ("src_tables", "dst_tables", "tok_begin", "tok_end", "exit_planes", "exit_offsets")
-        self._plan = self._arrays_sent = None
-        self._arrays = (arrays, {name: t.data_ptr() for name, t in zip(names, arrays) if t is not None})
+        self._plan = None
+        self._arrays = {0: (arrays, {name: t.data_ptr() for name, t in zip(names, arrays) if t is not None}, None)}
         self.has_exit = exit_planes is not None
         self.exit_count = exit_planes.numel() if exit_planes is not None else 0
         return self
 
     def as_struct(self) -> _lib.RltBatch:
-        g = self._ptr.get
+        """The RltBatch for launches on the current stream."""
+        on = _stream_ptr(None)
+        return self._struct(self._arrays_on(on, _lib.load_host().capture(on))[1])
+
+    def _struct(self, addresses) -> _lib.RltBatch:
+        g = addresses.get
         return _lib.RltBatch(
             self.num_requests, self.table_width, g("src_tables"), g("dst_tables"),
             g("tok_begin"), g("tok_end"), g("exit_planes"), g("exit_offsets"), self.exit_count,
