@@ -116,3 +116,32 @@ def test_host_checks_raise_what_the_reference_planner_raises(kh):
         mk(t, t, [(0, 12)], exit_planes=[[0, 1]])
     with pytest.raises(ValueError, match="one exit-plane array per request"):
         mk(t, t, [(0, 12)], exit_planes=[[0] * 12, [1] * 3])
+
+
+def test_a_pinned_buffer_belongs_to_whoever_acquired_it_until_it_is_released(monkeypatch):
+    from vllm_rlt_b200.kernels import kv_handoff
+
+    class Event:
+        fired = False
+
+        def record(self):
+            pass
+
+        def query(self):
+            return Event.fired
+
+    real = torch.empty
+    monkeypatch.setattr(torch, "empty", lambda *args, pin_memory=False, **kw: real(*args, **kw))
+    monkeypatch.setattr(torch.cuda, "Event", Event)
+    pool = kv_handoff._PinnedPool()
+    first = pool.acquire(1000)
+    first.release()
+    assert pool.acquire(1000) is not first  # the copy that reads it is not over
+    Event.fired = True
+    again = pool.acquire(1000)
+    assert again is first
+    other = pool.acquire(1000)  # another thread, before the first has recorded its copy
+    assert other is not first
+    other.release()
+    first.release()
+    assert pool.acquire(1 << 20).buffer.numel() == 1 << 20 and len(pool.buffers) == 2

@@ -155,7 +155,8 @@ class PoolView:
 class _Staging:
     """One pinned host buffer; reusable once the copy that read it has completed."""
 
-    def __init__(self, capacity: int):
+    def __init__(self, pool: "_PinnedPool", capacity: int):
+        self.pool = pool
         self.buffer = torch.empty(capacity, dtype=torch.uint8, pin_memory=True)
         self.event = None
 
@@ -165,24 +166,30 @@ class _Staging:
     def release(self) -> None:
         self.event = torch.cuda.Event()
         self.event.record()
+        self.pool.give(self)
 
 
 class _PinnedPool:
-    """Pinned staging buffers are costly to allocate (a driver call each), so they are kept and reused."""
+    """Pinned staging buffers are costly to allocate (a driver call each), so up to ``KEPT`` of them are kept and reused. One that
+    has been acquired is out of the pool until it is released: another thread cannot get it meanwhile."""
+
+    KEPT = 64
 
     def __init__(self):
         self.buffers: list[_Staging] = []
+        self._lock = threading.Lock()
 
     def acquire(self, size: int) -> _Staging:
-        for b in self.buffers:
-            if b.buffer.numel() >= size and b.free():
-                b.event = None
-                return b
-        capacity = 1 << max(16, (size - 1).bit_length())
-        b = _Staging(capacity)
-        if len(self.buffers) < 64:
-            self.buffers.append(b)
-        return b
+        with self._lock:
+            for i, b in enumerate(self.buffers):
+                if b.buffer.numel() >= size and b.free():
+                    return self.buffers.pop(i)
+        return _Staging(self, 1 << max(16, (size - 1).bit_length()))
+
+    def give(self, b: _Staging) -> None:
+        with self._lock:
+            if len(self.buffers) < self.KEPT:
+                self.buffers.append(b)
 
 
 _PINNED = _PinnedPool()
