@@ -297,7 +297,9 @@ RLT_API int rlt_kv_copy_segments(const int64_t* segments, int32_t count, rlt_str
  * V and scale rows of the exit plane into every deeper plane of the same pool,
  * for the layers whose bit is set in layer_mask (0 = all layers; the reference
  * copies its recurrent_layers). rows is a device int32[count][3]; tables is the
- * device int32[num_requests][planes][table_width] of the pool. One launch.
+ * device int32[num_requests][planes][table_width] of the pool. One launch, or a
+ * few where the rows are more than the blocks of one grid (89 million rows of
+ * 24 layers with 4 KiB each).
  *
  * Replaces KVCacheManager.finalize_token (vllm_rlt/core/kv_cache_manager.py:1053-1076)
  * and the finalize_kernel launches of ModelRunner.finalize_many

@@ -187,3 +187,18 @@ def test_op_loader_registers_the_ops_once_and_fails_loudly_when_unbuilt(monkeypa
     with pytest.raises(OSError):
         _lib.load_ops()
     _lib.load_ops.cache_clear()
+
+
+def test_finalize_has_no_limit_on_its_rows(lib):
+    """More rows than one grid of blocks can serve: without a device the call gets as far as asking for one. (Where there is one the
+    made-up addresses must not be launched on.)"""
+    import torch
+
+    from vllm_rlt_b200 import _lib
+
+    if torch.cuda.is_available():
+        pytest.skip("for machines without a GPU")
+    region = _lib.RltRegion(1 << 20, 1 << 30, 24 * 16 * 4096, 16 * 4096, 4096)
+    pool = _lib.RltPool(region, _lib.RltRegion(None, None, 0, 0, 0), 64, 16, 24, 4)
+    for count in (1, 89_000_000, 90_000_000, 2**31 - 1):
+        assert lib.rlt_kv_finalize(C.byref(pool), 0x1000, 1, 4, 0x2000, count, 0, None, None) == _lib.RLT_E_CUDA, count

@@ -40,3 +40,26 @@ def test_finalize_at_the_edges_of_its_groups(kind, shape, rows):
     kh.kv_finalize(full_view(gp), torch.from_numpy(tables).cuda(), torch.tensor(todo, dtype=torch.int32, device="cuda"), status=status)
     kh.raise_for_status(status)
     assert_pools_equal(gp, P)
+
+
+def test_rows_beyond_one_launch_are_served_and_reported_by_their_place_in_the_list():
+    from vllm_rlt_b200.kernels import kv_handoff as kh
+
+    one_launch = 1 << 28
+    if torch.cuda.mem_get_info()[0] < 5 << 30:
+        pytest.skip("needs 5 GiB of free device memory")
+    key, value = (torch.randn(6, 1, 4, 1, 16, device="cuda").to(torch.bfloat16) for _ in range(2))
+    want = [t.clone() for t in (key, value)]
+    rows = torch.empty(one_launch + 5, 3, dtype=torch.int32, device="cuda")
+    rows[:] = torch.tensor([0, 1, 0], dtype=torch.int32)  # the deepest plane: nothing to copy
+    for at, position in ((0, 0), (one_launch - 1, 5), (one_launch, 2), (one_launch + 4, 7)):
+        rows[at, 1], rows[at, 2] = 0, position
+        for t in want:
+            t[3 + position // 4, 0, position % 4] = t[1 - position // 4, 0, position % 4]
+    rows[one_launch + 2, 1] = 2  # no such plane
+    tables = torch.tensor([[[1, 0], [3, 4]]], dtype=torch.int32, device="cuda")
+    status = kh.new_status()
+    before = kh.kernel_launches()
+    kh.kv_finalize(kh.PoolView.from_tensors(key, value, 2), tables, rows, status=status)
+    assert status.tolist() == [3, one_launch + 2, 0, 2] and kh.kernel_launches() == before + 2
+    assert torch.equal(key, want[0]) and torch.equal(value, want[1])

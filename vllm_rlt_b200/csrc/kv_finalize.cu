@@ -20,6 +20,8 @@
 //
 // HBM roofline: each selected (layer, tensor) row is read once and written once per deeper plane.
 
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace rlt {
@@ -47,10 +49,12 @@ struct FinalizeParams {
   int table_width, num_requests;
   const int* rows;                // [n][3]: request index, exit plane, token position
   int n;
+  int first_row;                  // of this launch in the caller's list
   int* status;
 };
 
 constexpr int kGroupRows = 16;
+constexpr long long kMostRows = 1ll << 28;  // of one launch: three times a row's index stays in 32 bits
 
 // Vectors per thread: one of 32 or 16 bytes, more of the narrow ones.
 template <typename T>
@@ -77,7 +81,7 @@ __device__ __forceinline__ void fill_deeper(const FinalizeParams& p, const Final
   if (row >= p.n) return;
   const int request = p.rows[3 * row], e = p.rows[3 * row + 1], position = p.rows[3 * row + 2];
   if (request < 0 || request >= p.num_requests || e < 0 || e >= p.planes || position < 0 || position >= p.table_width * p.block_size) {
-    if (say && slot == 0) report(p.status, RLT_STATUS_BAD_PLANE, row, position, e);
+    if (say && slot == 0) report(p.status, RLT_STATUS_BAD_PLANE, p.first_row + row, position, e);
     return;
   }
   // the deeper planes of this CTA's chunk (all of them, unless the launch is small)
@@ -191,10 +195,7 @@ int rlt_kv_finalize(const RltPool* pool, const int32_t* tables, int32_t num_requ
   p.tables = tables;
   p.table_width = table_width;
   p.num_requests = num_requests;
-  p.rows = rows;
-  p.n = count;
   p.status = status;
-  const long long groups = (static_cast<long long>(count) + rlt::kGroupRows - 1) / rlt::kGroupRows;
   for (int g = 0; g < regions; ++g) {
     rlt::FinalizeRegion& rg = p.region[g];
     const int per = rlt::kThreads * (rg.vec_bytes == 32 ? rlt::vectors_of<rlt::Vec32>() : rg.vec_bytes == 16 ? rlt::vectors_of<uint4>()
@@ -203,21 +204,27 @@ int rlt_kv_finalize(const RltPool* pool, const int32_t* tables, int32_t num_requ
     rg.parts = static_cast<int>((vectors + per - 1) / per);
     p.parts += 2 * rg.parts;
   }
-  const long long grid = groups * p.parts;
-  if (grid > 0x7fffffffll) return RLT_E_LIMIT;
-  // A launch too small to fill the GPU is short of stores in flight where each thread has many planes to fill: the planes
-  // are then dealt to several CTAs, each of which reads the source rows (from L2, after the first) for itself. 8 rows of 32
-  // planes: 13.3 -> 10.0 us.
   int sms = 0;
   const int rc = rlt::sm_count(&sms);
   if (rc != RLT_OK) return rc;
-  p.plane_chunk = grid < 8ll * sms && p.planes > 8 ? 8 : p.planes;
-  const dim3 ctas(static_cast<unsigned>(grid), static_cast<unsigned>((p.planes + p.plane_chunk - 1) / p.plane_chunk));
   const bool wide = p.region[0].vec_bytes == 32 && (regions == 1 || p.region[1].vec_bytes == 32);
-  auto* kernel = ctas.y > 1 ? (wide ? rlt::finalize_kernel<true, true> : rlt::finalize_kernel<false, true>)
-                            : (wide ? rlt::finalize_kernel<true, false> : rlt::finalize_kernel<false, false>);
-  RLT_CUDA_TRY(rlt::launch_following(kernel, ctas, rlt::kThreads, reinterpret_cast<cudaStream_t>(stream), p));
-  rlt::g_launches.fetch_add(1, std::memory_order_relaxed);
+  // One launch, unless the rows need more CTAs than a grid holds (89 million rows of 24 layers with 4 KiB each).
+  const long long most = std::min(0x7fffffffll / p.parts * rlt::kGroupRows, rlt::kMostRows);
+  for (long long first = 0; first < count; first += most) {
+    p.rows = rows + 3 * first;
+    p.first_row = static_cast<int>(first);
+    p.n = static_cast<int>(std::min<long long>(most, count - first));
+    const long long grid = static_cast<long long>((p.n + rlt::kGroupRows - 1) / rlt::kGroupRows) * p.parts;
+    // A launch too small to fill the GPU is short of stores in flight where each thread has many planes to fill: the planes
+    // are then dealt to several CTAs, each of which reads the source rows (from L2, after the first) for itself. 8 rows of 32
+    // planes: 13.3 -> 10.0 us.
+    p.plane_chunk = grid < 8ll * sms && p.planes > 8 ? 8 : p.planes;
+    const dim3 ctas(static_cast<unsigned>(grid), static_cast<unsigned>((p.planes + p.plane_chunk - 1) / p.plane_chunk));
+    auto* kernel = ctas.y > 1 ? (wide ? rlt::finalize_kernel<true, true> : rlt::finalize_kernel<false, true>)
+                              : (wide ? rlt::finalize_kernel<true, false> : rlt::finalize_kernel<false, false>);
+    RLT_CUDA_TRY(rlt::launch_following(kernel, ctas, rlt::kThreads, reinterpret_cast<cudaStream_t>(stream), p));
+    rlt::g_launches.fetch_add(1, std::memory_order_relaxed);
+  }
   return RLT_OK;
 }
 
