@@ -3,10 +3,16 @@
 Everything is compiled for sm_100a only, with explicit ``nvcc`` / ``g++``
 commands, into files that sit inside the package directory so that they travel
 with a source snapshot. Nothing is cached outside the tree.
+
+Several processes may ask for a build at once, as workers that start together
+do: one compiles, the others wait for it and find its result, and a file that
+is being written has another name than the one that is loaded.
 """
 
 from __future__ import annotations
 
+import contextlib
+import fcntl
 import hashlib
 import os
 import shutil
@@ -75,6 +81,30 @@ def _run(cmd: list[str], show: bool = False) -> None:
         print(proc.stdout + proc.stderr)
 
 
+@contextlib.contextmanager
+def _alone():
+    """No other process builds in this tree meanwhile. The system lets go of the lock when its holder ends, however it ends."""
+    with open(PACKAGE / ".build.lock", "w") as lock:
+        fcntl.flock(lock, fcntl.LOCK_EX)
+        yield
+
+
+def _compile(target: Path, command, fingerprint: str, force: bool, show: bool = False) -> None:
+    """Run ``command(output)`` if ``target`` is not what ``fingerprint`` stands for (``force``: in any case)."""
+    if not force and not _stale(target, fingerprint):
+        return
+    with _alone():
+        if not force and not _stale(target, fingerprint):
+            return  # another process has built it meanwhile
+        fresh = target.with_name(f".{target.name}.{os.getpid()}")
+        try:
+            _run(command(fresh), show=show)
+            os.replace(fresh, target)
+        finally:
+            fresh.unlink(missing_ok=True)
+        _record(target, fingerprint)
+
+
 def build_library(force: bool = False, verbose: bool = False) -> Path:
     """Compile the C-ABI library (no torch types, static cudart)."""
     target = PACKAGE / LIB_NAME
@@ -83,12 +113,12 @@ def build_library(force: bool = False, verbose: bool = False) -> Path:
                       CSRC / "internal.h", CSRC / "slot_pool.h", INCLUDE / "rlt_kv_handoff.h"]
     flags = [*ARCH, "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC,-fvisibility=hidden"]
     fingerprint = _fingerprint(flags, deps)
-    if force or verbose or _stale(target, fingerprint):
-        cmd = [_nvcc(), *flags, f"-I{INCLUDE}", "-shared", "-o", str(target), *map(str, sources), "-ldl"]
-        if verbose:
-            cmd.insert(1, "-Xptxas=-v")
-        _run(cmd, show=verbose)
-        _record(target, fingerprint)
+
+    def command(output: Path) -> list[str]:
+        say = ["-Xptxas=-v"] if verbose else []
+        return [_nvcc(), *say, *flags, f"-I{INCLUDE}", "-shared", "-o", str(output), *map(str, sources), "-ldl"]
+
+    _compile(target, command, fingerprint, force or verbose, show=verbose)
     return target
 
 
@@ -105,15 +135,16 @@ def _build_torch_module(name: str, source_name: str, headers: list[Path], force:
     flags = ["-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={abi}",
              f"-DTORCH_EXTENSION_NAME={target.stem}", f"torch={torch.__version__}"]
     fingerprint = _fingerprint(flags, deps)
-    if force or _stale(target, fingerprint):
+
+    def command(output: Path) -> list[str]:
         includes = [f"-I{p}" for p in cpp_extension.include_paths("cuda")] + [f"-I{INCLUDE}", f"-I{CSRC}"]
         includes.append(f"-I{sysconfig.get_paths()['include']}")
         torch_lib = Path(torch.__file__).parent / "lib"
         libraries = ["-ltorch", "-ltorch_cpu", "-lc10", "-ltorch_cuda", "-lc10_cuda"] + (["-ltorch_python"] if python else [])
-        cmd = ["g++", *flags[:-1], *includes, str(source), "-o", str(target),
-               f"-L{PACKAGE}", "-l:" + LIB_NAME, f"-L{torch_lib}", *libraries, "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{torch_lib}"]
-        _run(cmd)
-        _record(target, fingerprint)
+        return ["g++", *flags[:-1], *includes, str(source), "-o", str(output),
+                f"-L{PACKAGE}", "-l:" + LIB_NAME, f"-L{torch_lib}", *libraries, "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{torch_lib}"]
+
+    _compile(target, command, fingerprint, force)
     return target
 
 

@@ -191,6 +191,20 @@ def load_host():
     return module
 
 
+def on_demand(module: dict, **makers):
+    """A module's ``__getattr__`` for classes whose bases are compiled: each is made when it is first asked for, so that importing the
+    module loads (and, in a tree that was never built, compiles) nothing. ``module`` is its ``globals()``."""
+
+    def __getattr__(name):
+        if name not in makers:
+            raise AttributeError(f"module {module['__name__']!r} has no attribute {name!r}")
+        made = makers[name]()
+        made.__qualname__ = name
+        return module.setdefault(name, made)
+
+    return __getattr__
+
+
 class RltError(RuntimeError):
     def __init__(self, code: int, where: str):
         lib = load()
