@@ -63,3 +63,14 @@ def test_rows_beyond_one_launch_are_served_and_reported_by_their_place_in_the_li
     kh.kv_finalize(kh.PoolView.from_tensors(key, value, 2), tables, rows, status=status)
     assert status.tolist() == [3, one_launch + 2, 0, 2] and kh.kernel_launches() == before + 2
     assert torch.equal(key, want[0]) and torch.equal(value, want[1])
+
+
+def test_a_layer_past_the_ones_that_can_be_selected_is_refused_in_words():
+    from vllm_rlt_b200.kernels import kv_handoff as kh
+
+    cache = torch.zeros(2, 70, 4, 1, 16, dtype=torch.bfloat16, device="cuda")
+    tables = torch.zeros(1, 2, 1, dtype=torch.int32, device="cuda")
+    rows = torch.zeros(1, 3, dtype=torch.int32, device="cuda")
+    for layers in ([69], [64], None):
+        with pytest.raises(ValueError, match="limit"):
+            kh.kv_finalize(kh.PoolView.from_tensors(cache, cache.clone(), 2), tables, rows, layers=layers)

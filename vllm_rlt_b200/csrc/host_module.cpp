@@ -99,6 +99,12 @@ long long integer(PyObject* o) {
   return v;
 }
 
+// A position or size: a fraction is refused, not cut off.
+long long index_of(PyObject* o) {
+  const Ref n(PyNumber_Index(o));
+  return integer(n.p);
+}
+
 int32_t int32_of(long long v) {
   if (v < INT32_MIN || v > INT32_MAX) fail(PyExc_OverflowError, "block id or exit plane out of bounds for int32");
   return static_cast<int32_t>(v);
@@ -388,7 +394,7 @@ PyObject* make_plan(PyObject* const* a) {
       if (count < plan->end[r]) bad_value(kCover);
     }
   }
-  plan->make_records();
+  if (plan->src.given || plan->dst.given) plan->make_records();  // no tables, nothing to move: the entry points say so
   const Ref list(PyList_New(n));
   for (int r = 0; r < n; ++r) {
     PyObject* pair = Py_BuildValue("LL", static_cast<long long>(plan->begin[r]), static_cast<long long>(plan->end[r]));
@@ -642,7 +648,7 @@ PyObject* finalize(PyObject* const* a) {
   const int32_t *table_data = tables->data_ptr<int32_t>(), *row_data = rows->data_ptr<int32_t>();
   const auto requests = static_cast<int32_t>(tables->size(0)), width = static_cast<int32_t>(tables->size(2));
   const auto count = static_cast<int32_t>(rows->size(0));
-  const uint64_t mask = PyLong_AsUnsignedLongLong(a[4]);
+  const uint64_t mask = PyLong_AsUnsignedLongLongMask(a[4]);  // a layer past the 64th: the library says that the pool has too many
   auto* status = static_cast<int32_t*>(data_of(a[5]));
   const rlt_stream_t stream = stream_of(a[6]);
   return PyLong_FromLong(unlocked([&] { return rlt_kv_finalize(pool, table_data, requests, width, row_data, count, mask, status, stream); }));
@@ -840,7 +846,7 @@ PyObject* fill(PyObject* const* a) {
   if (!PyList_CheckExact(values) && !PyTuple_CheckExact(values)) Py_RETURN_NONE;
   const int64_t start = integer(a[1]);
   const Py_ssize_t n = PySequence_Fast_GET_SIZE(values);
-  if (!t.is_cpu() || t.dim() != 1 || !t.is_contiguous() || start < 0 || start + n > t.size(0)) Py_RETURN_NONE;
+  if (!t.is_cpu() || t.dim() != 1 || !t.is_contiguous() || start < 0 || start > t.size(0) - n) Py_RETURN_NONE;
   PyObject** items = PySequence_Fast_ITEMS(values);
   auto whole = [](PyObject* o, long long* v) {
     if (!PyLong_CheckExact(o)) return false;
@@ -878,10 +884,10 @@ PyObject* fill(PyObject* const* a) {
 PyObject* row_slice(PyObject* const* a) {
   const at::Tensor& t = some_tensor(a[0]);
   if (!PyLong_CheckExact(a[1]) || t.dim() != 2) Py_RETURN_NONE;
-  int64_t index = integer(a[1]);
-  const int64_t start = integer(a[2]), n = integer(a[3]);
+  int64_t index = index_of(a[1]);
+  const int64_t start = index_of(a[2]), n = integer(a[3]);
   index += index < 0 ? t.size(0) : 0;
-  if (index < 0 || index >= t.size(0) || start < 0 || start + n > t.size(1)) Py_RETURN_NONE;
+  if (index < 0 || index >= t.size(0) || start < 0 || start > t.size(1) - n) Py_RETURN_NONE;
   return THPVariable_Wrap(plain_view(t, t.storage_offset() + index * t.stride(0) + start * t.stride(1), n, t.stride(1)));
 }
 
@@ -987,7 +993,7 @@ PyObject* encode_chunk(PyObject* const* a) {
     if (PySequence_Fast_GET_SIZE(request.p) != 4) bad_value("a request is (source, target, start, end)");
     const Ref source(PySequence_Fast(PySequence_Fast_GET_ITEM(request.p, 0), "block tables must be a sequence"));
     const Ref target(PySequence_Fast(PySequence_Fast_GET_ITEM(request.p, 1), "block tables must be a sequence"));
-    const int64_t start = integer(PySequence_Fast_GET_ITEM(request.p, 2)), end = integer(PySequence_Fast_GET_ITEM(request.p, 3));
+    const int64_t start = index_of(PySequence_Fast_GET_ITEM(request.p, 2)), end = index_of(PySequence_Fast_GET_ITEM(request.p, 3));
     const Py_ssize_t ns = PySequence_Fast_GET_SIZE(source.p), nt = PySequence_Fast_GET_SIZE(target.p);
     if (ns == 0 || nt == 0 || start < 0 || start >= end) bad_value("invalid KV range");
     const int64_t first = page_size > 0 ? start / page_size : 0;
@@ -1016,7 +1022,7 @@ PyObject* encode_chunk(PyObject* const* a) {
   for (Py_ssize_t i = 0; i < PySequence_Fast_GET_SIZE(extra.p); ++i) {
     const Ref triple(PySequence_Fast(PySequence_Fast_GET_ITEM(extra.p, i), "a range is (source, target, bytes)"));
     if (PySequence_Fast_GET_SIZE(triple.p) != 3) bad_value("a range is (source, target, bytes)");
-    for (int k = 0; k < 3; ++k) put(out, static_cast<int64_t>(integer(PySequence_Fast_GET_ITEM(triple.p, k))));
+    for (int k = 0; k < 3; ++k) put(out, static_cast<int64_t>(index_of(PySequence_Fast_GET_ITEM(triple.p, k))));
   }
   return PyBytes_FromStringAndSize(out.data(), static_cast<Py_ssize_t>(out.size()));
 }
@@ -1028,7 +1034,7 @@ struct RequestRecords {
   int words;
   int64_t requests = 0, before = 0, blocks = 0, width = 1;
   RequestRecords(const RltPool* s, const RltPool* d) : src(s), dst(d), words(kRecordHeader + s->num_planes + d->num_planes) {}
-  bool fits(int64_t pages) const { return (blocks + pages) * words * 4 <= (1 << 20) && requests < RLT_MAX_REQUESTS; }
+  bool fits(int64_t pages) const { return pages <= (1 << 20) && (blocks + pages) * words * 4 <= (1 << 20) && requests < RLT_MAX_REQUESTS; }
   bool valid(const int32_t* ids, int64_t n, const RltPool* pool) const {
     bool ok = true;
     for (int64_t i = 0; i < n; ++i) ok &= static_cast<uint32_t>(ids[i]) < static_cast<uint32_t>(pool->num_blocks);
@@ -1198,7 +1204,7 @@ PyObject* pull_chunk(PyObject* const* a) {
       for (Py_ssize_t k = 0; k < PySequence_Fast_GET_SIZE(spans.p) && !found; ++k) {
         const Ref s(PySequence_Fast(PySequence_Fast_GET_ITEM(spans.p, k), "a span is (low, high, base)"));
         const int64_t lo = integer(PySequence_Fast_GET_ITEM(s.p, 0)), hi = integer(PySequence_Fast_GET_ITEM(s.p, 1));
-        found = lo <= extra[i] && extra[i] + extra[i + 2] <= hi;
+        found = lo <= extra[i] && extra[i] <= hi && extra[i + 2] >= 0 && extra[i + 2] <= hi - extra[i];
         if (found) extra[i] += integer(PySequence_Fast_GET_ITEM(s.p, 2)) - lo;
       }
       if (!found) Py_RETURN_NONE;
@@ -1249,7 +1255,7 @@ PyObject* pack_segments(PyObject* const* a) {
     if (PySequence_Fast_GET_SIZE(s.p) < 2 || PySequence_Fast_GET_SIZE(d.p) < 2) bad_value("a descriptor is (address, bytes, device)");
     const int64_t bytes = integer(PySequence_Fast_GET_ITEM(s.p, 1)), to = integer(PySequence_Fast_GET_ITEM(d.p, 0));
     if (bytes != integer(PySequence_Fast_GET_ITEM(d.p, 1))) bad_value("incompatible source/target KV geometry");
-    auto inside = [&](size_t k) { return span[k] <= to && to + bytes <= span[k + 1]; };
+    auto inside = [&](size_t k) { return span[k] <= to && to <= span[k + 1] && bytes <= span[k + 1] - to; };
     if (hit >= span.size() || !inside(hit)) {
       for (hit = 0; hit < span.size() && !inside(hit); hit += 3) {
       }
