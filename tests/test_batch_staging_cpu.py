@@ -145,3 +145,32 @@ def test_a_pinned_buffer_belongs_to_whoever_acquired_it_until_it_is_released(mon
     other.release()
     first.release()
     assert pool.acquire(1 << 20).buffer.numel() == 1 << 20 and len(pool.buffers) == 2
+
+
+def test_the_events_of_a_batch_are_recorded_and_waited_for_on_the_device_that_launches(monkeypatch):
+    """A launch on one device may read the records of a batch on another; a default stream has the same address (0) on both."""
+    import types
+
+    from vllm_rlt_b200.kernels import kv_handoff
+
+    log, current = [], [1]
+
+    class Event:
+        def __init__(self, timed, device, stream):
+            log.append(("record", device, stream))
+
+        def order(self, device, stream):
+            log.append(("order", device, stream))
+
+    monkeypatch.setattr(kv_handoff._lib, "load_host", lambda: types.SimpleNamespace(event=Event))
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: current[0])
+    memory = types.SimpleNamespace(device=types.SimpleNamespace(index=1), data_ptr=lambda: 64)
+    sent = kv_handoff._Sent(memory, 0)
+    for device, stream in ((1, 0), (0, 0), (1, 7), (0, 0)):
+        current[0] = device
+        assert sent.before(stream, 0) == 64
+        sent.after(stream, 0)
+    used = [("order", 0, 0), ("record", 0, 0)]
+    assert log == [("record", 1, 0), *used, ("order", 1, 7), ("record", 1, 7), *used]
+    del log[:], sent
+    assert log == [("order", 1, 0)] * 2

@@ -1497,9 +1497,11 @@ PyObject* event_synchronize(PyObject* self, PyObject* const*) {
   check_code(unlocked([&] { return rlt_event_wait(event); }));
   Py_RETURN_NONE;
 }
+// order(device, stream): what is queued on that device's stream from now on comes after the event
 PyObject* event_order(PyObject* self, PyObject* const* a) {
   RltEvent* event = reinterpret_cast<EventObject*>(self)->event;
-  const rlt_stream_t stream = stream_of(a[0]);
+  const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(integer(a[0])));
+  const rlt_stream_t stream = stream_of(a[1]);
   check_code(unlocked([&] { return rlt_event_order(event, stream); }));
   Py_RETURN_NONE;
 }
@@ -1515,7 +1517,7 @@ void event_dealloc(PyObject* self) {
   PyObject_Free(self);
   Py_DECREF(type);
 }
-PyMethodDef kEventMethods[] = {RLT_METHOD("query", event_query, 0), RLT_METHOD("synchronize", event_synchronize, 0), RLT_METHOD("order", event_order, 1),
+PyMethodDef kEventMethods[] = {RLT_METHOD("query", event_query, 0), RLT_METHOD("synchronize", event_synchronize, 0), RLT_METHOD("order", event_order, 2),
                                RLT_METHOD("elapsed_time", event_elapsed_time, 1), {nullptr, nullptr, 0, nullptr}};
 PyType_Slot kEventSlots[] = {{Py_tp_dealloc, reinterpret_cast<void*>(event_dealloc)}, {Py_tp_methods, kEventMethods}, {0, nullptr}};
 PyType_Spec kEventType = {"_host.Event", sizeof(EventObject), 0, Py_TPFLAGS_DEFAULT | Py_TPFLAGS_DISALLOW_INSTANTIATION, kEventSlots};

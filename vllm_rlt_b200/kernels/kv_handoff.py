@@ -205,23 +205,31 @@ class _Sent:
         self.tensor, self.stream, self.capture = tensor, stream, capture
         self._event = _lib.load_host().event
         self._filled = self._event(False, tensor.device.index, stream)
-        self._used = {}  # other streams: an event behind the last use there
+        self._used = {}  # (device, stream) of the launches elsewhere: an event behind the last of them
+
+    def _elsewhere(self, stream: int):
+        """The launching device, which is the current one, and the stream, unless they are where the memory was filled."""
+        use = torch.cuda.current_device(), stream
+        return None if use == (self.tensor.device.index, self.stream) else use
 
     def before(self, stream: int, capture: int) -> int:
         if capture != self.capture:
             self._filled.synchronize()  # a graph cannot wait for what lies before it: its replays find the memory filled
-        elif stream != self.stream:
-            self._filled.order(stream)
+        else:
+            use = self._elsewhere(stream)
+            if use is not None:
+                self._filled.order(*use)
         return self.tensor.data_ptr()
 
     def after(self, stream: int, capture: int) -> None:
-        if stream != self.stream and not capture:  # (a batch outlives the graphs that use it)
-            self._used[stream] = self._event(False, self.tensor.device.index, stream)
+        use = self._elsewhere(stream)
+        if use is not None and not capture:  # (a batch outlives the graphs that use it)
+            self._used[use] = self._event(False, *use)
 
     def __del__(self):
         try:
             for event in self._used.values():
-                event.order(self.stream)
+                event.order(self.tensor.device.index, self.stream)
         except Exception:  # the caller's stream is gone, and with it whatever was queued there
             pass
 
