@@ -65,7 +65,7 @@ def test_full_size_exit_only_handoff_and_pack_scatter_round_trip():
     assert untouched_rows_keep_the_sentinel(w, dst)
     # a checksum of the whole destination pool (wrapping 64-bit sums): identical after both routes
     assert [int(t.view(torch.uint8).view(torch.int64).sum()) for t in (dst.key_cache, dst.value_cache)] == direct
-    del src, dst
+    del src, dst, sv, dv, batch  # the views hold the pools too: the next test needs their memory
     torch.cuda.empty_cache()
 
 
@@ -84,6 +84,7 @@ def test_the_reference_cpu_case_at_its_stated_size_against_the_oracle():
 
     layers, heads, dim, blocks, page, planes = shape = (24, 16, 128, 4096, 16, 4)
     pool_bytes = 2 * blocks * layers * page * heads * dim * 2
+    torch.cuda.empty_cache()
     if torch.cuda.mem_get_info(0)[0] < 4 * pool_bytes:
         pytest.skip("needs about 52 GiB of free device memory")
     rng = np.random.default_rng(20240)
