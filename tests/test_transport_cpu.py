@@ -4,6 +4,7 @@ Mirrors what the reference pins for its NIXL transport with a fake agent (tests/
 and what its connector tests expect of a transport (tests/test_transfer_connector.py:15-27).
 """
 
+import numpy as np
 import pytest
 import torch
 
@@ -222,10 +223,17 @@ def test_a_reader_that_has_not_finished_keeps_the_source_busy_and_blocks_close()
         t.close()
 
 
+def trimmed(source, target, start, end, block_size):
+    """A request's tables cut to the pages ``[start, end)`` touches, the range rebased onto them."""
+    first, last = start // block_size, (end - 1) // block_size
+    cut = lambda tables: tuple(table[first : last + 1] for table in tables)  # noqa: E731
+    return cut(source), cut(target), start - first * block_size, end - first * block_size
+
+
 def test_descriptors_are_cut_to_the_pages_of_the_chunk_and_round_trip():
     source = (tuple(range(100, 140)), tuple(range(200, 240)))
     target = (tuple(range(300, 340)), tuple(range(400, 440)))
-    s, t, lo, hi = tr.trim_request(source, target, 70, 101, 16)
+    s, t, lo, hi = trimmed(source, target, 70, 101, 16)
     assert (lo, hi) == (6, 37) and s == ((104, 105, 106), (204, 205, 206)) and t == ((304, 305, 306), (404, 405, 406))
     raw = tr.encode_chunk([(s, t, lo, hi)], [(1 << 40, 1 << 41, 64)], mode=0, layer_begin=2, layer_end=5, plane_begin=1, plane_end=2)
     assert len(raw) < 200
@@ -235,6 +243,11 @@ def test_descriptors_are_cut_to_the_pages_of_the_chunk_and_round_trip():
     assert where == dict(mode=0, layer_begin=2, layer_end=5, plane_begin=1, plane_end=2)
     with pytest.raises(ValueError, match="invalid KV range"):
         tr.encode_chunk([(s, t, 5, 5)], [])
+    # the cut that encoding makes by itself, given the page size, for tables of every kind
+    for kind in (tuple, list, lambda table: np.asarray(table, np.int32)):
+        whole = [tuple(kind(table) for table in side) for side in (source, target)]
+        for start, end in ((70, 101), (0, 640), (15, 17), (64, 80), (639, 640), (0, 1)):
+            assert tr.encode_chunk([(*whole, start, end)], [], page_size=16) == tr.encode_chunk([trimmed(source, target, start, end, 16)], [])
 
 
 def test_the_descriptor_ring_applies_back_pressure_and_reuses_space_in_order():

@@ -105,7 +105,7 @@ def encode_chunk(requests, extra, *, mode=0, layer_begin=0, layer_end=0, plane_b
     """A pull offer's descriptor: what the receiver needs to run the launch itself.
 
     ``requests`` is ``[(source tables, target tables, start, end)]``; given the page size, each request's tables are cut
-    down to the pages the range touches and the range is rebased onto them as ``trim_request`` does (block tables are only
+    down to the pages the range touches and the range is rebased onto them (block tables are only
     ever indexed by page, so the kernel's result is the same), which keeps a descriptor proportional to the chunk, not
     to the prompt. ``extra`` is ``[(source address, target address, bytes)]``.
 
@@ -133,13 +133,6 @@ def decode_chunk(raw: bytes):
         at += 24
     return requests, extra, dict(mode=mode, layer_begin=layer_begin, layer_end=layer_end, plane_begin=plane_begin,
                                  plane_end=plane_end)
-
-
-def trim_request(source, target, start, end, block_size):
-    """Cut a request's tables to the pages ``[start, end)`` touches and rebase the range onto them."""
-    first, last = start // block_size, (end - 1) // block_size
-    cut = lambda tables: tuple(table[first : last + 1] for table in tables)  # noqa: E731
-    return cut(source), cut(target), start - first * block_size, end - first * block_size
 
 
 class _RingWriter:
