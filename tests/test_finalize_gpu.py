@@ -97,8 +97,8 @@ def test_finalize_reports_rows_it_cannot_apply():
 
 @pytest.mark.parametrize("planes", [2, 32, 64, 65])
 def test_finalize_with_many_planes_fills_every_deeper_plane(planes):
-    """Up to 64 planes one unit loads a row once and stores it to every deeper plane; beyond that the
-    unit-per-target kernel runs. Both must leave the pool the oracle's ``finalize_token`` leaves."""
+    """A thread fills all deeper planes of its vector; in a launch this small they are dealt to several blocks, eight planes
+    each. The pool must be left as the oracle's ``finalize_token`` leaves it."""
     import random
 
     from vllm_rlt_b200.kernels import kv_handoff as kh

@@ -734,7 +734,9 @@ def test_dedup_pack_reports_a_negative_exit_plane_and_leaves_the_token_off_the_w
 @pytest.mark.parametrize("mode_name", ["exit_only", "dedup", "dedup_pack"])
 def test_an_exit_array_shorter_than_the_ranges_is_reported_and_never_read_past(mode_name):
     """RltBatch.exit_count bounds every read of exit_planes: a request whose offset + range end runs past the
-    array is reported as a bad range and skipped as a whole; the requests before it arrive untouched by that."""
+    array is reported as a bad range and skipped as a whole; the requests before it arrive untouched by that. This is about
+    the table-driven kernels, which serve a batch whose ``exit_count`` was set by hand: the records of the others are
+    made on the host, where an array that is too short is refused."""
     k = kh()
     kind, shape = SHAPES["ouro_bf16_small"]
     page, planes = shape[4], shape[5]
