@@ -35,15 +35,18 @@ METRIC = "kv_handoff_gbps"
 UNIT = "GB/s"
 FALLBACK_HBM_GBS = 6650.0
 # NVLink 5, one direction, per GPU. The nominal figure is what the fractions are quoted against; the other is one
-# builder-run peer-to-peer memcpy on a B200 pair, kept for context only (it is not a driver-written peak).
+# peer-to-peer memcpy measured on a B200 pair, kept for context only (not one of the measured peaks).
 NVLINK_NOMINAL_GBS = 900.0
 NVLINK_PEER_MEMCPY_GBS = 770.0
 # link bytes per payload byte for writes over NVLink (ncu: nvltx__bytes.sum / nvltx__bytes_data_user.sum of the handoff kernel)
 NVLINK_WRITE_OVERHEAD = 1.1875
 # the same for read responses when the destination GPU pulls (ncu: nvlrx__bytes.sum / nvlrx__bytes_data_user.sum)
 NVLINK_READ_OVERHEAD = 1.125
-# DRAM traffic per algorithmic byte of table_copy_kernel, from the ncu capture summarised under profiles/
-TRAFFIC_PER_ALGORITHMIC_BYTE = 0.98
+# DRAM traffic per algorithmic byte (ncu dram__bytes_read.sum + dram__bytes_write.sum, summarised under profiles/): of move_kernel by
+# mode at 8 requests, 14,864 tokens, where the last 50 MB of the writes were still in L2 when the kernel ended; of the table-driven
+# kernels at 2 requests
+TRAFFIC_PER_ALGORITHMIC_BYTE = {"exit_only": 0.992, "dedup": 0.997, "all": 0.998}
+TRAFFIC_OF_TABLE_KERNELS = 0.98
 
 
 # ------------------------------------------------------------------------------- helpers
@@ -528,15 +531,20 @@ def run_single(args):
     kh.raise_for_status(status)
 
     cpu = None if args.no_cpu_baseline else cpu_baseline_sample(w, max_tokens=args.cpu_tokens)
+    if args.variant == 0:
+        kernel, ratio = "move_kernel", TRAFFIC_PER_ALGORITHMIC_BYTE[args.mode]
+    else:
+        fan = w.extra.get("mode") == "dedup" and args.variant & 0xf not in (3, 4, 6)
+        kernel, ratio = "table_fan_kernel" if fan else "table_copy_kernel", TRAFFIC_OF_TABLE_KERNELS
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": 1, "steps": args.steps, "warmup": args.warmup,
         "ms_per_step": ms_per_step, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
         "dtype": "u8", "data": "synthetic", "config": config_of(w, args, {"variant": args.variant}),
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                     "traffic": TRAFFIC_PER_ALGORITHMIC_BYTE * algorithmic, "peak_source": peak_note,
-                     "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of a 2-request capture of the same "
-                                       "kernel (traffic / algorithmic = 0.98), scaled by tokens",
-                     "kernel": "move_kernel" if args.variant == 0 else "table_fan_kernel" if w.extra.get("mode") == "dedup" and args.variant & 0xf not in (3, 4, 6) else "table_copy_kernel",
+                     "traffic": ratio * algorithmic, "peak_source": peak_note,
+                     "traffic_source": f"ncu dram__bytes_read.sum + dram__bytes_write.sum of a capture of the same kernel with "
+                                       f"{'8' if args.variant == 0 else '2'} requests (traffic / algorithmic = {ratio}), scaled by tokens",
+                     "kernel": kernel,
                      "algorithmic_bytes_per_launch": algorithmic, "kernel_ms": avg_kernel_ms},
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": batch.metadata_bytes,
                 "d2h_bytes_per_step": 16, "ms_per_step": statistics.mean(e2e_times) * 1e3,
