@@ -172,10 +172,12 @@ RLT_API int rlt_kv_handoff(const RltPool* src, const RltPool* dst, const RltBatc
  * rlt_kv_handoff in RLT_MODE_ALL_PLANES for a caller whose block tables are still in HOST memory: the call turns
  * them into page records, which are parameters of the launch while they fit (30 KiB; 24 bytes and 4 per plane of
  * either side a page) and go through a staging slot of the library beyond that (pinned host memory and device memory,
- * 16 slots of 64 KiB per GPU, allocated at the first such call on that GPU). The arrays may be changed or freed as soon as it has returned. A batch whose tables and ranges exceed
- * rlt_kv_host_batch_limit() bytes gets RLT_E_LIMIT and nothing is queued: stage such a batch yourself and call
- * rlt_kv_handoff. When all 16 slots belong to launches that have not finished, the call waits for the oldest
- * on the host; for that reason, and because it may allocate, it is not for CUDA-graph capture.
+ * 16 slots of 64 KiB per GPU, allocated at the first such call on that GPU). The arrays may be changed or freed as
+ * soon as it has returned. A batch whose tables and ranges exceed rlt_kv_host_batch_limit() bytes gets RLT_E_LIMIT and
+ * nothing is queued: stage such a batch yourself and call rlt_kv_handoff. When all 16 slots belong to launches that
+ * have not finished, the call waits on the host for the one given out longest ago; calls of other threads that find a
+ * free slot are not held up by that. A slot serves one launch, so a batch that needs one is refused (RLT_E_CUDA) on a
+ * stream that is capturing a graph, before anything is queued.
  *
  * This is what a transfer worker calls per chunk: one request, tables of a few hundred entries, where the time to
  * stage them decides how soon after the producer's event the copy starts. It takes the place of the descriptor

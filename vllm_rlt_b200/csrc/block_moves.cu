@@ -630,9 +630,13 @@ extern "C" int rlt_move_blocks(int direction, const RltPool* src, const RltPool*
   p.status = opt->status;
   // Rounds of a piece. Where a plane's block is all a CTA looks up, one: the smaller the piece the closer the SMs stay
   // together. Kinds that fetch the page's record and work out exit planes first need more payload behind that: measured
-  // best at 2 for exit-only (29k tokens: 1.84 -> 1.75 ms), at about 12 / planes where planes are walked (6.4k tokens, four planes:
-  // 1.36 -> 1.23 ms; at 32 planes one round is best), at 8 for a dedup pack (1.86 -> 0.95 ms). A launch of fewer than eight
-  // waves takes the smallest piece that a larger one would split into: it is short of CTAs, not of payload per CTA.
+  // best at 2 for exit-only (29k tokens: 1.84 -> 1.75 ms), at 8 for a dedup pack (1.86 -> 0.95 ms). Where planes are walked, the
+  // more planes a round stores to the fewer rounds are needed, 12 / planes and at most 4. Dedup handoffs of 6 - 8.6 GB, us at
+  // 1 / 2 / 3 / 4 / 8 rounds: two planes 1,267 / 1,105 / 1,054 / 1,026 / 991 (so 8 would be 4 % faster there), three 1,199 /
+  // 1,093 / 1,053 / 1,036 / 1,039, four 1,295 / 1,234 / 1,226 / 1,227 / 1,240, six 1,289 / 1,270 / 1,267 / 1,270 / 1,281, eight
+  // 1,185 / 1,190 / 1,191 / 1,196 / 1,205, sixteen 1,282 / 1,295 / 1,298 / 1,307 / 1,321, 32 1,086 / 1,098 / 1,105 / 1,114 /
+  // 1,114; scatters of dedup images within 1 % of the same. A launch of fewer than eight waves takes the smallest piece that a
+  // larger one would split into: it is short of CTAs, not of payload per CTA.
   int sms = 0;
   const int found = sm_count(&sms);
   if (found != RLT_OK) return found;

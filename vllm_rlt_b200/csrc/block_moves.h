@@ -16,7 +16,8 @@
 constexpr int kRecordHeader = 6;
 constexpr int kRecordBad = -1;
 
-// Records up to this many bytes travel as kernel parameters: no staging slot, no copy, no event.
+// Records up to this many words travel as kernel parameters: no staging slot, no copy, no event. (The launch takes the smallest of
+// three parameter blocks that holds them.)
 constexpr int kInlineWords = 7680;
 constexpr int kInlineMediumWords = 1920;
 constexpr int kInlineSmallWords = 896;

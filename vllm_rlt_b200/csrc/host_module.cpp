@@ -101,6 +101,7 @@ long long integer(PyObject* o) {
 
 // A position or size: a fraction is refused, not cut off.
 long long index_of(PyObject* o) {
+  if (PyLong_CheckExact(o)) return integer(o);
   const Ref n(PyNumber_Index(o));
   return integer(n.p);
 }

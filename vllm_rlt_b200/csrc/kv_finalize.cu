@@ -15,8 +15,8 @@
 // mostly the same ones, so the lookups hit L1) and stores the vector to every deeper plane. The grid holds one CTA per 8 KiB
 // in that order: HBM is fastest while the SMs work close together (block_moves.cu has the measurements), and a decode step of
 // a few rows still reaches every SM. Nothing is shared inside a CTA: lists of rows and blocks in shared memory, with two
-// barriers before the first load, cost 7.4 us where this takes 6.2 (64 rows of four planes), 275 where it takes 271 (4,000 rows).
-// Measured before that, with persistent CTAs that scanned all rows' costs first: 12.6 and 324 us.
+// barriers before the first load, cost 8.5 us where this takes 6.2 (64 rows of four planes), 277 where it takes 274 (4,000 rows).
+// Measured before that, with persistent CTAs that scanned all rows' costs first: 13.8 and 322 us.
 //
 // HBM roofline: each selected (layer, tensor) row is read once and written once per deeper plane.
 
