@@ -82,3 +82,36 @@ def test_handoff_pack_and_scatter_from_records_equal_the_oracle(name, mode):
     for i, (s, e) in enumerate(ranges):
         ho.handoff_rows(P, D, tables[0][i], tables[1][i], s, e, mode=mode, exit_planes=exits[i])
     assert_pools_equal(gd, D)
+
+
+@pytest.mark.parametrize("wide", ["source", "destination"])
+def test_a_batch_with_more_planes_on_the_side_that_an_image_does_not_touch(wide):
+    """A dedup image of three planes, packed or scattered with a batch that also holds tables of 70 planes for the other side."""
+    from vllm_rlt_b200.kernels import kv_handoff as k
+
+    page, planes, many, lengths = 4, 3, 70, [30, 9]
+    P = oracle_pool("bf16", (2, 1, 16, 64, page, planes))
+    D = sentinel_destination("bf16", (2, 1, 16, 64, page, planes))
+    P.fill_random(np.random.default_rng(1))
+    rng, exits, others = random.Random(1), [], []
+    for i, n in enumerate(lengths):
+        assert P.allocate(f"r{i}", n) and D.allocate(f"r{i}", n)
+        exits.append([rng.randrange(planes) for _ in range(n)])
+        others.append([[rng.randrange(64) for _ in range(-(-n // page))] for _ in range(many)])
+        for pos in range(n):
+            P.finalize_token(f"r{i}", pos, exits[i][pos])
+    src, dst = ([pool.plane_block_tables(f"r{i}") for i in range(len(lengths))] for pool in (P, D))
+    ranges = [(0, n) for n in lengths]
+    gp, gd = GpuPool(P), GpuPool(D)
+    pack = k.HandoffBatch(src, others if wide == "destination" else None, ranges, block_size=page, exit_planes=exits)
+    scatter = k.HandoffBatch(others if wide == "source" else None, dst, ranges, block_size=page, exit_planes=exits)
+    status = k.new_status()
+    packed = torch.zeros(k.packed_bytes(gp.view(), pack.total_tokens, planes), dtype=torch.uint8, device="cuda")
+    k.kv_pack(gp.view(), pack, packed, mode=k.MODE_DEDUP, status=status, workspace=k.dedup_workspace(pack, planes))
+    want = np.concatenate([ho.pack_rows(P, t, s, e, mode=ho.MODE_DEDUP, exit_planes=x) for t, (s, e), x in zip(src, ranges, exits)])
+    assert np.array_equal(packed.cpu().numpy()[: want.size], want)
+    k.kv_scatter(packed, gd.view(), scatter, mode=k.MODE_DEDUP, status=status, workspace=k.dedup_workspace(scatter, planes))
+    k.raise_for_status(status)
+    for i, (s, e) in enumerate(ranges):
+        ho.handoff_rows(P, D, src[i], dst[i], s, e, mode=ho.MODE_DEDUP, exit_planes=exits[i])
+    assert_pools_equal(gd, D)

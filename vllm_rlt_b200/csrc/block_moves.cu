@@ -571,11 +571,13 @@ extern "C" int rlt_move_blocks(int direction, const RltPool* src, const RltPool*
     if (reinterpret_cast<uintptr_t>(opt->workspace) & 15u) return RLT_E_ALIGN;
     if (opt->workspace_bytes < dedup_workspace_bytes(m->num_requests, m->table_width, t.src_planes)) return RLT_E_LIMIT;
   }
-  if (opt->variant != 0 || opt->grid_limit != 0 || t.src_planes > 64 || t.dst_planes > 64) return RLT_MOVE_UNSUITED;
+  if (opt->variant != 0 || opt->grid_limit != 0 || t.src_planes > kMaxPlanes || t.dst_planes > kMaxPlanes) return RLT_MOVE_UNSUITED;
   if (dir != kDirect && (t.plane_begin != 0 || t.plane_count != t.dst_planes)) return RLT_MOVE_UNSUITED;
   if (t.block_size != m->block_size || (dir != kScatter && m->src_planes != t.src_planes) ||
       (dir != kPack && m->dst_planes != t.dst_planes))
     return RLT_MOVE_UNSUITED;
+  // a CTA lists a page's blocks on both sides, also on the one that this direction does not touch
+  if (m->src_planes > kMaxPlanes || m->dst_planes > kMaxPlanes) return RLT_MOVE_UNSUITED;
   if (t.dedup_wire && m->host_wire == nullptr) return RLT_MOVE_UNSUITED;
   if (m->blocks == 0) return RLT_OK;
 
