@@ -115,3 +115,22 @@ def test_a_batch_with_more_planes_on_the_side_that_an_image_does_not_touch(wide)
     for i, (s, e) in enumerate(ranges):
         ho.handoff_rows(P, D, src[i], dst[i], s, e, mode=ho.MODE_DEDUP, exit_planes=exits[i])
     assert_pools_equal(gd, D)
+
+
+@pytest.mark.parametrize("layers", [255, 256, 300])  # 4,096 pairs a page: 32-bit division of (layer, pair) ends at 256 layers
+def test_a_dedup_pack_of_many_layers_of_full_pages_on_many_planes(layers):
+    from vllm_rlt_b200.kernels import kv_handoff as k
+
+    planes = page = 64
+    key, value = (torch.randint(-30000, 30000, (planes + 1, layers, page, 1, 1), dtype=torch.int16, device="cuda") for _ in range(2))
+    blocks = torch.randperm(planes + 1)[:planes]
+    exits = torch.randint(0, planes, (page,))
+    exits[:60] = planes - 1
+    view = k.PoolView.from_tensors(key.view(torch.bfloat16), value.view(torch.bfloat16), planes)
+    batch = k.HandoffBatch([[[b] for b in blocks.tolist()]], None, [(0, page)], block_size=page, exit_planes=[exits.tolist()])
+    want = torch.cat([t[b, :, (exits >= p).cuda()].reshape(-1) for p, b in enumerate(blocks.tolist()) for t in (key, value)])
+    packed = torch.zeros(k.packed_bytes(view, page, planes), dtype=torch.uint8, device="cuda")
+    status, workspace = k.new_status(), k.dedup_workspace(batch, planes)
+    k.kv_pack(view, batch, packed, mode=k.MODE_DEDUP, status=status, workspace=workspace)
+    k.raise_for_status(status)
+    assert torch.equal(packed.view(torch.int16)[: want.numel()], want)

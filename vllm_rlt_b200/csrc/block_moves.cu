@@ -604,6 +604,9 @@ extern "C" int rlt_move_blocks(int direction, const RltPool* src, const RltPool*
     if ((row_vecs + 65536) * row_vecs >= (1ll << 32) || slice_vecs * t.src_planes >= (1ll << 30) ||
         static_cast<long long>(t.block_size) * t.block_size * p.slice_layers >= (1ll << 32))
       return RLT_MOVE_UNSUITED;
+    // the one of pack_pairs: (layers x pairs of a page) * pairs
+    const long long most_pairs = static_cast<long long>(t.block_size) * t.src_planes;
+    if (pairs && most_pairs * most_pairs * p.slice_layers >= (1ll << 32)) return RLT_MOVE_UNSUITED;
     rg.row_vecs = static_cast<int>(row_vecs);
     rg.row_magic = row_vecs == 1 ? 0u : div_magic(static_cast<uint32_t>(row_vecs));
     rg.slice_vecs = static_cast<int>(slice_vecs);
