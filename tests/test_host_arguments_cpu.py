@@ -46,3 +46,21 @@ def test_a_batch_without_tables_holds_no_records():
     batch = kh.HandoffBatch(None, None, [(0, 1 << 40)], block_size=16)
     assert batch.metadata_bytes == 0 and batch.total_tokens == 1 << 40
 
+
+
+def test_two_threads_that_ask_for_a_views_struct_get_one_that_stays():
+    from vllm_rlt_b200.kernels import kv_handoff as kh
+
+    seen = []
+
+    class View(kh.PoolView):
+        def as_struct(self):
+            struct = super().as_struct()
+            if not seen:  # the other thread comes in between, and has used its address already
+                seen.append(None)
+                seen[0] = self._address()
+            return struct
+
+    view = View(kh.Region(4096, 8192, 384, 128, 32), None, 8, 4, 3, 2, 0)
+    assert view._address() == seen[0] == view._address()
+

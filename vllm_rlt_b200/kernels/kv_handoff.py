@@ -136,8 +136,8 @@ class PoolView:
         hit = self.__dict__.get("_struct")
         if hit is None:
             struct = self.as_struct()
-            hit = (C.addressof(struct), struct)
-            object.__setattr__(self, "_struct", hit)
+            # one struct, also where two threads get here at once: an address that is in use stays good
+            hit = self.__dict__.setdefault("_struct", (C.addressof(struct), struct))
         return hit[0]
 
     @property
