@@ -162,7 +162,7 @@ def test_the_events_of_a_batch_are_recorded_and_waited_for_on_the_device_that_la
         def order(self, device, stream):
             log.append(("order", device, stream))
 
-    monkeypatch.setattr(kv_handoff._lib, "load_host", lambda: types.SimpleNamespace(event=Event))
+    monkeypatch.setattr(kv_handoff._lib, "load_host", lambda: types.SimpleNamespace(event=Event, capture=lambda stream: 0))
     monkeypatch.setattr(torch.cuda, "current_device", lambda: current[0])
     memory = types.SimpleNamespace(device=types.SimpleNamespace(index=1), data_ptr=lambda: 64)
     sent = kv_handoff._Sent(memory, 0)

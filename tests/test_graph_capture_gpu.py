@@ -124,3 +124,26 @@ def test_what_cannot_be_captured_is_refused_and_the_capture_goes_on():
     graph.replay()
     torch.cuda.synchronize()
     assert moved(pools, tables, 0, 1)
+
+
+def test_a_batch_dropped_while_its_stream_captures_leaves_the_capture_alone():
+    from vllm_rlt_b200.kernels import kv_handoff as kh
+
+    pages = 1000
+    pools, views, tables = single_plane(pages)
+    own, other = torch.cuda.Stream(), torch.cuda.Stream()
+    pools[0].key_cache.normal_()
+    pools[0].value_cache.normal_()
+    torch.cuda.synchronize()
+    dropped = kh.HandoffBatch(tables[0], tables[1], [(0, 4 * pages)], block_size=4, stream=own)
+    kept = kh.HandoffBatch(tables[1], tables[2], [(0, 4 * pages)], block_size=4, stream=own)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=own):
+        kh.kv_handoff(views[0], views[1], dropped, stream=other)  # outside the capture
+        del dropped
+        kh.kv_handoff(views[1], views[2], kept, stream=own)
+    torch.cuda.synchronize()
+    assert moved(pools, tables, 0, 1) and not moved(pools, tables, 1, 2)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert moved(pools, tables, 1, 2)

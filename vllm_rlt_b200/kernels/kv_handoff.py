@@ -228,8 +228,12 @@ class _Sent:
 
     def __del__(self):
         try:
+            capturing = self._used and _lib.load_host().capture(self.stream)
             for event in self._used.values():
-                event.order(self.tensor.device.index, self.stream)
+                if capturing:  # the stream's next work is a graph's, which cannot wait for this
+                    event.synchronize()
+                else:
+                    event.order(self.tensor.device.index, self.stream)
         except Exception:  # the caller's stream is gone, and with it whatever was queued there
             pass
 
