@@ -679,3 +679,12 @@ extern "C" int rlt_move_blocks(int direction, const RltPool* src, const RltPool*
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return RLT_OK;
 }
+
+extern "C" int rlt_load_moves(void) {
+  using namespace rlt;
+  RLT_CUDA_TRY(load_kernel(move_kernel<kPlaneToPlane, kInlineSmallWords>));
+  RLT_CUDA_TRY(load_kernel(move_kernel<kPlaneToPlane, kInlineMediumWords>));
+  RLT_CUDA_TRY(load_kernel(move_kernel<kPlaneToPlane, kInlineWords>));
+  RLT_CUDA_TRY(load_kernel(move_kernel<kPlaneToPlane, 1>));
+  return RLT_OK;
+}

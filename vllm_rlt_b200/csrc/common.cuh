@@ -59,6 +59,12 @@ inline cudaError_t launch_following(void (*kernel)(P...), dim3 grid, unsigned bl
   config.numAttrs = 1;
   return cudaLaunchKernelEx(&config, kernel, args...);
 }
+// Loads a kernel, if that has not been done.
+template <typename... P>
+inline cudaError_t load_kernel(void (*kernel)(P...)) {
+  cudaFuncAttributes unused;
+  return cudaFuncGetAttributes(&unused, kernel);
+}
 __device__ __forceinline__ void follow_stream() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -98,6 +104,46 @@ __device__ __forceinline__ uint32_t ld_stream(const uint32_t* p) { return __ldcs
 __device__ __forceinline__ void st_stream(uint32_t* p, uint32_t v) { __stcs(p, v); }
 __device__ __forceinline__ uint8_t ld_stream(const uint8_t* p) { return *p; }
 __device__ __forceinline__ void st_stream(uint8_t* p, uint8_t v) { *p = v; }
+
+// A CTA copies elements [0, n).
+template <typename T, int kUnroll = 4>
+__device__ __forceinline__ void stream_range(const char* __restrict__ src, char* __restrict__ dst, long long n) {
+  const T* s = reinterpret_cast<const T*>(src);
+  T* d = reinterpret_cast<T*>(dst);
+  for (long long base = threadIdx.x; base < n; base += kThreads * kUnroll) {
+    T regs[kUnroll];
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) {
+      const long long i = base + u * kThreads;
+      if (i < n) regs[u] = ld_stream(s + i);
+    }
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) {
+      const long long i = base + u * kThreads;
+      if (i < n) st_stream(d + i, regs[u]);
+    }
+  }
+}
+
+// A CTA copies one tile of a byte range. kWide: 32-byte accesses where both pointers allow. Pointers that are both 16-byte
+// aligned take the vector path with a byte tail; otherwise the widest element both pointers and the length allow.
+template <bool kWide>
+__device__ __forceinline__ void copy_piece(const char* src, char* dst, long long n) {
+  const unsigned long long both = reinterpret_cast<unsigned long long>(src) | reinterpret_cast<unsigned long long>(dst);
+  if (kWide && (both & 31ull) == 0) {
+    const long long body = n & ~31ll;
+    stream_range<Vec32, 2>(src, dst, body >> 5);
+    if (static_cast<long long>(threadIdx.x) < n - body) dst[body + threadIdx.x] = src[body + threadIdx.x];
+  } else if ((both & 15ull) == 0) {
+    const long long body = n & ~15ll;
+    stream_range<uint4>(src, dst, body >> 4);
+    if (static_cast<long long>(threadIdx.x) < n - body) dst[body + threadIdx.x] = src[body + threadIdx.x];
+  } else if (((both | static_cast<unsigned long long>(n)) & 3ull) == 0) {
+    stream_range<uint32_t>(src, dst, n >> 2);
+  } else {
+    stream_range<uint8_t>(src, dst, n);
+  }
+}
 
 // Inclusive prefix sum across the 32 lanes of a warp.
 __device__ __forceinline__ int warp_inclusive_scan(int v) {

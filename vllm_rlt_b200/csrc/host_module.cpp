@@ -1059,6 +1059,10 @@ struct RequestRecords {
     before += end - start;
   }
   int launch(const RltOptions& o, rlt_stream_t stream) const {
+    const RltBlockMoves m = moves();
+    return rlt_handoff_staged(src, dst, &m, &o, stream);
+  }
+  RltBlockMoves moves() const {
     RltBlockMoves m = {};
     m.host_records = records.data();
     m.blocks = static_cast<int32_t>(blocks);
@@ -1068,57 +1072,117 @@ struct RequestRecords {
     m.block_size = src->block_size;
     m.num_requests = static_cast<int32_t>(requests);
     m.table_width = static_cast<int32_t>(width);
-    return rlt_handoff_staged(src, dst, &m, &o, stream);
+    return m;
   }
 };
 
-// handoff_requests(source pool, destination pool, requests, layer_begin, layer_end, plane_begin, plane_end, device, stream) -> code of an
-// all-planes handoff of [(source tables, target tables, start, end)], or RLT_MOVE_UNSUITED (nothing queued) when something about the
-// requests looks wrong or their records do not fit the library's own staging: the general path then does it, or says what is wrong.
-PyObject* handoff_requests(PyObject* const* a) {
-  const auto* src = static_cast<const RltPool*>(address(a[0]));
-  const auto* dst = static_cast<const RltPool*>(address(a[1]));
-  const Ref requests(PySequence_Fast(a[2], "requests must be a sequence"));
-  const int64_t bs = src->block_size;
+// A mailbox message: slot address, 56-byte body, stamp.
+struct Message {
+  void* slot;
+  const uint8_t* body;
+  uint64_t stamp;
+  explicit Message(PyObject* const* a) : slot(address(a[0])) {
+    char* bytes = nullptr;
+    Py_ssize_t n = 0;
+    if (PyBytes_AsStringAndSize(a[1], &bytes, &n) != 0) throw Failure{};
+    if (n != 56) bad_value("a message body has 56 bytes");
+    body = reinterpret_cast<const uint8_t*>(bytes);
+    stamp = PyLong_AsUnsignedLongLong(a[2]);
+    if (PyErr_Occurred()) throw Failure{};
+  }
+  // Posted behind copies of `ranges`, [n](source, destination, bytes): with them where they are few and small.
+  int post(const std::vector<int64_t>& ranges, rlt_stream_t stream) const {
+    const int rc = rlt_post_behind(ranges.data(), static_cast<int32_t>(ranges.size() / 3), slot, body, stamp, stream);
+    return rc == RLT_E_LIMIT ? post_last(ranges, stream) : rc;
+  }
+
+ private:
+  int post_last(const std::vector<int64_t>& ranges, rlt_stream_t stream) const {
+    for (size_t i = 0; i < ranges.size(); i += 3) {
+      const int rc = rlt_kv_push(reinterpret_cast<void*>(ranges[i]), reinterpret_cast<void*>(ranges[i + 1]), ranges[i + 2], stream);
+      if (rc != RLT_OK) return rc;
+    }
+    return rlt_kv_post(slot, body, stamp, stream);
+  }
+};
+
+// The records of [(source tables, target tables, start, end)]; false where something about the requests looks wrong or the library's
+// own staging does not hold their records: the general path then does it, or says what is wrong.
+bool records_of(PyObject* sequence, RequestRecords& out) {
+  const Ref requests(PySequence_Fast(sequence, "requests must be a sequence"));
+  const int64_t bs = out.src->block_size;
   const Py_ssize_t n = PySequence_Fast_GET_SIZE(requests.p);
-  auto unsuited = [] { return PyLong_FromLong(RLT_MOVE_UNSUITED); };
-  if (n < 1 || bs < 1) return unsuited();
-  RequestRecords out(src, dst);
+  if (n < 1 || bs < 1) return false;
   Ints ids;
   for (Py_ssize_t r = 0; r < n; ++r) {
     const Ref request(PySequence_Fast(PySequence_Fast_GET_ITEM(requests.p, r), "a request is (source, target, start, end)"));
-    if (PySequence_Fast_GET_SIZE(request.p) < 4) return unsuited();
+    if (PySequence_Fast_GET_SIZE(request.p) < 4) return false;
     const int64_t start = integer(PySequence_Fast_GET_ITEM(request.p, 2)), end = integer(PySequence_Fast_GET_ITEM(request.p, 3));
-    if (start < 0 || start >= end) return unsuited();
+    if (start < 0 || start >= end) return false;
     const int64_t first = start / bs, pages = (end - 1) / bs - first + 1;
-    if (!out.fits(pages)) return unsuited();
+    if (!out.fits(pages)) return false;
     ids.clear();
     for (int side = 0; side < 2; ++side) {
-      const RltPool* pool = side == 0 ? src : dst;
+      const RltPool* pool = side == 0 ? out.src : out.dst;
       const Ref tables(PySequence_Fast(PySequence_Fast_GET_ITEM(request.p, side), "block tables must be a sequence"));
-      if (PySequence_Fast_GET_SIZE(tables.p) != pool->num_planes) return unsuited();
+      if (PySequence_Fast_GET_SIZE(tables.p) != pool->num_planes) return false;
       Py_ssize_t of_request = -1;
       const size_t at = ids.size();
       for (int p = 0; p < pool->num_planes; ++p) {
         PyObject* table = PySequence_Fast_GET_ITEM(tables.p, p);
         const Py_ssize_t held = length(table);
-        if (held < first + pages || (of_request >= 0 && held != of_request)) return unsuited();
+        if (held < first + pages || (of_request >= 0 && held != of_request)) return false;
         of_request = held;
         out.width = held > out.width ? held : out.width;
         append_range(table, first, first + pages, ids);
       }
-      if (!out.valid(ids.data() + at, static_cast<int64_t>(ids.size() - at), pool)) return unsuited();
+      if (!out.valid(ids.data() + at, static_cast<int64_t>(ids.size() - at), pool)) return false;
     }
     out.add(ids.data(), pages, 0, first, pages, start, end);
   }
+  return true;
+}
+
+RltOptions slice_of(PyObject* const* a) {  // layer_begin, layer_end, plane_begin, plane_end
   RltOptions o = {};
-  o.layer_begin = static_cast<int32_t>(integer(a[3]));
-  o.layer_end = static_cast<int32_t>(integer(a[4]));
-  o.plane_begin = static_cast<int32_t>(integer(a[5]));
-  o.plane_end = static_cast<int32_t>(integer(a[6]));
+  o.layer_begin = static_cast<int32_t>(integer(a[0]));
+  o.layer_end = static_cast<int32_t>(integer(a[1]));
+  o.plane_begin = static_cast<int32_t>(integer(a[2]));
+  o.plane_end = static_cast<int32_t>(integer(a[3]));
+  return o;
+}
+
+// handoff_requests(source pool, destination pool, requests, layer_begin, layer_end, plane_begin, plane_end, device, stream) -> code of an
+// all-planes handoff of the requests, or RLT_MOVE_UNSUITED (nothing queued) where records_of leaves them to the general path.
+PyObject* handoff_requests(PyObject* const* a) {
+  RequestRecords out(static_cast<const RltPool*>(address(a[0])), static_cast<const RltPool*>(address(a[1])));
+  if (!records_of(a[2], out)) return PyLong_FromLong(RLT_MOVE_UNSUITED);
+  const RltOptions o = slice_of(a + 3);
   const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(integer(a[7])));
   const rlt_stream_t stream = stream_of(a[8]);
   return PyLong_FromLong(unlocked([&] { return out.launch(o, stream); }));
+}
+
+// push_chunk(source pool, destination pool, requests, [(source address, destination address, bytes)], layer_begin, layer_end, plane_begin,
+//            plane_end, slot, body, stamp, device, stream) -> code of handoff_requests, with copies of the ranges and the message behind it
+PyObject* push_chunk(PyObject* const* a) {
+  RequestRecords out(static_cast<const RltPool*>(address(a[0])), static_cast<const RltPool*>(address(a[1])));
+  if (!records_of(a[2], out)) return PyLong_FromLong(RLT_MOVE_UNSUITED);
+  std::vector<int64_t> ranges;
+  const Ref list(PySequence_Fast(a[3], "ranges must be a sequence"));
+  for (Py_ssize_t i = 0; i < PySequence_Fast_GET_SIZE(list.p); ++i) {
+    const Ref range(PySequence_Fast(PySequence_Fast_GET_ITEM(list.p, i), "a range is (source, target, bytes)"));
+    if (PySequence_Fast_GET_SIZE(range.p) != 3) bad_value("a range is (source, target, bytes)");
+    for (int k = 0; k < 3; ++k) ranges.push_back(integer(PySequence_Fast_GET_ITEM(range.p, k)));
+  }
+  const RltOptions o = slice_of(a + 4);
+  const Message message(a + 8);
+  const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(integer(a[11])));
+  const rlt_stream_t stream = stream_of(a[12]);
+  return PyLong_FromLong(unlocked([&] {
+    const int rc = out.launch(o, stream);
+    return rc == RLT_OK ? message.post(ranges, stream) : rc;
+  }));
 }
 
 // A recorded event of the library's pool.
@@ -1313,6 +1377,12 @@ PyObject* post(PyObject* const* a) {
   return PyLong_FromLong(unlocked([&] { return rlt_kv_post(slot, reinterpret_cast<const uint8_t*>(body), stamp, stream); }));
 }
 
+// load_transport(device) -> code
+PyObject* load_transport(PyObject* const* a) {
+  const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(integer(a[0])));
+  return PyLong_FromLong(unlocked([] { return rlt_load_transport(); }));
+}
+
 // ------------------------------------------------------------------------------------------------ the module
 
 template <PyObject* (*kFunction)(PyObject* const*), int kArgs>
@@ -1351,6 +1421,8 @@ PyMethodDef kMethods[] = {
     RLT_ENTRY("pull_chunk", pull_chunk, 6),
     RLT_ENTRY("pack_segments", pack_segments, 3),
     RLT_ENTRY("copy_segments", copy_segments, 3),
+    RLT_ENTRY("push_chunk", push_chunk, 13),
+    RLT_ENTRY("load_transport", load_transport, 1),
     RLT_ENTRY("push", push, 5),
     RLT_ENTRY("post", post, 5),
     RLT_ENTRY("tensor_copy", tensor_copy, 3),

@@ -22,6 +22,17 @@ RLT_API int rlt_capture_id(rlt_stream_t stream, uint64_t* id);  // of the captur
 RLT_API int rlt_tensor_transfer_inline(const int64_t* descriptors, int32_t count, int32_t max_rows, int32_t max_cols,
                                        int32_t dtype, rlt_stream_t stream);
 
+// rlt_kv_post behind copies of a few small byte ranges, (source, destination, bytes) in HOST memory, in one launch.
+#define RLT_POST_RANGES 4
+#define RLT_POST_RANGE_BYTES 32768  // of all of them
+RLT_API int rlt_post_behind(const int64_t* ranges, int32_t count, void* slot, const uint8_t body[56], uint64_t stamp, rlt_stream_t stream);
+
+// Loads the kernels of a transfer worker on the current device. A kernel is otherwise loaded by its first launch, and that may wait for what
+// runs on the device by then: a message that should be queued behind a prefill would hold the host until the prefill has ended.
+RLT_API int rlt_load_transport(void);
+int rlt_load_moves(void);
+int rlt_load_segments(void);
+
 // rlt_kv_copy_segments with the (source, destination, bytes) triples in HOST memory: they travel as kernel parameters.
 #define RLT_INLINE_SEGMENTS 1024
 RLT_API int rlt_copy_segments_inline(const int64_t* triples, int32_t count, rlt_stream_t stream);

@@ -30,48 +30,7 @@ namespace {
 
 constexpr long long kTileBytes = 32 * 1024;   // of the persistent kernel: 16, 64 and 128 KiB, and 4 or 6 CTAs per SM, all measured slower
 constexpr long long kShortTile = 16 * 1024;   // of one CTA per tile
-constexpr int kUnroll = 4;
 constexpr int kCtasPerSm = 3;
-
-template <typename T, int kUnroll = rlt::kUnroll>
-__device__ __forceinline__ void stream_range(const char* __restrict__ src, char* __restrict__ dst, long long n) {
-  const T* s = reinterpret_cast<const T*>(src);
-  T* d = reinterpret_cast<T*>(dst);
-  for (long long base = threadIdx.x; base < n; base += kThreads * kUnroll) {
-    T regs[kUnroll];
-#pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
-      const long long i = base + u * kThreads;
-      if (i < n) regs[u] = ld_stream(s + i);
-    }
-#pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
-      const long long i = base + u * kThreads;
-      if (i < n) st_stream(d + i, regs[u]);
-    }
-  }
-}
-
-// One tile of one range. kWide: 32-byte accesses where both pointers allow (the persistent kernel measured slower with
-// them: 136 -> 140 us for 0.8 GB). Pointers that are both 16-byte aligned take the vector path with a byte tail;
-// otherwise the widest element both pointers and the length allow.
-template <bool kWide>
-__device__ __forceinline__ void copy_piece(const char* src, char* dst, long long n) {
-  const unsigned long long both = reinterpret_cast<unsigned long long>(src) | reinterpret_cast<unsigned long long>(dst);
-  if (kWide && (both & 31ull) == 0) {
-    const long long body = n & ~31ll;
-    stream_range<Vec32, 2>(src, dst, body >> 5);
-    if (static_cast<long long>(threadIdx.x) < n - body) dst[body + threadIdx.x] = src[body + threadIdx.x];
-  } else if ((both & 15ull) == 0) {
-    const long long body = n & ~15ll;
-    stream_range<uint4>(src, dst, body >> 4);
-    if (static_cast<long long>(threadIdx.x) < n - body) dst[body + threadIdx.x] = src[body + threadIdx.x];
-  } else if (((both | static_cast<unsigned long long>(n)) & 3ull) == 0) {
-    stream_range<uint32_t>(src, dst, n >> 2);
-  } else {
-    stream_range<uint8_t>(src, dst, n);
-  }
-}
 
 __global__ void __launch_bounds__(kThreads, 6) push_kernel(const char* src, char* dst, long long nbytes) {
   const long long at = static_cast<long long>(blockIdx.x) * kShortTile;
@@ -192,6 +151,15 @@ int rlt_copy_segments_inline(const int64_t* triples, int32_t count, rlt_stream_t
   return count <= 32    ? rlt::launch_inline<32>(triples, count, s)
          : count <= 256 ? rlt::launch_inline<256>(triples, count, s)
                         : rlt::launch_inline<RLT_INLINE_SEGMENTS>(triples, count, s);
+}
+
+int rlt_load_segments(void) {
+  using namespace rlt;
+  RLT_CUDA_TRY(load_kernel(push_kernel));
+  RLT_CUDA_TRY(load_kernel(inline_segments_kernel<32>));
+  RLT_CUDA_TRY(load_kernel(inline_segments_kernel<256>));
+  RLT_CUDA_TRY(load_kernel(inline_segments_kernel<RLT_INLINE_SEGMENTS>));
+  return RLT_OK;
 }
 
 int rlt_kv_copy_segments(const int64_t* segments, int32_t count, rlt_stream_t stream) {

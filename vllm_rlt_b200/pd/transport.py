@@ -315,6 +315,7 @@ class CudaBackend:
         self.stream = torch.cuda.Stream(self.device)
         self._where = (self.stream.device.index, self.stream.cuda_stream)  # what the compiled calls launch on
         self._host = _lib.load_host()
+        _lib.check(self._host.load_transport(self._where[0]), "rlt_load_transport")
 
     def order_after(self, event) -> None:
         """Make everything submitted from now on wait (on the device) for ``event``."""
@@ -432,6 +433,18 @@ class CudaBackend:
             kh.kv_handoff(src, dst, batch, mode=mode, layer_begin=layer_begin, layer_end=layer_end,
                           plane_begin=plane_begin, plane_end=plane_end, status=status)
         return (batch,)
+
+    def push_chunk(self, cache, peer_info, translate, requests, ranges, slot_ptr: int, body: bytes, stamp: int, *, layer_begin,
+                   layer_end, plane_begin, plane_end) -> bool:
+        """``handoff`` of every plane to the peer's pool, ``copy_ranges`` and ``post`` by one compiled call; False (nothing queued) where
+        the general path must do it or say what is wrong."""
+        src, dst = self._views_of(cache, peer_info, translate, False, False)
+        rc = self._host.push_chunk(src._address(), dst._address(), requests, ranges, layer_begin, layer_end, plane_begin, plane_end,
+                                   slot_ptr, body, stamp, *self._where)
+        if rc == _lib.MOVE_UNSUITED:
+            return False
+        _lib.check(rc, "rlt_kv_handoff")
+        return True
 
     def post(self, slot_ptr: int, body: bytes, stamp: int):
         _lib.check(self._host.post(slot_ptr, body, stamp, *self._where), "rlt_kv_post")
@@ -615,15 +628,21 @@ class B200Transport:
             return False
         return self._slot_free(link)
 
-    def _post(self, link: dict, body: bytes, *, from_host: bool = False) -> None:
-        if not from_host and link["box_ptr"] is None:
+    def _next_slot(self, link: dict) -> tuple[int, int]:
+        """Where this worker's device posts its next message on a link, and the stamp. The caller counts the message once it is queued."""
+        if link["box_ptr"] is None:
             link["box_ptr"] = self.backend.mailbox_address(self.peers[link["agent"]]["metadata"]["mailbox"])
-        link["stamp"] += 1
+        stamp = link["stamp"] + 1
+        return link["box_ptr"] + Mailbox.slot_offset(link["lane"], stamp), stamp
+
+    def _post(self, link: dict, body: bytes, *, from_host: bool = False) -> None:
         if from_host:
+            link["stamp"] += 1
             link["box"].post_from_host(link["lane"], link["stamp"], body)
         else:
-            at = Mailbox.slot_offset(link["lane"], link["stamp"])
-            self.backend.post(link["box_ptr"] + at, body, link["stamp"])
+            at, stamp = self._next_slot(link)
+            link["stamp"] = stamp
+            self.backend.post(at, body, stamp)
 
     def _tickets(self, handle, transfer_id, parts, keepalive, started) -> bool:
         now = time.monotonic()
@@ -702,12 +721,20 @@ class B200Transport:
             return self._offer(link, transfer_id, parts, requests, extra, where, after)
         body = Mailbox.encode(transfer_id, sequence, LANDED, count=len(parts))
         translate = link["translate"]
+        ranges = [(s, translate(d, n), n) for s, d, n in extra]
+        at_once = getattr(self.backend, "push_chunk", None) if mode == 0 and exit_planes is None and status is None else None
+        slot = self._next_slot(link) if at_once is not None else None
         started = self._order_after(after)
-        keep = tuple(self.backend.handoff(self.cache, self.peers[peer], translate, requests, exit_planes=exit_planes,
-                                          status=status, **where))
-        if extra:
-            keep += tuple(self.backend.copy_ranges([(s, translate(d, n), n) for s, d, n in extra]))
-        self._post(link, body)
+        keep = ()
+        if at_once is not None and at_once(self.cache, self.peers[peer], translate, requests, ranges, slot[0], body, slot[1],
+                                           layer_begin=layer_begin, layer_end=layer_end, plane_begin=plane_begin, plane_end=plane_end):
+            link["stamp"] = slot[1]
+        else:
+            keep = tuple(self.backend.handoff(self.cache, self.peers[peer], translate, requests, exit_planes=exit_planes,
+                                              status=status, **where))
+            if ranges:
+                keep += tuple(self.backend.copy_ranges(ranges))
+            self._post(link, body)
         return self._tickets(self.backend.event(), transfer_id, parts, keep, started)
 
     def _offer(self, link, transfer_id, parts, requests, extra, where, after) -> bool:
