@@ -80,6 +80,7 @@ constexpr int kTile = 256;
 
 template <typename S, typename D>
 __global__ void __launch_bounds__(kTile) segmented_transfer_kernel(const long long* __restrict__ descriptors) {
+  follow_stream();
   const long long* d = descriptors + 8ll * blockIdx.x;
   const S* src = reinterpret_cast<const S*>(d[0]);
   D* dst = reinterpret_cast<D*>(d[1]);
@@ -124,6 +125,7 @@ __global__ void __launch_bounds__(kTile) inline_transfer_kernel(const __grid_con
   const long long* d = table.d[blockIdx.x];
   const long long rows = d[2], cols = d[3], sr = d[4], sc = d[5], dr = d[6], dc = d[7];
   const long long c0 = blockIdx.z * kCols;
+  follow_stream();
   if (c0 >= cols) return;
   const int n = static_cast<int>(cols - c0 < kCols ? cols - c0 : kCols);
 #pragma unroll
@@ -138,7 +140,7 @@ template <typename T, int kCount>
 int launch_inline(const int64_t* descriptors, int count, dim3 grid, cudaStream_t stream) {
   InlineDescriptors<kCount> table;
   std::memcpy(table.d, descriptors, static_cast<size_t>(count) * sizeof(table.d[0]));
-  inline_transfer_kernel<T, kCount><<<grid, kTile, 0, stream>>>(table);
+  RLT_CUDA_TRY(launch_following(inline_transfer_kernel<T, kCount>, grid, kTile, stream, table));
   return RLT_OK;
 }
 
@@ -274,7 +276,7 @@ template <typename S, typename D>
 int launch_segmented(const long long* descriptors, int count, int max_rows, int max_cols, cudaStream_t stream) {
   const dim3 grid(count, (max_rows + kRows - 1) / kRows, (max_cols + kTile - 1) / kTile);
   if (grid.y > 65535u || grid.z > 65535u) return RLT_E_LIMIT;
-  segmented_transfer_kernel<S, D><<<grid, kTile, 0, stream>>>(descriptors);
+  RLT_CUDA_TRY(launch_following(segmented_transfer_kernel<S, D>, grid, kTile, stream, descriptors));
   return RLT_OK;
 }
 
