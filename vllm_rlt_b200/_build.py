@@ -139,6 +139,10 @@ def _build_torch_module(name: str, source_name: str, headers: list[Path], force:
     def command(output: Path) -> list[str]:
         includes = [f"-I{p}" for p in cpp_extension.include_paths("cuda")] + [f"-I{INCLUDE}", f"-I{CSRC}"]
         includes.append(f"-I{sysconfig.get_paths()['include']}")
+        if python:
+            import numpy
+
+            includes.append(f"-I{numpy.get_include()}")
         torch_lib = Path(torch.__file__).parent / "lib"
         libraries = ["-ltorch", "-ltorch_cpu", "-lc10", "-ltorch_cuda", "-lc10_cuda"] + (["-ltorch_python"] if python else [])
         return ["g++", *flags[:-1], *includes, str(source), "-o", str(output),

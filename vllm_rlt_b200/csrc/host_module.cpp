@@ -12,6 +12,8 @@
 #include <ATen/core/Tensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#define NPY_NO_DEPRECATED_API NPY_2_0_API_VERSION
+#include <numpy/arrayobject.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <cstddef>
@@ -115,6 +117,16 @@ bool is_int32(const Py_buffer& v) {
   return v.itemsize == 4 && v.format != nullptr && (std::strcmp(v.format, "i") == 0 || std::strcmp(v.format, "l") == 0);
 }
 
+// An int32 array of NumPy's, or nullptr. Its fields are read directly: asked for a buffer, NumPy describes the element type in a string each
+// time, 0.1 us an array, and a batch has one for every request and plane.
+PyArrayObject* int32_array(PyObject* o) {
+  if (!PyArray_Check(o)) return nullptr;
+  auto* array = reinterpret_cast<PyArrayObject*>(o);
+  const int type = PyArray_TYPE(array);
+  const bool whole = type == NPY_INT || (sizeof(long) == 4 && type == NPY_LONG);
+  return whole && PyArray_ISALIGNED(array) && PyArray_ISNOTSWAPPED(array) ? array : nullptr;
+}
+
 // Appends the int32 values of one table (or exit-plane array) to `out`; returns how many.
 Py_ssize_t append_ints(PyObject* o, Ints& out, const char* not_flat) {
   if (PyTuple_CheckExact(o) || PyList_CheckExact(o)) {
@@ -129,7 +141,21 @@ Py_ssize_t append_ints(PyObject* o, Ints& out, const char* not_flat) {
     }
     return n;
   }
+  auto copy = [&](const char* from, Py_ssize_t n, Py_ssize_t stride) {
+    const size_t at = out.size();
+    out.resize(at + static_cast<size_t>(n));
+    if (stride == 4) {
+      std::memcpy(out.data() + at, from, 4 * static_cast<size_t>(n));
+    } else {
+      for (Py_ssize_t i = 0; i < n; ++i) std::memcpy(&out[at + i], from + i * stride, 4);
+    }
+    return n;
+  };
   auto take = [&](PyObject* source) -> Py_ssize_t {
+    if (PyArrayObject* array = int32_array(source)) {
+      if (PyArray_NDIM(array) != 1) bad_value(not_flat);
+      return copy(PyArray_BYTES(array), PyArray_DIM(array, 0), PyArray_STRIDE(array, 0));
+    }
     Buffer b;
     if (PyObject_GetBuffer(source, &b.view, PyBUF_RECORDS_RO) != 0) {
       PyErr_Clear();
@@ -138,16 +164,7 @@ Py_ssize_t append_ints(PyObject* o, Ints& out, const char* not_flat) {
     b.held = true;
     if (b.view.ndim != 1) bad_value(not_flat);
     if (!is_int32(b.view)) return -1;
-    const Py_ssize_t n = b.view.shape[0], stride = b.view.strides[0];
-    const size_t at = out.size();
-    out.resize(at + static_cast<size_t>(n));
-    const char* from = static_cast<const char*>(b.view.buf);
-    if (stride == 4) {
-      std::memcpy(out.data() + at, from, 4 * static_cast<size_t>(n));
-    } else {
-      for (Py_ssize_t i = 0; i < n; ++i) std::memcpy(&out[at + i], from + i * stride, 4);
-    }
-    return n;
+    return copy(static_cast<const char*>(b.view.buf), b.view.shape[0], b.view.strides[0]);
   };
   Py_ssize_t n = take(o);
   if (n >= 0) return n;
@@ -595,32 +612,47 @@ PyObject* move(PyObject* const* a) {
 
 // handoff_host(source pool, destination pool, source tables, destination tables, begin, end, layer_begin, layer_end,
 //              plane_begin, plane_end, status, stream) -> code
-PyObject* handoff_host(PyObject* const* a) {
-  Buffer b[4];
-  for (int i = 0; i < 4; ++i) {
-    if (PyObject_GetBuffer(a[2 + i], &b[i].view, PyBUF_FORMAT | PyBUF_STRIDES) != 0) {
-      PyErr_Clear();
-      bad_value("host tables and ranges must be C-contiguous int32 arrays");
+struct HostArray {
+  const int32_t* data;
+  int dims;
+  const Py_ssize_t* shape;
+  Buffer buffer;
+  explicit HostArray(PyObject* o) {
+    if (PyArrayObject* array = int32_array(o); array != nullptr && PyArray_IS_C_CONTIGUOUS(array)) {
+      data = static_cast<const int32_t*>(PyArray_DATA(array));
+      dims = PyArray_NDIM(array);
+      shape = PyArray_DIMS(array);
+      return;
     }
-    b[i].held = true;
-    if (!is_int32(b[i].view) || !PyBuffer_IsContiguous(&b[i].view, 'C'))
-      bad_value("host tables and ranges must be C-contiguous int32 arrays");
+    constexpr const char* kWanted = "host tables and ranges must be C-contiguous int32 arrays";
+    if (PyObject_GetBuffer(o, &buffer.view, PyBUF_FORMAT | PyBUF_STRIDES) != 0) {
+      PyErr_Clear();
+      bad_value(kWanted);
+    }
+    buffer.held = true;
+    if (!is_int32(buffer.view) || !PyBuffer_IsContiguous(&buffer.view, 'C')) bad_value(kWanted);
+    data = static_cast<const int32_t*>(buffer.view.buf);
+    dims = buffer.view.ndim;
+    shape = buffer.view.shape;
   }
-  const Py_buffer &s = b[0].view, &d = b[1].view;
-  if (s.ndim != 3) bad_value("host tables must be [requests, planes, width]");
+};
+
+PyObject* handoff_host(PyObject* const* a) {
+  const HostArray s(a[2]), d(a[3]), begin(a[4]), end(a[5]);
+  if (s.dims != 3) bad_value("host tables must be [requests, planes, width]");
   const Py_ssize_t n = s.shape[0];
-  auto one_per_request = [&](const Py_buffer& v) { return v.ndim == 1 && v.shape[0] == n; };
-  if (d.ndim != 3 || d.shape[0] != n || d.shape[2] != s.shape[2] || !one_per_request(b[2].view) || !one_per_request(b[3].view))
+  auto one_per_request = [&](const HostArray& v) { return v.dims == 1 && v.shape[0] == n; };
+  if (d.dims != 3 || d.shape[0] != n || d.shape[2] != s.shape[2] || !one_per_request(begin) || !one_per_request(end))
     bad_value("source and destination tables must agree in requests and width, one range per request");
   RltHostBatch hb = {};
   hb.num_requests = static_cast<int32_t>(n);
   hb.table_width = static_cast<int32_t>(s.shape[2]);
   hb.src_planes = static_cast<int32_t>(s.shape[1]);
   hb.dst_planes = static_cast<int32_t>(d.shape[1]);
-  hb.src_tables = static_cast<const int32_t*>(s.buf);
-  hb.dst_tables = static_cast<const int32_t*>(d.buf);
-  hb.tok_begin = static_cast<const int32_t*>(b[2].view.buf);
-  hb.tok_end = static_cast<const int32_t*>(b[3].view.buf);
+  hb.src_tables = s.data;
+  hb.dst_tables = d.data;
+  hb.tok_begin = begin.data;
+  hb.tok_end = end.data;
   RltOptions o = {};
   o.layer_begin = static_cast<int32_t>(integer(a[6]));
   o.layer_end = static_cast<int32_t>(integer(a[7]));
@@ -1605,6 +1637,7 @@ PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, kMethods, nu
 }  // namespace
 
 PyMODINIT_FUNC PyInit__host(void) {
+  if (_import_array() < 0) return nullptr;
   PyObject* module = PyModule_Create(&kModule);
   if (module == nullptr) return nullptr;
   g_event_type = reinterpret_cast<PyTypeObject*>(PyType_FromSpec(&kEventType));
