@@ -76,6 +76,25 @@ __device__ __forceinline__ void follow_stream() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// Asks L2 for [from, from + bytes), both multiples of 16: nobody waits for it. A kernel launched as above may ask for what it is going to
+// read before follow_stream(), while the kernel ahead of it finishes and memory falls idle: what that one still writes it writes to
+// L2 as well, so nothing stale is ever read. Only for memory of this GPU: another GPU's would cross the link and not be kept.
+__device__ __forceinline__ void prefetch_l2(const char* from, int bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(from), "r"(bytes) : "memory");
+}
+// CTAs ahead of its own that a CTA asks for the source of, where that is worked out from the kernel's parameters alone. It keeps reads coming in
+// the moment between a CTA's end and the next one's first load. Copies of 32 MiB - 1 GiB in 16 KiB pieces, TB/s without / own piece /
+// 148, 296 and 592 CTAs ahead as well: 5.82 / 6.36 / 6.65, 6.64, 6.55; 6.71 / 6.79 / 6.82, 6.77, 6.60; 6.87 / 6.92 / 6.89, 6.86, 6.68.
+// With the records of block_moves.cu 74 is as good or better than 148 in every case tried (1 GB of FP8 pages: 1,101 / 1,090 / 1,086 us
+// at none, own, 74; 1,087 at 148, 1,107 at 592).
+constexpr unsigned kPrefetchAhead = 74;
+// Bytes that a launch reads and writes from which on it asks. Below that all of them may well be in L2 since they were last used, where asking
+// costs a little and gains nothing. us without / with, three pairs of buffers in turn: 24 MB float32 -> bfloat16 3.04 / 3.14, a layer
+// slice of 26 MB 4.19 / 4.42 and of 32 MB 5.70 / 5.71; 42 MB 8.8 / 8.0, 48 MB int64 -> int32 8.45 / 7.07, 1.2 GB 172 / 169.
+constexpr long long kPrefetchBytes = 32 << 20;
+// Whether a launch that moves so many bytes asks for its source, which has to be in memory of the current device (0.07 us to find out).
+bool prefetches(const void* src, long long bytes);
+
 // First error wins: later reports leave the status words alone.
 __device__ __forceinline__ void report(int32_t* status, int code, int a, int b, int c) {
   if (status == nullptr) return;

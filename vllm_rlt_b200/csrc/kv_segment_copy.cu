@@ -32,8 +32,18 @@ constexpr long long kTileBytes = 32 * 1024;   // of the persistent kernel: 16, 6
 constexpr long long kShortTile = 16 * 1024;   // of one CTA per tile
 constexpr int kCtasPerSm = 3;
 
-__global__ void __launch_bounds__(kThreads, 6) push_kernel(const char* src, char* dst, long long nbytes) {
+// Asks for the source of a tile, but for the bytes at its ends that share 16 with others.
+__device__ __forceinline__ void prefetch_tile(const char* src, long long n) {
+  const int skip = static_cast<int>(-reinterpret_cast<intptr_t>(src) & 15);
+  if (n >= skip + 16) prefetch_l2(src + skip, static_cast<int>(n - skip) & ~15);
+}
+
+__global__ void __launch_bounds__(kThreads, 6) push_kernel(const char* src, char* dst, long long nbytes, int prefetch) {
   const long long at = static_cast<long long>(blockIdx.x) * kShortTile;
+  if (prefetch && threadIdx.x < 2) {
+    const long long from = at + (threadIdx.x ? kPrefetchAhead * kShortTile : 0);
+    if (from < nbytes) prefetch_tile(src + from, min(kShortTile, nbytes - from));
+  }
   follow_stream();
   copy_piece<true>(src + at, dst + at, min(kShortTile, nbytes - at));
 }
@@ -46,22 +56,38 @@ struct Segment {
 template <int kCount>
 struct InlineSegments {
   int count;
+  int prefetch;
   int first_tile[kCount + 1];
   Segment segment[kCount];
 };
 
 template <int kCount>
 __global__ void __launch_bounds__(kThreads, 6) inline_segments_kernel(const __grid_constant__ InlineSegments<kCount> list) {
-  const int t = static_cast<int>(blockIdx.x);
-  int lo = 0, hi = list.count;  // last range whose first tile is at or before t
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (list.first_tile[mid] <= t) lo = mid; else hi = mid;
+  struct Tile {
+    const char* src;
+    char* dst;
+    long long bytes;
+  };
+  const auto tile_at = [&](int t) -> Tile {
+    int lo = 0, hi = list.count;  // last range whose first tile is at or before t
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (list.first_tile[mid] <= t) lo = mid; else hi = mid;
+    }
+    const Segment& s = list.segment[lo];
+    const long long at = static_cast<long long>(t - list.first_tile[lo]) * kShortTile;
+    return {s.src + at, s.dst + at, min(kShortTile, s.bytes - at)};
+  };
+  const Tile tile = tile_at(static_cast<int>(blockIdx.x));
+  if (list.prefetch) {
+    if (threadIdx.x == 0) prefetch_tile(tile.src, tile.bytes);
+    if (threadIdx.x == 32 && gridDim.x - blockIdx.x > kPrefetchAhead) {
+      const Tile next = tile_at(static_cast<int>(blockIdx.x + kPrefetchAhead));
+      prefetch_tile(next.src, next.bytes);
+    }
   }
-  const Segment s = list.segment[lo];
-  const long long at = static_cast<long long>(t - list.first_tile[lo]) * kShortTile;
   follow_stream();
-  copy_piece<true>(s.src + at, s.dst + at, min(kShortTile, s.bytes - at));
+  copy_piece<true>(tile.src, tile.dst, tile.bytes);
 }
 
 template <int kCount>
@@ -78,6 +104,7 @@ int launch_inline(const int64_t* triples, int count, cudaStream_t stream) {
   }
   if (list.count == 0) return RLT_OK;
   list.first_tile[list.count] = static_cast<int>(tiles);
+  list.prefetch = prefetches(list.segment[0].src, 2 * tiles * kShortTile);  // the ranges of one list come from one worker's memory
   RLT_CUDA_TRY(launch_following(inline_segments_kernel<kCount>, static_cast<unsigned>(tiles), kThreads, stream, list));
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return RLT_OK;
@@ -136,7 +163,8 @@ int rlt_kv_push(const void* src, void* dst, int64_t nbytes, rlt_stream_t stream)
   const long long tiles = (nbytes + rlt::kShortTile - 1) / rlt::kShortTile;
   if (tiles > 0x7fffffffll) return RLT_E_LIMIT;
   RLT_CUDA_TRY(rlt::launch_following(rlt::push_kernel, static_cast<unsigned>(tiles), rlt::kThreads, reinterpret_cast<cudaStream_t>(stream),
-                                     static_cast<const char*>(src), static_cast<char*>(dst), static_cast<long long>(nbytes)));
+                                     static_cast<const char*>(src), static_cast<char*>(dst), static_cast<long long>(nbytes),
+                                     static_cast<int>(rlt::prefetches(src, 2 * nbytes))));
   rlt::g_launches.fetch_add(1, std::memory_order_relaxed);
   return RLT_OK;
 }

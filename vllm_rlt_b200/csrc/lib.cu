@@ -21,6 +21,17 @@ int sm_count(int* out) {
   return RLT_OK;
 }
 
+bool prefetches(const void* src, long long bytes) {
+  if (bytes < kPrefetchBytes) return false;
+  cudaPointerAttributes of = {};
+  int device = -1;
+  if (cudaPointerGetAttributes(&of, src) != cudaSuccess || cudaGetDevice(&device) != cudaSuccess) {
+    cudaGetLastError();  // an address that nobody knows is no error here
+    return false;
+  }
+  return of.type == cudaMemoryTypeDevice && of.device == device;
+}
+
 }  // namespace rlt
 
 extern "C" {
