@@ -34,10 +34,18 @@ enum MoveKind {
   kExitToWire,     // pack, EXIT_ONLY
   kDedupToWire,    // pack, DEDUP
   kWireToPlane,    // scatter of an image with every plane
-  kDedupFromWire   // scatter of a dedup image: like kFanOut with the rows taken from the image
+  kDedupFromWire,  // scatter of a dedup image: like kFanOut with the rows taken from the image
+  // the same two with images whose rows are at odd places (load_image): kernels of their own, because the registers of that would cost the
+  // others 1 - 5 %
+  kDedupToOddWire,
+  kDedupFromOddWire
 };
 
-__host__ __device__ constexpr bool loops_planes(MoveKind k) { return k == kFanOut || k == kDedupFromWire; }
+__host__ __device__ constexpr bool by_token(MoveKind k) { return k == kExitToPlane || k == kExitToWire; }
+__host__ __device__ constexpr bool asks_ahead(MoveKind k) { return k == kPlaneToPlane || k == kPlaneToWire || k == kWireToPlane || by_token(k); }
+__host__ __device__ constexpr bool packs_dedup(MoveKind k) { return k == kDedupToWire || k == kDedupToOddWire; }
+__host__ __device__ constexpr bool scatters_dedup(MoveKind k) { return k == kDedupFromWire || k == kDedupFromOddWire; }
+__host__ __device__ constexpr bool loops_planes(MoveKind k) { return k == kFanOut || scatters_dedup(k); }
 
 struct MoveRegion {
   const char* src[2];  // K and V; the image for a scatter
@@ -45,7 +53,8 @@ struct MoveRegion {
   long long block_bytes;
   long long slice_at;  // byte offset of the layer slice inside a block
   int token_bytes;
-  int vec_bytes;       // 32, 16, 4 or 1
+  int vec_bytes;       // 32, 16, 4 or 1: what the pools' rows allow
+  int image_bytes;     // 16, 8 or 4: of one access to the image where the vectors have 16
   int row_vecs;
   unsigned row_magic;  // div_magic(row_vecs), 0 for one-vector rows
   int slice_vecs;      // vectors of the layer slice of one block
@@ -67,7 +76,6 @@ struct MoveParams {
   int words;         // int32 per record
   int blocks;
   int dst_at, exit_at;  // where a record's destination blocks and exit planes start
-  int prefetch;         // the source is asked for ahead of time
   const int* records;
   const int* wire;   // [blocks][planes]
   long long* wire_header;
@@ -119,17 +127,76 @@ struct PagePairs {
   unsigned short code[kMaxPlanes * kMaxBlockSize];
 };
 
-// Where vector `first + k` of a block's layer slice is: row (layer-major, token-minor), token, and vector inside the row.
-// k counts from the piece's first vector, whose row and offset are (row0, rem0): the multiplier split stays exact.
+// Where vector `k` behind the piece's first one is: row (layer-major, token-minor), token, and vector inside the row. The piece's rows are those of
+// `tokens` tokens from `t_lo` on, layer by layer: a whole block's, or only the ones in range. k counts from the piece's first vector, whose row and
+// offset are (row0, rem0): the multiplier split stays exact.
 struct RowAt {
   int layer, token, within;
 };
-__device__ __forceinline__ RowAt row_at(const MoveParams& p, const MoveRegion& rg, int row0, int rem0, int k) {
+__device__ __forceinline__ RowAt row_at(const MoveRegion& rg, int tokens, unsigned magic, int t_lo, int row0, int rem0, int k) {
   const unsigned j = static_cast<unsigned>(rem0 + k);
   const int q = rg.row_magic ? static_cast<int>(__umulhi(j, rg.row_magic)) : static_cast<int>(j);
   const int row = row0 + q;
-  const int layer = p.block_size == 1 ? row : static_cast<int>(__umulhi(static_cast<unsigned>(row), p.block_magic));
-  return {layer, row - layer * p.block_size, static_cast<int>(j) - q * rg.row_vecs};
+  const int layer = tokens == 1 ? row : static_cast<int>(__umulhi(static_cast<unsigned>(row), magic));
+  return {layer, t_lo + row - layer * tokens, static_cast<int>(j) - q * rg.row_vecs};
+}
+
+// A vector of the image; kSplit: in pieces of 8 or 4 bytes, because its rows follow one another whatever their size. (FP8 codes beside the scales
+// of an odd number of heads lie on 4-byte boundaries in the image and on 16-byte ones in the pool. Where a row is found by arithmetic, doing that for
+// 16 bytes and not for 4 halves the time: 15 prompts of 7 planes and 384-byte rows, dedup, packed in 309 us instead of 660 and scattered in 419
+// instead of 783; 56 prompts with every plane scattered in 470 instead of 708.)
+template <bool kSplit, typename T>
+__device__ __forceinline__ T load_image(const char* from, int bytes) {
+  if constexpr (!kSplit) {
+    return ld_stream(reinterpret_cast<const T*>(from));
+  } else {
+    static_assert(sizeof(T) == 16, "");
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(from);
+    if (bytes == 4) return T{w[0], w[1], w[2], w[3]};
+    const uint2 lo = *reinterpret_cast<const uint2*>(from), hi = *reinterpret_cast<const uint2*>(from + 8);
+    return T{lo.x, lo.y, hi.x, hi.y};
+  }
+}
+template <bool kSplit, typename T>
+__device__ __forceinline__ void store_image(char* to, const T& v, int bytes) {
+  if constexpr (!kSplit) {
+    st_stream(reinterpret_cast<T*>(to), v);
+  } else {
+    static_assert(sizeof(T) == 16, "");
+    uint32_t* w = reinterpret_cast<uint32_t*>(to);
+    if (bytes == 4) {
+      w[0] = v.x, w[1] = v.y, w[2] = v.z, w[3] = v.w;
+    } else {
+      *reinterpret_cast<uint2*>(to) = uint2{v.x, v.y};
+      *reinterpret_cast<uint2*>(to + 8) = uint2{v.z, v.w};
+    }
+  }
+}
+
+// `count` vectors of 16 bytes to a place in the image that is only a multiple of 4: the image's vectors are stored whole, and each is put together
+// from four words of the source, which lie in L1 by the second of them: 56 prompts with every plane packed in 454 us, 713 with 4-byte accesses on both
+// sides, 1,430 with the source's vectors stored in four parts each.
+__device__ __forceinline__ void copy_to_odd_place(const char* from, char* to, int count) {
+  const int skip = static_cast<int>(-reinterpret_cast<intptr_t>(to) & 15);
+  const int words = count * 4, head = skip / 4, body = (words - head) / 4, done = head + 4 * body;
+  const uint32_t* src = reinterpret_cast<const uint32_t*>(from);
+  constexpr int kU = 4;
+  for (int k0 = static_cast<int>(threadIdx.x); k0 < body; k0 += kThreads * kU) {
+    uint4 v[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const uint32_t* w = src + head + 4 * (k0 + u * kThreads);
+      if (k0 + u * kThreads < body) v[u] = uint4{w[0], w[1], w[2], w[3]};
+    }
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      if (k0 + u * kThreads < body) st_stream(reinterpret_cast<uint4*>(to + skip) + k0 + u * kThreads, v[u]);
+    }
+  }
+  const int i = static_cast<int>(threadIdx.x);
+  uint32_t* dst = reinterpret_cast<uint32_t*>(to);
+  if (i < head) dst[i] = src[i];
+  if (i < words - done) dst[done + i] = src[done + i];
 }
 
 __device__ __forceinline__ bool deep_carried(const MoveParams& p, int layer_rel) {
@@ -159,7 +226,7 @@ __device__ __forceinline__ long long wire_base(const MoveParams& p, const Piece&
 
 template <MoveKind K>
 __device__ __forceinline__ void fetch_page(const MoveParams& p, const MoveRegion& rg, const Piece& w, const int* wire, PageShared& s) {
-  constexpr bool kImage = K == kDedupToWire || K == kDedupFromWire;
+  constexpr bool kImage = packs_dedup(K) || scatters_dedup(K);
   const int tid = static_cast<int>(threadIdx.x);
   const int word = kRecordHeader + tid;
   if (word < p.words) {
@@ -196,9 +263,10 @@ __device__ __forceinline__ void fetch_page(const MoveParams& p, const MoveRegion
   }
 }
 
-template <typename T, MoveKind K>
+template <typename T, MoveKind K, bool kSplit>
 __device__ __forceinline__ void move_rows(const MoveParams& p, const MoveRegion& rg, const Piece& w, const PageShared& s) {
   constexpr int kU = flight_of<T>();
+  constexpr bool kFromImage = K == kWireToPlane, kToImage = K == kPlaneToWire || K == kExitToWire;
   const int first = w.index * rg.per;
   const int n_tok = w.t_hi - w.t_lo;
   const int sid = K == kWireToPlane || K == kExitToPlane || K == kExitToWire ? 0 : w.rec[kRecordHeader + w.plane];
@@ -233,27 +301,33 @@ __device__ __forceinline__ void move_rows(const MoveParams& p, const MoveRegion&
     const T* from = reinterpret_cast<const T*>(src) + first;
     T* to = reinterpret_cast<T*>(dst) + first;
     const int left = rg.slice_vecs - first;
+    if (kSplit && kToImage) {
+      if (left > 0) copy_to_odd_place(reinterpret_cast<const char*>(from), reinterpret_cast<char*>(to), min(left, rg.per));
+      return;
+    }
     for (int k0 = static_cast<int>(threadIdx.x); k0 < rg.per; k0 += kThreads * kU) {
 #pragma unroll
       for (int u = 0; u < kU; ++u) {
-        if (k0 + u * kThreads < left) regs[u] = ld_stream(from + k0 + u * kThreads);
+        if (k0 + u * kThreads < left) regs[u] = kFromImage ? load_image<kSplit, T>(reinterpret_cast<const char*>(from + k0 + u * kThreads), rg.image_bytes) : ld_stream(from + k0 + u * kThreads);
       }
 #pragma unroll
       for (int u = 0; u < kU; ++u) {
-        if (k0 + u * kThreads < left) st_stream(to + k0 + u * kThreads, regs[u]);
+        if (k0 + u * kThreads >= left) continue;
+        if (kToImage) store_image<kSplit>(reinterpret_cast<char*>(to + k0 + u * kThreads), regs[u], rg.image_bytes);
+        else st_stream(to + k0 + u * kThreads, regs[u]);
       }
     }
     return;
   }
   const int row0 = first / rg.row_vecs, rem0 = first - row0 * rg.row_vecs;
   for (int k0 = static_cast<int>(threadIdx.x); k0 < rg.per; k0 += kThreads * kU) {
-    T* to[kU];
+    char* to[kU];
 #pragma unroll
     for (int u = 0; u < kU; ++u) {
       const int k = k0 + u * kThreads;
       to[u] = nullptr;
       if (first + k >= rg.slice_vecs) continue;
-      const RowAt at = row_at(p, rg, row0, rem0, k);
+      const RowAt at = row_at(rg, p.block_size, p.block_magic, 0, row0, rem0, k);
       if (at.token < w.t_lo || at.token >= w.t_hi) continue;
       if (w.plane > 0 && !deep_carried(p, at.layer)) continue;
       const long long in_slice = static_cast<long long>(first + k) * static_cast<int>(sizeof(T));
@@ -277,12 +351,14 @@ __device__ __forceinline__ void move_rows(const MoveParams& p, const MoveRegion&
         if (block < 0) continue;
         from += block + rg.slice_at;
       }
-      to[u] = reinterpret_cast<T*>(dst + (K == kPlaneToWire || K == kExitToWire ? in_image : in_slice));
-      regs[u] = ld_stream(reinterpret_cast<const T*>(from));
+      to[u] = dst + (kToImage ? in_image : in_slice);
+      regs[u] = kFromImage ? load_image<kSplit, T>(from, rg.image_bytes) : ld_stream(reinterpret_cast<const T*>(from));
     }
 #pragma unroll
     for (int u = 0; u < kU; ++u) {
-      if (to[u] != nullptr) st_stream(to[u], regs[u]);
+      if (to[u] == nullptr) continue;
+      if (kToImage) store_image<kSplit>(to[u], regs[u], rg.image_bytes);
+      else st_stream(reinterpret_cast<T*>(to[u]), regs[u]);
     }
   }
 }
@@ -292,15 +368,20 @@ __device__ __forceinline__ void move_rows(const MoveParams& p, const MoveRegion&
 // first store.
 constexpr int kPlaneBatch = 4;
 
-template <typename T, MoveKind K>
+template <typename T, MoveKind K, bool kSplit>
 __device__ __forceinline__ void walk_planes(const MoveParams& p, const MoveRegion& rg, const Piece& w, const PageShared& s) {
   const int first = w.index * rg.per;
   const int row0 = first / rg.row_vecs, rem0 = first - row0 * rg.row_vecs;
   const int begin = p.plane_begin;
-  const int count = min(rg.per, rg.slice_vecs - first);
+  // A handoff goes through the rows in range only, a scatter through the block's: us of the one and the other, handoffs of 5 GB and two planes
+  // 854 / 872, of 480-byte rows 808 / 833, scatters of 5 GB and two planes 909 / 902, of a hundred pages 105 / 103.
+  constexpr bool kInRange = K == kFanOut;
+  const int tokens = kInRange ? w.t_hi - w.t_lo : p.block_size, t_lo = kInRange ? w.t_lo : 0;
+  const unsigned magic = !kInRange || tokens == p.block_size || tokens == 1 ? p.block_magic : 0xffffffffu / static_cast<unsigned>(tokens) + 1u;
+  const int count = min(rg.per, (kInRange ? p.slice_layers * tokens * rg.row_vecs : rg.slice_vecs) - first);
   for (int k = static_cast<int>(threadIdx.x); k < count; k += kThreads) {
-    const RowAt at = row_at(p, rg, row0, rem0, k);
-    if (at.token < w.t_lo || at.token >= w.t_hi) continue;
+    const RowAt at = row_at(rg, tokens, magic, t_lo, row0, rem0, k);
+    if (!kInRange && (at.token < w.t_lo || at.token >= w.t_hi)) continue;
     const int e = s.exit_plane[at.token];
     if (e < 0 || e >= p.src_planes) {
       report(p.status, RLT_STATUS_BAD_PLANE, w.request(), w.logical() * p.block_size + at.token, e);
@@ -308,7 +389,8 @@ __device__ __forceinline__ void walk_planes(const MoveParams& p, const MoveRegio
     }
     const char* src = rg.src[w.kv];
     char* dst = rg.dst[w.kv];
-    const long long in_slice = rg.slice_at + static_cast<long long>(first + k) * static_cast<int>(sizeof(T));
+    const int vec = kInRange ? (at.layer * p.block_size + at.token) * rg.row_vecs + at.within : first + k;
+    const long long in_slice = rg.slice_at + static_cast<long long>(vec) * static_cast<int>(sizeof(T));
     const int end = p.plane_end > 1 && !deep_carried(p, at.layer) ? 1 : p.plane_end;  // planes this row reaches
     if (begin >= end) continue;
     // source rows are those of planes [begin, begin + loads): plane p <- min(p, e)
@@ -334,7 +416,7 @@ __device__ __forceinline__ void walk_planes(const MoveParams& p, const MoveRegio
         ok[j] = j0 + j < loads;
         if (!ok[j]) continue;
         long long from;
-        if (K == kDedupFromWire) {
+        if (scatters_dedup(K)) {
           from = image_at(plane);
           ok[j] = from >= 0;
         } else {
@@ -343,7 +425,7 @@ __device__ __forceinline__ void walk_planes(const MoveParams& p, const MoveRegio
           ok[j] = from >= 0;
           from += in_slice;
         }
-        if (ok[j]) regs[j] = ld_stream(reinterpret_cast<const T*>(src + from));
+        if (ok[j]) regs[j] = scatters_dedup(K) ? load_image<kSplit, T>(src + from, rg.image_bytes) : ld_stream(reinterpret_cast<const T*>(src + from));
       }
 #pragma unroll
       for (int j = 0; j < kPlaneBatch; ++j) {
@@ -392,7 +474,7 @@ __device__ __forceinline__ int list_pairs(const MoveParams& p, const Piece& w, c
 
 // Dedup pack. What a page contributes differs from page to page, so its vectors - (layer, pair, vector of the row) - are
 // dealt to the page's CTAs in equal shares: every thread has something to copy, whatever the exit planes.
-template <typename T>
+template <typename T, bool kSplit>
 __device__ __forceinline__ void pack_pairs(const MoveParams& p, const MoveRegion& rg, const Piece& w, const PageShared& s,
                                            PagePairs& pairs) {
   constexpr int kU = flight_of<T>();
@@ -412,7 +494,7 @@ __device__ __forceinline__ void pack_pairs(const MoveParams& p, const MoveRegion
   char* dst = rg.dst[w.kv];
   for (int k0 = static_cast<int>(threadIdx.x); k0 < count; k0 += kThreads * kU) {
     T regs[kU];
-    T* to[kU];
+    char* to[kU];
 #pragma unroll
     for (int u = 0; u < kU; ++u) {
       const int k = k0 + u * kThreads;
@@ -435,11 +517,11 @@ __device__ __forceinline__ void pack_pairs(const MoveParams& p, const MoveRegion
       if (block < 0) continue;
       const int within = (static_cast<int>(j) - q * rg.row_vecs) * static_cast<int>(sizeof(T));
       regs[u] = ld_stream(reinterpret_cast<const T*>(src + block + (static_cast<long long>(layer) * p.block_size + token) * rg.token_bytes + within));
-      to[u] = reinterpret_cast<T*>(dst + image + within);
+      to[u] = dst + image + within;
     }
 #pragma unroll
     for (int u = 0; u < kU; ++u) {
-      if (to[u] != nullptr) st_stream(to[u], regs[u]);
+      if (to[u] != nullptr) store_image<kSplit>(to[u], regs[u], rg.image_bytes);
     }
   }
 }
@@ -477,7 +559,7 @@ __device__ __forceinline__ void prefetch_piece(const MoveParams& p, const Piece&
     if (K == kWireToPlane) {
       const long long before = static_cast<long long>(w.rec[4]) * p.dst_planes + static_cast<long long>(w.plane) * w.rec[5] + w.rec[3];
       const long long image = wire_base(p, w, rg, before, p.block_size);
-      if (image + static_cast<long long>(rg.slice_vecs) * rg.vec_bytes > p.packed_bytes) return;
+      if (rg.image_bytes < 16 || image + static_cast<long long>(rg.slice_vecs) * rg.vec_bytes > p.packed_bytes) return;
       src += image;
     } else {
       const int id = w.rec[kRecordHeader + w.plane];
@@ -499,18 +581,19 @@ __device__ __forceinline__ void prefetch_piece(const MoveParams& p, const Piece&
   }
 }
 
-template <typename T, MoveKind K>
+template <typename T, MoveKind K, bool kSplit = false>
 __device__ __forceinline__ void move_piece(const MoveParams& p, const MoveRegion& rg, const Piece& w, const PageShared& s, PagePairs& pairs) {
-  if constexpr (K == kDedupToWire) {
-    pack_pairs<T>(p, rg, w, s, pairs);
+  if constexpr (packs_dedup(K)) {
+    pack_pairs<T, kSplit>(p, rg, w, s, pairs);
   } else if constexpr (loops_planes(K)) {
-    walk_planes<T, K>(p, rg, w, s);
+    walk_planes<T, K, kSplit>(p, rg, w, s);
   } else {
-    move_rows<T, K>(p, rg, w, s);
+    move_rows<T, K, kSplit>(p, rg, w, s);
   }
 }
 
-template <MoveKind K, int kWords>
+// kAsk: the source is asked for ahead of time.
+template <MoveKind K, int kWords, bool kAsk>
 __global__ void __launch_bounds__(kThreads, loops_planes(K) ? 3 : 6) move_kernel(const __grid_constant__ MoveArgs<kWords> args) {
   const MoveParams& p = args.p;
   const int* records = kWords > 1 ? args.inline_words : p.records;
@@ -520,18 +603,15 @@ __global__ void __launch_bounds__(kThreads, loops_planes(K) ? 3 : 6) move_kernel
   // Records that are parameters may be read before the kernel ahead has ended, and tell where the source is. (Records in device memory would have
   // to be waited for first; asking for pieces further on then costs more than it gives: 29k tokens exit-only 1,758 -> 1,786 us.) Against
   // none: a layer slice of 42 MB 9.1 -> 8.2 us, of 0.2 GB 31.2 -> 29.7; 1,000 tokens exit-only 62.0 -> 60.3 and all planes 234 -> 230.
-  constexpr bool kPlain = K == kPlaneToPlane || K == kPlaneToWire || K == kWireToPlane;
-  if constexpr (kWords > 1 && (kPlain || K == kExitToPlane || K == kExitToWire)) {
-    if (p.prefetch) {
-      if (threadIdx.x < 32) prefetch_piece<K>(p, w);
-      // (for the rows that exit planes choose, one prefetch each, the pieces ahead are not worth their cost: 60.3 -> 60.5)
-      if (kPlain && threadIdx.x / 32 == 1 && gridDim.x - blockIdx.x > kPrefetchAhead)
-        prefetch_piece<K>(p, piece_at(p, records, blockIdx.x + kPrefetchAhead));
-    }
+  if constexpr (kAsk) {
+    if (threadIdx.x < 32) prefetch_piece<K>(p, w);
+    // (for the rows that exit planes choose, one prefetch each, the pieces ahead are not worth their cost: 60.3 -> 60.5)
+    if (!by_token(K) && threadIdx.x / 32 == 1 && gridDim.x - blockIdx.x > kPrefetchAhead)
+      prefetch_piece<K>(p, piece_at(p, records, blockIdx.x + kPrefetchAhead));
   }
   follow_stream();
   const int range = w.rec[2];
-  if ((K == kDedupToWire || K == kDedupFromWire) && blockIdx.x == 0 && threadIdx.x == 0) {
+  if ((packs_dedup(K) || scatters_dedup(K)) && blockIdx.x == 0 && threadIdx.x == 0) {
     p.wire_header[0] = p.wire_tokens;
     p.wire_header[1] = static_cast<long long>(p.blocks) * p.src_planes;
   }
@@ -543,11 +623,14 @@ __global__ void __launch_bounds__(kThreads, loops_planes(K) ? 3 : 6) move_kernel
   w.t_hi = range >> 8;
   __shared__ PageShared shared;  // not allocated where nothing touches it
   __shared__ PagePairs pairs;
-  if constexpr (loops_planes(K) || K == kExitToPlane || K == kExitToWire || K == kDedupToWire)
+  if constexpr (loops_planes(K) || K == kExitToPlane || K == kExitToWire || packs_dedup(K))
     fetch_page<K>(p, rg, w, wire + (w.rec - records) / p.words * p.src_planes, shared);
   if (rg.vec_bytes == 32) {
     move_piece<Vec32, K>(p, rg, w, shared, pairs);
   } else if (rg.vec_bytes == 16) {
+    if constexpr (K == kPlaneToWire || K == kExitToWire || K == kWireToPlane || K == kDedupToOddWire || K == kDedupFromOddWire) {
+      if (rg.image_bytes < 16) return move_piece<uint4, K, true>(p, rg, w, shared, pairs);
+    }
     move_piece<uint4, K>(p, rg, w, shared, pairs);
   } else if (rg.vec_bytes == 4) {
     move_piece<uint32_t, K>(p, rg, w, shared, pairs);
@@ -557,7 +640,7 @@ __global__ void __launch_bounds__(kThreads, loops_planes(K) ? 3 : 6) move_kernel
 }
 
 template <MoveKind K, int kWords>
-cudaError_t launch_move(const MoveParams& p, const RltBlockMoves& m, unsigned grid, cudaStream_t stream) {
+cudaError_t launch_move(const MoveParams& p, const RltBlockMoves& m, unsigned grid, bool ask, cudaStream_t stream) {
   MoveArgs<kWords> args;
   args.p = p;
   if (kWords > 1) {
@@ -566,24 +649,27 @@ cudaError_t launch_move(const MoveParams& p, const RltBlockMoves& m, unsigned gr
     if (m.host_wire != nullptr)
       std::memcpy(args.inline_words + n, m.host_wire, static_cast<size_t>(m.blocks) * p.src_planes * sizeof(int));
   }
-  return launch_following(move_kernel<K, kWords>, grid, kThreads, stream, args);
+  if constexpr (kWords > 1 && asks_ahead(K)) {
+    if (ask) return launch_following(move_kernel<K, kWords, true>, grid, kThreads, stream, args);
+  }
+  return launch_following(move_kernel<K, kWords, false>, grid, kThreads, stream, args);
 }
 
 template <MoveKind K>
-int launch_kind(const MoveParams& p, const RltBlockMoves& m, unsigned grid, cudaStream_t stream) {
+int launch_kind(const MoveParams& p, const RltBlockMoves& m, unsigned grid, bool ask, cudaStream_t stream) {
   const long long n = static_cast<long long>(m.blocks) * m.words + (m.host_wire ? static_cast<long long>(m.blocks) * p.src_planes : 0);
   // A parameter block is copied into the launch whole (a launch takes the host 2.4 us with 2 KiB, 3.6 with 8 and 6.6 with 32; a
   // copy of the records, the launch and an event 4.5, and the GPU 6 us more), so three sizes of it: the small one covers a few
   // hundred tokens, the medium one a thousand.
   cudaError_t launched;
   if (n <= kInlineSmallWords) {
-    launched = launch_move<K, kInlineSmallWords>(p, m, grid, stream);
+    launched = launch_move<K, kInlineSmallWords>(p, m, grid, ask, stream);
   } else if (n <= kInlineMediumWords) {
-    launched = launch_move<K, kInlineMediumWords>(p, m, grid, stream);
+    launched = launch_move<K, kInlineMediumWords>(p, m, grid, ask, stream);
   } else if (n <= kInlineWords) {
-    launched = launch_move<K, kInlineWords>(p, m, grid, stream);
+    launched = launch_move<K, kInlineWords>(p, m, grid, ask, stream);
   } else if (p.records != nullptr && (m.host_wire == nullptr || p.wire != nullptr)) {
-    launched = launch_move<K, 1>(p, m, grid, stream);
+    launched = launch_move<K, 1>(p, m, grid, ask, stream);
   } else {
     return RLT_E_INVALID;
   }
@@ -638,10 +724,10 @@ extern "C" int rlt_move_blocks(int direction, const RltPool* src, const RltPool*
   if (t.dedup_wire && m->host_wire == nullptr) return RLT_MOVE_UNSUITED;
   if (m->blocks == 0) return RLT_OK;
 
-  const MoveKind kind = dir == kDirect ? (dedup ? kFanOut : opt->mode == RLT_MODE_EXIT_ONLY ? kExitToPlane : kPlaneToPlane)
+  MoveKind kind = dir == kDirect ? (dedup ? kFanOut : opt->mode == RLT_MODE_EXIT_ONLY ? kExitToPlane : kPlaneToPlane)
                         : dir == kPack ? (dedup ? kDedupToWire : opt->mode == RLT_MODE_EXIT_ONLY ? kExitToWire : kPlaneToWire)
                                        : (dedup ? kDedupFromWire : kWireToPlane);
-  const bool planes = loops_planes(kind), pairs = kind == kDedupToWire;
+  const bool planes = loops_planes(kind), pairs = packs_dedup(kind);
   MoveParams p = {};
   p.slice_layers = t.layer_end - t.layer_begin;
   for (int g = 0; g < t.num_regions; ++g) {
@@ -654,7 +740,14 @@ extern "C" int rlt_move_blocks(int direction, const RltPool* src, const RltPool*
     rg.block_bytes = s.block_bytes;
     rg.slice_at = s.layer_bytes * t.layer_begin;
     rg.token_bytes = static_cast<int>(s.token_bytes);
-    rg.vec_bytes = s.wide_ok ? 32 : s.vec_bytes;
+    // of the pool's side; the image's rows lie on multiples of the largest power of two that divides all sizes in it
+    const uintptr_t rows_at = static_cast<uintptr_t>(s.token_bytes) | (dir == kScatter ? 0 : reinterpret_cast<uintptr_t>(s.src_key) | reinterpret_cast<uintptr_t>(s.src_value)) |
+                              (dir == kPack ? 0 : reinterpret_cast<uintptr_t>(s.dst_key) | reinterpret_cast<uintptr_t>(s.dst_value));
+    uintptr_t image_at = dir == kDirect ? 0 : reinterpret_cast<uintptr_t>(packed);
+    for (int h = 0; dir != kDirect && h < t.num_regions; ++h) image_at |= static_cast<uintptr_t>(t.region[h].token_bytes);
+    rg.image_bytes = image_at & 4u ? 4 : image_at & 8u ? 8 : 16;
+    rg.vec_bytes = (rows_at | image_at) & 3u ? 1 : ((rows_at | image_at) & 31u) == 0 ? 32 : (rows_at & 15u) == 0 ? 16 : 4;
+    if (rg.vec_bytes == 16 && rg.image_bytes < 16 && t.dedup_wire) kind = dir == kPack ? kDedupToOddWire : kDedupFromOddWire;
     const long long row_vecs = s.token_bytes / rg.vec_bytes;
     const long long slice_vecs = row_vecs * t.block_size * p.slice_layers;
     // the multiplier splits of row_at: (row_vecs + piece) * row_vecs and rows * block_size below 2^32
@@ -692,48 +785,68 @@ extern "C" int rlt_move_blocks(int direction, const RltPool* src, const RltPool*
   p.status = opt->status;
   // Rounds of a piece. Where a plane's block is all a CTA looks up, one: the smaller the piece the closer the SMs stay
   // together. Kinds that fetch the page's record and work out exit planes first need more payload behind that: measured
-  // best at 2 for exit-only (29k tokens: 1.84 -> 1.75 ms), at 8 for a dedup pack (1.86 -> 0.95 ms). Where planes are walked, the
+  // best at 2 for exit-only (29k tokens: 1.84 -> 1.75 ms), at 5 for a dedup pack (see below). Where planes are walked, the
   // more planes a round stores to the fewer rounds are needed, 12 / planes and at most 4. Dedup handoffs of 6 - 8.6 GB, us at
   // 1 / 2 / 3 / 4 / 8 rounds: two planes 1,267 / 1,105 / 1,054 / 1,026 / 991 (so 8 would be 4 % faster there), three 1,199 /
   // 1,093 / 1,053 / 1,036 / 1,039, four 1,295 / 1,234 / 1,226 / 1,227 / 1,240, six 1,289 / 1,270 / 1,267 / 1,270 / 1,281, eight
   // 1,185 / 1,190 / 1,191 / 1,196 / 1,205, sixteen 1,282 / 1,295 / 1,298 / 1,307 / 1,321, 32 1,086 / 1,098 / 1,105 / 1,114 /
   // 1,114; scatters of dedup images within 1 % of the same. A launch of fewer than eight waves takes the smallest piece that a
-  // larger one would split into: it is short of CTAs, not of payload per CTA.
+  // larger one would split into: it is short of CTAs, not of payload per CTA. A dedup pack, whose CTAs first list a page's pairs, stays with two
+  // rounds as long as those fill the GPU twice: 30 requests of 4 - 34 tokens 31.2 -> 29.1 us, 9 of 17 - 34 42.2 -> 31.1 (59 and 68 where the
+  // shares were made as if every page were full and every token on every plane).
   int sms = 0;
   const int found = sm_count(&sms);
   if (found != RLT_OK) return found;
-  const bool by_exit = kind == kExitToPlane || kind == kExitToWire;
-  int rounds = pairs ? 8 : planes ? std::max(1, std::min(4, 12 / p.dst_planes)) : by_exit ? 2 : 1;
+  int rounds = pairs ? 5 : planes ? std::max(1, std::min(4, 12 / p.dst_planes)) : by_token(kind) ? 2 : 1;
   long long grid = 0;
   for (;; rounds /= 2) {
     p.pieces = 0;
     for (int g = 0; g < t.num_regions; ++g) {
       MoveRegion& rg = p.region[g];
       rg.per = vectors_per_round(rg.vec_bytes, planes) * rounds;
-      const long long most = static_cast<long long>(rg.slice_vecs) * (pairs ? p.src_planes : 1);
+      const long long most = rg.slice_vecs;
       rg.pieces = static_cast<int>((most + rg.per - 1) / rg.per);
+      if (pairs) {
+        // What the pages contribute is known: their average is dealt out, in shares that end where layers do as far as possible (five prompts of
+        // four planes: 957 us in halves of a layer, 975 in 47 shares of 24 layers). No share of a full page may have more vectors than the
+        // multiplier split allows.
+        const long long layer = rg.row_vecs * ((m->wire_tokens + m->blocks - 1) / m->blocks), share = rg.per;
+        const long long count = layer >= share ? p.slice_layers * ((layer + share / 2) / share)
+                                               : std::max(1ll, p.slice_layers * layer / std::max(1ll, share / std::max(1ll, layer) * layer));
+        rg.pieces = static_cast<int>(std::max(count, (static_cast<long long>(rg.slice_vecs) * p.src_planes + 65535) / 65536));
+      }
       p.pieces += 2 * rg.pieces;
     }
     grid = static_cast<long long>(m->blocks) * p.grid_planes * p.pieces;
-    if (rounds == 1 || grid >= 8ll * sms * (planes ? 3 : 6)) break;
+    const long long waves = !pairs ? 8 : rounds == 2 ? 2 : 6;
+    if (rounds == 1 || grid >= waves * sms * (planes ? 3 : 6)) break;
   }
   if (grid > 0x7fffffffll) return RLT_MOVE_UNSUITED;
   long long bytes = 0;
   for (int g = 0; g < t.num_regions; ++g) bytes += 4ll * m->blocks * p.grid_planes * p.region[g].slice_vecs * p.region[g].vec_bytes;
-  p.prefetch = prefetches(p.region[0].src[0], bytes);
+  if (bytes >= kPrefetchBytes && asks_ahead(kind) && !by_token(kind)) {
+    // Only pages that are wholly in range are asked for where all rows of one come from one place. With few of those the asking costs more than it
+    // gives (51 prompts of 19 - 38 tokens in 64-token pages: 179 us without, 191 with it).
+    int whole = 0;
+    for (int b = 0; b < m->blocks; ++b) whole += m->host_records[static_cast<size_t>(b) * m->words + 2] == t.block_size << 8;
+    if (2 * whole < m->blocks) bytes = 0;
+  }
+  const bool ask = asks_ahead(kind) && prefetches(p.region[0].src[0], bytes);
 
   const cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   const unsigned ctas = static_cast<unsigned>(grid);
   int rc = RLT_E_INVALID;
   switch (kind) {
-    case kPlaneToPlane: rc = launch_kind<kPlaneToPlane>(p, *m, ctas, s); break;
-    case kExitToPlane: rc = launch_kind<kExitToPlane>(p, *m, ctas, s); break;
-    case kFanOut: rc = launch_kind<kFanOut>(p, *m, ctas, s); break;
-    case kPlaneToWire: rc = launch_kind<kPlaneToWire>(p, *m, ctas, s); break;
-    case kExitToWire: rc = launch_kind<kExitToWire>(p, *m, ctas, s); break;
-    case kDedupToWire: rc = launch_kind<kDedupToWire>(p, *m, ctas, s); break;
-    case kWireToPlane: rc = launch_kind<kWireToPlane>(p, *m, ctas, s); break;
-    case kDedupFromWire: rc = launch_kind<kDedupFromWire>(p, *m, ctas, s); break;
+    case kPlaneToPlane: rc = launch_kind<kPlaneToPlane>(p, *m, ctas, ask, s); break;
+    case kExitToPlane: rc = launch_kind<kExitToPlane>(p, *m, ctas, ask, s); break;
+    case kFanOut: rc = launch_kind<kFanOut>(p, *m, ctas, ask, s); break;
+    case kPlaneToWire: rc = launch_kind<kPlaneToWire>(p, *m, ctas, ask, s); break;
+    case kExitToWire: rc = launch_kind<kExitToWire>(p, *m, ctas, ask, s); break;
+    case kDedupToWire: rc = launch_kind<kDedupToWire>(p, *m, ctas, ask, s); break;
+    case kWireToPlane: rc = launch_kind<kWireToPlane>(p, *m, ctas, ask, s); break;
+    case kDedupFromWire: rc = launch_kind<kDedupFromWire>(p, *m, ctas, ask, s); break;
+    case kDedupToOddWire: rc = launch_kind<kDedupToOddWire>(p, *m, ctas, ask, s); break;
+    case kDedupFromOddWire: rc = launch_kind<kDedupFromOddWire>(p, *m, ctas, ask, s); break;
   }
   if (rc != RLT_OK) return rc;
   g_launches.fetch_add(1, std::memory_order_relaxed);
@@ -742,9 +855,12 @@ extern "C" int rlt_move_blocks(int direction, const RltPool* src, const RltPool*
 
 extern "C" int rlt_load_moves(void) {
   using namespace rlt;
-  RLT_CUDA_TRY(load_kernel(move_kernel<kPlaneToPlane, kInlineSmallWords>));
-  RLT_CUDA_TRY(load_kernel(move_kernel<kPlaneToPlane, kInlineMediumWords>));
-  RLT_CUDA_TRY(load_kernel(move_kernel<kPlaneToPlane, kInlineWords>));
-  RLT_CUDA_TRY(load_kernel(move_kernel<kPlaneToPlane, 1>));
+  RLT_CUDA_TRY(load_kernel(move_kernel<kPlaneToPlane, kInlineSmallWords, true>));
+  RLT_CUDA_TRY(load_kernel(move_kernel<kPlaneToPlane, kInlineSmallWords, false>));
+  RLT_CUDA_TRY(load_kernel(move_kernel<kPlaneToPlane, kInlineMediumWords, true>));
+  RLT_CUDA_TRY(load_kernel(move_kernel<kPlaneToPlane, kInlineMediumWords, false>));
+  RLT_CUDA_TRY(load_kernel(move_kernel<kPlaneToPlane, kInlineWords, true>));
+  RLT_CUDA_TRY(load_kernel(move_kernel<kPlaneToPlane, kInlineWords, false>));
+  RLT_CUDA_TRY(load_kernel(move_kernel<kPlaneToPlane, 1, false>));
   return RLT_OK;
 }
