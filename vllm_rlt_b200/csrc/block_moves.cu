@@ -658,8 +658,8 @@ cudaError_t launch_move(const MoveParams& p, const RltBlockMoves& m, unsigned gr
 template <MoveKind K>
 int launch_kind(const MoveParams& p, const RltBlockMoves& m, unsigned grid, bool ask, cudaStream_t stream) {
   const long long n = static_cast<long long>(m.blocks) * m.words + (m.host_wire ? static_cast<long long>(m.blocks) * p.src_planes : 0);
-  // A parameter block is copied into the launch whole (a launch takes the host 2.4 us with 2 KiB, 3.6 with 8 and 6.6 with 32; a
-  // copy of the records, the launch and an event 4.5, and the GPU 6 us more), so three sizes of it: the small one covers a few
+  // A parameter block is copied into the launch whole (a launch takes the host 1.85 us with 0.1 - 7 KiB, 2.2 with 16 and 3.1 with 31; a
+  // copy of the records, the launch and an event 4.5, and the GPU 9 - 16 us more), so three sizes of it: the small one covers a few
   // hundred tokens, the medium one a thousand.
   cudaError_t launched;
   if (n <= kInlineSmallWords) {

@@ -11,7 +11,8 @@
 // Where the host knows the sizes (push, and ranges that come from the host, whose triples are kernel parameters) the grid
 // holds one CTA per 16 KiB tile, in order: the hardware then keeps all SMs within a few MB of each other, which DRAM
 // rewards (block_moves.cu has the measurements). 0.4 GB read and written in 256 ranges of 1.5 MiB: 136 us with the persistent kernel
-// below, 120 here; a push of 1 GiB 343 -> 312 us (6.9 TB/s).
+// below, 120 here; a push of 1 GiB 343 -> 312 us (6.9 TB/s). Asking for the source ahead of time (prefetch_l2): 170 ranges of 1.5 MiB one
+// launch behind another 81.6 -> 78.0 us, a push of 64 MiB 18.1 -> 17.5.
 //
 // A list in device memory has sizes the host cannot see: a persistent grid strides over tiles of 32 KiB, every CTA computes the
 // exclusive scan of the per-range tile counts with warp-shuffle prefix sums in shared memory and finds a tile's range by
