@@ -46,6 +46,9 @@ int sm_count(int* out);
 // kernel calls follow_stream() before it touches any memory but its parameters: that returns when everything before it on the
 // stream has completed and is visible, and then lets the next such launch be set up behind this one. Saves most of the gap
 // between two short kernels; kernels launched the ordinary way, copies and events are ordered as ever.
+// What such a kernel reads may still be written by the one before it while it is being set up, so none of its pointers is __restrict__: that
+// would promise the compiler memory that nobody writes for as long as the kernel runs, and let it read ahead of the wait or through a cache
+// that is not coherent.
 template <typename T>
 struct Given {  // the type of the parameter, whatever is given for it
   using type = T;
@@ -132,7 +135,7 @@ __device__ __forceinline__ void st_stream(uint8_t* p, uint8_t v) { *p = v; }
 
 // A CTA copies elements [0, n).
 template <typename T, int kUnroll = 4>
-__device__ __forceinline__ void stream_range(const char* __restrict__ src, char* __restrict__ dst, long long n) {
+__device__ __forceinline__ void stream_range(const char* src, char* dst, long long n) {
   const T* s = reinterpret_cast<const T*>(src);
   T* d = reinterpret_cast<T*>(dst);
   for (long long base = threadIdx.x; base < n; base += kThreads * kUnroll) {

@@ -79,7 +79,7 @@ constexpr int kRows = 4;
 constexpr int kTile = 256;
 
 template <typename S, typename D>
-__global__ void __launch_bounds__(kTile) segmented_transfer_kernel(const long long* __restrict__ descriptors) {
+__global__ void __launch_bounds__(kTile) segmented_transfer_kernel(const long long* descriptors) {
   follow_stream();
   const long long* d = descriptors + 8ll * blockIdx.x;
   const S* src = reinterpret_cast<const S*>(d[0]);
@@ -162,7 +162,9 @@ int launch_inline(const int64_t* descriptors, int count, int max_rows, int max_c
 // 128 Mi elements int64 -> int32 253 -> 233 us (6.9 TB/s), float16 -> int32 143 -> 121, bfloat16 -> float16 and int64 303 -> 242;
 // int32 -> int32 views that start one element past an aligned one 233 -> 159.
 constexpr int kFlatGroups = 2;
-constexpr int kFlatSingles = 8;  // elements per thread where nothing is aligned
+// Elements per thread where nothing is aligned, all loaded before any is stored (64 Mi elements into views that start elsewhere than the source's,
+// us, one by one -> so: int32 -> int32 142 -> 78, float16 -> int32 142 -> 72, bfloat16 -> float32 139 -> 68).
+constexpr int kFlatSingles = 8;
 
 template <int kBytes>
 struct Bits;
@@ -210,16 +212,14 @@ constexpr int flat_width() {
 }
 
 template <typename S, typename D, typename E>
-__device__ __forceinline__ void one_element(const S* __restrict__ src, D* __restrict__ dst, E* __restrict__ secondary, long long i) {
-  const S v = src[i];
+__device__ __forceinline__ void put_element(S v, D* dst, E* secondary, long long i) {
   dst[i] = Convert<D, S>::run(v);
   if (secondary != nullptr) secondary[i] = Convert<E, S>::run(v);
 }
 
 // head: elements before the first aligned one, -1 if there is no such place.
 template <typename S, typename D, typename E>
-__global__ void __launch_bounds__(kTile) flat_transfer_kernel(const S* __restrict__ src, D* __restrict__ dst,
-                                                              E* __restrict__ secondary, long long n, int head, int prefetch) {
+__global__ void __launch_bounds__(kTile) flat_transfer_kernel(const S* src, D* dst, E* secondary, long long n, int head, int prefetch) {
   constexpr int N = 32 / (sizeof(S) > sizeof(D) ? (sizeof(S) > sizeof(E) ? sizeof(S) : sizeof(E))
                                                 : (sizeof(D) > sizeof(E) ? sizeof(D) : sizeof(E)));
   if (prefetch && threadIdx.x == 0) {  // (further on as well: a loss where more is read than written, 172 -> 215 us for 1.2 GB int64 -> int32)
@@ -231,9 +231,14 @@ __global__ void __launch_bounds__(kTile) flat_transfer_kernel(const S* __restric
   follow_stream();
   if (head < 0) {
     const long long first = static_cast<long long>(blockIdx.x) * (kTile * kFlatSingles) + threadIdx.x;
+    S in[kFlatSingles];
 #pragma unroll
     for (int k = 0; k < kFlatSingles; ++k) {
-      if (first + k * kTile < n) one_element(src, dst, secondary, first + k * kTile);
+      if (first + k * kTile < n) in[k] = src[first + k * kTile];
+    }
+#pragma unroll
+    for (int k = 0; k < kFlatSingles; ++k) {
+      if (first + k * kTile < n) put_element(in[k], dst, secondary, first + k * kTile);
     }
     return;
   }
@@ -262,7 +267,7 @@ __global__ void __launch_bounds__(kTile) flat_transfer_kernel(const S* __restric
   if (blockIdx.x == 0) {  // both ends: fewer than 2 N elements
     const long long tail = head + groups * N;
     const long long i = threadIdx.x < head ? threadIdx.x : tail + (threadIdx.x - head);
-    if (i < n && (i < head || i >= tail)) one_element(src, dst, secondary, i);
+    if (i < n && (i < head || i >= tail)) put_element(src[i], dst, secondary, i);
   }
 }
 
