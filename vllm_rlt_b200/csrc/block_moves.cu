@@ -650,7 +650,7 @@ cudaError_t launch_move(const MoveParams& p, const RltBlockMoves& m, unsigned gr
       std::memcpy(args.inline_words + n, m.host_wire, static_cast<size_t>(m.blocks) * p.src_planes * sizeof(int));
   }
   if constexpr (kWords > 1 && asks_ahead(K)) {
-    if (ask) return launch_following(move_kernel<K, kWords, true>, grid, kThreads, stream, args);
+    if (asking(ask)) return launch_following(move_kernel<K, kWords, true>, grid, kThreads, stream, args);
   }
   return launch_following(move_kernel<K, kWords, false>, grid, kThreads, stream, args);
 }

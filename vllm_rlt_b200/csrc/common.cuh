@@ -98,6 +98,27 @@ constexpr long long kPrefetchBytes = 32 << 20;
 // Whether a launch that moves so many bytes asks for its source, which has to be in memory of the current device (0.07 us to find out).
 bool prefetches(const void* src, long long bytes);
 
+// Which addresses are in memory of the current device. An allocation is looked up once, and a few at most: where ranges lie in more of them than
+// a worker's pools have tensors, the answer is no.
+class OwnMemory {
+ public:
+  bool holds(const void* from, long long bytes);
+
+ private:
+  static constexpr int kLookups = 8;
+  struct {
+    uintptr_t begin, end;
+  } known_[kLookups];
+  int count_ = 0, last_ = 0;
+};
+
+// Counts the launches that ask, for the tests.
+extern std::atomic<long long> g_asking, g_lookups;
+inline bool asking(bool yes) {
+  if (yes) g_asking.fetch_add(1, std::memory_order_relaxed);
+  return yes;
+}
+
 // First error wins: later reports leave the status words alone.
 __device__ __forceinline__ void report(int32_t* status, int code, int a, int b, int c) {
   if (status == nullptr) return;

@@ -22,6 +22,9 @@ RLT_API int rlt_capture_id(rlt_stream_t stream, uint64_t* id);  // of the captur
 RLT_API int rlt_tensor_transfer_inline(const int64_t* descriptors, int32_t count, int32_t max_rows, int32_t max_cols,
                                        int32_t dtype, rlt_stream_t stream);
 
+// How many launches of this process have asked L2 for their source ahead of time, and how many addresses were looked up for that.
+RLT_API void rlt_prefetch_counts(int64_t counts[2]);
+
 // rlt_kv_post behind copies of a few small byte ranges, (source, destination, bytes) in HOST memory, in one launch.
 #define RLT_POST_RANGES 4
 #define RLT_POST_RANGE_BYTES 32768  // of all of them

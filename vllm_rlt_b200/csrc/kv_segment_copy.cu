@@ -94,18 +94,23 @@ __global__ void __launch_bounds__(kThreads, 6) inline_segments_kernel(const __gr
 template <int kCount>
 int launch_inline(const int64_t* triples, int count, cudaStream_t stream) {
   InlineSegments<kCount> list;
-  long long tiles = 0;
+  long long tiles = 0, bytes = 0;
   list.count = 0;
   for (int i = 0; i < count; ++i) {
     if (triples[3 * i + 2] <= 0) continue;
     list.first_tile[list.count] = static_cast<int>(tiles);
     list.segment[list.count++] = {reinterpret_cast<const char*>(triples[3 * i]), reinterpret_cast<char*>(triples[3 * i + 1]), triples[3 * i + 2]};
     tiles += (triples[3 * i + 2] + kShortTile - 1) / kShortTile;
+    bytes += triples[3 * i + 2];
     if (tiles > 0x7fffffffll) return RLT_E_LIMIT;
   }
   if (list.count == 0) return RLT_OK;
   list.first_tile[list.count] = static_cast<int>(tiles);
-  list.prefetch = prefetches(list.segment[0].src, 2 * tiles * kShortTile);  // the ranges of one list come from one worker's memory
+  // Every range has to be in this GPU's memory: a list may take them from anywhere. (All of a worker's pools: one look-up a tensor.)
+  bool ask = 2 * bytes >= kPrefetchBytes;
+  OwnMemory mine;
+  for (int i = 0; ask && i < list.count; ++i) ask = mine.holds(list.segment[i].src, list.segment[i].bytes);
+  list.prefetch = asking(ask);
   RLT_CUDA_TRY(launch_following(inline_segments_kernel<kCount>, static_cast<unsigned>(tiles), kThreads, stream, list));
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return RLT_OK;
@@ -165,7 +170,7 @@ int rlt_kv_push(const void* src, void* dst, int64_t nbytes, rlt_stream_t stream)
   if (tiles > 0x7fffffffll) return RLT_E_LIMIT;
   RLT_CUDA_TRY(rlt::launch_following(rlt::push_kernel, static_cast<unsigned>(tiles), rlt::kThreads, reinterpret_cast<cudaStream_t>(stream),
                                      static_cast<const char*>(src), static_cast<char*>(dst), static_cast<long long>(nbytes),
-                                     static_cast<int>(rlt::prefetches(src, 2 * nbytes))));
+                                     static_cast<int>(rlt::asking(rlt::prefetches(src, 2 * nbytes)))));
   rlt::g_launches.fetch_add(1, std::memory_order_relaxed);
   return RLT_OK;
 }

@@ -1,5 +1,6 @@
 // Library-wide state and the information entry points.
 #include "common.cuh"
+#include "internal.h"
 
 namespace rlt {
 
@@ -21,15 +22,58 @@ int sm_count(int* out) {
   return RLT_OK;
 }
 
-bool prefetches(const void* src, long long bytes) {
-  if (bytes < kPrefetchBytes) return false;
+std::atomic<long long> g_asking{0}, g_lookups{0};
+
+namespace {
+
+bool own(const void* at) {
+  g_lookups.fetch_add(1, std::memory_order_relaxed);
   cudaPointerAttributes of = {};
   int device = -1;
-  if (cudaPointerGetAttributes(&of, src) != cudaSuccess || cudaGetDevice(&device) != cudaSuccess) {
+  if (cudaPointerGetAttributes(&of, at) != cudaSuccess || cudaGetDevice(&device) != cudaSuccess) {
     cudaGetLastError();  // an address that nobody knows is no error here
     return false;
   }
   return of.type == cudaMemoryTypeDevice && of.device == device;
+}
+
+// The allocation that holds an address; false where the driver does not say.
+bool allocation_of(uintptr_t at, unsigned long long* base, size_t* size) {
+  using GetRange = int (*)(unsigned long long*, size_t*, unsigned long long);
+  static const GetRange get = [] {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &fn, cudaEnableDefault, &found) != cudaSuccess || found != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      fn = nullptr;
+    }
+    return reinterpret_cast<GetRange>(fn);
+  }();
+  return get != nullptr && get(base, size, at) == 0 && *base <= at && at - *base < *size;
+}
+
+}  // namespace
+
+bool prefetches(const void* src, long long bytes) { return bytes >= kPrefetchBytes && own(src); }
+
+bool OwnMemory::holds(const void* from, long long bytes) {
+  uintptr_t at = reinterpret_cast<uintptr_t>(from);
+  const uintptr_t end = at + static_cast<uintptr_t>(bytes);
+  const auto in = [&](int k) { return known_[k].begin <= at && at < known_[k].end; };
+  while (at < end) {
+    if (last_ >= count_ || !in(last_)) {
+      for (last_ = 0; last_ < count_ && !in(last_); ++last_) {
+      }
+    }
+    if (last_ == count_) {
+      unsigned long long base = 0;
+      size_t size = 0;
+      if (count_ == kLookups || !own(reinterpret_cast<const void*>(at)) || !allocation_of(at, &base, &size)) return false;
+      known_[count_++] = {static_cast<uintptr_t>(base), static_cast<uintptr_t>(base) + size};
+    }
+    at = known_[last_].end;
+  }
+  return true;
 }
 
 }  // namespace rlt
@@ -51,6 +95,11 @@ const char* rlt_error_string(int code) {
 }
 
 int rlt_last_cuda_error(void) { return rlt::g_last_cuda_error; }
+
+void rlt_prefetch_counts(int64_t counts[2]) {
+  counts[0] = rlt::g_asking.load(std::memory_order_relaxed);
+  counts[1] = rlt::g_lookups.load(std::memory_order_relaxed);
+}
 
 int64_t rlt_kernel_launches(void) { return rlt::g_launches.load(std::memory_order_relaxed); }
 

@@ -299,7 +299,7 @@ int launch_flat_typed(const void* src, void* dst, void* secondary, long long n, 
   const long long grid = (n + per - 1) / per;
   if (grid > 0x7fffffffll) return RLT_E_LIMIT;
   const int64_t bytes = n * static_cast<int64_t>(sizeof(S) + sizeof(D) + (secondary != nullptr ? sizeof(E) : 0));
-  const int prefetch = head >= 0 && prefetches(src, bytes);
+  const int prefetch = asking(head >= 0 && prefetches(src, bytes));
   RLT_CUDA_TRY(launch_following(flat_transfer_kernel<S, D, E>, static_cast<unsigned>(grid), kTile, stream, static_cast<const S*>(src),
                                 static_cast<D*>(dst), static_cast<E*>(secondary), n, head, prefetch));
   return RLT_OK;
