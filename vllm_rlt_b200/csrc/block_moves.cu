@@ -655,9 +655,14 @@ cudaError_t launch_move(const MoveParams& p, const RltBlockMoves& m, unsigned gr
   return launch_following(move_kernel<K, kWords, false>, grid, kThreads, stream, args);
 }
 
+// int32 that the launch's parameters would have to hold.
+long long parameter_words(const MoveParams& p, const RltBlockMoves& m) {
+  return static_cast<long long>(m.blocks) * m.words + (m.host_wire ? static_cast<long long>(m.blocks) * p.src_planes : 0);
+}
+
 template <MoveKind K>
 int launch_kind(const MoveParams& p, const RltBlockMoves& m, unsigned grid, bool ask, cudaStream_t stream) {
-  const long long n = static_cast<long long>(m.blocks) * m.words + (m.host_wire ? static_cast<long long>(m.blocks) * p.src_planes : 0);
+  const long long n = parameter_words(p, m);
   // A parameter block is copied into the launch whole (a launch takes the host 1.85 us with 0.1 - 7 KiB, 2.2 with 16 and 3.1 with 31; a
   // copy of the records, the launch and an event 4.5, and the GPU 9 - 16 us more), so three sizes of it: the small one covers a few
   // hundred tokens, the medium one a thousand.
@@ -680,6 +685,34 @@ int launch_kind(const MoveParams& p, const RltBlockMoves& m, unsigned grid, bool
 int vectors_per_round(int vec_bytes, bool planes) {
   return kThreads * (vec_bytes == 32 ? unroll_of<Vec32>(planes) : vec_bytes == 16 ? unroll_of<uint4>(planes)
                      : vec_bytes == 4 ? unroll_of<uint32_t>(planes) : unroll_of<uint8_t>(planes));
+}
+
+// Whether a launch of a kind that can ask for its source does.
+bool asks(const MoveParams& p, const RltBlockMoves& m, MoveKind kind, int regions) {
+  if (parameter_words(p, m) > kInlineWords) return false;  // records in device memory would have to be waited for (move_kernel)
+  long long bytes = 0;
+  for (int g = 0; g < regions; ++g) bytes += 4ll * m.blocks * p.grid_planes * p.region[g].slice_vecs * p.region[g].vec_bytes;
+  if (bytes < kPrefetchBytes) return false;
+  if (by_token(kind)) {
+    // A prefetch per row costs a long launch more than the start of it gains: exit-only handoffs of 0.39 GB 61.9 us without, 60.3 with it, of 0.79 GB
+    // 121.9 and 122.7.
+    if (bytes > (512ll << 20)) return false;
+  } else {
+    // Only pages that are wholly in range are asked for where all rows of one come from one place. With few of those the asking costs more than it
+    // gives (51 prompts of 19 - 38 tokens in 64-token pages: 179 us without, 191 with it).
+    int whole = 0;
+    for (int b = 0; b < m.blocks; ++b) whole += m.host_records[static_cast<size_t>(b) * m.words + 2] == p.block_size << 8;
+    if (2 * whole < m.blocks) return false;
+  }
+  // every tensor that is asked for (an image: once)
+  for (int g = 0; g < regions; ++g) {
+    const MoveRegion& rg = p.region[g];
+    if (rg.vec_bytes < 16) continue;
+    if (!prefetches(rg.src[0], bytes)) return false;
+    if (kind == kWireToPlane) break;
+    if (!prefetches(rg.src[1], bytes)) return false;
+  }
+  return true;
 }
 
 }  // namespace
@@ -822,19 +855,7 @@ extern "C" int rlt_move_blocks(int direction, const RltPool* src, const RltPool*
     if (rounds == 1 || grid >= waves * sms * (planes ? 3 : 6)) break;
   }
   if (grid > 0x7fffffffll) return RLT_MOVE_UNSUITED;
-  long long bytes = 0;
-  for (int g = 0; g < t.num_regions; ++g) bytes += 4ll * m->blocks * p.grid_planes * p.region[g].slice_vecs * p.region[g].vec_bytes;
-  if (bytes >= kPrefetchBytes && asks_ahead(kind) && !by_token(kind)) {
-    // Only pages that are wholly in range are asked for where all rows of one come from one place. With few of those the asking costs more than it
-    // gives (51 prompts of 19 - 38 tokens in 64-token pages: 179 us without, 191 with it).
-    int whole = 0;
-    for (int b = 0; b < m->blocks; ++b) whole += m->host_records[static_cast<size_t>(b) * m->words + 2] == t.block_size << 8;
-    if (2 * whole < m->blocks) bytes = 0;
-  }
-  // A prefetch per row costs a long launch more than the start of it gains: exit-only handoffs of 0.39 GB 61.9 us without, 60.3 with it, of 0.79 GB
-  // 121.9 and 122.7.
-  if (by_token(kind) && bytes > (512ll << 20)) bytes = 0;
-  const bool ask = asks_ahead(kind) && prefetches(p.region[0].src[0], bytes);
+  const bool ask = asks_ahead(kind) && asks(p, *m, kind, t.num_regions);
 
   const cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   const unsigned ctas = static_cast<unsigned>(grid);
