@@ -687,6 +687,40 @@ int vectors_per_round(int vec_bytes, bool planes) {
                      : vec_bytes == 4 ? unroll_of<uint32_t>(planes) : unroll_of<uint8_t>(planes));
 }
 
+// How the pairs of a page are dealt to CTAs in a dedup pack. What the pages contribute is known, and the average is cut: a layer's pairs into a power
+// of two of shares, or whole layers put together, so that shares of an average page end where layers do. The first of these cuts that gives the GPU
+// enough CTAs is taken: the most that a share holds, in eighths of a round of 16 KiB, and the waves of six CTAs per SM that are enough.
+//
+// Every CTA first lists its page's pairs, so shares below 64 KiB lose more than a fuller GPU gains: 5 prompts on four planes, shares of 160 / 80 / 53 / 40 /
+// 32 KiB, 850 / 843 / 911 / 922 / 1,011 us. Three and seven shares a layer are worse than two and four: all tokens of 6 prompts on four planes, 2 / 3 / 4
+// shares 984 / 1,010 / 1,011; 16 planes, 4 / 7 / 8 shares 661 / 674 / 663. A launch of few waves is better with smaller ones: 700 tokens on four planes
+// (4.8 waves of 80 KiB) 115 -> 111 with 40 KiB; 2,500 on one plane (8.5 of 64) 153 -> 148 with 32, but 5,000 (17 of 64) stay; 300 on six planes (4.1 of 56)
+// 73 with 28 KiB, 71 when they stay; 100 on four (1.5 of 36) 24 with 18 KiB, 19.5 when they stay. Rows below 1 KiB take a CTA longer than larger ones do: 352 pages of
+// 384-byte rows on seven planes (4.8 waves of 120 KiB) 185 with shares of 48 KiB, 178 when they stay.
+//
+// Pages that contribute much more than the average get longer shares. More shares for every page, until the deepest one's are short, is
+// far worse (16 planes, 450 pages on one plane and 20 on all: 733 us so, 1,247 with at most twice the average's share, 1,924 with
+// at most its own; 1,330 where every page had the shares of a full one).
+struct PackCut {
+  int eighths, waves, waves_of_short_rows;
+};
+constexpr PackCut kPackCuts[] = {{70, 8, 4}, {35, 12, 12}, {30, 1, 1}, {15, 0, 0}};
+constexpr int kShortRow = 1024;
+
+int pack_shares(const MoveRegion& rg, const MoveParams& p, const RltBlockMoves& m, const PackCut& cut) {
+  const long long layer = std::max<long long>(1, rg.row_vecs * ((m.wire_tokens + m.blocks - 1) / m.blocks));
+  const long long most = vectors_per_round(rg.vec_bytes, false) * cut.eighths / 8;
+  long long count = p.slice_layers;
+  if (layer > most) {
+    for (long long share = layer; share > most; share = (share + 1) / 2) count *= 2;
+  } else {
+    const long long layers = most / layer;
+    count = (count + layers - 1) / layers;
+  }
+  // no share of a full page may have more vectors than the multiplier split of pack_pairs allows
+  return static_cast<int>(std::max(count, (static_cast<long long>(rg.slice_vecs) * p.src_planes + 65535) / 65536));
+}
+
 // Whether a launch of a kind that can ask for its source does.
 bool asks(const MoveParams& p, const RltBlockMoves& m, MoveKind kind, int regions) {
   if (parameter_words(p, m) > kInlineWords) return false;  // records in device memory would have to be waited for (move_kernel)
@@ -818,41 +852,36 @@ extern "C" int rlt_move_blocks(int direction, const RltPool* src, const RltPool*
   p.status = opt->status;
   // Rounds of a piece. Where a plane's block is all a CTA looks up, one: the smaller the piece the closer the SMs stay
   // together. Kinds that fetch the page's record and work out exit planes first need more payload behind that: measured
-  // best at 2 for exit-only (29k tokens: 1.84 -> 1.75 ms), at 5 for a dedup pack (see below). Where planes are walked, the
+  // best at 2 for exit-only (29k tokens: 1.84 -> 1.75 ms); a dedup pack has a rule of its own (pack_shares). Where planes are walked, the
   // more planes a round stores to the fewer rounds are needed, 12 / planes and at most 4. Dedup handoffs of 6 - 8.6 GB, us at
   // 1 / 2 / 3 / 4 / 8 rounds: two planes 1,267 / 1,105 / 1,054 / 1,026 / 991 (so 8 would be 4 % faster there), three 1,199 /
   // 1,093 / 1,053 / 1,036 / 1,039, four 1,295 / 1,234 / 1,226 / 1,227 / 1,240, six 1,289 / 1,270 / 1,267 / 1,270 / 1,281, eight
   // 1,185 / 1,190 / 1,191 / 1,196 / 1,205, sixteen 1,282 / 1,295 / 1,298 / 1,307 / 1,321, 32 1,086 / 1,098 / 1,105 / 1,114 /
   // 1,114; scatters of dedup images within 1 % of the same. A launch of fewer than eight waves takes the smallest piece that a
-  // larger one would split into: it is short of CTAs, not of payload per CTA. A dedup pack, whose CTAs first list a page's pairs, stays with two
-  // rounds as long as those fill the GPU twice: 30 requests of 4 - 34 tokens 31.2 -> 29.1 us, 9 of 17 - 34 42.2 -> 31.1 (59 and 68 where the
-  // shares were made as if every page were full and every token on every plane).
+  // larger one would split into: it is short of CTAs, not of payload per CTA.
   int sms = 0;
   const int found = sm_count(&sms);
   if (found != RLT_OK) return found;
-  int rounds = pairs ? 5 : planes ? std::max(1, std::min(4, 12 / p.dst_planes)) : by_token(kind) ? 2 : 1;
+  int rounds = planes ? std::max(1, std::min(4, 12 / p.dst_planes)) : by_token(kind) ? 2 : 1;
+  const PackCut* cut = kPackCuts;  // the last of them ends the search
   long long grid = 0;
-  for (;; rounds /= 2) {
+  for (;;) {
     p.pieces = 0;
     for (int g = 0; g < t.num_regions; ++g) {
       MoveRegion& rg = p.region[g];
       rg.per = vectors_per_round(rg.vec_bytes, planes) * rounds;
-      const long long most = rg.slice_vecs;
-      rg.pieces = static_cast<int>((most + rg.per - 1) / rg.per);
-      if (pairs) {
-        // What the pages contribute is known: their average is dealt out, in shares that end where layers do as far as possible (five prompts of
-        // four planes: 957 us in halves of a layer, 975 in 47 shares of 24 layers). No share of a full page may have more vectors than the
-        // multiplier split allows.
-        const long long layer = rg.row_vecs * ((m->wire_tokens + m->blocks - 1) / m->blocks), share = rg.per;
-        const long long count = layer >= share ? p.slice_layers * ((layer + share / 2) / share)
-                                               : std::max(1ll, p.slice_layers * layer / std::max(1ll, share / std::max(1ll, layer) * layer));
-        rg.pieces = static_cast<int>(std::max(count, (static_cast<long long>(rg.slice_vecs) * p.src_planes + 65535) / 65536));
-      }
+      rg.pieces = pairs ? pack_shares(rg, p, *m, *cut) : (rg.slice_vecs + rg.per - 1) / rg.per;
       p.pieces += 2 * rg.pieces;
     }
     grid = static_cast<long long>(m->blocks) * p.grid_planes * p.pieces;
-    const long long waves = !pairs ? 8 : rounds == 2 ? 2 : 6;
-    if (rounds == 1 || grid >= waves * sms * (planes ? 3 : 6)) break;
+    const long long wave = static_cast<long long>(sms) * (planes ? 3 : 6);
+    if (pairs) {
+      if (grid >= wave * (p.region[0].token_bytes < kShortRow ? cut->waves_of_short_rows : cut->waves)) break;
+      ++cut;
+    } else {
+      if (rounds == 1 || grid >= 8 * wave) break;
+      rounds /= 2;
+    }
   }
   if (grid > 0x7fffffffll) return RLT_MOVE_UNSUITED;
   const bool ask = asks_ahead(kind) && asks(p, *m, kind, t.num_regions);
