@@ -113,7 +113,7 @@ struct Piece {
 // A page's record as the kinds that choose planes per token use it: fetched by the CTA in one round, then looked up in
 // shared memory (a chain of global lookups, token -> exit plane -> block, would cost a CTA this short as much time as its
 // payload).
-constexpr int kMaxPlanes = 64;
+constexpr int kMaxPlanes = kMaxRecordPlanes;
 struct PageShared {
   long long src[kMaxPlanes];  // byte offset of each plane's block, -1 if the id is outside the pool
   long long dst[kMaxPlanes];

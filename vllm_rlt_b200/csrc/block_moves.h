@@ -16,6 +16,9 @@
 constexpr int kRecordHeader = 6;
 constexpr int kRecordBad = -1;
 
+// Pools of more planes are served by the table-driven kernels.
+constexpr int kMaxRecordPlanes = 64;
+
 // Records up to this many words travel as kernel parameters: no staging slot, no copy, no event. (The launch takes the smallest of
 // three parameter blocks that holds them.)
 constexpr int kInlineWords = 7680;

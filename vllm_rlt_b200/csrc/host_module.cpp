@@ -1409,10 +1409,11 @@ PyObject* post(PyObject* const* a) {
   return PyLong_FromLong(unlocked([&] { return rlt_kv_post(slot, reinterpret_cast<const uint8_t*>(body), stamp, stream); }));
 }
 
-// load_transport(device) -> code
+// load_transport(device, planes) -> code
 PyObject* load_transport(PyObject* const* a) {
   const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(integer(a[0])));
-  return PyLong_FromLong(unlocked([] { return rlt_load_transport(); }));
+  const auto planes = static_cast<int32_t>(integer(a[1]));
+  return PyLong_FromLong(unlocked([&] { return rlt_load_transport(planes); }));
 }
 
 // ------------------------------------------------------------------------------------------------ the module
@@ -1454,7 +1455,7 @@ PyMethodDef kMethods[] = {
     RLT_ENTRY("pack_segments", pack_segments, 3),
     RLT_ENTRY("copy_segments", copy_segments, 3),
     RLT_ENTRY("push_chunk", push_chunk, 13),
-    RLT_ENTRY("load_transport", load_transport, 1),
+    RLT_ENTRY("load_transport", load_transport, 2),
     RLT_ENTRY("push", push, 5),
     RLT_ENTRY("post", post, 5),
     RLT_ENTRY("tensor_copy", tensor_copy, 3),

@@ -30,9 +30,11 @@ RLT_API void rlt_prefetch_counts(int64_t counts[2]);
 #define RLT_POST_RANGE_BYTES 32768  // of all of them
 RLT_API int rlt_post_behind(const int64_t* ranges, int32_t count, void* slot, const uint8_t body[56], uint64_t stamp, rlt_stream_t stream);
 
-// Loads the kernels of a transfer worker on the current device. A kernel is otherwise loaded by its first launch, and that may wait for what
-// runs on the device by then: a message that should be queued behind a prefill would hold the host until the prefill has ended.
-RLT_API int rlt_load_transport(void);
+// Loads what a transfer worker launches, on the current device, for pools of so many planes. The kernels of a source file are otherwise loaded by the
+// first launch of any of them, and that waits for what runs on the device by then: a message that should be queued behind a prefill would
+// hold the host until the prefill has ended. (The other kernels of a file do not wait once one of them has been loaded.)
+RLT_API int rlt_load_transport(int32_t planes);
+int rlt_load_tables(void);
 int rlt_load_moves(void);
 int rlt_load_segments(void);
 

@@ -11,6 +11,7 @@
 
 #include <cstring>
 
+#include "block_moves.h"
 #include "common.cuh"
 #include "internal.h"
 
@@ -118,10 +119,14 @@ int rlt_post_behind(const int64_t* ranges, int32_t count, void* slot, const uint
   return RLT_OK;
 }
 
-int rlt_load_transport(void) {
+int rlt_load_transport(int32_t planes) {
   RLT_CUDA_TRY(rlt::load_kernel(rlt::post_kernel));
   const int rc = rlt_load_segments();
-  return rc == RLT_OK ? rlt_load_moves() : rc;
+  if (rc != RLT_OK) return rc;
+  // The table-driven kernels bring 4.2 MB of device memory with them, so only for the pools that need them; where that does not fit, the first
+  // launch will say so.
+  if (planes > kMaxRecordPlanes && rlt_load_tables() != RLT_OK) (void)cudaGetLastError();
+  return rlt_load_moves();
 }
 
 int rlt_kv_wait(const uint64_t* flag, uint64_t value, int64_t timeout_ns, int32_t* status, rlt_stream_t stream) {

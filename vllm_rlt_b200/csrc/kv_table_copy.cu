@@ -44,6 +44,7 @@
 
 #include "block_moves.h"
 #include "common.cuh"
+#include "internal.h"
 #include "slot_pool.h"
 #include "table_params.cuh"
 
@@ -1311,6 +1312,13 @@ int rlt_kv_pack_dedup_static(const RltPool* src, const RltBatch* batch, const Rl
 int64_t rlt_kv_static_plan_entries(void) { return rlt::kStaticPlanEntries; }
 
 int64_t rlt_kv_host_batch_limit(void) { return static_cast<int64_t>(rlt::kHostSlotBytes); }
+
+int rlt_load_tables(void) {
+  using namespace rlt;
+  RLT_CUDA_TRY(load_kernel(table_copy_kernel<4, true, false>));
+  RLT_CUDA_TRY(load_kernel(table_fan_kernel<4>));
+  return RLT_OK;
+}
 
 int rlt_handoff_staged(const RltPool* src, const RltPool* dst, const RltBlockMoves* moves, const RltOptions* options,
                        rlt_stream_t stream) {

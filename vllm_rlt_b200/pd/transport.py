@@ -300,7 +300,7 @@ class CudaBackend:
 
     device_ordered = True
 
-    def __init__(self, device):
+    def __init__(self, device, planes: int = 1):
         import torch
 
         from . import peer as peerlib
@@ -315,7 +315,7 @@ class CudaBackend:
         self.stream = torch.cuda.Stream(self.device)
         self._where = (self.stream.device.index, self.stream.cuda_stream)  # what the compiled calls launch on
         self._host = _lib.load_host()
-        _lib.check(self._host.load_transport(self._where[0]), "rlt_load_transport")
+        _lib.check(self._host.load_transport(self._where[0], planes), "rlt_load_transport")
 
     def order_after(self, event) -> None:
         """Make everything submitted from now on wait (on the device) for ``event``."""
@@ -526,7 +526,7 @@ class B200Transport:
         self.config = config
         self.name = name
         self.cache = cache
-        self.backend = backend if backend is not None else CudaBackend(cache.key_cache.device)
+        self.backend = backend if backend is not None else CudaBackend(cache.key_cache.device, cache.storage_depths)
         # True: submissions may carry a producer event that the copy waits for on the device (``after=``)
         self.device_ordered = getattr(self.backend, "device_ordered", False) is True
         self.direction = default_direction() if direction is None else direction
