@@ -102,14 +102,21 @@ bool prefetches(const void* src, long long bytes);
 // a worker's pools have tensors, the answer is no.
 class OwnMemory {
  public:
-  bool holds(const void* from, long long bytes);
+  bool holds(const void* from, long long bytes) {
+    const uintptr_t at = reinterpret_cast<uintptr_t>(from), size = static_cast<uintptr_t>(bytes);
+    for (int k = 0; k < count_; ++k) {
+      if (at - known_[k].begin < known_[k].size && size <= known_[k].size - (at - known_[k].begin)) return true;
+    }
+    return look_up(at, size);
+  }
 
  private:
   static constexpr int kLookups = 8;
+  bool look_up(uintptr_t at, uintptr_t size);
   struct {
-    uintptr_t begin, end;
+    uintptr_t begin, size;
   } known_[kLookups];
-  int count_ = 0, last_ = 0;
+  int count_ = 0;
 };
 
 // Counts the launches that ask, for the tests.

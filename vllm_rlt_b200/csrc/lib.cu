@@ -1,4 +1,6 @@
 // Library-wide state and the information entry points.
+#include <cuda.h>
+
 #include "common.cuh"
 #include "internal.h"
 
@@ -24,54 +26,53 @@ int sm_count(int* out) {
 
 std::atomic<long long> g_asking{0}, g_lookups{0};
 
-namespace {
-
-bool own(const void* at) {
+bool prefetches(const void* src, long long bytes) {
+  if (bytes < kPrefetchBytes) return false;
   g_lookups.fetch_add(1, std::memory_order_relaxed);
   cudaPointerAttributes of = {};
   int device = -1;
-  if (cudaPointerGetAttributes(&of, at) != cudaSuccess || cudaGetDevice(&device) != cudaSuccess) {
+  if (cudaPointerGetAttributes(&of, src) != cudaSuccess || cudaGetDevice(&device) != cudaSuccess) {
     cudaGetLastError();  // an address that nobody knows is no error here
     return false;
   }
   return of.type == cudaMemoryTypeDevice && of.device == device;
 }
 
-// The allocation that holds an address; false where the driver does not say.
-bool allocation_of(uintptr_t at, unsigned long long* base, size_t* size) {
-  using GetRange = int (*)(unsigned long long*, size_t*, unsigned long long);
-  static const GetRange get = [] {
+// The allocation that holds an address, if it is memory of the current device. One call of the driver's (0.06 us) where the runtime would take two.
+static bool own_allocation(uintptr_t at, uintptr_t* begin, uintptr_t* size) {
+  using Attributes = CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+  static const Attributes ask = [] {
     void* fn = nullptr;
     cudaDriverEntryPointQueryResult found;
-    if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &fn, cudaEnableDefault, &found) != cudaSuccess || found != cudaDriverEntryPointSuccess) {
+    if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &fn, cudaEnableDefault, &found) != cudaSuccess || found != cudaDriverEntryPointSuccess) {
       cudaGetLastError();
       fn = nullptr;
     }
-    return reinterpret_cast<GetRange>(fn);
+    return reinterpret_cast<Attributes>(fn);
   }();
-  return get != nullptr && get(base, size, at) == 0 && *base <= at && at - *base < *size;
+  g_lookups.fetch_add(1, std::memory_order_relaxed);
+  unsigned type = 0, managed = 0;  // (the driver writes four bytes for either)
+  int of = -1, device = -2;
+  CUdeviceptr base = 0;
+  size_t bytes = 0;
+  CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL, CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+  void* where[] = {&type, &of, &managed, &base, &bytes};
+  if (ask == nullptr || ask(5, what, where, at) != CUDA_SUCCESS || cudaGetDevice(&device) != cudaSuccess) return false;
+  *begin = base;
+  *size = bytes;
+  return type == CU_MEMORYTYPE_DEVICE && managed == 0 && of == device && base <= at && at - base < bytes;
 }
 
-}  // namespace
-
-bool prefetches(const void* src, long long bytes) { return bytes >= kPrefetchBytes && own(src); }
-
-bool OwnMemory::holds(const void* from, long long bytes) {
-  uintptr_t at = reinterpret_cast<uintptr_t>(from);
-  const uintptr_t end = at + static_cast<uintptr_t>(bytes);
-  const auto in = [&](int k) { return known_[k].begin <= at && at < known_[k].end; };
-  while (at < end) {
-    if (last_ >= count_ || !in(last_)) {
-      for (last_ = 0; last_ < count_ && !in(last_); ++last_) {
-      }
+bool OwnMemory::look_up(uintptr_t at, uintptr_t size) {
+  for (const uintptr_t end = at + size; at < end;) {
+    int k = 0;
+    while (k < count_ && at - known_[k].begin >= known_[k].size) ++k;
+    if (k == count_) {
+      if (count_ == kLookups || !own_allocation(at, &known_[k].begin, &known_[k].size)) return false;
+      ++count_;
     }
-    if (last_ == count_) {
-      unsigned long long base = 0;
-      size_t size = 0;
-      if (count_ == kLookups || !own(reinterpret_cast<const void*>(at)) || !allocation_of(at, &base, &size)) return false;
-      known_[count_++] = {static_cast<uintptr_t>(base), static_cast<uintptr_t>(base) + size};
-    }
-    at = known_[last_].end;
+    at = known_[k].begin + known_[k].size;
   }
   return true;
 }
