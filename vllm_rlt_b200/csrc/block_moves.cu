@@ -728,9 +728,9 @@ bool asks(const MoveParams& p, const RltBlockMoves& m, MoveKind kind, int region
   for (int g = 0; g < regions; ++g) bytes += 4ll * m.blocks * p.grid_planes * p.region[g].slice_vecs * p.region[g].vec_bytes;
   if (bytes < kPrefetchBytes) return false;
   if (by_token(kind)) {
-    // A prefetch per row costs a long launch more than the start of it gains: exit-only handoffs of 0.39 GB 61.9 us without, 60.3 with it, of 0.79 GB
-    // 121.9 and 122.7.
-    if (bytes > (512ll << 20)) return false;
+    // A prefetch per row costs a long launch more than the start of it gains. Exit-only handoffs one behind another, us without / with it: 39 MB
+    // 6.7 / 6.6, 79 MB 11.9 / 11.0, 0.20 GB 30.8 / 29.2, 0.39 GB 60.8 / 59.1, 0.47 GB 73.4 / 73.7, 0.59 GB 90.6 / 90.7, 1.2 GB 178.7 / 180.1.
+    if (bytes > (448ll << 20)) return false;
   } else {
     // Only pages that are wholly in range are asked for where all rows of one come from one place. With few of those the asking costs more than it
     // gives (51 prompts of 19 - 38 tokens in 64-token pages: 179 us without, 191 with it).

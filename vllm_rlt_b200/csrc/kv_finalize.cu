@@ -55,9 +55,9 @@ struct FinalizeParams {
 
 constexpr int kGroupRows = 16;
 // Deeper planes whose blocks are looked up together with the source's, before the source is read: rows -> blocks -> payload are three dependent
-// accesses then, not four and one more per plane. us at none / 2 / 3 (which no longer fits the registers of eight CTAs per SM): one row
-// 2.12 / 1.98 / 2.05, 64 rows of four planes 5.94 / 5.85 / 6.06, 8 and 1,200 rows of 32 planes 10.4 / 10.0 / 11.0 and 809 / 791 / 845, 4,000
-// rows of four planes 271.7 / 271.9 / 277.3.
+// accesses then, not four and one more per plane. us at none / 2, launches one behind another in a graph: one row 1.88 / 1.81, 64 rows of four planes
+// 6.35 / 6.28, 8, 64 and 1,200 rows of 32 planes with geometric exits 6.78 / 6.54, 24.8 / 24.5 and 403 / 395, 300 rows of eight planes of 1 KiB 12.8 /
+// 12.6, 4,000 rows of four planes 273.0 / 273.1. (3 no longer fits the registers of eight CTAs per SM: 4,000 rows 2 % slower.)
 constexpr int kAhead = 2;
 constexpr long long kMostRows = 1ll << 28;  // of one launch: three times a row's index stays in 32 bits
 
