@@ -123,8 +123,10 @@ def test_handoffs_ask_while_their_records_are_parameters():
 def test_pages_that_are_mostly_not_full_are_not_asked_for():
     from vllm_rlt_b200.kernels import kv_handoff as kh
 
-    assert handoff(1, 12, kh.MODE_ALL_PLANES, page=64, tokens=63)[0] == (0, 0)
-    assert handoff(2, 12, kh.MODE_ALL_PLANES, page=64, tokens=65)[0] == (1, 2)
+    assert handoff(1, 12, kh.MODE_ALL_PLANES, page=64, tokens=47)[0] == (0, 0)
+    assert handoff(1, 12, kh.MODE_ALL_PLANES, page=64, tokens=48)[0] == (1, 2)
+    assert handoff(2, 12, kh.MODE_ALL_PLANES, page=64, tokens=65)[0] == (0, 0)  # every second one is whole
+    assert handoff(2, 12, kh.MODE_ALL_PLANES, page=64, tokens=96)[0] == (1, 2)
 
 
 def test_pool_tensors_elsewhere():

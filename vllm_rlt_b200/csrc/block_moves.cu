@@ -732,11 +732,17 @@ bool asks(const MoveParams& p, const RltBlockMoves& m, MoveKind kind, int region
     // 6.7 / 6.6, 79 MB 11.9 / 11.0, 0.20 GB 30.8 / 29.2, 0.39 GB 60.8 / 59.1, 0.47 GB 73.4 / 73.7, 0.59 GB 90.6 / 90.7, 1.2 GB 178.7 / 180.1.
     if (bytes > (448ll << 20)) return false;
   } else {
-    // Only pages that are wholly in range are asked for where all rows of one come from one place. With few of those the asking costs more than it
-    // gives (51 prompts of 19 - 38 tokens in 64-token pages: 179 us without, 191 with it).
-    int whole = 0;
-    for (int b = 0; b < m.blocks; ++b) whole += m.host_records[static_cast<size_t>(b) * m.words + 2] == p.block_size << 8;
-    if (2 * whole < m.blocks) return false;
+    // Where all rows of a page come from one place, only pages that are wholly in range are asked for, and the blocks of the others partly idle.
+    // Much of that and asking costs more than it gives. Prompts of two pages of 4 KiB rows, us without / with it, by the share of the pages' tokens that
+    // is in range: handoffs, 32-token pages, 0.55 983 / 1,021, 0.65 930 / 946, 0.75 921 / 911, 0.85 923 / 912; 64-token pages, 0.51 708 / 727, 0.72 799 / 801,
+    // 0.75 901 / 889; 16-token pages, 0.53 120.1 / 121.6, 0.75 558 / 552. Packs 0.55 1,003 / 1,053, 0.65 927 / 950, 0.75 912 / 906, but in 64-token pages
+    // 0.75 894 / 905 and 0.85 912 / 904; scatters like packs. FP8 in 16-token pages, 0.56 433 / 441, 0.75 578 / 569.
+    long long used = 0;
+    for (int b = 0; b < m.blocks; ++b) {
+      const int range = m.host_records[static_cast<size_t>(b) * m.words + 2];
+      if (range != kRecordBad) used += (range >> 8) - (range & 0xff);
+    }
+    if (4 * used < 3ll * m.blocks * p.block_size) return false;
   }
   // every tensor that is asked for (an image: once)
   for (int g = 0; g < regions; ++g) {
